@@ -195,8 +195,10 @@ pq_status pq_ci_diag(pq_ci_handle *h, double *out_device) {
   return PQ_OK;
 }
 
+// on_device: C and S are device memory, where a single FP64 vector is its own interleaved block and sigma reads
+// and writes it in place (page-locked host memory is converted, so that the gathers stay on the device)
 static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, double *S, int64_t lds,
-                              int32_t precision) {
+                              int32_t precision, bool on_device) {
   if (!h || !C || !S || nvec < 1 || ldc < h->n_dets || lds < h->n_dets) {
     set_error("pq_ci_sigma: bad arguments (nvec=%d, ldc=%lld, lds=%lld, n_dets=%lld)", nvec, (long long)ldc,
               (long long)lds, (long long)(h ? h->n_dets : 0));
@@ -210,6 +212,14 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
   for (int v0 = 0; v0 < nvec; v0 += 4) {
     int nv = nvec - v0 < 4 ? nvec - v0 : 4;
     int nvp = il_width(h, nv, precision);
+    if (on_device && nvp == 1 && precision == PQ_FP64) {
+      const double *c = C + (size_t)v0 * ldc;
+      double *s = S + (size_t)v0 * lds;
+      if (s + h->n_dets <= c || c + h->n_dets <= s) {  // sigma over its own input needs the copies below
+        PQ_TRY(ci_sigma_il(h, c, s, 1, precision, 0.0));
+        continue;
+      }
+    }
     size_t bytes = esz * (size_t)nvp * (size_t)(h->n_dets + 1);
     PQ_TRY(h->x_il.ensure(bytes));
     PQ_TRY(h->y_il.ensure(bytes));
@@ -223,7 +233,7 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
 pq_status pq_ci_sigma(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, double *S, int64_t lds,
                       int32_t precision) {
   clear_error();
-  return sigma_device(h, C, ldc, nvec, S, lds, precision);
+  return sigma_device(h, C, ldc, nvec, S, lds, precision, true);
 }
 
 // Device address of a page-locked (pinned or registered) host buffer; NULL for pageable memory.
@@ -250,7 +260,7 @@ pq_status pq_ci_sigma_host(pq_ci_handle *h, const double *C, int64_t ldc, int32_
   // on all SMs instead of one copy engine.
   const void *mc = mapped_host(C), *ms = mapped_host(S);
   if (mc && ms && getenv("PQ_SIGMA_HOST_STAGED") == nullptr) {
-    PQ_TRY(sigma_device(h, (const double *)mc, ldc, nvec, (double *)ms, lds, precision));
+    PQ_TRY(sigma_device(h, (const double *)mc, ldc, nvec, (double *)ms, lds, precision, false));
     PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
     return PQ_OK;
   }
@@ -267,7 +277,7 @@ pq_status pq_ci_sigma_host(pq_ci_handle *h, const double *C, int64_t ldc, int32_
       PQ_CUDA_TRY(cudaMemcpyAsync(dc + (size_t)v * n, C + (size_t)v * ldc, sizeof(double) * n, cudaMemcpyHostToDevice,
                                   h->stream));
   }
-  PQ_TRY(sigma_device(h, dc, n, nvec, ds, n, precision));
+  PQ_TRY(sigma_device(h, dc, n, nvec, ds, n, precision, true));
   if (lds == n) {
     PQ_CUDA_TRY(cudaMemcpyAsync(S, ds, sizeof(double) * (size_t)n * nvec, cudaMemcpyDeviceToHost, h->stream));
   } else {

@@ -90,6 +90,12 @@ template <> struct VecIO<double, 2> {
     *reinterpret_cast<double2 *>(p) = make_double2(r[0], r[1]);
   }
 };
+template <> struct VecIO<double, 3> {
+  static __device__ __forceinline__ void ld(const double *p, double (&r)[3]) {
+    r[0] = __ldg(p), r[1] = __ldg(p + 1), r[2] = __ldg(p + 2);
+  }
+  static __device__ __forceinline__ void st(double *p, const double (&r)[3]) { p[0] = r[0], p[1] = r[1], p[2] = r[2]; }
+};
 template <> struct VecIO<double, 4> {
   static __device__ __forceinline__ void ld(const double *p, double (&r)[4]) {
     double2 v0 = __ldg(reinterpret_cast<const double2 *>(p));
@@ -354,15 +360,17 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvp, int prec
   if (h->n_species == 2) return ci_sigma2_il(h, X, Y, nvp, precision, shift);
   if (precision == PQ_FP32 && allow_scratch && h->fp32_v2) return ci_sigma32_v2(h, X, Y, nvp, shift);
   if (precision == PQ_FP64) {
+    if (h->rows) return ci_sigma_rows(h, X, Y, nvp, shift);
     if (nvp == 1) return sigma_dispatch<double, 1>(h, (const double *)X, (double *)Y, shift);
     if (nvp == 2) return sigma_dispatch<double, 2>(h, (const double *)X, (double *)Y, shift);
+    if (nvp == 3) return sigma_dispatch<double, 3>(h, (const double *)X, (double *)Y, shift);
     if (nvp == 4) return sigma_dispatch<double, 4>(h, (const double *)X, (double *)Y, shift);
   } else if (precision == PQ_FP32) {
     if (nvp == 1) return sigma_dispatch<float, 1>(h, (const float *)X, (float *)Y, shift);
     if (nvp == 2) return sigma_dispatch<float, 2>(h, (const float *)X, (float *)Y, shift);
     if (nvp == 4) return sigma_dispatch<float, 4>(h, (const float *)X, (float *)Y, shift);
   }
-  set_error("unsupported interleave width %d / precision %d (widths 1, 2, 4)", nvp, precision);
+  set_error("unsupported interleave width %d / precision %d (widths 1, 2, 4, in FP64 also 3)", nvp, precision);
   return PQ_ERR_ARG;
 }
 

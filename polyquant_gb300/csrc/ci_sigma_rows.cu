@@ -1,0 +1,439 @@
+// FP64 sigma = H C of one species with one warp (or one CTA) per determinant.
+//
+// Reference: src/ci/detset/direct_singleparticle.cpp:238-372, the elements of
+// slater_condon_singleparticle.cpp:53-175 (as ci_sigma.cu applies them).
+//
+// The kernel of ci_sigma.cu gives every determinant one thread of a CTA that
+// covers 256 beta strings of one alpha string.  That fills the chip only when
+// the beta rows are long and there are many determinants.  A truncated space
+// has mostly rows of one beta string (in CISD every doubly excited alpha string
+// goes with the Fermi beta string alone), so its CTAs ran one live thread
+// through some 10^3 connections, and a small full space has fewer
+// determinants than the chip has warps.  Here the 32 lanes of a warp share one
+// determinant's connections, and determinants with more than HEAVY
+// connections (the Fermi determinant of a truncated space has all of them) are
+// shared by the 8 warps of the CTA.
+//
+// A truncated space keeps the pairs with level(alpha) + level(beta) <= limit.
+// A single moves a string's level by -1, 0 or +1 and a double by -2 .. +2, so
+// with the entries of each string grouped by that change the partners that are
+// in the list are a prefix of the groups, and the alpha-beta doubles are three
+// rectangles (alpha group) x (prefix of the beta groups): no entry is looked
+// up in vain and no lane idles inside a rectangle.  The grouped copies hold
+// the partner's row offset (alpha) or string (beta), and the opposite-spin
+// Coulomb sums of the singles come from tables [string][pair].
+//
+// Bound: FP64 pipe and L2 gathers.  CISD of 5a5b in 24 orbitals (12 636
+// determinants, 11.2 M elements), three roots: 144 us a sigma against 3914 us
+// with the thread-per-determinant kernel, 0.47 TFLOP/s; full CI of water in 7
+// orbitals (441 determinants), one root: 18 against 41 us.
+#include <algorithm>
+
+#include "pq_bits.cuh"
+#include "pq_internal.h"
+
+namespace pq {
+
+// Grouped tables of one spin list and the Coulomb sums of its strings.
+struct SigmaRows {
+  struct Side {
+    DevBuf s1;    // int2 {partner (row offset for alpha, string for beta), info}, grouped by level change
+    DevBuf s1_F;  // same-spin part of the element
+    DevBuf s2, s2_D;
+    DevBuf cum;   // per string 8 x int32: ends of the 3 groups of singles and the 5 groups of doubles
+    DevBuf lvl;
+    DevBuf coul;  // [string][pair]: sum over the string's orbitals k of (pair of the other spin | kk)
+  };
+  Side side[2];
+  DevBuf row;  // alpha string of every determinant
+  int lim = 0;
+};
+
+void rows_delete(SigmaRows *r) { delete r; }
+
+namespace rows {
+
+constexpr int WARPS = 8;
+constexpr int HEAVY = 1536;  // connections above which the CTA shares a determinant
+constexpr int U = 4;         // gathers in flight per lane
+
+struct Side {
+  const int64_t *o1, *o2;
+  const int2 *s1;
+  const double *F;
+  const int32_t *s2;
+  const double *D;
+  const int4 *cum;
+  const int32_t *lvl;
+  const double *coul;
+};
+
+struct Args {
+  Side a, b;
+  const int32_t *row;
+  const int64_t *rowoff;
+  const double *eab, *diag;
+  double shift;
+  int npair, lim;
+  int64_t n;
+  const double *X;
+  double *Y;
+};
+
+template <int NV> __device__ __forceinline__ void load_x(const double *X, int64_t j, double (&x)[NV]) {
+  const double *p = X + j * NV;
+  if constexpr (NV == 2 || NV == 4) {
+#pragma unroll
+    for (int v = 0; v < NV; v += 2) {
+      const double2 d = __ldg(reinterpret_cast<const double2 *>(p + v));
+      x[v] = d.x, x[v + 1] = d.y;
+    }
+  } else {
+#pragma unroll
+    for (int v = 0; v < NV; v++) x[v] = __ldg(p + v);
+  }
+}
+
+__device__ __forceinline__ double flip(double v, int neg) {
+  return __hiloint2double(__double2hiint(v) ^ (neg << 31), __double2loint(v));
+}
+
+// One determinant's connection classes: list bounds after the level limits.
+struct Det {
+  int64_t I, rowI, a1, a2, b1, b2;
+  int ia, ib;
+  int ca1[4], cb1[4];     // group starts of the singles (ca1[0] = 0)
+  int na1, na2, nb1, nb2;  // kept singles and doubles of either spin
+  int nbx[3];              // kept beta singles beside an alpha single of group g
+  int total;
+};
+
+__device__ __forceinline__ Det load_det(const Args &p, int64_t I) {
+  Det d;
+  d.I = I;
+  d.ia = p.row[I];
+  d.rowI = p.rowoff[d.ia];
+  d.ib = (int)(I - d.rowI);
+  d.a1 = p.a.o1[d.ia], d.a2 = p.a.o2[d.ia];
+  d.b1 = p.b.o1[d.ib], d.b2 = p.b.o2[d.ib];
+  const int slack = min(p.lim - p.a.lvl[d.ia] - p.b.lvl[d.ib], 4);  // >= 0 for a determinant of the list
+  const int4 x0 = p.a.cum[2 * d.ia], x1 = p.a.cum[2 * d.ia + 1];
+  const int4 y0 = p.b.cum[2 * d.ib], y1 = p.b.cum[2 * d.ib + 1];
+  d.ca1[0] = 0, d.ca1[1] = x0.x, d.ca1[2] = x0.y, d.ca1[3] = x0.z;
+  d.cb1[0] = 0, d.cb1[1] = y0.x, d.cb1[2] = y0.y, d.cb1[3] = y0.z;
+  // a group of change c is kept when c <= slack
+  d.na1 = slack >= 1 ? x0.z : x0.y;
+  d.nb1 = slack >= 1 ? y0.z : y0.y;
+  d.na2 = slack >= 2 ? x1.w : (slack == 1 ? x1.z : x1.y);
+  d.nb2 = slack >= 2 ? y1.w : (slack == 1 ? y1.z : y1.y);
+  d.total = 1 + d.na1 + d.nb1 + d.na2 + d.nb2;
+#pragma unroll
+  for (int g = 0; g < 3; g++) {
+    // alpha change g - 1 leaves slack - (g - 1) for the beta change
+    const int s = slack - (g - 1);
+    d.nbx[g] = s >= 1 ? y0.z : (s == 0 ? y0.y : (s == -1 ? y0.x : 0));
+    d.total += (d.ca1[g + 1] - d.ca1[g]) * d.nbx[g];
+  }
+  return d;
+}
+
+// acc += c x for U list entries at t0 + u * nth of a list of `cnt`; entry(t, idx) returns the element and the
+// partner.  Entries past the end load nothing.
+template <int NV, typename E>
+__device__ __forceinline__ void gather(const Args &p, double (&acc)[NV], int t0, int nth, int cnt, E &&entry) {
+  for (int t = t0; t - t0 < cnt; t += U * nth) {
+    double c[U], x[U][NV];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      c[u] = 0.0;
+#pragma unroll
+      for (int v = 0; v < NV; v++) x[u][v] = 0.0;
+      if (t + u * nth < cnt) {
+        int64_t j;
+        c[u] = entry(t + u * nth, j);
+        load_x<NV>(p.X, j, x[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (t - t0 + u * nth < cnt) {  // uniform over the sharing threads: lane 0's entry exists
+#pragma unroll
+        for (int v = 0; v < NV; v++) acc[v] = fma(c[u], x[u][v], acc[v]);
+      }
+  }
+}
+
+// the part of thread tid of nth of determinant d's row of H times X
+template <int NV>
+__device__ __forceinline__ void accumulate(const Args &p, const Det &d, int tid, int nth, double (&acc)[NV]) {
+  if (tid == 0) {
+    double x[NV];
+    load_x<NV>(p.X, d.I, x);
+    const double h = p.diag[d.I] - p.shift;
+#pragma unroll
+    for (int v = 0; v < NV; v++) acc[v] = h * x[v];
+  }
+  gather<NV>(p, acc, tid, nth, d.na1, [&](int t, int64_t &j) {
+    const int2 e = __ldg(p.a.s1 + d.a1 + t);
+    j = (int64_t)e.x + d.ib;
+    return flip(__ldg(p.a.F + d.a1 + t) + __ldg(p.b.coul + (int64_t)d.ib * p.npair + (e.y >> 1)), e.y & 1);
+  });
+  gather<NV>(p, acc, tid, nth, d.nb1, [&](int t, int64_t &j) {
+    const int2 e = __ldg(p.b.s1 + d.b1 + t);
+    j = d.rowI + e.x;
+    return flip(__ldg(p.b.F + d.b1 + t) + __ldg(p.a.coul + (int64_t)d.ia * p.npair + (e.y >> 1)), e.y & 1);
+  });
+  gather<NV>(p, acc, tid, nth, d.na2, [&](int t, int64_t &j) {
+    j = (int64_t)__ldg(p.a.s2 + d.a2 + t) + d.ib;
+    return __ldg(p.a.D + d.a2 + t);
+  });
+  gather<NV>(p, acc, tid, nth, d.nb2, [&](int t, int64_t &j) {
+    j = d.rowI + __ldg(p.b.s2 + d.b2 + t);
+    return __ldg(p.b.D + d.b2 + t);
+  });
+#pragma unroll
+  for (int g = 0; g < 3; g++) {
+    const int nb = d.nbx[g], cnt = (d.ca1[g + 1] - d.ca1[g]) * nb;
+    if (cnt == 0) continue;
+    // entry t is (alpha single t / nb, beta single t % nb); stepping by nth adds (qs, rs) with a carry
+    const int qs = nth / nb, rs = nth - qs * nb;
+    int ea = tid / nb, eb = tid - ea * nb;
+    const int2 *la = p.a.s1 + d.a1 + d.ca1[g], *lb = p.b.s1 + d.b1;
+    gather<NV>(p, acc, tid, nth, cnt, [&](int, int64_t &j) {
+      const int2 a = __ldg(la + ea), b = __ldg(lb + eb);
+      ea += qs, eb += rs;
+      if (eb >= nb) eb -= nb, ea++;
+      j = (int64_t)a.x + b.x;
+      return flip(__ldg(p.eab + (int64_t)(a.y >> 1) * p.npair + (b.y >> 1)), (a.y ^ b.y) & 1);
+    });
+  }
+}
+
+// Sum of acc over the warp: the halving steps also halve the number of values a lane carries, so four roots take
+// 6 additions instead of 20 on the FP64 pipe.  The sum of root v ends in lane root_lane(v), in acc[0].
+template <int NV> __device__ __forceinline__ void warp_sum(double (&acc)[NV], int lane) {
+  int w = 16;
+  if constexpr (NV >= 3) {
+    const bool hi = lane & 16;
+    const double x3 = NV == 4 ? acc[NV - 1] : 0.0;
+    const double s0 = hi ? acc[0] : acc[2], s1 = hi ? acc[1] : x3;
+    const double k0 = hi ? acc[2] : acc[0], k1 = hi ? x3 : acc[1];
+    acc[0] = k0 + __shfl_xor_sync(0xffffffffu, s0, 16);
+    acc[1] = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
+    w = 8;
+  }
+  if constexpr (NV >= 2) {
+    const bool hi = lane & w;
+    const double s = hi ? acc[0] : acc[1], k = hi ? acc[1] : acc[0];
+    acc[0] = k + __shfl_xor_sync(0xffffffffu, s, w);
+    w >>= 1;
+  }
+  for (; w; w >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], w);
+}
+template <int NV> __device__ __forceinline__ int root_of_lane(int lane) {  // -1: the lane holds no root
+  if (NV == 1) return lane == 0 ? 0 : -1;
+  if (NV == 2) return (lane & 15) == 0 ? lane >> 4 : -1;
+  const int v = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
+  return (lane & 7) == 0 && v < NV ? v : -1;
+}
+
+template <int NV> __global__ void __launch_bounds__(32 * WARPS, 3) sigma_rows_kernel(Args p) {
+  __shared__ double part[WARPS][4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t I0 = (int64_t)blockIdx.x * WARPS, I = I0 + warp;
+  bool heavy = false;
+  if (I < p.n) {
+    const Det d = load_det(p, I);
+    heavy = d.total > HEAVY;
+    if (!heavy) {
+      double acc[NV];
+#pragma unroll
+      for (int v = 0; v < NV; v++) acc[v] = 0.0;
+      accumulate<NV>(p, d, lane, 32, acc);
+      warp_sum<NV>(acc, lane);
+      const int v = root_of_lane<NV>(lane);
+      if (v >= 0) p.Y[I * NV + v] = acc[0];
+    }
+  }
+  if (!__syncthreads_or(heavy)) return;
+  for (int k = 0; k < WARPS && I0 + k < p.n; k++) {
+    const Det d = load_det(p, I0 + k);
+    if (d.total <= HEAVY) continue;  // the same for every thread
+    double acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) acc[v] = 0.0;
+    accumulate<NV>(p, d, threadIdx.x, 32 * WARPS, acc);
+    warp_sum<NV>(acc, lane);
+    const int v = root_of_lane<NV>(lane);
+    if (v >= 0) part[warp][v] = acc[0];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+      double s = 0.0;
+      for (int w = 0; w < WARPS; w++) s += part[w][threadIdx.x];
+      p.Y[d.I * NV + threadIdx.x] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// Entries of each string grouped by level change, in table order inside a group: warp per string.
+// key[J] is what a grouped entry stores for partner J (its row offset, or J itself when NULL).
+__global__ void __launch_bounds__(128) group_kernel(int64_t n_str, const int32_t *lvl, const int64_t *key,
+                                                    const int64_t *o1, const int32_t *J1, const int32_t *info1,
+                                                    const double *F1, const int64_t *o2, const int32_t *J2,
+                                                    const double *D2, int2 *s1, double *F, int32_t *s2, double *D,
+                                                    int32_t *cum) {
+  const int lane = threadIdx.x & 31;
+  const int64_t I = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (I >= n_str) return;
+  const int l0 = lvl[I];
+  int64_t w = o1[I];
+  for (int g = 0; g < 3; g++) {
+    for (int64_t e0 = o1[I]; e0 < o1[I + 1]; e0 += 32) {
+      const int64_t e = e0 + lane;
+      const int J = e < o1[I + 1] ? J1[e] : -1;
+      const bool take = J >= 0 && lvl[J] - l0 == g - 1;
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take) {
+        const int64_t o = w + __popc(m & ((1u << lane) - 1u));
+        s1[o] = make_int2(key ? (int)key[J] : J, info1[e]);
+        F[o] = F1[e];
+      }
+      w += __popc(m);
+    }
+    if (lane == 0) cum[8 * I + g] = (int32_t)(w - o1[I]);
+  }
+  w = o2[I];
+  for (int g = 0; g < 5; g++) {
+    for (int64_t e0 = o2[I]; e0 < o2[I + 1]; e0 += 32) {
+      const int64_t e = e0 + lane;
+      const int J = e < o2[I + 1] ? J2[e] : -1;
+      const bool take = J >= 0 && lvl[J] - l0 == g - 2;
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take) {
+        const int64_t o = w + __popc(m & ((1u << lane) - 1u));
+        s2[o] = key ? (int)key[J] : J;
+        D[o] = D2[e];
+      }
+      w += __popc(m);
+    }
+    if (lane == 0) cum[8 * I + 3 + g] = (int32_t)(w - o2[I]);
+  }
+}
+
+// coul[string][pair] = sum over the string's occupied orbitals k of E[pair * rs + kk * cs]
+__global__ void __launch_bounds__(256) coulomb_kernel(const double *E, int npair, int64_t rs, int64_t cs,
+                                                      const uint64_t *str, const uint64_t *str_hi, int64_t n_str,
+                                                      double *coul) {
+  const int64_t total = (int64_t)npair * n_str;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t s = i / npair;
+    const int pr = (int)(i - s * npair);
+    double c = 0.0;
+    for_occ(str[s], hiword(str_hi, s), [&](int k) { c += E[pr * rs + (int64_t)(k * (k + 3) / 2) * cs]; });
+    coul[i] = c;
+  }
+}
+
+__global__ void __launch_bounds__(128) row_kernel(const int64_t *rowoff, const int32_t *rowlen, int64_t na, int32_t *row) {
+  for (int64_t a = blockIdx.x; a < na; a += gridDim.x)
+    for (int b = threadIdx.x; b < rowlen[a]; b += blockDim.x) row[rowoff[a] + b] = (int32_t)a;
+}
+
+}  // namespace rows
+
+// Rule.  Truncated spaces always take this kernel (32-bit determinant indices, Coulomb tables of at most 1 GiB).
+// Full spaces take it up to ROWS_FULL_MAX determinants, where the other kernel has too few threads to hide the
+// latency of its serial walk; beyond, that one's staged coefficients and coalesced alpha rows win.  us a sigma
+// (whole call, four roots), this kernel / the other: 441 determinants 22 / 78, 4 900 55 / 126, 15 876 159 / 170,
+// 63 504 657 / 619, 213 444 2955 / 2328.
+constexpr int64_t ROWS_FULL_MAX = 1 << 15;
+constexpr size_t ROWS_COUL_MAX = (size_t)1 << 30;
+
+pq_status ci_sigma_rows_build(pq_ci_handle *h) {
+  using namespace rows;
+  if (h->n_species != 1 || h->n_dets <= 0 || h->n_dets > 0x7fffffffLL) return PQ_OK;
+  if (h->full && h->n_dets > ROWS_FULL_MAX) return PQ_OK;
+  const int npair = h->npair[0];
+  for (int sp = 0; sp < 2; sp++)
+    if (sizeof(double) * (size_t)npair * (size_t)h->tab[0][sp].n_str > ROWS_COUL_MAX) return PQ_OK;
+  cudaStream_t st = h->stream;
+  std::unique_ptr<SigmaRows, void (*)(SigmaRows *)> r(new (std::nothrow) SigmaRows(), rows_delete);
+  if (!r) {
+    set_error("host allocation failed");
+    return PQ_ERR_OOM;
+  }
+  r->lim = std::min(h->desc.ex_level[0][2], h->desc.max_collective);
+  for (int sp = 0; sp < 2; sp++) {
+    const SpinTablesDev &t = h->tab[0][sp];
+    SigmaRows::Side &s = r->side[sp];
+    PQ_TRY(upload(s.lvl, h->lvl[0][sp], st));
+    PQ_TRY(s.s1.alloc(sizeof(int2) * (t.n1 + 1)));
+    PQ_TRY(s.s1_F.alloc(sizeof(double) * (t.n1 + 1)));
+    PQ_TRY(s.s2.alloc(sizeof(int32_t) * (t.n2 + 1)));
+    PQ_TRY(s.s2_D.alloc(sizeof(double) * (t.n2 + 1)));
+    PQ_TRY(s.cum.alloc(sizeof(int32_t) * 8 * t.n_str));
+    PQ_TRY(s.coul.alloc(sizeof(double) * (size_t)npair * t.n_str));
+    group_kernel<<<(unsigned)((t.n_str + 3) / 4), 128, 0, st>>>(
+        t.n_str, s.lvl.as<int32_t>(), sp == 0 ? h->d_rowoff.as<int64_t>() : nullptr, t.s1_off.as<int64_t>(),
+        t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(),
+        t.s2_J.as<int32_t>(), t.s2_D64.as<double>(), s.s1.as<int2>(), s.s1_F.as<double>(), s.s2.as<int32_t>(),
+        s.s2_D.as<double>(), s.cum.as<int32_t>());
+    PQ_CUDA_TRY(cudaGetLastError());
+    // strings of this spin stand beside singles of the other one: eab is [pair_alpha][pair_beta]
+    const int64_t total = (int64_t)npair * t.n_str;
+    coulomb_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 152 * 16), 256, 0, st>>>(
+        h->d_eab64.as<double>(), npair, sp == 0 ? 1 : npair, sp == 0 ? npair : 1, t.str.as<uint64_t>(),
+        t.str_hi.as<uint64_t>(), t.n_str, s.coul.as<double>());
+    PQ_CUDA_TRY(cudaGetLastError());
+  }
+  const int64_t na = h->tab[0][0].n_str;
+  PQ_TRY(r->row.alloc(sizeof(int32_t) * h->n_dets));
+  row_kernel<<<(unsigned)std::min<int64_t>(na, 152 * 16), 128, 0, st>>>(h->d_rowoff.as<int64_t>(),
+                                                                       h->d_rowlen.as<int32_t>(), na, r->row.as<int32_t>());
+  PQ_CUDA_TRY(cudaGetLastError());
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  h->rows = std::move(r);
+  return PQ_OK;
+}
+
+pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift) {
+  using namespace rows;
+  const SigmaRows &r = *h->rows;
+  Args p{};
+  Side *out[2] = {&p.a, &p.b};
+  for (int sp = 0; sp < 2; sp++) {
+    const SpinTablesDev &t = h->tab[0][sp];
+    const SigmaRows::Side &s = r.side[sp];
+    *out[sp] = {t.s1_off.as<int64_t>(), t.s2_off.as<int64_t>(), s.s1.as<int2>(),  s.s1_F.as<double>(),
+                s.s2.as<int32_t>(),     s.s2_D.as<double>(),    s.cum.as<int4>(), s.lvl.as<int32_t>(),
+                s.coul.as<double>()};
+  }
+  p.row = r.row.as<int32_t>();
+  p.rowoff = h->d_rowoff.as<int64_t>();
+  p.eab = h->d_eab64.as<double>();
+  p.diag = h->d_diag.as<double>();
+  p.shift = shift;
+  p.npair = h->npair[0];
+  p.lim = r.lim;
+  p.n = h->n_dets;
+  p.X = (const double *)X;
+  p.Y = (double *)Y;
+  const unsigned grid = (unsigned)((p.n + WARPS - 1) / WARPS);
+  if (nvp == 1)
+    sigma_rows_kernel<1><<<grid, 32 * WARPS, 0, h->stream>>>(p);
+  else if (nvp == 2)
+    sigma_rows_kernel<2><<<grid, 32 * WARPS, 0, h->stream>>>(p);
+  else if (nvp == 3)
+    sigma_rows_kernel<3><<<grid, 32 * WARPS, 0, h->stream>>>(p);
+  else if (nvp == 4)
+    sigma_rows_kernel<4><<<grid, 32 * WARPS, 0, h->stream>>>(p);
+  else {
+    set_error("sigma: unsupported interleave width %d (widths 1 to 4)", nvp);
+    return PQ_ERR_ARG;
+  }
+  PQ_CUDA_TRY(cudaGetLastError());
+  return PQ_OK;
+}
+
+}  // namespace pq

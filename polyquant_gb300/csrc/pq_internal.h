@@ -79,6 +79,8 @@ struct SpinTablesDev {
 
 struct SameSpinGemm;  // ci_sigma32_ss.cu
 void ss_delete(SameSpinGemm *g);
+struct SigmaRows;  // ci_sigma_rows.cu
+void rows_delete(SigmaRows *r);
 
 }  // namespace pq
 
@@ -123,6 +125,8 @@ struct pq_ci_handle {
   bool fp32_tc = false;  // the FP32 full-CI sigma uses the tensor-core alpha-beta path
   bool fp32_ss = false;  // ... and the same-spin doubles as tensor-core GEMMs (ci_sigma32_ss.cu)
   std::unique_ptr<pq::SameSpinGemm, void (*)(pq::SameSpinGemm *)> ss{nullptr, pq::ss_delete};
+  // FP64 sigma with a warp per determinant (ci_sigma_rows.cu); empty where ci_sigma.cu's kernel runs
+  std::unique_ptr<pq::SigmaRows, void (*)(pq::SigmaRows *)> rows{nullptr, pq::rows_delete};
   // two species: addressing of the product space (see ci_two.cu)
   std::vector<int32_t> e_a, e_b;        // species-0 (alpha, beta) string pair of each kept pair ie
   std::vector<int64_t> ebase;           // first determinant of pair ie's species-1 block
@@ -164,19 +168,18 @@ pq_status ci_ham_rows2(pq_ci_handle *h, double thr, int32_t *cnt, const int64_t 
 // allow_scratch = false keeps sigma on kernels that need no work memory beyond X and Y
 pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int precision, double shift,
                       bool allow_scratch = true);
+// ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
+pq_status ci_sigma_rows_build(pq_ci_handle *h);
+pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
 // ci_explicit.cu: sigma with the explicit matrix (FP64, interleaved vectors)
 pq_status ci_ham_spmv(pq_ci_handle *h, const void *X, void *Y, int nvp);
 // exact FP64 columns H[:, dets[c]] into column-major W (one species)
 pq_status ci_unit_columns(pq_ci_handle *h, const std::vector<int64_t> &dets, double *W);
 // ci_element.cu: exact H_IJ of n pairs (host index arrays, host output)
 pq_status ci_elements(pq_ci_handle *h, int64_t n, const int64_t *I, const int64_t *J, double *out);
-// interleave width of a block of nv <= 4 vectors: 1, 2 or 4; two-species spaces take 3 in FP64 (their FP64
-// sigma is bound by the FP64 pipe, so a padded fourth root would only add FMAs), while in FP32 four roots
-// load as one 16-byte vector
-inline int il_width(const pq_ci_handle *h, int nv, int precision) {
-  if (nv == 3 && h->n_species == 2 && precision == PQ_FP64) return 3;
-  return nv == 1 ? 1 : (nv == 2 ? 2 : 4);
-}
+// interleave width of a block of nv <= 4 vectors: three FP64 vectors stay three (FP64 sigma is bound by the FP64
+// pipe, so a padded fourth would only add FMAs), three FP32 vectors take four (one 16-byte load)
+inline int il_width(const pq_ci_handle *, int nv, int precision) { return nv == 3 && precision == PQ_FP32 ? 4 : nv; }
 // ci_sigma32.cu
 bool sigma32_v2_applicable(const pq_ci_handle *h);
 pq_status ci_sigma32_v2(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
