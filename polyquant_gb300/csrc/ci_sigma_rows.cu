@@ -29,134 +29,38 @@
 // orbitals (441 determinants), one root: 18 against 41 us.
 #include <algorithm>
 
-#include "pq_bits.cuh"
-#include "pq_internal.h"
+#include "ci_rows.cuh"
 
 namespace pq {
-
-// Grouped tables of one spin list and the Coulomb sums of its strings.
-struct SigmaRows {
-  struct Side {
-    DevBuf s1;    // int2 {partner (row offset for alpha, string for beta), info}, grouped by level change
-    DevBuf s1_F;  // same-spin part of the element
-    DevBuf s2, s2_D;
-    DevBuf cum;   // per string 8 x int32: ends of the 3 groups of singles and the 5 groups of doubles
-    DevBuf lvl;
-    DevBuf coul;  // [string][pair]: sum over the string's orbitals k of (pair of the other spin | kk)
-  };
-  Side side[2];
-  DevBuf row;  // alpha string of every determinant
-  int lim = 0;
-};
 
 void rows_delete(SigmaRows *r) { delete r; }
 
 namespace rows {
 
-constexpr int WARPS = 8;
-constexpr int HEAVY = 1536;  // connections above which the CTA shares a determinant
-constexpr int U = 4;         // gathers in flight per lane
+constexpr int U = 4;  // gathers in flight per lane
 
-struct Side {
-  const int64_t *o1, *o2;
-  const int2 *s1;
-  const double *F;
-  const int32_t *s2;
-  const double *D;
-  const int4 *cum;
-  const int32_t *lvl;
-  const double *coul;
-};
-
-struct Args {
-  Side a, b;
-  const int32_t *row;
-  const int64_t *rowoff;
-  const double *eab, *diag;
-  double shift;
-  int npair, lim;
-  int64_t n;
-  const double *X;
-  double *Y;
-};
-
-template <int NV> __device__ __forceinline__ void load_x(const double *X, int64_t j, double (&x)[NV]) {
-  const double *p = X + j * NV;
-  if constexpr (NV == 2 || NV == 4) {
-#pragma unroll
-    for (int v = 0; v < NV; v += 2) {
-      const double2 d = __ldg(reinterpret_cast<const double2 *>(p + v));
-      x[v] = d.x, x[v + 1] = d.y;
-    }
-  } else {
-#pragma unroll
-    for (int v = 0; v < NV; v++) x[v] = __ldg(p + v);
-  }
-}
-
-__device__ __forceinline__ double flip(double v, int neg) {
-  return __hiloint2double(__double2hiint(v) ^ (neg << 31), __double2loint(v));
-}
-
-// One determinant's connection classes: list bounds after the level limits.
-struct Det {
-  int64_t I, rowI, a1, a2, b1, b2;
-  int ia, ib;
-  int ca1[4], cb1[4];     // group starts of the singles (ca1[0] = 0)
-  int na1, na2, nb1, nb2;  // kept singles and doubles of either spin
-  int nbx[3];              // kept beta singles beside an alpha single of group g
-  int total;
-};
-
-__device__ __forceinline__ Det load_det(const Args &p, int64_t I) {
-  Det d;
-  d.I = I;
-  d.ia = p.row[I];
-  d.rowI = p.rowoff[d.ia];
-  d.ib = (int)(I - d.rowI);
-  d.a1 = p.a.o1[d.ia], d.a2 = p.a.o2[d.ia];
-  d.b1 = p.b.o1[d.ib], d.b2 = p.b.o2[d.ib];
-  const int slack = min(p.lim - p.a.lvl[d.ia] - p.b.lvl[d.ib], 4);  // >= 0 for a determinant of the list
-  const int4 x0 = p.a.cum[2 * d.ia], x1 = p.a.cum[2 * d.ia + 1];
-  const int4 y0 = p.b.cum[2 * d.ib], y1 = p.b.cum[2 * d.ib + 1];
-  d.ca1[0] = 0, d.ca1[1] = x0.x, d.ca1[2] = x0.y, d.ca1[3] = x0.z;
-  d.cb1[0] = 0, d.cb1[1] = y0.x, d.cb1[2] = y0.y, d.cb1[3] = y0.z;
-  // a group of change c is kept when c <= slack
-  d.na1 = slack >= 1 ? x0.z : x0.y;
-  d.nb1 = slack >= 1 ? y0.z : y0.y;
-  d.na2 = slack >= 2 ? x1.w : (slack == 1 ? x1.z : x1.y);
-  d.nb2 = slack >= 2 ? y1.w : (slack == 1 ? y1.z : y1.y);
-  d.total = 1 + d.na1 + d.nb1 + d.na2 + d.nb2;
-#pragma unroll
-  for (int g = 0; g < 3; g++) {
-    // alpha change g - 1 leaves slack - (g - 1) for the beta change
-    const int s = slack - (g - 1);
-    d.nbx[g] = s >= 1 ? y0.z : (s == 0 ? y0.y : (s == -1 ? y0.x : 0));
-    d.total += (d.ca1[g + 1] - d.ca1[g]) * d.nbx[g];
-  }
-  return d;
-}
-
-// acc += c x for U list entries at t0 + u * nth of a list of `cnt`; entry(t, idx) returns the element and the
-// partner.  Entries past the end load nothing.
-template <int NV, typename E>
-__device__ __forceinline__ void gather(const Args &p, double (&acc)[NV], int t0, int nth, int cnt, E &&entry) {
-  for (int t = t0; t - t0 < cnt; t += U * nth) {
+// acc += c x over the entries tid, tid + nth, ... of a list of n, U of them in flight; entries past the end load
+// nothing
+template <int NV, typename M>
+__device__ __forceinline__ void gather(const Args &p, double (&acc)[NV], int tid, int nth, int n, M &&make) {
+  if (n == 0) return;
+  auto entry = make(tid, nth);
+  for (int t0 = 0; t0 < n; t0 += U * nth) {
     double c[U], x[U][NV];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       c[u] = 0.0;
 #pragma unroll
       for (int v = 0; v < NV; v++) x[u][v] = 0.0;
-      if (t + u * nth < cnt) {
+      if (t0 + u * nth + tid < n) {
         int64_t j;
-        c[u] = entry(t + u * nth, j);
+        c[u] = entry(j);
         load_x<NV>(p.X, j, x[u]);
       }
     }
 #pragma unroll
     for (int u = 0; u < U; u++)
-      if (t - t0 + u * nth < cnt) {  // uniform over the sharing threads: lane 0's entry exists
+      if (t0 + u * nth < n) {  // the same for all threads that share the list
 #pragma unroll
         for (int v = 0; v < NV; v++) acc[v] = fma(c[u], x[u][v], acc[v]);
       }
@@ -173,40 +77,7 @@ __device__ __forceinline__ void accumulate(const Args &p, const Det &d, int tid,
 #pragma unroll
     for (int v = 0; v < NV; v++) acc[v] = h * x[v];
   }
-  gather<NV>(p, acc, tid, nth, d.na1, [&](int t, int64_t &j) {
-    const int2 e = __ldg(p.a.s1 + d.a1 + t);
-    j = (int64_t)e.x + d.ib;
-    return flip(__ldg(p.a.F + d.a1 + t) + __ldg(p.b.coul + (int64_t)d.ib * p.npair + (e.y >> 1)), e.y & 1);
-  });
-  gather<NV>(p, acc, tid, nth, d.nb1, [&](int t, int64_t &j) {
-    const int2 e = __ldg(p.b.s1 + d.b1 + t);
-    j = d.rowI + e.x;
-    return flip(__ldg(p.b.F + d.b1 + t) + __ldg(p.a.coul + (int64_t)d.ia * p.npair + (e.y >> 1)), e.y & 1);
-  });
-  gather<NV>(p, acc, tid, nth, d.na2, [&](int t, int64_t &j) {
-    j = (int64_t)__ldg(p.a.s2 + d.a2 + t) + d.ib;
-    return __ldg(p.a.D + d.a2 + t);
-  });
-  gather<NV>(p, acc, tid, nth, d.nb2, [&](int t, int64_t &j) {
-    j = d.rowI + __ldg(p.b.s2 + d.b2 + t);
-    return __ldg(p.b.D + d.b2 + t);
-  });
-#pragma unroll
-  for (int g = 0; g < 3; g++) {
-    const int nb = d.nbx[g], cnt = (d.ca1[g + 1] - d.ca1[g]) * nb;
-    if (cnt == 0) continue;
-    // entry t is (alpha single t / nb, beta single t % nb); stepping by nth adds (qs, rs) with a carry
-    const int qs = nth / nb, rs = nth - qs * nb;
-    int ea = tid / nb, eb = tid - ea * nb;
-    const int2 *la = p.a.s1 + d.a1 + d.ca1[g], *lb = p.b.s1 + d.b1;
-    gather<NV>(p, acc, tid, nth, cnt, [&](int, int64_t &j) {
-      const int2 a = __ldg(la + ea), b = __ldg(lb + eb);
-      ea += qs, eb += rs;
-      if (eb >= nb) eb -= nb, ea++;
-      j = (int64_t)a.x + b.x;
-      return flip(__ldg(p.eab + (int64_t)(a.y >> 1) * p.npair + (b.y >> 1)), (a.y ^ b.y) & 1);
-    });
-  }
+  for_lists(p, d, [&](int n, auto &&make) { gather<NV>(p, acc, tid, nth, n, make); });
 }
 
 // Sum of acc over the warp: the halving steps also halve the number of values a lane carries, so four roots take
@@ -342,21 +213,17 @@ __global__ void __launch_bounds__(128) row_kernel(const int64_t *rowoff, const i
 
 }  // namespace rows
 
-// Rule.  Truncated spaces always take this kernel (32-bit determinant indices, Coulomb tables of at most 1 GiB).
-// Full spaces take it up to ROWS_FULL_MAX determinants, where the other kernel has too few threads to hide the
-// latency of its serial walk; beyond, that one's staged coefficients and coalesced alpha rows win.  us a sigma
-// (whole call, four roots), this kernel / the other: 441 determinants 22 / 78, 4 900 55 / 126, 15 876 159 / 170,
-// 63 504 657 / 619, 213 444 2955 / 2328.
+// Rule.  Truncated spaces always take this kernel (32-bit determinant indices).  Full spaces take it up to
+// ROWS_FULL_MAX determinants, where the other kernel has too few threads to hide the latency of its serial walk;
+// beyond, that one's staged coefficients and coalesced alpha rows win.  us a sigma (whole call, four roots), this
+// kernel / the other: 441 determinants 22 / 78, 4 900 55 / 126, 15 876 159 / 170, 63 504 657 / 619, 213 444
+// 2955 / 2328.
 constexpr int64_t ROWS_FULL_MAX = 1 << 15;
-constexpr size_t ROWS_COUL_MAX = (size_t)1 << 30;
+constexpr size_t ROWS_COUL_MAX = (size_t)1 << 30;  // larger Coulomb tables are summed in the kernel instead
 
-pq_status ci_sigma_rows_build(pq_ci_handle *h) {
+pq_status rows_make(pq_ci_handle *h, std::unique_ptr<SigmaRows, void (*)(SigmaRows *)> &out) {
   using namespace rows;
-  if (h->n_species != 1 || h->n_dets <= 0 || h->n_dets > 0x7fffffffLL) return PQ_OK;
-  if (h->full && h->n_dets > ROWS_FULL_MAX) return PQ_OK;
   const int npair = h->npair[0];
-  for (int sp = 0; sp < 2; sp++)
-    if (sizeof(double) * (size_t)npair * (size_t)h->tab[0][sp].n_str > ROWS_COUL_MAX) return PQ_OK;
   cudaStream_t st = h->stream;
   std::unique_ptr<SigmaRows, void (*)(SigmaRows *)> r(new (std::nothrow) SigmaRows(), rows_delete);
   if (!r) {
@@ -373,15 +240,15 @@ pq_status ci_sigma_rows_build(pq_ci_handle *h) {
     PQ_TRY(s.s2.alloc(sizeof(int32_t) * (t.n2 + 1)));
     PQ_TRY(s.s2_D.alloc(sizeof(double) * (t.n2 + 1)));
     PQ_TRY(s.cum.alloc(sizeof(int32_t) * 8 * t.n_str));
-    PQ_TRY(s.coul.alloc(sizeof(double) * (size_t)npair * t.n_str));
     group_kernel<<<(unsigned)((t.n_str + 3) / 4), 128, 0, st>>>(
         t.n_str, s.lvl.as<int32_t>(), sp == 0 ? h->d_rowoff.as<int64_t>() : nullptr, t.s1_off.as<int64_t>(),
         t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(),
         t.s2_J.as<int32_t>(), t.s2_D64.as<double>(), s.s1.as<int2>(), s.s1_F.as<double>(), s.s2.as<int32_t>(),
         s.s2_D.as<double>(), s.cum.as<int32_t>());
     PQ_CUDA_TRY(cudaGetLastError());
-    // strings of this spin stand beside singles of the other one: eab is [pair_alpha][pair_beta]
     const int64_t total = (int64_t)npair * t.n_str;
+    if (sizeof(double) * (size_t)total > ROWS_COUL_MAX) continue;
+    PQ_TRY(s.coul.alloc(sizeof(double) * (size_t)total));
     coulomb_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 152 * 16), 256, 0, st>>>(
         h->d_eab64.as<double>(), npair, sp == 0 ? 1 : npair, sp == 0 ? npair : 1, t.str.as<uint64_t>(),
         t.str_hi.as<uint64_t>(), t.n_str, s.coul.as<double>());
@@ -393,30 +260,42 @@ pq_status ci_sigma_rows_build(pq_ci_handle *h) {
                                                                        h->d_rowlen.as<int32_t>(), na, r->row.as<int32_t>());
   PQ_CUDA_TRY(cudaGetLastError());
   PQ_CUDA_TRY(cudaStreamSynchronize(st));
-  h->rows = std::move(r);
+  out = std::move(r);
   return PQ_OK;
 }
 
-pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift) {
-  using namespace rows;
-  const SigmaRows &r = *h->rows;
-  Args p{};
-  Side *out[2] = {&p.a, &p.b};
+rows::Args rows_args(const pq_ci_handle *h, const SigmaRows &r) {
+  rows::Args p{};
+  rows::Side *out[2] = {&p.a, &p.b};
+  p.npair = h->npair[0];
   for (int sp = 0; sp < 2; sp++) {
     const SpinTablesDev &t = h->tab[0][sp];
     const SigmaRows::Side &s = r.side[sp];
-    *out[sp] = {t.s1_off.as<int64_t>(), t.s2_off.as<int64_t>(), s.s1.as<int2>(),  s.s1_F.as<double>(),
-                s.s2.as<int32_t>(),     s.s2_D.as<double>(),    s.cum.as<int4>(), s.lvl.as<int32_t>(),
-                s.coul.as<double>()};
+    // strings of one spin stand beside singles of the other: eab is [pair_alpha][pair_beta]
+    *out[sp] = {t.s1_off.as<int64_t>(), t.s2_off.as<int64_t>(), s.s1.as<int2>(),     s.s1_F.as<double>(),
+                s.s2.as<int32_t>(),     s.s2_D.as<double>(),    s.cum.as<int4>(),    s.lvl.as<int32_t>(),
+                s.coul.as<double>(),    t.str.as<uint64_t>(),   t.str_hi.as<uint64_t>(),
+                sp == 0 ? 1 : p.npair,  sp == 0 ? p.npair : 1};
   }
   p.row = r.row.as<int32_t>();
   p.rowoff = h->d_rowoff.as<int64_t>();
   p.eab = h->d_eab64.as<double>();
   p.diag = h->d_diag.as<double>();
-  p.shift = shift;
-  p.npair = h->npair[0];
   p.lim = r.lim;
   p.n = h->n_dets;
+  return p;
+}
+
+pq_status ci_sigma_rows_build(pq_ci_handle *h) {
+  if (h->n_species != 1 || h->n_dets <= 0 || h->n_dets > 0x7fffffffLL) return PQ_OK;
+  if (h->full && h->n_dets > ROWS_FULL_MAX) return PQ_OK;
+  return rows_make(h, h->rows);
+}
+
+pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift) {
+  using namespace rows;
+  Args p = rows_args(h, *h->rows);
+  p.shift = shift;
   p.X = (const double *)X;
   p.Y = (double *)Y;
   const unsigned grid = (unsigned)((p.n + WARPS - 1) / WARPS);
