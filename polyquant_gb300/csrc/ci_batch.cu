@@ -23,7 +23,6 @@
 // captured once as a CUDA graph and replayed.  The launch shape (warps per
 // CTA, rows per work unit) is chosen by timing candidates on a sample of the
 // group's work units.
-#include <cublas_v2.h>
 
 #include <algorithm>
 #include <chrono>
@@ -1203,23 +1202,13 @@ pq_status pq_ci_batch_davidson(pq_ci_batch *b, const pq_davidson_params *p, size
     groups.back().push_back(pi);
     used += need;
   }
-  cublasHandle_t cb = nullptr;
-  if (cublasCreate(&cb) != CUBLAS_STATUS_SUCCESS) {
-    set_error("cublasCreate failed");
-    return PQ_ERR_CUDA;
-  }
-  cublasSetStream(cb, b->stream);
-  struct CbGuard {
-    cublasHandle_t c;
-    ~CbGuard() { cublasDestroy(c); }
-  } guard{cb};
   pq_status overall = PQ_OK;
   b->all.reset();  // the sigma-call plan may assume another width
   for (const auto &grp : groups) {
     std::vector<std::unique_ptr<DavidsonRun>> runs;
     for (int pi : grp) {
       runs.emplace_back(new DavidsonRun());
-      pq_status s = runs.back()->init(b->h[pi], *p, cb);
+      pq_status s = runs.back()->init(b->h[pi], *p);
       if (s != PQ_OK) {
         set_error("problem %d: %s", pi, pq_last_error());
         return s;

@@ -9,15 +9,13 @@
 // the converged energies only.
 //
 // All subspace algebra (Gram-Schmidt, projections, Ritz vectors, residual
-// norms, preconditioner denominators) is FP64 on the device through cuBLAS;
-// the Rayleigh matrix eigenproblem (at most a few hundred rows) is solved on
+// norms, preconditioner denominators) is FP64 on the device in the tall-skinny
+// kernels below; the Rayleigh matrix eigenproblem (at most a few hundred rows) is solved on
 // the host in FP64.  With precision = PQ_FP32 the sigma vectors of new search
 // directions come from the FP32 kernel applied to (H - s) with s the current
 // lowest Ritz value, and every restart recomputes the Ritz vectors' sigma in
 // FP64 ("residual refinement"), so reported energies and residual norms are
 // always exact FP64 Rayleigh quotients and residuals.
-#include <cublas_v2.h>
-
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -28,15 +26,6 @@
 #include "pq_internal.h"
 
 namespace pq {
-
-#define PQ_CUBLAS_TRY(call)                                                          \
-  do {                                                                               \
-    cublasStatus_t cs_ = (call);                                                     \
-    if (cs_ != CUBLAS_STATUS_SUCCESS) {                                              \
-      set_error("%s failed: cublas status %d (%s:%d)", #call, (int)cs_, __FILE__, __LINE__); \
-      return PQ_ERR_CUDA;                                                            \
-    }                                                                                \
-  } while (0)
 
 // Cyclic Jacobi eigensolver for a small symmetric matrix (column-major n x n).
 // Eigenvalues ascending in w, eigenvectors in the columns of Z.
@@ -88,16 +77,229 @@ static void jacobi_eigh(int n, std::vector<double> A, std::vector<double> &w, st
   Z.swap(Zs);
 }
 
-// C[:, j] = op(A) B[:, j] for j < q, one DGEMV per column.  A is the tall
-// n x m block of V or W (n up to ~1e9 rows, m <= a few dozen columns): DGEMV
-// streams it at the FP64 FMA rate, while DGEMM on these shapes runs an order
-// of magnitude slower.
-static pq_status tall_skinny(cublasHandle_t cb, cublasOperation_t op, int64_t n, int m, const double *A,
-                             const double *B, int64_t ldb, int q, double *C, int64_t ldc) {
-  const double one = 1.0, zero = 0.0;
-  for (int j = 0; j < q; j++)
-    PQ_CUBLAS_TRY(cublasDgemv(cb, op, (int)n, m, &one, A, (int)n, B + (size_t)j * ldb, 1, &zero, C + (size_t)j * ldc, 1));
-  return PQ_OK;
+// ---- tall-skinny kernels: n rows (up to ~2^31), m <= a few dozen columns, leading dimension n
+//
+// For large n all of these run at the FP64 pipe's rate, as library DGEMV did.  For the n of small solves they were
+// bound by launches, host synchronisations and the serial tail of the norms: a four-root solve of a 10-orbital full
+// CI (63 504 determinants) issued 448 norms of 35 us and about 500 DGEMV and dot launches.  Here one launch does
+// what belongs together (Ritz vectors, residuals and their norms; all projections of a vector and its norm), sums
+// are finished by the last block to arrive, in block order, so results do not vary between runs, and Gram-Schmidt
+// takes its decisions on the device.  That solve takes 21.4 ms against 41.4, 9.4 of them in sigma (before: the same 9.4).
+constexpr int TS_THREADS = 256;
+constexpr int TS_MI = 8, TS_Q = 4;  // register tile of the products: columns of V x columns of the other block
+
+// Sums of K (a power of two, at most 32) values over a warp in K - 1 exchanges and log2(32 / K) full steps; lane l
+// ends with value l % K in acc[0].
+template <int K> __device__ __forceinline__ void warp_sums(double (&acc)[K], int lane) {
+#pragma unroll
+  for (int h = K / 2; h; h >>= 1) {
+    const bool up = lane & h;
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const double send = up ? acc[i] : acc[i + h], keep = up ? acc[i + h] : acc[i];
+      acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  }
+#pragma unroll
+  for (int w = K; w < 32; w <<= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], w);
+}
+
+// Sum of acc over all blocks of gridDim.x: block partials in part[block][K]; returns true in the threads of the last
+// block to arrive, whose threads 0 .. K - 1 hold the totals in *tot.  cnt is a counter at zero, left at zero.
+template <int K>
+__device__ __forceinline__ bool grid_sums(double (&acc)[K], double *part, unsigned *cnt, double *tot) {
+  __shared__ double red[TS_THREADS / 32][K];
+  __shared__ double fin[TS_THREADS];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  warp_sums<K>(acc, lane);
+  if (lane < K) red[warp][lane] = acc[0];
+  __syncthreads();
+  if (threadIdx.x < K) {
+    double s = 0.0;
+    for (int w = 0; w < TS_THREADS / 32; w++) s += red[w][threadIdx.x];
+    part[(int64_t)blockIdx.x * K + threadIdx.x] = s;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(cnt, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  // K sums over the blocks, TS_THREADS / K threads each
+  double s = 0.0;
+#pragma unroll 4
+  for (unsigned b = threadIdx.x / K; b < gridDim.x; b += TS_THREADS / K) s += __ldcg(part + (int64_t)b * K + threadIdx.x % K);
+  fin[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = TS_THREADS / 2; w >= K; w >>= 1) {  // w is a multiple of K: values stay apart
+    if ((int)threadIdx.x < w) fin[threadIdx.x] += fin[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x < K) *tot = fin[threadIdx.x];
+  if (threadIdx.x == 0) *cnt = 0;
+  return true;
+}
+
+// out[i + j * ldo] = A[:, i] . S[:, j], i < m, j < q: tiles of TS_MI x TS_Q over blockIdx.y and blockIdx.z
+__global__ void __launch_bounds__(TS_THREADS) gram_kernel(const double *A, const double *S, int64_t n, int m, int q,
+                                                         double *part, unsigned *cnt, double *out, int ldo) {
+  const int i0 = blockIdx.y * TS_MI, j0 = blockIdx.z * TS_Q;
+  const int mi = min(TS_MI, m - i0), qj = min(TS_Q, q - j0);
+  A += (int64_t)i0 * n;
+  S += (int64_t)j0 * n;
+  double acc[TS_MI * TS_Q];
+#pragma unroll
+  for (int t = 0; t < TS_MI * TS_Q; t++) acc[t] = 0.0;
+  for (int64_t r = (int64_t)blockIdx.x * TS_THREADS + threadIdx.x; r < n; r += (int64_t)gridDim.x * TS_THREADS) {
+    double a[TS_MI], s[TS_Q];
+#pragma unroll
+    for (int i = 0; i < TS_MI; i++) a[i] = i < mi ? A[r + i * n] : 0.0;
+#pragma unroll
+    for (int j = 0; j < TS_Q; j++) s[j] = j < qj ? S[r + j * n] : 0.0;
+#pragma unroll
+    for (int j = 0; j < TS_Q; j++)
+      if (j < qj)
+#pragma unroll
+        for (int i = 0; i < TS_MI; i++)
+          if (i < mi) acc[j * TS_MI + i] = fma(a[i], s[j], acc[j * TS_MI + i]);
+  }
+  const int tile = blockIdx.z * gridDim.y + blockIdx.y;
+  double tot;
+  if (!grid_sums<TS_MI * TS_Q>(acc, part + (int64_t)tile * gridDim.x * (TS_MI * TS_Q), cnt + tile, &tot)) return;
+  if (threadIdx.x < TS_MI * TS_Q) {
+    const int i = threadIdx.x % TS_MI, j = threadIdx.x / TS_MI;
+    if (i < mi && j < qj) out[(i0 + i) + (int64_t)(j0 + j) * ldo] = tot;
+  }
+}
+
+// out[:, j] = A[:, 0:m] Z[:, j], j < q (Z column-major, leading dimension m); tiles of TS_Q columns over blockIdx.y
+__global__ void __launch_bounds__(TS_THREADS) rotate_kernel(const double *A, const double *Z, int64_t n, int m, int q,
+                                                           double *out) {
+  const int j0 = blockIdx.y * TS_Q, qj = min(TS_Q, q - j0);
+  Z += (int64_t)j0 * m;
+  for (int64_t r = (int64_t)blockIdx.x * TS_THREADS + threadIdx.x; r < n; r += (int64_t)gridDim.x * TS_THREADS) {
+    double x[TS_Q] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int i = 0; i < m; i++) {
+      const double a = A[r + i * n];
+#pragma unroll
+      for (int j = 0; j < TS_Q; j++)
+        if (j < qj) x[j] = fma(a, __ldg(Z + i + (int64_t)j * m), x[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < TS_Q; j++)
+      if (j < qj) out[r + (int64_t)(j0 + j) * n] = x[j];
+  }
+}
+
+// X = V Z, R = W Z - X theta and |R_j|^2 for k Ritz pairs (zt holds Z, m x k, then theta)
+__global__ void __launch_bounds__(TS_THREADS) ritz_kernel(const double *V, const double *W, const double *zt, int64_t n,
+                                                         int m, int k, double *X, double *R, double *part,
+                                                         unsigned *cnt, double *rn2) {
+  const int j0 = blockIdx.y * TS_Q, qj = min(TS_Q, k - j0);
+  const double *Z = zt + (int64_t)j0 * m, *theta = zt + (int64_t)m * k + j0;
+  double acc[TS_Q] = {0.0, 0.0, 0.0, 0.0};
+  for (int64_t r = (int64_t)blockIdx.x * TS_THREADS + threadIdx.x; r < n; r += (int64_t)gridDim.x * TS_THREADS) {
+    double x[TS_Q] = {0.0, 0.0, 0.0, 0.0}, y[TS_Q] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int i = 0; i < m; i++) {
+      const double v = V[r + i * n], w = W[r + i * n];
+#pragma unroll
+      for (int j = 0; j < TS_Q; j++)
+        if (j < qj) {
+          const double z = __ldg(Z + i + (int64_t)j * m);
+          x[j] = fma(v, z, x[j]);
+          y[j] = fma(w, z, y[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < TS_Q; j++)
+      if (j < qj) {
+        const double d = fma(-__ldg(theta + j), x[j], y[j]);
+        X[r + (int64_t)(j0 + j) * n] = x[j];
+        R[r + (int64_t)(j0 + j) * n] = d;
+        acc[j] = fma(d, d, acc[j]);
+      }
+  }
+  double tot;
+  if (!grid_sums<TS_Q>(acc, part + (int64_t)blockIdx.y * gridDim.x * TS_Q, cnt + blockIdx.y, &tot)) return;
+  if ((int)threadIdx.x < qj) rn2[j0 + threadIdx.x] = tot;
+}
+
+// Gram-Schmidt of one vector t against the mm columns of V, on the device: squared norms of t before and after the
+// passes, and the number of columns of V, which grows when t is appended.
+struct GsState {
+  double n0, n1, n2;
+  int mm;
+};
+// the second pass is left out when the first kept at least 1/sqrt(2) of the norm (t is then orthogonal to working
+// precision)
+__device__ __forceinline__ bool gs_kept(const GsState &s) { return sqrt(s.n1) >= 0.70710678118654752 * sqrt(s.n0); }
+
+// coef[i] = V[:, i] . t for i < mm, and in the first pass n0 = t . t as one more column
+__global__ void __launch_bounds__(TS_THREADS) gs_dots_kernel(const double *V, const double *t, int64_t n, int pass,
+                                                            GsState *st, double *part, unsigned *cnt, double *coef) {
+  const int mm = st->mm, i0 = blockIdx.y * TS_MI;
+  if (i0 > mm || (pass == 1 && gs_kept(*st))) return;  // the same for every block of this column tile
+  const int mi = min(TS_MI, mm + 1 - i0);
+  V += (int64_t)i0 * n;
+  double acc[TS_MI];
+#pragma unroll
+  for (int i = 0; i < TS_MI; i++) acc[i] = 0.0;
+  for (int64_t r = (int64_t)blockIdx.x * TS_THREADS + threadIdx.x; r < n; r += (int64_t)gridDim.x * TS_THREADS) {
+    const double x = t[r];
+    double a[TS_MI];
+#pragma unroll
+    for (int i = 0; i < TS_MI; i++) a[i] = i >= mi ? 0.0 : (i0 + i < mm ? V[r + i * n] : x);
+#pragma unroll
+    for (int i = 0; i < TS_MI; i++)
+      if (i < mi) acc[i] = fma(a[i], x, acc[i]);
+  }
+  double tot;
+  if (!grid_sums<TS_MI>(acc, part + (int64_t)blockIdx.y * gridDim.x * TS_MI, cnt + blockIdx.y, &tot)) return;
+  if ((int)threadIdx.x < mi) {
+    if (i0 + (int)threadIdx.x < mm)
+      coef[i0 + threadIdx.x] = tot;
+    else if (pass == 0)
+      st->n0 = tot;
+  }
+}
+
+// t -= V coef; n1 (n2 in the second pass) = t . t
+__global__ void __launch_bounds__(TS_THREADS) gs_update_kernel(const double *V, double *t, int64_t n, int pass, GsState *st,
+                                                              double *part, unsigned *cnt, const double *coef) {
+  if (pass == 1 && gs_kept(*st)) return;
+  const int mm = st->mm;
+  double acc[1] = {0.0};
+  for (int64_t r = (int64_t)blockIdx.x * TS_THREADS + threadIdx.x; r < n; r += (int64_t)gridDim.x * TS_THREADS) {
+    double x = t[r];
+#pragma unroll 8
+    for (int i = 0; i < mm; i++) x = fma(-__ldg(coef + i), V[r + (int64_t)i * n], x);
+    t[r] = x;
+    acc[0] = fma(x, x, acc[0]);
+  }
+  double tot;
+  if (!grid_sums<1>(acc, part, cnt, &tot)) return;
+  if (threadIdx.x == 0) (pass == 0 ? st->n1 : st->n2) = tot;
+}
+
+// V[:, mm] = t / |t| unless t was (numerically) in the span of V
+__global__ void __launch_bounds__(TS_THREADS) gs_append_kernel(double *V, const double *t, int64_t n, GsState *st, unsigned *cnt) {
+  const double nrm0 = sqrt(st->n0), nrm = sqrt(gs_kept(*st) ? st->n1 : st->n2);
+  const int mm = st->mm;
+  if (!(nrm0 > 0.0) || !isfinite(nrm0) || !(nrm > 1e-8 * nrm0) || nrm < 1e-300) return;
+  const double inv = 1.0 / nrm;
+  double *v = V + (int64_t)mm * n;
+  for (int64_t r = (int64_t)blockIdx.x * TS_THREADS + threadIdx.x; r < n; r += (int64_t)gridDim.x * TS_THREADS) v[r] = t[r] * inv;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(cnt, 1u) == gridDim.x - 1) {  // every block has read mm
+      *cnt = 0;
+      st->mm = mm + 1;
+    }
+  }
 }
 
 __global__ void unit_vectors_kernel(double *V, int64_t n, const int64_t *idx, int m) {
@@ -158,16 +360,17 @@ __global__ void __launch_bounds__(SEL_THREADS) select_final_kernel(const ValIdx 
   if (threadIdx.x == 0) sel[j] = best;
 }
 
-// T[:, j] = R[:, j] / (theta_j - D)   (diagonal preconditioner)
-__global__ void precondition_kernel(const double *R, const double *D, const double *theta, int64_t n, int k,
-                                    double *T) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n * k; i += stride) {
-    int64_t c = i / n, r = i - c * n;
-    double den = theta[c] - D[r];
+// T[:, j] = R[:, root_j] / (theta_j - D)   (diagonal preconditioner)
+__global__ void __launch_bounds__(256) precondition_kernel(const double *R, const double *D, const double2 *th, int64_t n,
+                                                          double *T) {
+  const int c = blockIdx.y;
+  const double theta = th[c].x;
+  R += (int64_t)th[c].y * n;
+  T += (int64_t)c * n;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+    double den = theta - D[r];
     if (fabs(den) < 1e-8) den = den < 0 ? -1e-8 : 1e-8;
-    T[i] = R[i] / den;
+    T[r] = R[r] / den;
   }
 }
 
@@ -184,7 +387,7 @@ __global__ void unshift_kernel(const float *Y, int nvp, int nv, const double *V,
 // whenever sigma vectors are needed (a SigmaRequest), so one driver can serve a
 // single problem and a lockstep batch of problems with one sigma launch per
 // iteration.
-pq_status DavidsonRun::init(pq_ci_handle *hh, const pq_davidson_params &pp, ::cublasContext *shared_cb) {
+pq_status DavidsonRun::init(pq_ci_handle *hh, const pq_davidson_params &pp) {
   t_start = std::chrono::steady_clock::now();
   h = hh;
   p = pp;
@@ -200,7 +403,7 @@ pq_status DavidsonRun::init(pq_ci_handle *hh, const pq_davidson_params &pp, ::cu
     return PQ_ERR_ARG;
   }
   if (n > 0x7fffffffLL) {
-    set_error("davidson: n_dets beyond the 32-bit cuBLAS dimension limit");
+    set_error("davidson: n_dets beyond 2^31 - 1");
     return PQ_ERR_ARG;
   }
   m0 = std::max(p.num_subspace_vec, k);
@@ -216,22 +419,20 @@ pq_status DavidsonRun::init(pq_ci_handle *hh, const pq_davidson_params &pp, ::cu
   tol = p.convergence_E > 0 ? p.convergence_E : 1e-6;
   switch_tol = std::max(tol, 1e-5);
   phase32 = p.precision == PQ_FP32;
-  if (shared_cb) {
-    cb = shared_cb;
-  } else {
-    if (cublasCreate(&cb) != CUBLAS_STATUS_SUCCESS) {
-      set_error("cublasCreate failed");
-      return PQ_ERR_CUDA;
-    }
-    own_cb = true;
-    PQ_CUBLAS_TRY(cublasSetStream(cb, st));
-  }
   PQ_TRY(V.alloc(sizeof(double) * (size_t)n * mmax));
   PQ_TRY(W.alloc(sizeof(double) * (size_t)n * mmax));
   PQ_TRY(X.alloc(sizeof(double) * (size_t)n * k));
   PQ_TRY(R.alloc(sizeof(double) * (size_t)n * k));
   PQ_TRY(T.alloc(sizeof(double) * (size_t)n * std::max(k, m0)));
-  PQ_TRY(dth.alloc(sizeof(double) * std::max(k, 8)));
+  PQ_TRY(dth.alloc(sizeof(double) * 2 * std::max(k, 8)));
+  {
+    const int tiles = (mmax / TS_MI + 1) * ((std::max(m0, k) + TS_Q - 1) / TS_Q);
+    PQ_TRY(part.alloc(sizeof(double) * (size_t)ts_grid() * tiles * TS_MI * TS_Q));
+    PQ_TRY(cnt.alloc(sizeof(unsigned) * tiles));
+    PQ_CUDA_TRY(cudaMemsetAsync(cnt.ptr, 0, sizeof(unsigned) * tiles, st));
+    PQ_TRY(gs.alloc(sizeof(GsState)));
+    PQ_TRY(coef.alloc(sizeof(double) * (size_t)(mmax + 1)));
+  }
   theta.assign(k, 0.0);
   rnorm.assign(k, 0.0);
   // initial subspace: unit vectors at the m0 smallest diagonal elements (ties by index), selected on the device
@@ -305,17 +506,21 @@ pq_status DavidsonRun::advance() {
     PQ_TRY(rayleigh(m, G));
     jacobi_eigh(m, G, w, Z);
     for (int i = 0; i < k; i++) theta[i] = w[i];
-    PQ_TRY(tmp.ensure(sizeof(double) * (size_t)m * k));
-    std::vector<double> Yk(Z.begin(), Z.begin() + (size_t)m * k);
-    PQ_CUDA_TRY(cudaMemcpyAsync(tmp.ptr, Yk.data(), sizeof(double) * m * k, cudaMemcpyHostToDevice, st));
-    // X = V Y, R = W Y - X theta
-    PQ_TRY(tall_skinny(cb, CUBLAS_OP_N, n, m, V.as<double>(), tmp.as<double>(), m, k, X.as<double>(), n));
-    PQ_TRY(tall_skinny(cb, CUBLAS_OP_N, n, m, W.as<double>(), tmp.as<double>(), m, k, R.as<double>(), n));
+    // X = V Y, R = W Y - X theta and the residual norms
+    std::vector<double> zt(Z.begin(), Z.begin() + (size_t)m * k);
+    zt.insert(zt.end(), theta.begin(), theta.end());
+    PQ_TRY(tmp.ensure(sizeof(double) * (zt.size() + k)));
+    double *rn2 = tmp.as<double>() + zt.size();
+    PQ_CUDA_TRY(cudaMemcpyAsync(tmp.ptr, zt.data(), sizeof(double) * zt.size(), cudaMemcpyHostToDevice, st));
+    ritz_kernel<<<dim3(ts_grid(), (k + TS_Q - 1) / TS_Q), TS_THREADS, 0, st>>>(
+        V.as<double>(), W.as<double>(), tmp.as<double>(), n, m, k, X.as<double>(), R.as<double>(), part.as<double>(),
+        cnt.as<unsigned>(), rn2);
+    PQ_CUDA_TRY(cudaGetLastError());
+    PQ_CUDA_TRY(cudaMemcpyAsync(rnorm.data(), rn2, sizeof(double) * k, cudaMemcpyDeviceToHost, st));
+    PQ_CUDA_TRY(cudaStreamSynchronize(st));
     double maxr = 0.0;
     for (int i = 0; i < k; i++) {
-      double mt = -theta[i];
-      PQ_CUBLAS_TRY(cublasDaxpy(cb, (int)n, &mt, X.as<double>() + (size_t)i * n, 1, R.as<double>() + (size_t)i * n, 1));
-      PQ_CUBLAS_TRY(cublasDnrm2(cb, (int)n, R.as<double>() + (size_t)i * n, 1, &rnorm[i]));
+      rnorm[i] = std::sqrt(rnorm[i]);
       maxr = std::max(maxr, rnorm[i]);
     }
     if (p.verbose) {
@@ -361,7 +566,7 @@ pq_status DavidsonRun::advance() {
       std::vector<double> Zr(Z.begin(), Z.begin() + (size_t)m * r);
       PQ_CUDA_TRY(cudaMemcpyAsync(tmp.ptr, Zr.data(), sizeof(double) * m * r, cudaMemcpyHostToDevice, st));
       PQ_TRY(T.ensure(sizeof(double) * (size_t)n * r));
-      PQ_TRY(tall_skinny(cb, CUBLAS_OP_N, n, m, V.as<double>(), tmp.as<double>(), m, r, T.as<double>(), n));
+      PQ_TRY(rotate(V.as<double>(), m, r));
       PQ_CUDA_TRY(cudaMemcpyAsync(V.ptr, T.ptr, sizeof(double) * n * r, cudaMemcpyDeviceToDevice, st));
       if (refine) {
         // FP64 residual refinement: exact sigma of the restart vectors
@@ -369,7 +574,7 @@ pq_status DavidsonRun::advance() {
         request(V.as<double>(), W.as<double>(), r, PQ_FP64, 0.0, AFTER_REFINE);
         return PQ_OK;
       }
-      PQ_TRY(tall_skinny(cb, CUBLAS_OP_N, n, m, W.as<double>(), tmp.as<double>(), m, r, T.as<double>(), n));
+      PQ_TRY(rotate(W.as<double>(), m, r));
       PQ_CUDA_TRY(cudaMemcpyAsync(W.ptr, T.ptr, sizeof(double) * n * r, cudaMemcpyDeviceToDevice, st));
       // the rotated Rayleigh matrix Z_r^T G Z_r is diag(w) (Z diagonalises G)
       for (int j = 0; j < r; j++)
@@ -379,18 +584,17 @@ pq_status DavidsonRun::advance() {
       continue;
     }
     // corrections for unconverged roots
-    int nt = 0;
-    std::vector<double> th_u;
-    for (int i = 0; i < k; i++) {
-      if (rnorm[i] < tol) continue;
-      PQ_CUDA_TRY(cudaMemcpyAsync(T.as<double>() + (size_t)nt * n, R.as<double>() + (size_t)i * n, sizeof(double) * n,
-                                  cudaMemcpyDeviceToDevice, st));
-      th_u.push_back(theta[i]);
-      nt++;
-    }
-    PQ_CUDA_TRY(cudaMemcpyAsync(dth.ptr, th_u.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, st));
-    precondition_kernel<<<grid(), 256, 0, st>>>(T.as<double>(), h->d_diag.as<double>(), dth.as<double>(), n, nt,
-                                                T.as<double>());
+    std::vector<double> th_u;  // (theta, root) of each
+    for (int i = 0; i < k; i++)
+      if (!(rnorm[i] < tol)) {
+        th_u.push_back(theta[i]);
+        th_u.push_back((double)i);
+      }
+    const int nt = (int)th_u.size() / 2;
+    PQ_CUDA_TRY(cudaMemcpyAsync(dth.ptr, th_u.data(), sizeof(double) * th_u.size(), cudaMemcpyHostToDevice, st));
+    if (nt > 0)
+      precondition_kernel<<<dim3(grid(), nt), 256, 0, st>>>(R.as<double>(), h->d_diag.as<double>(), dth.as<double2>(), n,
+                                                          T.as<double>());
     PQ_CUDA_TRY(cudaGetLastError());
     int added = 0;
     PQ_TRY(orthonormalize_append(m, nt, &added));
@@ -423,8 +627,11 @@ pq_status DavidsonRun::outputs(double *energies, double *vecs) {
   return PQ_OK;
 }
 
-DavidsonRun::~DavidsonRun() {
-  if (cb && own_cb) cublasDestroy(cb);
+// T[:, 0:r] = A[:, 0:m] Z with Z (m x r) in tmp
+pq_status DavidsonRun::rotate(const double *A, int mm, int r) {
+  rotate_kernel<<<dim3(ts_grid(), (r + TS_Q - 1) / TS_Q), TS_THREADS, 0, st>>>(A, tmp.as<double>(), n, mm, r, T.as<double>());
+  PQ_CUDA_TRY(cudaGetLastError());
+  return PQ_OK;
 }
 
 // G = V[:, 0:m]^T W[:, 0:m] on the host, kept across iterations in Gk
@@ -436,8 +643,14 @@ pq_status DavidsonRun::rayleigh(int mm, std::vector<double> &G) {
   if (g_valid < mm) {
     const int c0 = g_valid, nc = mm - c0;
     PQ_TRY(tmp.ensure(sizeof(double) * (size_t)mm * nc));
-    PQ_TRY(tall_skinny(cb, CUBLAS_OP_T, n, mm, V.as<double>(), W.as<double>() + (size_t)c0 * n, n, nc,
-                       tmp.as<double>(), mm));
+    // at most max(m0, k) columns at a time, as many as the partial sums were sized for
+    for (int j = 0; j < nc; j += std::max(m0, k)) {
+      const int q = std::min(nc - j, std::max(m0, k));
+      gram_kernel<<<dim3(ts_grid(), (mm + TS_MI - 1) / TS_MI, (q + TS_Q - 1) / TS_Q), TS_THREADS, 0, st>>>(
+          V.as<double>(), W.as<double>() + (size_t)(c0 + j) * n, n, mm, q, part.as<double>(), cnt.as<unsigned>(),
+          tmp.as<double>() + (size_t)j * mm, mm);
+      PQ_CUDA_TRY(cudaGetLastError());
+    }
     std::vector<double> B((size_t)mm * nc);
     PQ_CUDA_TRY(cudaMemcpyAsync(B.data(), tmp.ptr, sizeof(double) * mm * nc, cudaMemcpyDeviceToHost, st));
     PQ_CUDA_TRY(cudaStreamSynchronize(st));
@@ -456,34 +669,28 @@ pq_status DavidsonRun::rayleigh(int mm, std::vector<double> &G) {
   return PQ_OK;
 }
 
-// Orthonormalise columns T[:, 0:kk] against V[:, 0:mm] and each other (two
-// classical Gram-Schmidt passes); accepted columns are appended to V.
+// Orthonormalise columns T[:, 0:kk] against V[:, 0:mm] and each other (classical Gram-Schmidt, a second pass
+// where the first lost norm); accepted columns are appended to V.  Every decision is taken on the device; the host
+// reads the new column count once.
 pq_status DavidsonRun::orthonormalize_append(int mm0, int kk, int *added) {
-  const double one = 1.0, mone = -1.0, zero = 0.0;
-  PQ_TRY(coef.ensure(sizeof(double) * (size_t)(mm0 + kk) * 2));
-  int mm = mm0;
+  GsState s{0.0, 0.0, 0.0, mm0};
+  GsState *gd = gs.as<GsState>();
+  PQ_CUDA_TRY(cudaMemcpyAsync(gd, &s, sizeof(s), cudaMemcpyHostToDevice, st));
   for (int j = 0; j < kk; j++) {
     double *t = T.as<double>() + (size_t)j * n;
-    double nrm0 = 0.0;
-    PQ_CUBLAS_TRY(cublasDnrm2(cb, (int)n, t, 1, &nrm0));
-    if (!(nrm0 > 0.0) || !std::isfinite(nrm0)) continue;
-    // classical Gram-Schmidt, repeated once unless the first pass kept at
-    // least 1/sqrt(2) of the norm (then t is orthogonal to working precision)
-    double nrm = nrm0;
+    const dim3 dots(ts_grid(), (unsigned)((mm0 + j + 1 + TS_MI - 1) / TS_MI));
     for (int pass = 0; pass < 2; pass++) {
-      const double before = nrm;
-      PQ_CUBLAS_TRY(cublasDgemv(cb, CUBLAS_OP_T, (int)n, mm, &one, V.as<double>(), (int)n, t, 1, &zero, coef.as<double>(), 1));
-      PQ_CUBLAS_TRY(cublasDgemv(cb, CUBLAS_OP_N, (int)n, mm, &mone, V.as<double>(), (int)n, coef.as<double>(), 1, &one, t, 1));
-      PQ_CUBLAS_TRY(cublasDnrm2(cb, (int)n, t, 1, &nrm));
-      if (nrm >= 0.70710678118654752 * before) break;
+      gs_dots_kernel<<<dots, TS_THREADS, 0, st>>>(V.as<double>(), t, n, pass, gd, part.as<double>(), cnt.as<unsigned>(),
+                                                 coef.as<double>());
+      gs_update_kernel<<<ts_grid(), TS_THREADS, 0, st>>>(V.as<double>(), t, n, pass, gd, part.as<double>(),
+                                                        cnt.as<unsigned>(), coef.as<double>());
     }
-    if (!(nrm > 1e-8 * nrm0) || nrm < 1e-300) continue;
-    double inv = 1.0 / nrm;
-    PQ_CUBLAS_TRY(cublasDscal(cb, (int)n, &inv, t, 1));
-    PQ_CUDA_TRY(cudaMemcpyAsync(V.as<double>() + (size_t)mm * n, t, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-    mm++;
+    gs_append_kernel<<<ts_grid(), TS_THREADS, 0, st>>>(V.as<double>(), t, n, gd, cnt.as<unsigned>());
   }
-  *added = mm - mm0;
+  PQ_CUDA_TRY(cudaGetLastError());
+  PQ_CUDA_TRY(cudaMemcpyAsync(&s, gd, sizeof(s), cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  *added = s.mm - mm0;
   return PQ_OK;
 }
 

@@ -11,8 +11,6 @@
 #include "pq_ci.h"
 #include "pq_ints.h"
 
-struct cublasContext;  // cuBLAS handle type (cublasHandle_t)
-
 // Orbitals per species: strings are held as at most two 64-bit words.
 #define PQ_MAX_ORB 128
 
@@ -213,11 +211,9 @@ pq_status sigma_request_single(pq_ci_handle *h, const SigmaRequest &r);
 class DavidsonRun {
  public:
   enum Stage { NONE, AFTER_INIT, AFTER_REFINE, AFTER_NEW };
-  // shared_cb: a cuBLAS handle bound to h->stream that the run borrows (else it creates its own)
-  pq_status init(pq_ci_handle *h, const pq_davidson_params &p, ::cublasContext *shared_cb = nullptr);
+  pq_status init(pq_ci_handle *h, const pq_davidson_params &p);
   pq_status advance();  // after the pending request was evaluated
   pq_status outputs(double *energies, double *vecs);
-  ~DavidsonRun();
   bool pending = false, done = false;
   SigmaRequest req{};
   pq_status result = PQ_NOT_CONVERGED;
@@ -232,12 +228,14 @@ class DavidsonRun {
   pq_status finish_state(pq_status r);
   pq_status rayleigh(int m, std::vector<double> &G);
   pq_status orthonormalize_append(int m, int k, int *added);
+  pq_status rotate(const double *A, int mm, int r);
+  // blocks of the tall-skinny kernels: two per SM, fewer where 256 rows each already cover n
+  unsigned ts_grid() const { return (unsigned)((n + 255) / 256 < 152 * 2 ? (n + 255) / 256 : 152 * 2); }
   unsigned grid() const { return (unsigned)((n + 255) / 256 < 152 * 16 ? (n + 255) / 256 : 152 * 16); }
   pq_davidson_params p{};
   cudaStream_t st = nullptr;
-  ::cublasContext *cb = nullptr;
-  bool own_cb = false;
   DevBuf V, W, X, R, T, tmp, dth, didx, coef;
+  DevBuf part, cnt, gs;  // partial sums, arrival counters and Gram-Schmidt state of the tall-skinny kernels
   std::vector<double> Z, Gk;  // Ritz rotation; Rayleigh matrix (mmax x mmax, first g_valid columns valid)
   int g_valid = 0;
   int k = 0, m0 = 0, mmax = 0, m = 0, it = 0, r_restart = 0;
