@@ -10,8 +10,9 @@
 // where M_{la si}[mu][nu] = (mu nu|la si) and N_{ij}[la][si] = H1[la si][ij].
 // Work = 4 n_ao^3 npair + 4 n_ao^3 npair flops for equal sizes.
 //
-// PQ_XFORM_FP64 issues the batched GEMMs through cuBLAS (plain FP64 library
-// GEMMs); the split-precision tensor-core modes are in ao2mo_tc.cu.
+// PQ_XFORM_FP64 runs on the tensor cores by exact digit products up to 256
+// functions (ao2mo_f64.cu) and issues the batched GEMMs through cuBLAS beyond
+// that; the split-precision tensor-core modes are in ao2mo_tc.cu.
 #include <cublas_v2.h>
 
 #include <algorithm>
@@ -154,6 +155,9 @@ pq_status ao2mo_fp64(const double *eri_ao, int layout, int64_t n_ao_a, int64_t n
   return PQ_OK;
 }
 
+// ao2mo_tc.cu
+pq_status ao2mo_f64_shared(const double *eri_ao, int layout, int64_t n_ao_a, int64_t n_ao_b, const double *Ca, int64_t lda,
+                           int64_t nmo_a, const double *Cb, int64_t ldb, int64_t nmo_b, double *eri_mo, cudaStream_t st);
 pq_status ao2mo_tc(const double *eri_ao, int layout, int64_t n_ao, const double *Ca, int64_t lda, int64_t nmo,
                    int mode, double *eri_mo, cudaStream_t st);
 
@@ -183,6 +187,9 @@ extern "C" pq_status pq_ao2mo(const double *eri_ao, int32_t layout, int64_t n_ao
     return PQ_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
+  // up to 256 functions the digit products are exact in FP32 accumulators; larger bases take the library DGEMM
+  if (mode == PQ_XFORM_FP64 && n_ao_a <= 256 && n_ao_b <= 256)
+    return ao2mo_f64_shared(eri_ao, layout, n_ao_a, n_ao_b, C_a, ldc_a, n_mo_a, C_b, ldc_b, n_mo_b, eri_mo, st);
   if (mode == PQ_XFORM_FP64)
     return ao2mo_fp64(eri_ao, layout, n_ao_a, n_ao_b, C_a, ldc_a, n_mo_a, C_b, ldc_b, n_mo_b, eri_mo, st);
   if (mode == PQ_XFORM_BF16X3 || mode == PQ_XFORM_TF32X3) {

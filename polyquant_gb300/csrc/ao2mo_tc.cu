@@ -599,9 +599,41 @@ static pq_status run_gemm(const Operand &A, const Operand &B, bool a_batched, bo
 // each call synchronises its stream before it returns).  pq_ao2mo_release_workspace frees them.
 struct Ao2moWorkspace {
   DevBuf full, cth, ctl, sh, sl, uh, ul, H1, H1t, Erow, err;
+  Ao2moF64 f64;
+  void release() {
+    for (DevBuf *b : {&full, &cth, &ctl, &sh, &sl, &uh, &ul, &H1, &H1t, &Erow, &err}) b->release();
+    f64.release();
+  }
 };
 static std::mutex g_ws_mu;
 static Ao2moWorkspace g_ws[64];
+
+long long ao2mo_wait_cycles() { return g_gemm_wait_cycles; }
+
+// FP64 mode through the shared workspace.  A device that is too full for it gives the buffers of earlier calls back
+// and tries once more.
+pq_status ao2mo_f64_shared(const double *eri_ao, int layout, int64_t n_ao_a, int64_t n_ao_b, const double *Ca, int64_t lda,
+                           int64_t nmo_a, const double *Cb, int64_t ldb, int64_t nmo_b, double *eri_mo, cudaStream_t st) {
+  int dev = 0;
+  PQ_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) {
+    set_error("pq_ao2mo: device ordinal %d out of range", dev);
+    return PQ_ERR_STATE;
+  }
+  std::lock_guard<std::mutex> lock(g_ws_mu);
+  auto run = [&] {
+    return ao2mo_f64(g_ws[dev].f64, eri_ao, layout, n_ao_a, n_ao_b, Ca, lda, nmo_a, Cb, ldb, nmo_b, eri_mo, st);
+  };
+  pq_status s = run();
+  if (s == PQ_ERR_OOM) {
+    PQ_CUDA_TRY(cudaStreamSynchronize(st));
+    g_ws[dev].release();
+    cudaGetLastError();
+    s = run();
+    if (s == PQ_OK) clear_error();
+  }
+  return s;
+}
 
 template <bool TF32>
 static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, const double *C, int64_t ldc, int64_t nm,
@@ -733,8 +765,7 @@ extern "C" pq_status pq_ao2mo_release_workspace(void) {
     pq::set_error("pq_ao2mo_release_workspace: no current device");
     return PQ_ERR_STATE;
   }
-  pq::Ao2moWorkspace &w = pq::g_ws[dev];
-  for (pq::DevBuf *b : {&w.full, &w.cth, &w.ctl, &w.sh, &w.sl, &w.uh, &w.ul, &w.H1, &w.H1t, &w.Erow, &w.err}) b->release();
+  pq::g_ws[dev].release();
   return PQ_OK;
 }
 

@@ -196,6 +196,19 @@ pq_status ci_from_il(pq_ci_handle *h, const void *Y, int v0, int nv, int nvp, in
 pq_status ci_davidson(pq_ci_handle *h, const pq_davidson_params *p, double *energies, double *vecs,
                       pq_davidson_report *rep);
 
+// ao2mo_f64.cu: FP64 transform by digit products on the tensor cores (n_ao <= 256) and its work buffers, which
+// belong to the per-device workspace of ao2mo_tc.cu
+struct Ao2moF64 {
+  DevBuf ct, s, u, e, h1, err;
+  void release() {
+    for (DevBuf *b : {&ct, &s, &u, &e, &h1, &err}) b->release();
+  }
+};
+pq_status ao2mo_f64(Ao2moF64 &w, const double *eri_ao, int layout, int64_t n_ao_a, int64_t n_ao_b, const double *Ca,
+                    int64_t lda, int64_t nmo_a, const double *Cb, int64_t ldb, int64_t nmo_b, double *eri_mo,
+                    cudaStream_t st);
+long long ao2mo_wait_cycles();
+
 // A pending sigma evaluation of a Davidson run: dst = H src for cnt columns
 // (column-major, leading dimension n_dets); FP32 requests use (H - shift) in
 // FP32 and add shift * src back in FP64.
