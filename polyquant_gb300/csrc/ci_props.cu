@@ -10,15 +10,22 @@
 // occupied orbitals of the chosen spin, and phase C_I C_J on (k, l) and
 // (l, k) for each single of that spin between I and an earlier J (hole k in
 // I, particle l).
-// Thread <-> determinant (one species: grid of alpha strings x beta blocks;
-// two species: CTA per species-0 pair, threads over its species-1 block),
-// per-block reduction in shared memory, then one atomic per block and entry.
-// With two species each property is evaluated for the chosen species with
+// One species: both properties are sums over pairs of strings that differ by
+// one orbital pair, so the singles of each spin are kept once more as lists by
+// orbital pair (PairLists).  The alpha 1-RDM is then a sum of dot products of
+// rows of C, the beta one a sum over column pairs of rows staged in shared
+// memory, and <S^2> runs, pair by pair, over alpha moves up against beta moves
+// down; sums stay in registers per pair and meet in one atomic per warp or
+// block.  The former kernels, thread per determinant, added every product to a
+// shared-memory matrix by FP64 atomics and searched each beta partner along
+// its string's list.  Four states and two 1-RDMs of FCI(12o, 6a6b): 359 us
+// against 5212.
+// Two species: CTA per species-0 pair, threads over its species-1 block, with
 // the other species' strings held fixed, as in the reference's per-species
 // loops.
 #include <algorithm>
+#include <new>
 
-#include "ci_conn.cuh"
 #include "pq_bits.cuh"
 #include "pq_internal.h"
 
@@ -27,103 +34,335 @@ namespace pq {
 constexpr int PROP_THREADS = 128;
 constexpr int S2_MAXV = 8;
 
-__global__ void __launch_bounds__(PROP_THREADS) s2_kernel(ConnArgs a, int na, const double *C, int64_t ldc, int nvec,
-                                                          double *out) {
-  __shared__ double red[S2_MAXV][PROP_THREADS / 32];
-  const int ia = blockIdx.x;
-  double acc[S2_MAXV];
-#pragma unroll
-  for (int v = 0; v < S2_MAXV; v++) acc[v] = 0.0;
-  for (int ib = blockIdx.y * blockDim.x + threadIdx.x; ia < na && ib < a.rowlen[ia]; ib += gridDim.y * blockDim.x) {
-    const ConnRow r = conn_row(a, ia, ib);
-    double cI[S2_MAXV];
-#pragma unroll
-    for (int v = 0; v < S2_MAXV; v++) cI[v] = v < nvec ? C[r.I + v * ldc] : 0.0;
-    const uint64_t open = r.am ^ r.bm, openh = r.amh ^ r.bmh;
-    const int n_open = popc2(open, openh), n_a = popc2(open & r.am, openh & r.amh);
-    const double sz = n_a - 0.5 * n_open;
-    const double d = n_a + sz * (sz - 1.0);
-#pragma unroll
-    for (int v = 0; v < S2_MAXV; v++) acc[v] += cI[v] * cI[v] * d;
-    for (int s = 0; s < r.n1a; s++) {
-      const int Ja = a.a1_J[r.a1b + s], infa = a.a1_info[r.a1b + s];
-      const uint64_t jam = a.astr[Ja], jamh = hiword(a.astr_hi, Ja);
-      const int ha = first_set(r.am & ~jam, r.amh & ~jamh), pa = first_set(jam & ~r.am, jamh & ~r.amh);
-      if (!occupied(r.bm, r.bmh, pa) || occupied(r.bm, r.bmh, ha)) continue;
-      uint64_t jbm = r.bm, jbmh = r.bmh;
-      flip_orb(jbm, jbmh, pa);
-      flip_orb(jbm, jbmh, ha);
-      for (int q = 0; q < r.n1b; q++) {
-        const int Jb = a.b1_J[r.b1b + q];
-        if (a.bstr[Jb] != jbm || hiword(a.bstr_hi, Jb) != jbmh) continue;
-        if (Jb < a.rowlen[Ja]) {
-          const int64_t J = a.rowoff[Ja] + Jb;
-          const double ph = ((infa ^ a.b1_info[r.b1b + q]) & 1) ? -1.0 : 1.0;
-#pragma unroll
-          for (int v = 0; v < S2_MAXV; v++)
-            if (v < nvec) acc[v] -= ph * cI[v] * C[J + v * ldc];
-        }
-        break;
+// ---- one species ------------------------------------------------------------
+// Singles of one spin by orbital pair q = idx2(i, j), i > j: every unordered pair of strings that differ by a move
+// between i and j, at the string with the larger index, in its order: {I << 1 | phase, J << 1 | (I holds i)}; for
+// i = j the strings that hold i, {I << 1, I << 1}.
+struct PairLists {
+  DevBuf off[2], ent[2];     // int64 [npair + 1], uint2
+  std::vector<int64_t> hoff[2];
+  DevBuf out;                // sums of a call
+};
+void pairs_delete(PairLists *p) { delete p; }
+
+// warp per pair: counts (ent == NULL) or writes its list
+__global__ void __launch_bounds__(128) pair_lists_kernel(int npair, int64_t n_str, const uint64_t *str,
+                                                         const uint64_t *str_hi, const int64_t *s1_off,
+                                                         const int32_t *s1_J, const int32_t *s1_info, int64_t *cnt,
+                                                         const int64_t *off, uint2 *ent) {
+  const int lane = threadIdx.x & 31, q = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (q >= npair) return;
+  int i = 0;
+  while ((i + 1) * (i + 2) / 2 <= q) i++;
+  const int j = q - i * (i + 1) / 2;
+  int64_t w = ent ? off[q] : 0;
+  for (int64_t I0 = 0; I0 < n_str; I0 += 32) {
+    const int64_t I = I0 + lane;
+    bool there = false;
+    uint2 e = make_uint2(0u, 0u);
+    if (I < n_str) {
+      const uint64_t m = str[I], mh = hiword(str_hi, I);
+      const bool hi = occupied(m, mh, i);
+      if (i == j) {
+        there = hi;
+        e = make_uint2((uint32_t)I << 1, (uint32_t)I << 1);
+      } else if (hi != occupied(m, mh, j)) {
+        for (int64_t s = s1_off[I]; s < s1_off[I + 1]; s++)
+          if (s1_info[s] >> 1 == q) {
+            const int J = s1_J[s];
+            there = J < I;
+            e = make_uint2((uint32_t)I << 1 | (uint32_t)(s1_info[s] & 1), (uint32_t)J << 1 | (uint32_t)hi);
+            break;  // a string moves between i and j in one direction only
+          }
       }
     }
+    const unsigned b = __ballot_sync(0xffffffffu, there);
+    if (ent && there) ent[w + __popc(b & ((1u << lane) - 1u))] = e;
+    w += __popc(b);
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int v = 0; v < S2_MAXV; v++) {
-    double x = acc[v];
-    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[v][w] = x;
+  if (!ent && lane == 0) cnt[q] = w;
+}
+
+__device__ __forceinline__ double xflip(double v, uint32_t neg) {
+  return __hiloint2double(__double2hiint(v) ^ (int)(neg << 31), __double2loint(v));
+}
+__device__ __forceinline__ double warp_total(double x) {
+  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// pair that holds entry e of a list
+__device__ __forceinline__ int pair_of(const int64_t *off, int npair, int64_t e) {
+  int lo = 0, hi = npair;  // off[lo] <= e < off[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (off[mid] <= e)
+      lo = mid;
+    else
+      hi = mid;
   }
-  __syncthreads();
-  if (threadIdx.x < nvec) {
-    double x = 0.0;
-    for (int i = 0; i < PROP_THREADS / 32; i++) x += red[threadIdx.x][i];
-    atomicAdd(out + threadIdx.x, x);
+  return lo;
+}
+
+// Alpha 1-RDM: sum over the list of pair q of phase * (row I . row J), warp per ROWS_PER entries
+constexpr int ROWS_PER = 8;
+__global__ void __launch_bounds__(256) rdm_rows_kernel(const int64_t *off, const uint2 *ent, int npair, int64_t n_ent,
+                                                       const int64_t *rowoff, const int32_t *rowlen, const double *C,
+                                                       double *out) {
+  const int lane = threadIdx.x & 31;
+  int64_t e = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * ROWS_PER;
+  const int64_t e1 = min(e + ROWS_PER, n_ent);
+  if (e >= e1) return;
+  int q = pair_of(off, npair, e);
+  while (e < e1) {
+    while (off[q + 1] <= e) q++;
+    double acc = 0.0;
+    for (const int64_t stop = min(e1, off[q + 1]); e < stop; e++) {
+      const uint2 x = __ldg(ent + e);
+      const int64_t I = x.x >> 1, J = x.y >> 1;
+      const double *ri = C + rowoff[I], *rj = C + rowoff[J];
+      const int len = min(rowlen[I], rowlen[J]);
+      double part = 0.0;
+#pragma unroll 4
+      for (int b = lane; b < len; b += 32) part = fma(__ldg(ri + b), __ldg(rj + b), part);
+      acc += xflip(part, x.x & 1u);
+    }
+    acc = warp_total(acc);
+    if (lane == 0 && acc != 0.0) atomicAdd(out + q, acc);
   }
 }
 
-// rdm[k + l * n] (column-major n x n), spin 0 = alpha, 1 = beta
-__global__ void __launch_bounds__(PROP_THREADS) rdm1_kernel(ConnArgs a, int na, int n, int spin, const double *C,
-                                                            double *rdm) {
-  extern __shared__ double acc[];  // n x n
-  for (int i = threadIdx.x; i < n * n; i += blockDim.x) acc[i] = 0.0;
+// Beta 1-RDM: block per R rows, held in shared memory as [column][R] (R = 0: one row, read from global memory); the
+// warps share the pairs.  A list is in the order of its larger column, so it ends at the longest row.
+template <int R>
+__global__ void __launch_bounds__(512) rdm_cols_kernel(const int64_t *off, const uint2 *ent, int npair, int64_t na,
+                                                       const int64_t *rowoff, const int32_t *rowlen, const double *C,
+                                                       double *out) {
+  constexpr int RR = R == 0 ? 1 : R;
+  extern __shared__ __align__(16) double xs[];
+  const int64_t a0 = (int64_t)blockIdx.x * RR;
+  int len[RR], longest = 0;
+#pragma unroll
+  for (int r = 0; r < RR; r++) {
+    len[r] = a0 + r < na ? rowlen[a0 + r] : 0;
+    longest = max(longest, len[r]);
+  }
+  if (R > 0) {
+#pragma unroll
+    for (int r = 0; r < RR; r++) {
+      const double *row = C + (len[r] ? rowoff[a0 + r] : 0);
+      for (int b = threadIdx.x; b < longest; b += blockDim.x) xs[b * RR + r] = b < len[r] ? row[b] : 0.0;
+    }
+    __syncthreads();
+  }
+  const double *x0 = R > 0 ? xs : C + rowoff[a0];
+  const int lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < npair; q += blockDim.x >> 5) {
+    double acc = 0.0;
+    const int64_t e1 = off[q + 1];
+    for (int64_t e = off[q]; e < e1; e += 32) {
+      uint2 x = make_uint2(0u, 0u);
+      bool in = e + lane < e1;
+      if (in) x = __ldg(ent + e + lane);
+      in = in && (int)(x.x >> 1) < longest;
+      const int first = (int)(__shfl_sync(0xffffffffu, x.x, 0) >> 1);  // the smallest of the 32
+      if (first >= longest) break;
+      const int I = in ? (int)(x.x >> 1) : 0, J = in ? (int)(x.y >> 1) : 0;
+#pragma unroll
+      for (int r = 0; r < RR; r++)
+        if (first < len[r]) {  // the same for the warp; a column past a shorter row reads the stored zero
+          const double c = in ? xflip(x0[I * RR + r], x.x & 1u) : 0.0, d = in ? x0[J * RR + r] : 0.0;
+          acc = fma(c, d, acc);
+        }
+    }
+    acc = warp_total(acc);
+    if (lane == 0 && acc != 0.0) atomicAdd(out + q, acc);
+  }
+}
+
+// <S^2>, diagonal: sum of C_I^2 (s_z^2 + (n_alpha + n_beta)/2 - doubly occupied orbitals); block per alpha string
+__global__ void __launch_bounds__(PROP_THREADS) s2_diag_kernel(const uint64_t *astr, const uint64_t *astr_hi,
+                                                              const uint64_t *bstr, const uint64_t *bstr_hi,
+                                                              const int64_t *rowoff, const int32_t *rowlen, double d0,
+                                                              const double *C, int64_t ldc, int nvec, double *out) {
+  __shared__ double red[PROP_THREADS / 32][S2_MAXV], dd[129];
+  for (int k = threadIdx.x; k < 129; k += blockDim.x) dd[k] = d0 - k;
   __syncthreads();
-  const int ia = blockIdx.x;
-  for (int ib = blockIdx.y * blockDim.x + threadIdx.x; ia < na && ib < a.rowlen[ia]; ib += gridDim.y * blockDim.x) {
-    const ConnRow r = conn_row(a, ia, ib);
-    const double cI = C[r.I];
-    const uint64_t mine = spin == 0 ? r.am : r.bm, mineh = spin == 0 ? r.amh : r.bmh;
-    const double c2 = cI * cI;
-    if (fabs(c2) > 1e-16) for_occ(mine, mineh, [&](int o) { atomicAdd(acc + o * (n + 1), c2); });
-    const int ns = spin == 0 ? r.n1a : r.n1b;
-    for (int s = 0; s < ns; s++) {
-      int64_t J = -1;
-      int info;
-      uint64_t jm, jmh;
-      if (spin == 0) {
-        const int Ja = a.a1_J[r.a1b + s];
-        info = a.a1_info[r.a1b + s];
-        jm = a.astr[Ja];
-        jmh = hiword(a.astr_hi, Ja);
-        if (r.ib < a.rowlen[Ja]) J = a.rowoff[Ja] + r.ib;
-      } else {
-        const int Jb = a.b1_J[r.b1b + s];
-        info = a.b1_info[r.b1b + s];
-        jm = a.bstr[Jb];
-        jmh = hiword(a.bstr_hi, Jb);
-        if (Jb < a.rowlen[r.ia]) J = a.rowoff[r.ia] + Jb;
+  const int64_t ia = blockIdx.x, row = rowoff[ia];
+  const uint64_t am = astr[ia], amh = hiword(astr_hi, ia);
+  double acc[S2_MAXV];
+#pragma unroll
+  for (int v = 0; v < S2_MAXV; v++) acc[v] = 0.0;
+  for (int b = threadIdx.x; b < rowlen[ia]; b += blockDim.x) {
+    const double d = dd[popc2(am & bstr[b], amh & hiword(bstr_hi, b))];
+#pragma unroll
+    for (int v = 0; v < S2_MAXV; v++)
+      if (v < nvec) {
+        const double c = C[row + b + v * ldc];
+        acc[v] = fma(c * c, d, acc[v]);
       }
-      if (J < 0 || J > r.I) continue;  // each pair once, from the later determinant
-      const double c = ((info & 1) ? -cI : cI) * C[J];
-      if (fabs(c) <= 1e-16) continue;
-      const int k = first_set(mine & ~jm, mineh & ~jmh), l = first_set(jm & ~mine, jmh & ~mineh);
-      atomicAdd(acc + k + l * n, c);
-      atomicAdd(acc + l + k * n, c);
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int v = 0; v < S2_MAXV; v++)
+    if (v < nvec) {
+      const double x = warp_total(acc[v]);
+      if (lane == 0) red[w][v] = x;
+    }
+  __syncthreads();
+  if ((int)threadIdx.x < nvec) {
+    double x = 0.0;
+    for (int i = 0; i < PROP_THREADS / 32; i++) x += red[i][threadIdx.x];
+    if (x != 0.0) atomicAdd(out + threadIdx.x, x);
+  }
+}
+
+// <S^2>, spin flips: each unordered pair of determinants (A_lo, B_hi), (A_hi, B_lo) of a pair of orbitals, where lo
+// and hi are the strings that hold the lower and the higher of the two, adds -2 phase C C.  Warp per FLIP_PER alpha
+// entries, lanes over the beta list of the same pair.
+constexpr int FLIP_PER = 4;
+__global__ void __launch_bounds__(256) s2_flip_kernel(const int64_t *aoff, const uint2 *aent, const int64_t *boff,
+                                                      const uint2 *bent, int npair, int64_t n_ent,
+                                                      const int64_t *rowoff, const int32_t *rowlen, const double *C,
+                                                      int64_t ldc, int nvec, double *out) {
+  __shared__ double red[8][S2_MAXV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double acc[S2_MAXV];
+#pragma unroll
+  for (int v = 0; v < S2_MAXV; v++) acc[v] = 0.0;
+  int64_t e = ((int64_t)blockIdx.x * 8 + warp) * FLIP_PER;
+  const int64_t e1 = min(e + FLIP_PER, n_ent);
+  int q = e < e1 ? pair_of(aoff, npair, e) : 0;
+  int i = 0;
+  while ((i + 1) * (i + 2) / 2 <= q) i++;
+  for (; e < e1; e++) {
+    while (aoff[q + 1] <= e) {
+      q++;
+      if ((i + 1) * (i + 2) / 2 <= q) i++;
+    }
+    if (q == i * (i + 3) / 2) continue;  // i = j
+    const uint2 x = __ldg(aent + e);
+    const int I = (int)(x.x >> 1), J = (int)(x.y >> 1);
+    const int alo = (x.y & 1u) ? J : I, ahi = (x.y & 1u) ? I : J;
+    const int64_t rlo = rowoff[alo], rhi = rowoff[ahi];
+    const int llo = rowlen[alo], lhi = rowlen[ahi];
+    for (int64_t f = boff[q] + lane; f < boff[q + 1]; f += 32) {
+      const uint2 y = __ldg(bent + f);
+      const int K = (int)(y.x >> 1), L = (int)(y.y >> 1);
+      const int blo = (y.y & 1u) ? L : K, bhi = (y.y & 1u) ? K : L;
+      if (bhi >= llo || blo >= lhi) continue;
+#pragma unroll
+      for (int v = 0; v < S2_MAXV; v++)
+        if (v < nvec)
+          acc[v] = fma(xflip(__ldg(C + rlo + bhi + v * ldc), (x.x ^ y.x) & 1u), __ldg(C + rhi + blo + v * ldc), acc[v]);
     }
   }
+#pragma unroll
+  for (int v = 0; v < S2_MAXV; v++)
+    if (v < nvec) {
+      const double s = warp_total(acc[v]);
+      if (lane == 0) red[warp][v] = s;
+    }
   __syncthreads();
-  for (int i = threadIdx.x; i < n * n; i += blockDim.x)
-    if (acc[i] != 0.0) atomicAdd(rdm + i, acc[i]);
+  if ((int)threadIdx.x < nvec) {
+    double s = 0.0;
+    for (int w = 0; w < 8; w++) s += red[w][threadIdx.x];
+    if (s != 0.0) atomicAdd(out + threadIdx.x, -2.0 * s);
+  }
+}
+
+// the pair lists of a handle, made on the first property call
+static pq_status pair_lists(pq_ci_handle *h) {
+  if (h->pairs) return PQ_OK;
+  std::unique_ptr<PairLists, void (*)(PairLists *)> p(new (std::nothrow) PairLists(), pairs_delete);
+  if (!p) {
+    set_error("host allocation failed");
+    return PQ_ERR_OOM;
+  }
+  const int npair = h->npair[0];
+  cudaStream_t st = h->stream;
+  PQ_TRY(p->out.alloc(sizeof(double) * std::max(npair, S2_MAXV)));
+  DevBuf cnt;
+  PQ_TRY(cnt.alloc(sizeof(int64_t) * npair));
+  const unsigned grid = (unsigned)((npair + 3) / 4);
+  for (int sp = 0; sp < 2; sp++) {
+    const SpinTablesDev &t = h->tab[0][sp];
+    auto run = [&](int64_t *c, const int64_t *o, uint2 *e) -> pq_status {
+      pair_lists_kernel<<<grid, 128, 0, st>>>(npair, t.n_str, t.str.as<uint64_t>(), t.str_hi.as<uint64_t>(),
+                                             t.s1_off.as<int64_t>(), t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), c, o, e);
+      PQ_CUDA_TRY(cudaGetLastError());
+      return PQ_OK;
+    };
+    PQ_TRY(run(cnt.as<int64_t>(), nullptr, nullptr));
+    std::vector<int64_t> &o = p->hoff[sp];
+    o.assign(npair + 1, 0);
+    PQ_CUDA_TRY(cudaMemcpyAsync(o.data() + 1, cnt.ptr, sizeof(int64_t) * npair, cudaMemcpyDeviceToHost, st));
+    PQ_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int q = 0; q < npair; q++) o[q + 1] += o[q];
+    PQ_TRY(upload(p->off[sp], o, st));
+    PQ_TRY(p->ent[sp].alloc(sizeof(uint2) * (size_t)(o[npair] + 1)));
+    PQ_TRY(run(nullptr, p->off[sp].as<int64_t>(), p->ent[sp].as<uint2>()));
+  }
+  h->pairs = std::move(p);
+  return PQ_OK;
+}
+
+// <S^2> of nvec <= S2_MAXV states into the device sums of the lists
+static pq_status s2_one(pq_ci_handle *h, const double *C, int64_t ldc, int nvec) {
+  const PairLists &p = *h->pairs;
+  const SpinTablesDev &A = h->tab[0][0], &B = h->tab[0][1];
+  const int npair = h->npair[0], na = h->desc.n_alpha[0], nb = h->desc.n_beta[0];
+  cudaStream_t st = h->stream;
+  double *out = p.out.as<double>();
+  const double sz = 0.5 * (na - nb);
+  PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * S2_MAXV, st));
+  s2_diag_kernel<<<(unsigned)A.n_str, PROP_THREADS, 0, st>>>(
+      A.str.as<uint64_t>(), A.str_hi.as<uint64_t>(), B.str.as<uint64_t>(), B.str_hi.as<uint64_t>(),
+      h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), sz * sz + 0.5 * (na + nb), C, ldc, nvec, out);
+  const int64_t n_ent = p.hoff[0][npair];
+  if (n_ent > 0)
+    s2_flip_kernel<<<(unsigned)((n_ent + 8 * FLIP_PER - 1) / (8 * FLIP_PER)), 256, 0, st>>>(
+        p.off[0].as<int64_t>(), p.ent[0].as<uint2>(), p.off[1].as<int64_t>(), p.ent[1].as<uint2>(), npair, n_ent,
+        h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), C, ldc, nvec, out);
+  PQ_CUDA_TRY(cudaGetLastError());
+  return PQ_OK;
+}
+
+// 1-RDM sums by pair into the device sums of the lists
+static pq_status rdm_one(pq_ci_handle *h, const double *C, int spin) {
+  const PairLists &p = *h->pairs;
+  const int npair = h->npair[0];
+  cudaStream_t st = h->stream;
+  double *out = p.out.as<double>();
+  const int64_t *ro = h->d_rowoff.as<int64_t>();
+  const int32_t *rl = h->d_rowlen.as<int32_t>();
+  PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * npair, st));
+  const int64_t *off = p.off[spin].as<int64_t>();
+  const uint2 *ent = p.ent[spin].as<uint2>();
+  const int64_t n_ent = p.hoff[spin][npair], na = h->tab[0][0].n_str;
+  if (n_ent == 0) return PQ_OK;
+  if (spin == 0) {
+    const int64_t per = 8 * ROWS_PER;
+    rdm_rows_kernel<<<(unsigned)((n_ent + per - 1) / per), 256, 0, st>>>(off, ent, npair, n_ent, ro, rl, C, out);
+    PQ_CUDA_TRY(cudaGetLastError());
+    return PQ_OK;
+  }
+  // as many rows per block as 100 KB of shared memory hold, while the blocks still cover the chip twice
+  const int64_t longest = *std::max_element(h->rowlen.begin(), h->rowlen.end());
+  const size_t row = sizeof(double) * (size_t)longest;
+  auto run = [&](auto kern, int R) -> pq_status {
+    const size_t smem = row * R;
+    if (smem > 48 * 1024) PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t rows = std::max(R, 1);
+    kern<<<(unsigned)((na + rows - 1) / rows), 512, smem, st>>>(off, ent, npair, na, ro, rl, C, out);
+    PQ_CUDA_TRY(cudaGetLastError());
+    return PQ_OK;
+  };
+  if (8 * row <= 100 * 1024 && na >= 8 * 304) return run(rdm_cols_kernel<8>, 8);
+  if (4 * row <= 100 * 1024 && na >= 4 * 304) return run(rdm_cols_kernel<4>, 4);
+  if (2 * row <= 200 * 1024) return run(rdm_cols_kernel<2>, 2);
+  if (row <= 200 * 1024) return run(rdm_cols_kernel<1>, 1);
+  return run(rdm_cols_kernel<0>, 0);
 }
 
 // ---- two species: determinant (a0, b0, a1, b1) of the product space built
@@ -291,25 +530,25 @@ pq_status pq_ci_s2(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, 
     return PQ_ERR_ARG;
   }
   const int ns = h->n_species;
-  DevBuf out;
-  PQ_TRY(out.alloc(sizeof(double) * S2_MAXV));
+  DevBuf own;
+  if (ns == 1)
+    PQ_TRY(pair_lists(h));
+  else
+    PQ_TRY(own.alloc(sizeof(double) * S2_MAXV));
+  double *out = ns == 1 ? h->pairs->out.as<double>() : own.as<double>();
   std::vector<double> part(S2_MAXV);
   for (int sp = 0; sp < ns; sp++)
     for (int v0 = 0; v0 < nvec; v0 += S2_MAXV) {
       const int c = std::min(S2_MAXV, nvec - v0);
-      PQ_CUDA_TRY(cudaMemsetAsync(out.ptr, 0, sizeof(double) * S2_MAXV, h->stream));
       if (ns == 1) {
-        const ConnArgs a = make_conn_args(h);
-        const int na = (int)h->rowlen.size();
-        const int maxlen = *std::max_element(h->rowlen.begin(), h->rowlen.end());
-        const dim3 grid((unsigned)na, (unsigned)std::min((maxlen + PROP_THREADS - 1) / PROP_THREADS, 65535));
-        s2_kernel<<<grid, PROP_THREADS, 0, h->stream>>>(a, na, C + (size_t)v0 * ldc, ldc, c, out.as<double>());
+        PQ_TRY(s2_one(h, C + (size_t)v0 * ldc, ldc, c));
       } else {
+        PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * S2_MAXV, h->stream));
         s2_two_kernel<<<(unsigned)h->e_a.size(), PROP_THREADS, 0, h->stream>>>(make_two(h), sp, C + (size_t)v0 * ldc,
-                                                                               ldc, c, out.as<double>());
+                                                                               ldc, c, out);
+        PQ_CUDA_TRY(cudaGetLastError());
       }
-      PQ_CUDA_TRY(cudaGetLastError());
-      PQ_CUDA_TRY(cudaMemcpyAsync(part.data(), out.ptr, sizeof(double) * c, cudaMemcpyDeviceToHost, h->stream));
+      PQ_CUDA_TRY(cudaMemcpyAsync(part.data(), out, sizeof(double) * c, cudaMemcpyDeviceToHost, h->stream));
       PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
       for (int v = 0; v < c; v++) s2[(size_t)(v0 + v) * ns + sp] = part[v];
     }
@@ -323,23 +562,24 @@ pq_status pq_ci_rdm1(pq_ci_handle *h, const double *C, int32_t species, int32_t 
     return PQ_ERR_ARG;
   }
   const int n = h->n_orb[species];
+  if (h->n_species == 1) {
+    PQ_TRY(pair_lists(h));
+    PQ_TRY(rdm_one(h, C, spin));
+    std::vector<double> d(h->npair[0]);
+    PQ_CUDA_TRY(cudaMemcpyAsync(d.data(), h->pairs->out.ptr, sizeof(double) * d.size(), cudaMemcpyDeviceToHost, h->stream));
+    PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    for (int i = 0, q = 0; i < n; i++)
+      for (int j = 0; j <= i; j++, q++) rdm[i + (size_t)j * n] = rdm[j + (size_t)i * n] = d[q];
+    return PQ_OK;
+  }
   DevBuf out;
   PQ_TRY(out.alloc(sizeof(double) * n * n));
   PQ_CUDA_TRY(cudaMemsetAsync(out.ptr, 0, sizeof(double) * n * n, h->stream));
   const size_t smem = sizeof(double) * n * n;
-  if (h->n_species == 1) {
-    const ConnArgs a = make_conn_args(h);
-    const int na = (int)h->rowlen.size();
-    const int maxlen = *std::max_element(h->rowlen.begin(), h->rowlen.end());
-    const dim3 grid((unsigned)na, (unsigned)std::min((maxlen + PROP_THREADS - 1) / PROP_THREADS, 65535));
-    if (smem > 48 * 1024) PQ_CUDA_TRY(cudaFuncSetAttribute(rdm1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    rdm1_kernel<<<grid, PROP_THREADS, smem, h->stream>>>(a, na, n, spin, C, out.as<double>());
-  } else {
-    if (smem > 48 * 1024)
-      PQ_CUDA_TRY(cudaFuncSetAttribute(rdm1_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    rdm1_two_kernel<<<(unsigned)h->e_a.size(), PROP_THREADS, smem, h->stream>>>(make_two(h), species, spin, n, C,
-                                                                               out.as<double>());
-  }
+  if (smem > 48 * 1024)
+    PQ_CUDA_TRY(cudaFuncSetAttribute(rdm1_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  rdm1_two_kernel<<<(unsigned)h->e_a.size(), PROP_THREADS, smem, h->stream>>>(make_two(h), species, spin, n, C,
+                                                                             out.as<double>());
   PQ_CUDA_TRY(cudaGetLastError());
   PQ_CUDA_TRY(cudaMemcpyAsync(rdm, out.ptr, sizeof(double) * n * n, cudaMemcpyDeviceToHost, h->stream));
   PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));

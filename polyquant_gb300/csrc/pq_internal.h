@@ -79,6 +79,8 @@ struct SameSpinGemm;  // ci_sigma32_ss.cu
 void ss_delete(SameSpinGemm *g);
 struct SigmaRows;  // ci_sigma_rows.cu
 void rows_delete(SigmaRows *r);
+struct PairLists;  // ci_props.cu
+void pairs_delete(PairLists *p);
 
 }  // namespace pq
 
@@ -125,6 +127,8 @@ struct pq_ci_handle {
   std::unique_ptr<pq::SameSpinGemm, void (*)(pq::SameSpinGemm *)> ss{nullptr, pq::ss_delete};
   // FP64 sigma with a warp per determinant (ci_sigma_rows.cu); empty where ci_sigma.cu's kernel runs
   std::unique_ptr<pq::SigmaRows, void (*)(pq::SigmaRows *)> rows{nullptr, pq::rows_delete};
+  // singles by orbital pair, made by the first property call of a one-species handle (ci_props.cu)
+  std::unique_ptr<pq::PairLists, void (*)(pq::PairLists *)> pairs{nullptr, pq::pairs_delete};
   // two species: addressing of the product space (see ci_two.cu)
   std::vector<int32_t> e_a, e_b;        // species-0 (alpha, beta) string pair of each kept pair ie
   std::vector<int64_t> ebase;           // first determinant of pair ie's species-1 block
