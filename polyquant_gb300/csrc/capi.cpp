@@ -212,6 +212,22 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
   for (int v0 = 0; v0 < nvec; v0 += 4) {
     int nv = nvec - v0 < 4 ? nvec - v0 : 4;
     int nvp = il_width(h, nv, precision);
+    if (precision == PQ_FP64 && h->fp64_tc && !h->use_explicit) {
+      bool done = false;
+      if (on_device) {
+        PQ_TRY(ci_sigma64_block(h, C + (size_t)v0 * ldc, ldc, nv, S + (size_t)v0 * lds, lds, &done));
+      } else {
+        // page-locked host columns pass through device columns, copied by the conversion kernels
+        const size_t n = (size_t)h->n_dets, block = sizeof(double) * nv * (n + 1);
+        PQ_TRY(h->x_il.ensure(block));
+        PQ_TRY(h->y_il.ensure(block));
+        double *x = h->x_il.as<double>(), *y = h->y_il.as<double>();
+        for (int v = 0; v < nv; v++) PQ_TRY(ci_to_il(h, C, ldc, v0 + v, 1, 1, PQ_FP64, x + v * n));
+        PQ_TRY(ci_sigma64_block(h, x, n, nv, y, n, &done));
+        for (int v = 0; v < nv && done; v++) PQ_TRY(ci_from_il(h, y + v * n, v0 + v, 1, 1, PQ_FP64, S, lds));
+      }
+      if (done) continue;
+    }
     if (on_device && nvp == 1 && precision == PQ_FP64) {
       const double *c = C + (size_t)v0 * ldc;
       double *s = S + (size_t)v0 * lds;
@@ -305,7 +321,7 @@ pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes) {
     return PQ_ERR_ARG;
   }
   *bytes = (int64_t)(h->x_il.bytes + h->y_il.bytes + h->x_t.bytes + h->z_t.bytes + h->tc_btab.bytes + h->tc_aux.bytes +
-                     h->tc_toff.bytes + h->tc_tinfo.bytes + h->host_c.bytes + h->host_s.bytes + ci_sigma32_ss_bytes(h));
+                     h->tc_toff.bytes + h->tc_tinfo.bytes + h->host_c.bytes + h->host_s.bytes + ci_sigma32_ss_bytes(h) + sigma64_bytes(h));
   return PQ_OK;
 }
 

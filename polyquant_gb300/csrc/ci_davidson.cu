@@ -701,6 +701,11 @@ pq_status sigma_request_single(pq_ci_handle *h, const SigmaRequest &r) {
   const unsigned g = (unsigned)std::min<int64_t>((n + 255) / 256, 152 * 16);
   for (int v0 = 0; v0 < r.cnt; v0 += 4) {
     const int c = std::min(4, r.cnt - v0), nvp = il_width(h, c, r.precision);
+    if (r.precision == PQ_FP64) {
+      bool done = false;
+      PQ_TRY(ci_sigma64_block(h, r.src + (size_t)v0 * n, n, c, r.dst + (size_t)v0 * n, n, &done));
+      if (done) continue;
+    }
     const size_t esz = r.precision == PQ_FP64 ? sizeof(double) : sizeof(float);
     PQ_TRY(h->x_il.ensure(esz * nvp * (size_t)(n + 1)));
     PQ_TRY(h->y_il.ensure(esz * nvp * (size_t)(n + 1)));

@@ -460,7 +460,9 @@ pq_status ci_build(pq_ci_handle *h) {
   h->fp32_v2 = sigma32_v2_applicable(h) && getenv("PQ_SIGMA32_GATHER") == nullptr;
   h->fp32_tc = h->fp32_v2 && sigma32_tc_applicable(h) && getenv("PQ_SIGMA32_NO_TC") == nullptr;
   h->fp32_ss = h->fp32_tc && sigma32_ss_applicable(h) && getenv("PQ_SIGMA32_NO_SS") == nullptr;
-  return ci_sigma_rows_build(h);
+  PQ_TRY(ci_sigma_rows_build(h));
+  h->fp64_tc = sigma64_applicable(h) && getenv("PQ_SIGMA64_GATHER") == nullptr;
+  return PQ_OK;
 }
 
 }  // namespace pq

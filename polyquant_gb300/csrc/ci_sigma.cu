@@ -51,6 +51,7 @@ template <typename T> struct SigmaArgs {
   int64_t nblk_b;
   const T *X;
   T *Y;
+  const int *gate;  // not NULL: run only if it holds a nonzero value
 };
 
 // vector loads/stores of NV consecutive values
@@ -130,6 +131,7 @@ constexpr int SIGMA_CHUNK = 8;
 // working set stays small).  Needs TAB, J < 2^22, pair < 512, <= PK singles.
 template <typename T, int NV, bool FULL, bool TAB, int PK>
 __global__ void __launch_bounds__(SIGMA_THREADS, (PK > 0 ? 2 : 1)) sigma_one_species_kernel(SigmaArgs<T> p) {
+  if (p.gate && *p.gate == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *Wa = reinterpret_cast<T *>(smem_raw);
   T *Jrow = Wa + p.npair;
@@ -312,7 +314,7 @@ static pq_status launch_sigma(const SigmaArgs<T> &a, int64_t na, size_t smem, cu
 }
 
 template <typename T, int NV>
-static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift) {
+static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift, const int *gate = nullptr) {
   SigmaArgs<T> a{};
   a.a = make_view<T>(h->tab[0][0]);
   a.b = make_view<T>(h->tab[0][1]);
@@ -328,6 +330,7 @@ static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift)
   a.nblk_b = (nb + SIGMA_THREADS - 1) / SIGMA_THREADS;
   a.X = X;
   a.Y = Y;
+  a.gate = gate;
   size_t base = sizeof(T) * ((size_t)a.npair + (size_t)a.max1a * a.n_orb);
   size_t tab = sizeof(T) * (size_t)a.max1a * a.npair;
   const bool use_tab = base + tab <= 100 * 1024;
@@ -352,6 +355,25 @@ static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift)
   if (pk == 32) return launch_sigma<T, NV, false, true, 32>(a, na, smem, st);
   if (pk == 64) return launch_sigma<T, NV, false, true, 64>(a, na, smem, st);
   return use_tab ? launch_sigma<T, NV, false, true, 0>(a, na, smem, st) : launch_sigma<T, NV, false, false, 0>(a, na, smem, st);
+}
+
+pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, const int *gate) {
+  return sigma_dispatch<double, 1>(h, C, S, 0.0, gate);
+}
+
+pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool *done) {
+  *done = false;
+  if (!h->fp64_tc || h->use_explicit) return PQ_OK;
+  const double *c1 = C + (size_t)(nv - 1) * ldc + h->n_dets, *s1 = S + (size_t)(nv - 1) * lds + h->n_dets;
+  if (C < s1 && S < c1) return PQ_OK;
+  const pq_status s = ci_sigma64(h, C, ldc, nv, S, lds);
+  if (s == PQ_ERR_OOM) {
+    cudaGetLastError();
+    clear_error();
+    return PQ_OK;
+  }
+  *done = s == PQ_OK;
+  return s;
 }
 
 pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvp, int precision, double shift,

@@ -1,0 +1,989 @@
+// FP64 sigma = H C of one-species full CI on the tcgen05 tensor cores.
+//
+// Reference: sigma_one_species_class_singleshot (src/ci/detset/direct_singleparticle.cpp:238-372) with the elements
+// of slater_condon_singleparticle.cpp:4-175.  The kernel of ci_sigma.cu applies them one by one on the FP64 pipe,
+// which this GPU runs at 1/64 of its FP32 rate (1.1 TFLOP/s), and is bound by it.  Here every product is a sum of 34
+// exact FP16 digit products (digits9 in pq_digits.cuh), so the FP64 pipe only adds finished sums.
+//
+// In the full product space, with e_P = E_pq + E_qp (or E_pp) for an orbital pair P, H splits into
+//   diagonal      sigma  = (E_alpha + E_beta) C                               same-spin energies of the strings
+//   same spin     sigma += H_a C + C H_b^T      dense over the strings: singles (same-spin part) and doubles
+//   opposite spin sigma += sum_PQ (P|Q) e_P^alpha C e_Q^beta    alpha-beta doubles, the Coulomb part of the singles
+//                                                               and of the diagonal
+// x64_digits_kernel splits C once, planes [digit][root][Ia][Ib], and writes the diagonal term.  ss64_kernel is a GEMM
+// over those planes for either spin.  ab64_kernel forms, per alpha string Ia and tile of 128 beta strings Jb,
+//   D[Jb][Q] = sum_{(Ja, P): e_P Ja = +-Ia} +-(P|Q) C(Ja, Jb)       K = singles and occupied orbitals of Ia
+// with both operands fetched by TMA row gathers (rows of C's planes by Ja, signed rows of the integral digits by P),
+// and adds the entries of D into sigma(Ia, Ib) along the lists of e_Q.  The gathered rows run along Jb and Q, so both
+// operands are M- and N-major and nothing is converted or transposed on the way.
+//
+// Errors.  A sum of digits leaves out less than 2^-64 of K max|C| max|W|.  D goes through shared memory as 64-bit
+// integers with one exponent per tile, 56 bits below the tile's largest entry, and sums of its entries are exact.  An
+// element-by-element FP64 sum rounds each of its terms at 2^-53 of the partial sum, which holds the diagonal (-147
+// C_I at 14 orbitals).  2-norm error against 64-bit references: see the numbers at the end of this comment.
+//
+// Non-finite input (or integrals), and a bounded wait that runs out, raise a device flag; the element-by-element
+// kernel is launched behind with that flag as its condition and then computes the whole result, as before.
+//
+// Measured, four roots of FCI(14o, 7a7b): S64_NOW
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <new>
+#include <utility>
+#include <vector>
+
+#include "pq_bits.cuh"
+#include "pq_digits.cuh"
+#include "pq_internal.h"
+#include "pq_tc.cuh"
+
+namespace pq {
+
+struct Sigma64 {
+  struct Side {
+    DevBuf d;                 // digits of the dense same-spin H: [digit][I][np]
+    int64_t n = 0, np = 0;    // strings, row length
+    DevBuf kt_off, kt_list;   // K chunks of 32 with an entry, per row tile (64 rows alpha, 128 rows beta)
+    int win = 2;              // chunks of a window that holds at most 80 entries of a row
+  };
+  Side side[2];
+  bool shared = false;        // beta uses alpha's matrix
+  DevBuf w;                   // digits of (P|Q): [digit][2 P + sign; a zero row last][pass x 64]
+  DevBuf klist;               // per alpha string kp x {row of C, row of w}
+  int kp = 0, npass = 1, wq = 0;
+  DevBuf toff, tent;          // scatter lists per (pass, beta tile)
+  DevBuf hi;                  // high words of max|.|: same-spin H alpha, beta, integrals
+  DevBuf xd, aux;             // digits of C; gate and high word of max|C| per root
+  int sms = 0;
+  size_t bytes() const {
+    size_t b = w.bytes + klist.bytes + toff.bytes + tent.bytes + hi.bytes + xd.bytes + aux.bytes;
+    for (const Side &s : side) b += s.d.bytes + s.kt_off.bytes + s.kt_list.bytes;
+    return b;
+  }
+};
+void sigma64_delete(Sigma64 *s) { delete s; }
+
+namespace s64 {
+
+using namespace tcx;
+namespace dg = digits9;
+
+constexpr int KMAX = 80;                     // products of one exact sum
+constexpr int BM = 128, BN = 64;             // accumulator tile of one order
+constexpr int EPI_WARPS = 16, EPI = 32 * EPI_WARPS;
+constexpr int THREADS = 64 + EPI;            // producer warp, MMA warp, epilogue warps
+enum { ERR_WAIT = 2 };
+
+// exponent of a plane from the high word of its largest magnitude
+__device__ __forceinline__ int plane_exp(const uint32_t *hi) { return digits::exponent_of(__ldg(hi)); }
+
+// The 11 MMAs of one K step of 16: digit i of A times digits 0 .. min(6, 7 - i) of B, which lie `bstep` bytes apart and
+// form one operand of up to 256 rows; order l accumulates in columns 64 l.  FIRST: the tile's first step.  bdesc(j)
+// and adesc(i) give the descriptors.
+template <typename A, typename B>
+__device__ __forceinline__ void mma_step(uint32_t tmem, A &&adesc, B &&bdesc, uint32_t major, bool first) {
+#pragma unroll
+  for (int i = 0; i < dg::N; i++) {
+    const int n = (dg::ORDERS - i < dg::N ? dg::ORDERS - i : dg::N);  // digits of B
+    if (i == 1 && first) {
+      // order 7 begins here, the others were begun by digit 0
+      mma_f16(tmem + 64, adesc(1), bdesc(0), idesc_f16(256) | major, 1u);
+      mma_f16(tmem + 5 * 64, adesc(1), bdesc(4), idesc_f16(128) | major, 1u);
+      mma_f16(tmem + 7 * 64, adesc(1), bdesc(6), idesc_f16(64) | major, 0u);
+      continue;
+    }
+    const uint32_t acc = (first && i == 0) ? 0u : 1u;
+    mma_f16(tmem + i * 64, adesc(i), bdesc(0), idesc_f16((n < 4 ? n : 4) * 64) | major, acc);
+    if (n > 4) mma_f16(tmem + (i + 4) * 64, adesc(i), bdesc(4), idesc_f16((n - 4) * 64) | major, acc);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- digits of C
+
+__global__ void __launch_bounds__(256) x64_absmax_kernel(const double *C, int64_t ldc, int64_t n, uint32_t *hi) {
+  const double *c = C + (int64_t)blockIdx.y * ldc;
+  uint32_t m = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    m = max(m, (uint32_t)__double2hiint(c[i]) & 0x7fffffffu);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(hi + blockIdx.y, m);
+}
+
+// planes [digit][v][Ia][nbp] of the nv columns of C and S = (E_alpha + E_beta) C; block per (alpha string, root)
+__global__ void __launch_bounds__(256) x64_digits_kernel(const double *C, int64_t ldc, int64_t na, int64_t nb, int64_t nbp,
+                                                        int nv, const uint32_t *xhi, const uint32_t *hi,
+                                                        const double *ea, const double *eb, unsigned short *xd, double *S,
+                                                        int64_t lds, int *gate) {
+  const int64_t ia = blockIdx.x;
+  const int v = blockIdx.y;
+  const int e = plane_exp(xhi + v);
+  if (e == digits::BAD || plane_exp(hi) == digits::BAD || plane_exp(hi + 1) == digits::BAD || plane_exp(hi + 2) == digits::BAD) {
+    if (threadIdx.x == 0) *gate = 1;
+    return;
+  }
+  const double *c = C + v * ldc + ia * nb;
+  double *s = S + v * lds + ia * nb;
+  const double da = ea[ia];
+  const int64_t plane = (int64_t)nv * na * nbp;
+  unsigned short *row = xd + ((int64_t)v * na + ia) * nbp;
+  for (int64_t b = 2 * threadIdx.x; b < nb; b += 2 * blockDim.x) {
+    const double x0 = c[b], x1 = b + 1 < nb ? c[b + 1] : 0.0;
+    unsigned short d0[dg::N], d1[dg::N];
+    dg::to_half(digits::fixed_point<dg::BITS>(x0, e), d0);
+    dg::to_half(digits::fixed_point<dg::BITS>(x1, e), d1);
+#pragma unroll
+    for (int i = 0; i < dg::N; i++) *reinterpret_cast<ushort2 *>(row + i * plane + b) = make_ushort2(d0[i], d1[i]);
+    s[b] = (da + eb[b]) * x0;
+    if (b + 1 < nb) s[b + 1] = (da + eb[b + 1]) * x1;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- opposite spin
+
+constexpr int A_DIGIT = BM * 16 * 2;                // 4 KB: one digit of 128 beta strings x 16 K values
+constexpr int A_STAGE = dg::N * A_DIGIT;            // 28 KB
+constexpr int A_STAGES = 3;
+constexpr int B_BYTES = dg::N * KMAX * 128;         // 70 KB: all digits of 64 pairs x K
+constexpr int LDS_D = BN + 1;                       // row length of the staged D
+constexpr int D_BYTES = BM * LDS_D * 8;             // 65 KB
+constexpr int AB_BARS = 2 * A_STAGES + 9;
+constexpr int GATHER_WARPS = 4;                     // warp 0 and the last three
+constexpr int AB_THREADS = THREADS + 32 * (GATHER_WARPS - 1);
+constexpr int AB_SMEM = A_STAGES * A_STAGE + B_BYTES + D_BYTES + GATHER_WARPS * KMAX * 8 + AB_BARS * 8 + 64 + 1024;
+static_assert(AB_SMEM <= 232448, "shared memory per CTA");
+
+struct AbArgs {
+  int64_t na, nb, items;
+  int nv, vsplit;            // vsplit: an item is one root of (alpha string, pass), else all of them
+  int npass, wq, kp, wrows;  // wrows: rows of one digit of w
+  int m_tiles;
+  const int2 *klist;
+  const int32_t *toff;
+  const int4 *tent;
+  const uint32_t *xhi, *whi;
+  double *S;
+  int64_t lds;
+  int *gate;
+};
+
+// sum 2^e for an integer, rounded once or twice (outside the normal range)
+__device__ __forceinline__ double pow2_scale(int e) {
+  return e > -1022 && e < 1023 ? __hiloint2double((e + 1023) << 20, 0) : scalbn(1.0, e);
+}
+
+// Roles: warp 0 gathers (its lanes share the row gathers of a stage), warp 1 lane 0 issues MMAs, warps 2 .. 17 drain
+// and scatter.  Per tile the epilogue finds the largest |D| from the four leading orders, so that the tile's entries
+// become 57-bit integers; stages them; releases the accumulators; and sums the entries of each target.  Every wait is
+// an mbarrier wait with a budget; one that runs out raises the gate and the CTA winds down.
+__global__ void __launch_bounds__(AB_THREADS, 1)
+    ab64_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, AbArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  unsigned char *sa = smem, *sb = sa + A_STAGES * A_STAGE;
+  int64_t *sd = reinterpret_cast<int64_t *>(sb + B_BYTES);
+  int2 *kl_all = reinterpret_cast<int2 *>(reinterpret_cast<unsigned char *>(sd) + D_BYTES);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(kl_all + GATHER_WARPS * KMAX);
+  uint64_t *a_full = bars, *a_empty = bars + A_STAGES, *b_full = bars + 2 * A_STAGES, *b_empty = b_full + 1;
+  uint64_t *acc_full = b_full + 2, *acc_empty = b_full + 3, *max_full = b_full + 4, *d_full = b_full + 5, *d_empty = b_full + 6;
+  uint64_t *drain = b_full + 7;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + AB_BARS);
+  uint32_t *tmax = tmem_slot + 1;  // [2]
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 3);
+  if (*g.gate) return;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < A_STAGES; i++) {
+      mbar_init(smem_u32(a_full + i), 1);
+      mbar_init(smem_u32(a_empty + i), 1);
+    }
+    mbar_init(smem_u32(b_full), 1);
+    mbar_init(smem_u32(b_empty), 1);
+    mbar_init(smem_u32(acc_full), 1);
+    mbar_init(smem_u32(acc_empty), EPI_WARPS);
+    mbar_init(smem_u32(max_full), EPI_WARPS);
+    mbar_init(smem_u32(d_full), EPI_WARPS);
+    mbar_init(smem_u32(d_empty), EPI_WARPS);
+    mbar_init(smem_u32(drain), 1);
+    tmax[0] = tmax[1] = 0;
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const int steps = g.kp / 16;
+  auto fail = [&] {
+    *g.gate = ERR_WAIT;
+    *abort_flag = 1;
+  };
+  // item -> alpha string, pass, roots v0 .. v1 - 1
+  auto item_of = [&](int64_t it, int64_t &ia, int &p, int &v0, int &v1) {
+    v0 = 0, v1 = g.nv;
+    if (g.vsplit) {
+      v0 = (int)(it % g.nv), v1 = v0 + 1;
+      it /= g.nv;
+    }
+    ia = it / g.npass;
+    p = (int)(it - ia * g.npass);
+  };
+
+  if (warp == 0 || warp >= 2 + EPI_WARPS) {
+    // ---- gather warps
+    const int pw = warp == 0 ? 0 : warp - (1 + EPI_WARPS);
+    int2 *kl = kl_all + pw * KMAX;  // this warp's copy of the item's K list
+    int gs = 0, nit = 0;
+    bool ok = true;
+    for (int64_t it = blockIdx.x; it < g.items && ok; it += gridDim.x, nit++) {
+      int64_t ia;
+      int p, v0, v1;
+      item_of(it, ia, p, v0, v1);
+      __syncwarp();
+      for (int k = lane; k < g.kp; k += 32) kl[k] = __ldg(g.klist + ia * g.kp + k);
+      __syncwarp();
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(b_empty), (uint32_t)(nit & 1) ^ 1u, WAIT_CYCLES)) && !*abort_flag;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      if (pw == 0 && lane == 0) mbar_expect_tx(smem_u32(b_full), dg::N * g.kp * 128);
+      __syncwarp();
+      for (int i = GATHER_WARPS * lane + pw; i < dg::N * (g.kp / 4); i += 32 * GATHER_WARPS) {
+        const int d = i / (g.kp / 4), k = 4 * (i - d * (g.kp / 4));
+        const int r = d * g.wrows;
+        tma_gather4(smem_u32(sb) + d * g.kp * 128 + k * 128, &mapW, p * BN, r + kl[k].y, r + kl[k + 1].y, r + kl[k + 2].y,
+                    r + kl[k + 3].y, smem_u32(b_full));
+      }
+      for (int v = v0; v < v1 && ok; v++)
+        for (int t = 0; t < g.m_tiles && ok; t++)
+          for (int s = 0; s < steps; s++, gs++) {
+            const int slot = gs % A_STAGES;
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(a_empty + slot), (uint32_t)((gs / A_STAGES) & 1) ^ 1u, WAIT_CYCLES) &&
+                                             !*abort_flag);
+            if (!ok) break;
+            if (pw == 0 && lane == 0) mbar_expect_tx(smem_u32(a_full + slot), A_STAGE);
+            __syncwarp();
+            // 56 gathers: digit, half of the 128 strings, group of four K values
+            for (int i = GATHER_WARPS * lane + pw; i < dg::N * 8; i += 32 * GATHER_WARPS) {
+              const int d = i >> 3, h = (i >> 2) & 1, k = 4 * (i & 3);
+              const int2 *q = kl + 16 * s + k;
+              const int y = (int)((int64_t)(d * g.nv + v) * g.na);
+              tma_gather4(smem_u32(sa + slot * A_STAGE) + d * A_DIGIT + h * (A_DIGIT / 2) + k * 128, &mapX, t * BM + h * 64,
+                          y + q[0].x, y + q[1].x, y + q[2].x, y + q[3].x, smem_u32(a_full + slot));
+            }
+          }
+    }
+    if (!ok) {
+      if (lane == 0) fail();
+    }
+    // the gathers in flight land before the CTA exits
+    if (pw == 0 && lane == 0) {
+      for (int j = gs > A_STAGES ? gs - A_STAGES : 0; j < gs; j++)
+        mbar_wait(smem_u32(a_full + (j % A_STAGES)), (uint32_t)((j / A_STAGES) & 1), WAIT_CYCLES);
+      if (nit > 0) mbar_wait(smem_u32(b_full), (uint32_t)((nit - 1) & 1), WAIT_CYCLES);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int gs = 0, nit = 0, seq = 0;
+      bool ok = true;
+      for (int64_t it = blockIdx.x; it < g.items && ok; it += gridDim.x, nit++) {
+        int64_t ia;
+        int p, v0, v1;
+        item_of(it, ia, p, v0, v1);
+        ok = mbar_wait(smem_u32(b_full), (uint32_t)(nit & 1), WAIT_CYCLES) && !*abort_flag;
+        for (int u = 0; u < (v1 - v0) * g.m_tiles && ok; u++, seq++) {
+          ok = mbar_wait(smem_u32(acc_empty), (uint32_t)(seq & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          for (int s = 0; s < steps; s++, gs++) {
+            const int slot = gs % A_STAGES;
+            ok = mbar_wait(smem_u32(a_full + slot), (uint32_t)((gs / A_STAGES) & 1), WAIT_CYCLES);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_u32(sa + slot * A_STAGE), b = smem_u32(sb) + s * 2048;
+            const uint32_t bstep = (uint32_t)g.kp * 128;
+            mma_step(
+                tmem, [&](int i) { return smem_desc_mn(a + i * A_DIGIT, A_DIGIT / 2); },
+                [&](int j) { return smem_desc_mn(b + j * bstep, bstep); }, IDESC_A_MN | IDESC_B_MN, s == 0);
+            mma_commit(smem_u32(a_empty + slot));
+          }
+          if (ok) mma_commit(smem_u32(acc_full));
+        }
+        if (ok) mma_commit(smem_u32(b_empty));
+      }
+      if (!ok) fail();
+      mma_commit(smem_u32(drain));
+      mbar_wait(smem_u32(drain), 0, WAIT_CYCLES);
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue
+    const int q4 = warp & 3, part = (warp - 2) >> 2, te = threadIdx.x - 64;
+    const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16);
+    int64_t *drow = sd + (int64_t)(q4 * 32 + lane) * LDS_D;
+    auto wait_all = [&](uint64_t *bar, int phase) {
+      return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), (uint32_t)(phase & 1), WAIT_CYCLES) && !*abort_flag);
+    };
+    int seq = 0;
+    bool ok = true;
+    const int ew = plane_exp(g.whi);
+    for (int64_t it = blockIdx.x; it < g.items && ok; it += gridDim.x) {
+      int64_t ia;
+      int p, v0, v1;
+      item_of(it, ia, p, v0, v1);
+      for (int v = v0; v < v1 && ok; v++) {
+        const int ex = plane_exp(g.xhi + v);
+        double *srow = g.S + v * g.lds + ia * g.nb;
+        for (int t = 0; t < g.m_tiles; t++, seq++) {
+          const int tl = p * g.m_tiles + t, k0 = __ldg(g.toff + tl), k1 = __ldg(g.toff + tl + 1);
+          ok = wait_all(acc_full, seq);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          // largest |D|, in units of order 3
+          float m = 0.0f;
+          for (int c0 = 8 * part; c0 < g.wq; c0 += 32) {
+            uint32_t a[4][8];
+#pragma unroll
+            for (int l = 0; l < 4; l++) tmem_ld8(taddr + l * BN + c0, a[l]);
+            tmem_wait();
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+              float f = __uint_as_float(a[0][c]);
+#pragma unroll
+              for (int l = 1; l < 4; l++) f = fmaf(f, 512.0f, __uint_as_float(a[l][c]));
+              m = fmaxf(m, fabsf(f));
+            }
+          }
+          const uint32_t wm = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+          if (lane == 0) {
+            atomicMax(tmax + (seq & 1), wm);
+            mbar_arrive(smem_u32(max_full));
+          }
+          ok = wait_all(max_full, seq);
+          if (!ok) break;
+          // |T| < (m (1 + 2^-20) + 2^17) 2^36 with the orders behind; the entries of T >> sh are below 2^56
+          const float mx = __uint_as_float(*(volatile uint32_t *)(tmax + (seq & 1))) * 1.00001f + 131072.0f;
+          const int sh = max(0, (int)(__float_as_uint(mx) >> 23) - 126 + 36 - 56);
+          ok = wait_all(d_empty, seq ^ 1);  // the last tile's entries have been summed
+          if (!ok) break;
+          if (te == 0) tmax[(seq + 1) & 1] = 0;
+          for (int c0 = 8 * part; c0 < g.wq; c0 += 32) {
+            uint32_t a[dg::ORDERS][8];
+#pragma unroll
+            for (int l = 0; l < dg::ORDERS; l++) tmem_ld8(taddr + l * BN + c0, a[l]);
+            tmem_wait();
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+              float f[dg::ORDERS];
+#pragma unroll
+              for (int l = 0; l < dg::ORDERS; l++) f[l] = __uint_as_float(a[l][c]);
+              int64_t hi, lo;
+              dg::combine(f, hi, lo);
+              drow[c0 + c] = (sh <= 36 ? hi << (36 - sh) : hi >> (sh - 36)) + (lo >> sh);
+            }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(smem_u32(acc_empty));
+            mbar_arrive(smem_u32(d_full));
+          }
+          ok = wait_all(d_full, seq);
+          if (!ok) break;
+          const double scale = pow2_scale(ex + ew - 77 + sh);
+          for (int kb = k0 + te; kb < k1; kb += 2 * EPI) {
+            int4 ent[2];
+            ent[0] = __ldg(g.tent + kb);
+            ent[1] = kb + EPI < k1 ? __ldg(g.tent + kb + EPI) : make_int4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+              const int n = ent[u].x >> 16;
+              if (n == 0) continue;
+              const uint32_t w3[3] = {(uint32_t)ent[u].y, (uint32_t)ent[u].z, (uint32_t)ent[u].w};
+              int64_t sum = 0;
+#pragma unroll
+              for (int i = 0; i < 6; i++)
+                if (i < n) {
+                  // phase << 13 | beta string << 6 | pair
+                  const uint32_t en = (w3[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+                  const int64_t x = sd[((en >> 6) & 127u) * LDS_D + (en & 63u)];
+                  sum += (en & 8192u) ? -x : x;
+                }
+              atomicAdd(srow + (ent[u].x & 0xffff), (double)sum * scale);
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(d_empty));
+        }
+      }
+    }
+    if (!ok && lane == 0) fail();
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------- same spin
+
+constexpr int SS_A = BM * 64, SS_B = BN * 64;                  // one digit of 32 K values: 8 KB, 4 KB
+constexpr int SS_STAGE = dg::N * (SS_A + SS_B);                // 84 KB
+constexpr int SS_STAGES = 2;
+constexpr int SS_BARS = 2 * SS_STAGES + 3;
+constexpr int SS_SMEM = SS_STAGES * SS_STAGE + SS_BARS * 8 + 64 + 1024;
+
+struct SsArgs {
+  int64_t na, nb;
+  int nv, m_tiles, n_tiles;   // tiles of 128 beta strings, of 64 alpha strings
+  int64_t tiles;
+  int win;                    // chunks per exact window
+  int64_t a_plane, b_plane;   // rows of one digit of either operand
+  const int32_t *kt_off, *kt_list;
+  const uint32_t *xhi, *dhi;
+  double *S;
+  int64_t lds;
+  int *gate;
+};
+
+// Y[v][Ia][Ib] += sum_Ja Ha[Ia][Ja] X[v][Ja][Ib]   (ALPHA: A = planes of C along Ib, B = rows of Ha)
+//              or sum_Jb Hb[Ib][Jb] X[v][Ia][Jb]   (A = rows of Hb, B = rows (v, Ia) of C)
+// Accumulator rows are beta strings, columns alpha strings, so sigma is read and written in whole lines.  The sums of
+// a window of K chunks (at most 80 entries of a row of H) are exact; the epilogue adds windows as 96-bit integers.
+template <bool ALPHA>
+__global__ void __launch_bounds__(THREADS, 1)
+    ss64_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, SsArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + SS_STAGES * SS_STAGE);
+  uint64_t *full = bars, *empty = bars + SS_STAGES, *accf = bars + 2 * SS_STAGES, *acce = accf + 1, *drain = accf + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + SS_BARS);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  if (*g.gate) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < SS_STAGES; i++) {
+      mbar_init(smem_u32(full + i), 1);
+      mbar_init(smem_u32(empty + i), 1);
+    }
+    mbar_init(smem_u32(accf), 1);
+    mbar_init(smem_u32(acce), EPI_WARPS);
+    mbar_init(smem_u32(drain), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  auto fail = [&] {
+    *g.gate = ERR_WAIT;
+    *abort_flag = 1;
+  };
+  // tile -> root, beta tile, alpha tile; the alpha tile varies fastest
+  auto tile_of = [&](int64_t t, int &v, int &mt, int &nt) {
+    nt = (int)(t % g.n_tiles);
+    t /= g.n_tiles;
+    mt = (int)(t % g.m_tiles);
+    v = (int)(t / g.m_tiles);
+  };
+  auto row_tile = [&](int mt, int nt) { return ALPHA ? nt : mt; };
+  // end of the window that starts at list position j
+  auto window_end = [&](int j, int k1) {
+    const int w = __ldg(g.kt_list + j) / g.win;
+    int e = j + 1;
+    while (e < k1 && __ldg(g.kt_list + e) / g.win == w) e++;
+    return e;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int gs = 0;
+      bool ok = true;
+      for (int64_t t = blockIdx.x; t < g.tiles && ok; t += gridDim.x) {
+        int v, mt, nt;
+        tile_of(t, v, mt, nt);
+        const int rt = row_tile(mt, nt), k1 = g.kt_off[rt + 1];
+        for (int j = g.kt_off[rt]; j < k1; j++, gs++) {
+          const int slot = gs % SS_STAGES;
+          ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((gs / SS_STAGES) & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
+          if (!ok) break;
+          const uint32_t a = smem_u32(smem + slot * SS_STAGE), b = a + dg::N * SS_A, bar = smem_u32(full + slot);
+          const int k = g.kt_list[j] * 32;
+          mbar_expect_tx(bar, SS_STAGE);
+          for (int d = 0; d < dg::N; d++) {
+            if (ALPHA) {
+              const int y = (int)(d * g.a_plane + (int64_t)v * g.na) + k;  // rows Ja of the plane
+              tma_load_2d(a + d * SS_A, &mapA, mt * BM, y, bar);
+              tma_load_2d(a + d * SS_A + SS_A / 2, &mapA, mt * BM + 64, y, bar);
+              tma_load_2d(b + d * SS_B, &mapB, k, (int)(d * g.b_plane) + nt * BN, bar);
+            } else {
+              tma_load_2d(a + d * SS_A, &mapA, k, (int)(d * g.a_plane) + mt * BM, bar);
+              tma_load_2d(b + d * SS_B, &mapB, k, (int)(d * g.b_plane + (int64_t)v * g.na) + nt * BN, bar);
+            }
+          }
+        }
+      }
+      if (!ok) fail();
+      for (int j = gs > SS_STAGES ? gs - SS_STAGES : 0; j < gs; j++)
+        mbar_wait(smem_u32(full + (j % SS_STAGES)), (uint32_t)((j / SS_STAGES) & 1), WAIT_CYCLES);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int gs = 0, seq = 0;
+      bool ok = true;
+      for (int64_t t = blockIdx.x; t < g.tiles && ok; t += gridDim.x) {
+        int v, mt, nt;
+        tile_of(t, v, mt, nt);
+        const int rt = row_tile(mt, nt), k1 = g.kt_off[rt + 1];
+        for (int j = g.kt_off[rt]; j < k1 && ok; seq++) {
+          const int e = window_end(j, k1);
+          ok = mbar_wait(smem_u32(acce), (uint32_t)(seq & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          for (int j0 = j; j < e; j++, gs++) {
+            const int slot = gs % SS_STAGES;
+            ok = mbar_wait(smem_u32(full + slot), (uint32_t)((gs / SS_STAGES) & 1), WAIT_CYCLES);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_u32(smem + slot * SS_STAGE), b = a + dg::N * SS_A;
+#pragma unroll
+            for (int s = 0; s < 2; s++)
+              mma_step(
+                  tmem,
+                  [&](int i) {
+                    return ALPHA ? smem_desc_mn(a + i * SS_A + s * 2048, SS_A / 2) : smem_desc_k64(a + i * SS_A + s * 32);
+                  },
+                  [&](int i) { return smem_desc_k64(b + i * SS_B + s * 32); }, ALPHA ? IDESC_A_MN : 0u, j == j0 && s == 0);
+            mma_commit(smem_u32(empty + slot));
+          }
+          if (ok) mma_commit(smem_u32(accf));
+        }
+      }
+      if (!ok) fail();
+      mma_commit(smem_u32(drain));
+      mbar_wait(smem_u32(drain), 0, WAIT_CYCLES);
+    }
+    __syncwarp();
+  } else {
+    const int q4 = warp & 3, part = (warp - 2) >> 2;
+    const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + 16 * part;
+    int seq = 0;
+    bool ok = true;
+    const int ed = plane_exp(g.dhi);
+    for (int64_t t = blockIdx.x; t < g.tiles && ok; t += gridDim.x) {
+      int v, mt, nt;
+      tile_of(t, v, mt, nt);
+      const int rt = row_tile(mt, nt), k0 = g.kt_off[rt], k1 = g.kt_off[rt + 1];
+      if (k0 == k1) continue;
+      // sums of T >> 4 over the windows: 64-bit high part, 32-bit low part
+      int64_t sh[16];
+      uint32_t sl[16];
+#pragma unroll
+      for (int c = 0; c < 16; c++) sh[c] = 0, sl[c] = 0;
+      for (int j = k0; j < k1; seq++) {
+        j = window_end(j, k1);
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(accf), (uint32_t)(seq & 1), WAIT_CYCLES) && !*abort_flag);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c0 = 0; c0 < 16; c0 += 4) {
+          uint32_t a[dg::ORDERS][4];
+#pragma unroll
+          for (int l = 0; l < dg::ORDERS; l++) tmem_ld4(taddr + l * BN + c0, a[l]);
+          tmem_wait();
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            float f[dg::ORDERS];
+#pragma unroll
+            for (int l = 0; l < dg::ORDERS; l++) f[l] = __uint_as_float(a[l][c]);
+            int64_t hi, lo;
+            dg::combine(f, hi, lo);
+            lo >>= 4;
+            const uint32_t l32 = (uint32_t)lo, s = sl[c0 + c] + l32;
+            sh[c0 + c] += hi + (lo >> 32) + (s < l32);
+            sl[c0 + c] = s;
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(acce));
+      }
+      if (!ok) break;
+      const int64_t ib = (int64_t)mt * BM + q4 * 32 + lane;
+      const int e = plane_exp(g.xhi + v) + ed - 73;  // T counts 2^(e - 4)
+      if (ib < g.nb)
+#pragma unroll
+        for (int c = 0; c < 16; c++) {
+          const int64_t ia = (int64_t)nt * BN + 16 * part + c;
+          if (ia < g.na) {
+            double *y = g.S + v * g.lds + ia * g.nb + ib;
+            *y += digits::to_double(sh[c], (int64_t)sl[c], e);
+          }
+        }
+    }
+    if (!ok && lane == 0) fail();
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------- tables
+
+__global__ void __launch_bounds__(256) absmax_kernel(const double *x, int64_t n, uint32_t *hi) {
+  uint32_t m = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    m = max(m, (uint32_t)__double2hiint(x[i]) & 0x7fffffffu);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(hi, m);
+}
+
+// Row I of the dense same-spin H (digits, zeroed before): singles with their phase and doubles; flags of the
+// (row tile, chunk) blocks with an entry; and the largest number of a row's entries in aligned windows of 2, 4, 8, 16
+// chunks.  Shared memory: one counter per chunk.
+__global__ void __launch_bounds__(128) dense_kernel(const int64_t *o1, const int32_t *J1, const int32_t *info1,
+                                                   const double *F1, const int64_t *o2, const int32_t *J2,
+                                                   const double *D2, int64_t n, int64_t np, const uint32_t *hi, int chunks,
+                                                   int tile_rows, unsigned short *d, uint8_t *flags, int *wmax) {
+  extern __shared__ int cnt[];
+  const int64_t I = blockIdx.x;
+  const int e = plane_exp(hi);
+  for (int c = threadIdx.x; c < chunks; c += blockDim.x) cnt[c] = 0;
+  __syncthreads();
+  auto put = [&](int J, double x) {
+    atomicAdd(cnt + J / 32, 1);
+    flags[(I / tile_rows) * chunks + J / 32] = 1;
+    if (!d || e == digits::BAD) return;
+    unsigned short h[dg::N];
+    dg::to_half(digits::fixed_point<dg::BITS>(x, e), h);
+#pragma unroll
+    for (int i = 0; i < dg::N; i++) d[((int64_t)i * n + I) * np + J] = h[i];
+  };
+  for (int64_t k = o1[I] + threadIdx.x; k < o1[I + 1]; k += blockDim.x) put(J1[k], (info1[k] & 1) ? -F1[k] : F1[k]);
+  for (int64_t k = o2[I] + threadIdx.x; k < o2[I + 1]; k += blockDim.x) put(J2[k], D2[k]);
+  __syncthreads();
+  for (int l = 0; l < 4; l++) {
+    const int L = 2 << l;
+    int m = 0;
+    for (int w = threadIdx.x * L; w < chunks; w += blockDim.x * L) {
+      int s = 0;
+      for (int c = w; c < min(w + L, chunks); c++) s += cnt[c];
+      m = max(m, s);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(wmax + l, m);
+  }
+}
+
+// digits of (P|Q): rows 2 P and 2 P + 1 (negated) of each digit, a zero row behind; pair Q in column
+// 64 (Q / wq) + Q % wq
+__global__ void w_kernel(const double *eab, int npair, int wq, int ncol, const uint32_t *hi, unsigned short *w) {
+  const int64_t rows = 2 * npair + 1, i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * ncol) return;
+  const int r = (int)(i / ncol), c = (int)(i - (int64_t)r * ncol);
+  const int Q = (c / BN) * wq + c % BN, e = plane_exp(hi);
+  int64_t t = 0;
+  if (c % BN < wq && Q < npair && r < 2 * npair && e != digits::BAD)
+    t = digits::fixed_point<dg::BITS>(eab[(int64_t)(r >> 1) * npair + Q], e);
+  if (r & 1) t = -t;
+  unsigned short h[dg::N];
+  dg::to_half(t, h);
+#pragma unroll
+  for (int k = 0; k < dg::N; k++) w[((int64_t)k * rows + r) * ncol + c] = h[k];
+}
+
+// K list of each alpha string: its singles, its occupied orbitals, then the zero row
+__global__ void klist_kernel(const int64_t *o1, const int32_t *J1, const int32_t *info1, const uint64_t *str, int64_t na,
+                             int kp, int npair, int2 *kl) {
+  const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (I >= na) return;
+  int2 *o = kl + I * kp;
+  int k = 0;
+  for (int64_t s = o1[I]; s < o1[I + 1]; s++) o[k++] = make_int2(J1[s], info1[s]);
+  for (uint64_t m = str[I]; m; m &= m - 1) {
+    const int p = __ffsll((long long)m) - 1;
+    o[k++] = make_int2((int)I, (p * (p + 3) / 2) << 1);
+  }
+  for (; k < kp; k++) o[k] = make_int2((int)I, 2 * npair);
+}
+
+}  // namespace s64
+
+// One-species full CI of more than 32 768 determinants (below, ci_sigma_rows.cu), singles and occupied orbitals of an
+// alpha string within one exact sum of 80, 16-bit beta strings in the scatter lists, dense same-spin matrices of at
+// most 4 GiB of digits that are at least 2.5 % filled (a digit product of a zero costs 1/60 of an FP64 FMA).
+bool sigma64_applicable(const pq_ci_handle *h) {
+  if (h->n_species != 1 || !h->full || h->wide || h->rows) return false;
+  const SpinTablesDev &a = h->tab[0][0], &b = h->tab[0][1];
+  if (a.max1 + h->desc.n_alpha[0] > s64::KMAX || b.n_str >= 65536) return false;
+  for (int sp = 0; sp < 2; sp++) {
+    const SpinTablesDev &t = h->tab[0][sp];
+    const double n = (double)t.n_str;
+    if (14.0 * n * (n + 64) > 4.3e9 || (double)(t.n1 + t.n2) < 0.025 * n * n) return false;
+  }
+  return 2.0 * a.n_str * 7 * 4 < 2e9;  // plane rows are 32-bit TMA coordinates
+}
+
+size_t sigma64_bytes(const pq_ci_handle *h) { return h->s64 ? h->s64->bytes() : 0; }
+
+static PFN_cuTensorMapEncodeTiled_v12000 s64_encode_fn() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      return (PFN_cuTensorMapEncodeTiled_v12000)p;
+    return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
+  }();
+  return fn;
+}
+
+// FP16 matrix of `rows` rows of `cols` values, ld values apart; reads outside give zeros
+static pq_status s64_map(CUtensorMap *m, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_cols,
+                         int box_rows) {
+  auto fn = s64_encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled is not available from the driver");
+    return PQ_ERR_CUDA;
+  }
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, es[2] = {1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, es,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d): %lld x %lld", (int)r, (long long)rows, (long long)cols);
+    return PQ_ERR_CUDA;
+  }
+  return PQ_OK;
+}
+
+static int64_t up64(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
+
+// Dense same-spin H of one spin list in the role of alpha (64-row tiles) or beta (128-row tiles).  digits = false only
+// makes the chunk lists (the matrix is the other side's).
+static pq_status s64_side(pq_ci_handle *h, Sigma64 &S, int sp, bool with_digits) {
+  using namespace s64;
+  const SpinTablesDev &t = h->tab[0][sp];
+  Sigma64::Side &d = S.side[sp];
+  cudaStream_t st = h->stream;
+  d.n = t.n_str;
+  d.np = up64(t.n_str, 64);
+  const int chunks = (int)((d.n + 31) / 32), tile_rows = sp == 0 ? BN : BM;
+  const int64_t rt = (d.n + tile_rows - 1) / tile_rows;
+  if (with_digits) {
+    const size_t bytes = 2 * (size_t)dg::N * d.n * d.np;
+    PQ_TRY(d.d.alloc(bytes));
+    PQ_CUDA_TRY(cudaMemsetAsync(d.d.ptr, 0, bytes, st));
+  }
+  DevBuf flags, wmax;
+  PQ_TRY(flags.alloc((size_t)rt * chunks));
+  PQ_TRY(wmax.alloc(4 * sizeof(int)));
+  PQ_CUDA_TRY(cudaMemsetAsync(flags.ptr, 0, (size_t)rt * chunks, st));
+  PQ_CUDA_TRY(cudaMemsetAsync(wmax.ptr, 0, 4 * sizeof(int), st));
+  uint32_t *hi = S.hi.as<uint32_t>() + sp;
+  const unsigned g1 = (unsigned)std::min<int64_t>((t.n1 + 255) / 256, 1216), g2 = (unsigned)std::min<int64_t>((t.n2 + 255) / 256, 1216);
+  if (t.n1) absmax_kernel<<<g1, 256, 0, st>>>(t.s1_F64.as<double>(), t.n1, hi);
+  if (t.n2) absmax_kernel<<<g2, 256, 0, st>>>(t.s2_D64.as<double>(), t.n2, hi);
+  dense_kernel<<<(unsigned)d.n, 128, chunks * sizeof(int), st>>>(
+      t.s1_off.as<int64_t>(), t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(),
+      t.s2_J.as<int32_t>(), t.s2_D64.as<double>(), d.n, d.np, hi, chunks, tile_rows,
+      with_digits ? d.d.as<unsigned short>() : nullptr, flags.as<uint8_t>(), wmax.as<int>());
+  PQ_CUDA_TRY(cudaGetLastError());
+  std::vector<uint8_t> f((size_t)rt * chunks);
+  int wm[4];
+  PQ_CUDA_TRY(cudaMemcpyAsync(f.data(), flags.ptr, f.size(), cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaMemcpyAsync(wm, wmax.ptr, sizeof(wm), cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  d.win = 2;
+  for (int l = 1; l < 4; l++)
+    if (wm[l] <= KMAX) d.win = 2 << l;
+  std::vector<int32_t> off(rt + 1, 0), list;
+  for (int64_t r = 0; r < rt; r++) {
+    for (int c = 0; c < chunks; c++)
+      if (f[(size_t)r * chunks + c]) list.push_back(c);
+    off[r + 1] = (int32_t)list.size();
+  }
+  if (list.empty()) list.push_back(0);
+  PQ_TRY(upload(d.kt_off, off, st));
+  PQ_TRY(upload(d.kt_list, list, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  return PQ_OK;
+}
+
+// Scatter lists per (pass, tile of 128 beta strings): targets in ascending order, each with its contributions (six to
+// an entry): the singles of the tile's strings by pair, and their occupied orbitals onto themselves.
+static pq_status s64_lists(pq_ci_handle *h, Sigma64 &S) {
+  using namespace s64;
+  const SpinTablesDev &t = h->tab[0][1];
+  cudaStream_t st = h->stream;
+  std::vector<int64_t> off(t.n_str + 1);
+  std::vector<int32_t> J(t.n1 + 1), info(t.n1 + 1);
+  PQ_CUDA_TRY(cudaMemcpyAsync(off.data(), t.s1_off.ptr, off.size() * 8, cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaMemcpyAsync(J.data(), t.s1_J.ptr, t.n1 * 4, cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaMemcpyAsync(info.data(), t.s1_info.ptr, t.n1 * 4, cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  const int tiles = (int)((t.n_str + BM - 1) / BM);
+  std::vector<std::vector<uint32_t>> items((size_t)S.npass * tiles);  // target << 16 | contribution
+  const std::vector<uint64_t> &str = h->str[0][1];
+  for (int64_t b = 0; b < t.n_str; b++) {
+    auto put = [&](int64_t target, int pair, int neg) {
+      const int p = pair / S.wq, q = pair - p * S.wq;
+      items[(size_t)p * tiles + b / BM].push_back((uint32_t)target << 16 | (uint32_t)neg << 13 | (uint32_t)(b % BM) << 6 |
+                                                  (uint32_t)q);
+    };
+    for (int64_t s = off[b]; s < off[b + 1]; s++) put(J[s], info[s] >> 1, info[s] & 1);
+    for (uint64_t m = str[b]; m; m &= m - 1) {
+      const int k = __builtin_ctzll(m);
+      put(b, k * (k + 3) / 2, 0);
+    }
+  }
+  std::vector<int32_t> toff(items.size() + 1, 0);
+  std::vector<int4> ent;
+  for (size_t i = 0; i < items.size(); i++) {
+    std::vector<uint32_t> &v = items[i];
+    std::sort(v.begin(), v.end());
+    for (size_t u = 0; u < v.size();) {
+      const uint32_t target = v[u] >> 16;
+      uint32_t c[6] = {0, 0, 0, 0, 0, 0};
+      int n = 0;
+      while (u < v.size() && v[u] >> 16 == target && n < 6) c[n++] = v[u++] & 0xffffu;
+      ent.push_back(make_int4((int)(target | (uint32_t)n << 16), (int)(c[0] | c[1] << 16), (int)(c[2] | c[3] << 16),
+                              (int)(c[4] | c[5] << 16)));
+    }
+    if (ent.size() > (size_t)INT32_MAX / 2) {
+      set_error("FP64 full-CI sigma: scatter lists too large");
+      return PQ_ERR_ARG;
+    }
+    toff[i + 1] = (int32_t)ent.size();
+  }
+  if (ent.empty()) ent.push_back(make_int4(0, 0, 0, 0));
+  PQ_TRY(upload(S.toff, toff, st));
+  PQ_TRY(upload(S.tent, ent, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  return PQ_OK;
+}
+
+static pq_status s64_prepare(pq_ci_handle *h) {
+  using namespace s64;
+  if (h->s64) return PQ_OK;
+  std::unique_ptr<Sigma64, void (*)(Sigma64 *)> S(new (std::nothrow) Sigma64(), sigma64_delete);
+  if (!S) {
+    set_error("host allocation failed");
+    return PQ_ERR_OOM;
+  }
+  cudaStream_t st = h->stream;
+  const pq_ci_desc &d = h->desc;
+  const SpinTablesDev &a = h->tab[0][0];
+  const int npair = h->npair[0];
+  PQ_TRY(S->hi.alloc(16));
+  PQ_CUDA_TRY(cudaMemsetAsync(S->hi.ptr, 0, 16, st));
+  // identical spin lists with identical integrals share the matrix
+  S->shared = !h->selected && h->n_blocks[0] == 1 && d.n_alpha[0] == d.n_beta[0] && d.ex_level[0][0] == d.ex_level[0][1];
+  PQ_TRY(s64_side(h, *S, 0, true));
+  PQ_TRY(s64_side(h, *S, 1, !S->shared));
+  S->npass = (npair + BN - 1) / BN;
+  S->wq = (npair + S->npass - 1) / S->npass;
+  const int ncol = S->npass * BN;
+  uint32_t *whi = S->hi.as<uint32_t>() + 2;
+  absmax_kernel<<<32, 256, 0, st>>>(h->d_eab64.as<double>(), (int64_t)npair * npair, whi);
+  PQ_TRY(S->w.alloc(2 * (size_t)dg::N * (2 * npair + 1) * ncol));
+  w_kernel<<<(unsigned)(((int64_t)(2 * npair + 1) * ncol + 255) / 256), 256, 0, st>>>(h->d_eab64.as<double>(), npair, S->wq,
+                                                                                    ncol, whi, S->w.as<unsigned short>());
+  S->kp = (int)up64(a.max1 + d.n_alpha[0], 16);
+  if (S->kp == 0) S->kp = 16;
+  PQ_TRY(S->klist.alloc(sizeof(int2) * (size_t)a.n_str * S->kp));
+  klist_kernel<<<(unsigned)((a.n_str + 127) / 128), 128, 0, st>>>(a.s1_off.as<int64_t>(), a.s1_J.as<int32_t>(),
+                                                                a.s1_info.as<int32_t>(), a.str.as<uint64_t>(), a.n_str, S->kp,
+                                                                npair, S->klist.as<int2>());
+  PQ_CUDA_TRY(cudaGetLastError());
+  PQ_TRY(s64_lists(h, *S));
+  PQ_TRY(S->aux.alloc(64));
+  int dev = 0;
+  PQ_CUDA_TRY(cudaGetDevice(&dev));
+  PQ_CUDA_TRY(cudaDeviceGetAttribute(&S->sms, cudaDevAttrMultiProcessorCount, dev));
+  PQ_CUDA_TRY(cudaFuncSetAttribute(ab64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AB_SMEM));
+  PQ_CUDA_TRY(cudaFuncSetAttribute(ss64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM));
+  PQ_CUDA_TRY(cudaFuncSetAttribute(ss64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM));
+  h->s64 = std::move(S);
+  return PQ_OK;
+}
+
+// S[:, 0:nv] = H C[:, 0:nv] for nv <= 4 columns of device memory; C and S must not overlap
+pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds) {
+  using namespace s64;
+  PQ_TRY(s64_prepare(h));
+  Sigma64 &z = *h->s64;
+  cudaStream_t st = h->stream;
+  const int64_t na = h->tab[0][0].n_str, nb = h->tab[0][1].n_str, n = h->n_dets, nbp = up64(nb, 64);
+  PQ_TRY(z.xd.ensure(2 * (size_t)dg::N * nv * na * nbp));
+  int *gate = z.aux.as<int>();
+  uint32_t *xhi = z.aux.as<uint32_t>() + 4, *hi = z.hi.as<uint32_t>();
+  PQ_CUDA_TRY(cudaMemsetAsync(z.aux.ptr, 0, 64, st));
+  x64_absmax_kernel<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 152 * 4), nv), 256, 0, st>>>(C, ldc, n, xhi);
+  // beta's exponent word is alpha's when they share the matrix (same entries)
+  x64_digits_kernel<<<dim3((unsigned)na, nv), 256, 0, st>>>(C, ldc, na, nb, nbp, nv, xhi, hi, h->tab[0][0].e_same64.as<double>(),
+                                                          h->tab[0][1].e_same64.as<double>(), z.xd.as<unsigned short>(), S,
+                                                          lds, gate);
+  PQ_CUDA_TRY(cudaGetLastError());
+  const Sigma64::Side &A = z.side[0], &B = z.side[1];
+  const DevBuf &db = z.shared ? A.d : B.d;
+  SsArgs g{};
+  g.na = na, g.nb = nb, g.nv = nv;
+  g.m_tiles = (int)((nb + BM - 1) / BM);
+  g.n_tiles = (int)((na + BN - 1) / BN);
+  g.tiles = (int64_t)nv * g.m_tiles * g.n_tiles;
+  g.xhi = xhi;
+  g.S = S, g.lds = lds, g.gate = gate;
+  const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, z.sms);
+  CUtensorMap ma, mb;
+  const int64_t xrows = (int64_t)dg::N * nv * na;
+  // alpha: strips of 64 beta strings of 32 rows Ja; rows of Ha
+  PQ_TRY(s64_map(&ma, z.xd.ptr, xrows, nb, nbp, 64, 32));
+  PQ_TRY(s64_map(&mb, A.d.ptr, dg::N * A.n, A.n, A.np, 32, BN));
+  g.win = A.win;
+  g.a_plane = (int64_t)nv * na, g.b_plane = A.n;
+  g.kt_off = A.kt_off.as<int32_t>(), g.kt_list = A.kt_list.as<int32_t>();
+  g.dhi = hi;
+  ss64_kernel<true><<<grid, THREADS, SS_SMEM, st>>>(ma, mb, g);
+  // beta: rows of Hb; rows (v, Ia) of C
+  PQ_TRY(s64_map(&ma, db.ptr, dg::N * B.n, B.n, B.np, 32, BM));
+  PQ_TRY(s64_map(&mb, z.xd.ptr, xrows, nb, nbp, 32, BN));
+  g.win = B.win;
+  g.a_plane = B.n, g.b_plane = (int64_t)nv * na;
+  g.kt_off = B.kt_off.as<int32_t>(), g.kt_list = B.kt_list.as<int32_t>();
+  g.dhi = z.shared ? hi : hi + 1;
+  ss64_kernel<false><<<grid, THREADS, SS_SMEM, st>>>(ma, mb, g);
+  PQ_CUDA_TRY(cudaGetLastError());
+  AbArgs x{};
+  const int ncol = z.npass * BN, wrows = 2 * h->npair[0] + 1;
+  PQ_TRY(s64_map(&ma, z.xd.ptr, xrows, nb, nbp, 64, 1));
+  PQ_TRY(s64_map(&mb, z.w.ptr, (int64_t)dg::N * wrows, ncol, ncol, 64, 1));
+  x.na = na, x.nb = nb, x.nv = nv;
+  x.npass = z.npass, x.wq = z.wq, x.kp = z.kp, x.wrows = wrows;
+  x.m_tiles = g.m_tiles;
+  // few items: one per root, so that the last round of CTAs is short
+  x.vsplit = na * z.npass < 8 * z.sms;
+  x.items = na * z.npass * (x.vsplit ? nv : 1);
+  x.klist = z.klist.as<int2>();
+  x.toff = z.toff.as<int32_t>();
+  x.tent = z.tent.as<int4>();
+  x.xhi = xhi, x.whi = hi + 2;
+  x.S = S, x.lds = lds, x.gate = gate;
+  ab64_kernel<<<(unsigned)std::min<int64_t>(x.items, z.sms), AB_THREADS, AB_SMEM, st>>>(ma, mb, x);
+  PQ_CUDA_TRY(cudaGetLastError());
+  for (int v = 0; v < nv; v++) PQ_TRY(ci_sigma_gated(h, C + (size_t)v * ldc, S + (size_t)v * lds, gate));
+  return PQ_OK;
+}
+
+}  // namespace pq

@@ -26,12 +26,12 @@ __device__ __forceinline__ int exponent_of(uint32_t hi) {
   return ex == 0x7ff ? BAD : ex - 1022;
 }
 
-// round(x 2^(62 - e)) for |x| < 2^e, by integer arithmetic (the FP64 pipe runs at 1/64 of the integer rate)
-__device__ __forceinline__ int64_t fixed_point(double x, int e) {
+// round(x 2^(BITS - e)) for |x| < 2^e, by integer arithmetic (the FP64 pipe runs at 1/64 of the integer rate)
+template <int BITS = 62> __device__ __forceinline__ int64_t fixed_point(double x, int e) {
   const uint64_t b = (uint64_t)__double_as_longlong(x);
   const int ex = (int)((b >> 52) & 0x7ff);
   const uint64_t mant = (b & 0xfffffffffffffULL) | (ex ? 1ULL << 52 : 0ULL);
-  const int sh = (ex ? ex : 1) - e - 1013;  // <= 9
+  const int sh = (ex ? ex : 1) - e - 1075 + BITS;  // <= BITS - 53
   uint64_t t;
   if (sh >= 0)
     t = mant << sh;
@@ -94,4 +94,36 @@ __device__ __forceinline__ double to_double(int64_t hi, int64_t lo, int e) {
 }
 
 }  // namespace digits
+
+// The same with seven signed base-512 digits (|d_0| <= 128, the others <= 256, exact in FP16) and eight orders, 34
+// digit products, for sums of at most 80 products: t = round(x 2^(61 - e)) = sum_i d_i 512^(6 - i).  Orders 0 .. 3 stay
+// below 2^24 for 80 terms, a rounding of order l >= 4 is below 2^-55 of the largest possible sum; the products left
+// out are below 2^-67 of the two maxima each.
+namespace digits9 {
+
+constexpr int N = 7, ORDERS = 8, BITS = 61;
+
+// the seven digits of t as FP16 bits
+__device__ __forceinline__ void to_half(int64_t t, unsigned short (&d)[N]) {
+  uint64_t off = 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) off |= 256ULL << (9 * k);
+  const uint64_t u = (uint64_t)t + off;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    const unsigned f = (unsigned)(u >> (9 * (N - 1 - i))) & 511u;
+    d[i] = __half_as_ushort(__hsub(__ushort_as_half((unsigned short)(0x6400u | f)), __ushort_as_half((unsigned short)0x6500)));
+  }
+}
+
+// sum_l 512^(7 - l) a_l as hi 2^36 + lo; 512 a_0 + a_1 stays in 32 bits
+__device__ __forceinline__ void combine(const float (&a)[ORDERS], int64_t &hi, int64_t &lo) {
+  int v[ORDERS];
+#pragma unroll
+  for (int l = 0; l < ORDERS; l++) v[l] = __float2int_rn(a[l]);
+  hi = digits::mad_wide(v[0] * 512 + v[1], 1 << 18, digits::mad_wide(v[2], 512, v[3]));
+  lo = (digits::mad_wide(v[4], 512, v[5]) << 18) + digits::mad_wide(v[6], 512, v[7]);
+}
+
+}  // namespace digits9
 }  // namespace pq

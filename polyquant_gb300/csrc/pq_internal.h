@@ -79,6 +79,8 @@ struct SameSpinGemm;  // ci_sigma32_ss.cu
 void ss_delete(SameSpinGemm *g);
 struct SigmaRows;  // ci_sigma_rows.cu
 void rows_delete(SigmaRows *r);
+struct Sigma64;  // ci_sigma64.cu
+void sigma64_delete(Sigma64 *s);
 struct PairLists;  // ci_props.cu
 void pairs_delete(PairLists *p);
 
@@ -127,6 +129,9 @@ struct pq_ci_handle {
   std::unique_ptr<pq::SameSpinGemm, void (*)(pq::SameSpinGemm *)> ss{nullptr, pq::ss_delete};
   // FP64 sigma with a warp per determinant (ci_sigma_rows.cu); empty where ci_sigma.cu's kernel runs
   std::unique_ptr<pq::SigmaRows, void (*)(pq::SigmaRows *)> rows{nullptr, pq::rows_delete};
+  // FP64 full-CI sigma on the tensor cores (ci_sigma64.cu), its tables made by the first such call
+  bool fp64_tc = false;
+  std::unique_ptr<pq::Sigma64, void (*)(pq::Sigma64 *)> s64{nullptr, pq::sigma64_delete};
   // singles by orbital pair, made by the first property call of a one-species handle (ci_props.cu)
   std::unique_ptr<pq::PairLists, void (*)(pq::PairLists *)> pairs{nullptr, pq::pairs_delete};
   // two species: addressing of the product space (see ci_two.cu)
@@ -173,6 +178,15 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int pre
 // ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
 pq_status ci_sigma_rows_build(pq_ci_handle *h);
 pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
+// ci_sigma64.cu: S = H C for at most 4 columns of device memory that do not overlap (FP64, column-major)
+bool sigma64_applicable(const pq_ci_handle *h);
+pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds);
+size_t sigma64_bytes(const pq_ci_handle *h);
+// ci_sigma.cu: the element-by-element kernel on one column, if *gate is not zero when it runs
+pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, const int *gate);
+// FP64 sigma of a block of at most 4 columns in device memory, by the tensor cores where they apply (*done tells; the
+// explicit matrix, overlapping buffers and full device memory leave the block to the interleaved kernels)
+pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool *done);
 // ci_explicit.cu: sigma with the explicit matrix (FP64, interleaved vectors)
 pq_status ci_ham_spmv(pq_ci_handle *h, const void *X, void *Y, int nvp);
 // exact FP64 columns H[:, dets[c]] into column-major W (one species)
