@@ -312,6 +312,20 @@ pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32
     set_error("pq_ci_sigma_interleaved: NULL argument");
     return PQ_ERR_ARG;
   }
+  if (precision == PQ_FP64 && h->fp64_tc && (nvec == 1 || nvec == 2 || nvec == 4) && !(h->use_explicit && diag_shift == 0.0)) {
+    const double *x = (const double *)X;
+    double *y = (double *)Y;
+    const int64_t len = h->n_dets * nvec;
+    if (x + len <= y || y + len <= x) {
+      const pq_status s = ci_sigma64(h, x, nvec, 1, nvec, diag_shift, y, nvec, 1);
+      if (s != PQ_ERR_OOM) return s;
+      clear_error();
+    }
+  }
+  if (h->n_species == 1 && nvec == 3 && !(precision == PQ_FP64 && h->use_explicit && diag_shift == 0.0)) {
+    set_error("unsupported interleave width %d / precision %d (widths 1, 2, 4)", nvec, precision);
+    return PQ_ERR_ARG;
+  }
   return ci_sigma_il(h, X, Y, nvec, precision, diag_shift);
 }
 

@@ -357,8 +357,11 @@ static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift,
   return use_tab ? launch_sigma<T, NV, false, true, 0>(a, na, smem, st) : launch_sigma<T, NV, false, false, 0>(a, na, smem, st);
 }
 
-pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, const int *gate) {
-  return sigma_dispatch<double, 1>(h, C, S, 0.0, gate);
+pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate) {
+  if (nvp == 1) return sigma_dispatch<double, 1>(h, C, S, shift, gate);
+  if (nvp == 2) return sigma_dispatch<double, 2>(h, C, S, shift, gate);
+  if (nvp == 3) return sigma_dispatch<double, 3>(h, C, S, shift, gate);
+  return sigma_dispatch<double, 4>(h, C, S, shift, gate);
 }
 
 pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool *done) {
@@ -366,7 +369,7 @@ pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv
   if (!h->fp64_tc || h->use_explicit) return PQ_OK;
   const double *c1 = C + (size_t)(nv - 1) * ldc + h->n_dets, *s1 = S + (size_t)(nv - 1) * lds + h->n_dets;
   if (C < s1 && S < c1) return PQ_OK;
-  const pq_status s = ci_sigma64(h, C, ldc, nv, S, lds);
+  const pq_status s = ci_sigma64(h, C, 1, ldc, nv, 0.0, S, 1, lds);
   if (s == PQ_ERR_OOM) {
     cudaGetLastError();
     clear_error();

@@ -20,12 +20,19 @@
 // Errors.  A sum of digits leaves out less than 2^-64 of K max|C| max|W|.  D goes through shared memory as 64-bit
 // integers with one exponent per tile, 56 bits below the tile's largest entry, and sums of its entries are exact.  An
 // element-by-element FP64 sum rounds each of its terms at 2^-53 of the partial sum, which holds the diagonal (-147
-// C_I at 14 orbitals).  2-norm error against 64-bit references: see the numbers at the end of this comment.
+// C_I at 14 orbitals).
+// Against a 64-bit evaluation of the second-quantised form the 2-norm error is 7e-16 at 13 and 14 orbitals, where the
+// element kernel's is 2.4e-15 and 2.8e-15.
 //
 // Non-finite input (or integrals), and a bounded wait that runs out, raise a device flag; the element-by-element
 // kernel is launched behind with that flag as its condition and then computes the whole result, as before.
 //
-// Measured, four roots of FCI(14o, 7a7b): S64_NOW
+// Measured against the element-by-element kernel: four roots of FCI(14o, 7a7b) 50.1 / 345.6 ms (opposite spin 29, same
+// spin 2 x 10, digits 0.3), one root of FCI(13o, 6a5b) 1.86 / 17.0 ms, four roots of FCI(12o, 6a6b) 3.7 / 18.2,
+// FCI(11o, 5a5b) 0.95 / 2.33, FCI(10o, 5a5b) 0.21 / 0.61 ms.  Bound: the epilogue of the opposite-spin kernel, in clocks
+// per tile and pass of FCI(14o): MMAs 5.6 k, which overlap the sums of the entries (4.0 k), then the drain (4.6 k: the
+// integer arithmetic of eight orders), which cannot overlap MMAs because eight orders fill TMEM; the drain likewise in
+// ss64_kernel.  With one gather warp a tile took 17 k (75 clocks a row gather), with three 11 k.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -101,20 +108,21 @@ __device__ __forceinline__ void mma_step(uint32_t tmem, A &&adesc, B &&bdesc, ui
 
 // ---------------------------------------------------------------------------------------------- digits of C
 
-__global__ void __launch_bounds__(256) x64_absmax_kernel(const double *C, int64_t ldc, int64_t n, uint32_t *hi) {
-  const double *c = C + (int64_t)blockIdx.y * ldc;
+__global__ void __launch_bounds__(256) x64_absmax_kernel(const double *C, int64_t es, int64_t vs, int64_t n, uint32_t *hi) {
+  const double *c = C + (int64_t)blockIdx.y * vs;
   uint32_t m = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    m = max(m, (uint32_t)__double2hiint(c[i]) & 0x7fffffffu);
+    m = max(m, (uint32_t)__double2hiint(c[i * es]) & 0x7fffffffu);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) atomicMax(hi + blockIdx.y, m);
 }
 
-// planes [digit][v][Ia][nbp] of the nv columns of C and S = (E_alpha + E_beta) C; block per (alpha string, root)
-__global__ void __launch_bounds__(256) x64_digits_kernel(const double *C, int64_t ldc, int64_t na, int64_t nb, int64_t nbp,
+// planes [digit][v][Ia][nbp] of nv vectors and S = (E_alpha + E_beta - shift) C; block per (alpha string, root).
+// Vector v of determinant I lies at C[I es + v vs], of sigma at S[I ses + v svs].
+__global__ void __launch_bounds__(256) x64_digits_kernel(const double *C, int64_t es, int64_t vs, int64_t na, int64_t nb, int64_t nbp,
                                                         int nv, const uint32_t *xhi, const uint32_t *hi,
-                                                        const double *ea, const double *eb, unsigned short *xd, double *S,
-                                                        int64_t lds, int *gate) {
+                                                        const double *ea, const double *eb, double shift,
+                                                        unsigned short *xd, double *S, int64_t ses, int64_t svs, int *gate) {
   const int64_t ia = blockIdx.x;
   const int v = blockIdx.y;
   const int e = plane_exp(xhi + v);
@@ -122,20 +130,20 @@ __global__ void __launch_bounds__(256) x64_digits_kernel(const double *C, int64_
     if (threadIdx.x == 0) *gate = 1;
     return;
   }
-  const double *c = C + v * ldc + ia * nb;
-  double *s = S + v * lds + ia * nb;
-  const double da = ea[ia];
+  const double *c = C + v * vs + ia * nb * es;
+  double *s = S + v * svs + ia * nb * ses;
+  const double da = ea[ia] - shift;
   const int64_t plane = (int64_t)nv * na * nbp;
   unsigned short *row = xd + ((int64_t)v * na + ia) * nbp;
   for (int64_t b = 2 * threadIdx.x; b < nb; b += 2 * blockDim.x) {
-    const double x0 = c[b], x1 = b + 1 < nb ? c[b + 1] : 0.0;
+    const double x0 = c[b * es], x1 = b + 1 < nb ? c[(b + 1) * es] : 0.0;
     unsigned short d0[dg::N], d1[dg::N];
     dg::to_half(digits::fixed_point<dg::BITS>(x0, e), d0);
     dg::to_half(digits::fixed_point<dg::BITS>(x1, e), d1);
 #pragma unroll
     for (int i = 0; i < dg::N; i++) *reinterpret_cast<ushort2 *>(row + i * plane + b) = make_ushort2(d0[i], d1[i]);
-    s[b] = (da + eb[b]) * x0;
-    if (b + 1 < nb) s[b + 1] = (da + eb[b + 1]) * x1;
+    s[b * ses] = (da + eb[b]) * x0;
+    if (b + 1 < nb) s[(b + 1) * ses] = (da + eb[b + 1]) * x1;
   }
 }
 
@@ -148,8 +156,8 @@ constexpr int B_BYTES = dg::N * KMAX * 128;         // 70 KB: all digits of 64 p
 constexpr int LDS_D = BN + 1;                       // row length of the staged D
 constexpr int D_BYTES = BM * LDS_D * 8;             // 65 KB
 constexpr int AB_BARS = 2 * A_STAGES + 9;
-constexpr int GATHER_WARPS = 4;                     // warp 0 and the last three
-constexpr int AB_THREADS = THREADS + 32 * (GATHER_WARPS - 1);
+constexpr int GATHER_WARPS = 3;                     // warp 0 and the last two
+constexpr int AB_THREADS = 32 * (GATHER_WARPS + 1 + EPI_WARPS);
 constexpr int AB_SMEM = A_STAGES * A_STAGE + B_BYTES + D_BYTES + GATHER_WARPS * KMAX * 8 + AB_BARS * 8 + 64 + 1024;
 static_assert(AB_SMEM <= 232448, "shared memory per CTA");
 
@@ -163,7 +171,7 @@ struct AbArgs {
   const int4 *tent;
   const uint32_t *xhi, *whi;
   double *S;
-  int64_t lds;
+  int64_t es, vs;            // strides of sigma over determinants and roots
   int *gate;
 };
 
@@ -172,7 +180,11 @@ __device__ __forceinline__ double pow2_scale(int e) {
   return e > -1022 && e < 1023 ? __hiloint2double((e + 1023) << 20, 0) : scalbn(1.0, e);
 }
 
-// Roles: warp 0 gathers (its lanes share the row gathers of a stage), warp 1 lane 0 issues MMAs, warps 2 .. 17 drain
+constexpr int ZERO_SLOT = BN, ZERO2 = ZERO_SLOT | ZERO_SLOT << 16;  // D[0][64], which stays zero
+constexpr int NPRE = 3;  // list entries per epilogue thread loaded ahead of a tile
+
+// Roles: warp 0 and the last two gather (their lanes share the row gathers of a stage; one warp
+// issues a gather in about 75 clocks), warp 1 lane 0 issues MMAs, warps 2 .. 17 drain
 // and scatter.  Per tile the epilogue finds the largest |D| from the four leading orders, so that the tile's entries
 // become 57-bit integers; stages them; releases the accumulators; and sums the entries of each target.  Every wait is
 // an mbarrier wait with a budget; one that runs out raises the gate and the CTA winds down.
@@ -207,6 +219,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     mbar_init(smem_u32(d_empty), EPI_WARPS);
     mbar_init(smem_u32(drain), 1);
     tmax[0] = tmax[1] = 0;
+    sd[ZERO_SLOT] = 0;
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -338,15 +351,20 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
       item_of(it, ia, p, v0, v1);
       for (int v = v0; v < v1 && ok; v++) {
         const int ex = plane_exp(g.xhi + v);
-        double *srow = g.S + v * g.lds + ia * g.nb;
+        double *srow = g.S + v * g.vs + ia * g.nb * g.es;
         for (int t = 0; t < g.m_tiles; t++, seq++) {
           const int tl = p * g.m_tiles + t, k0 = __ldg(g.toff + tl), k1 = __ldg(g.toff + tl + 1);
+          // this thread's first list entries, on their way during the MMAs
+          const int4 NO_ENTRY = make_int4(0, ZERO2, ZERO2, ZERO2);
+          int4 pre[NPRE];
+#pragma unroll
+          for (int u = 0; u < NPRE; u++) pre[u] = k0 + te + u * EPI < k1 ? __ldg(g.tent + k0 + te + u * EPI) : NO_ENTRY;
           ok = wait_all(acc_full, seq);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           // largest |D|, in units of order 3
           float m = 0.0f;
-          for (int c0 = 8 * part; c0 < g.wq; c0 += 32) {
+          for (int c0 = 8 * part; c0 < g.wq; c0 += 2 * EPI_WARPS) {
             uint32_t a[4][8];
 #pragma unroll
             for (int l = 0; l < 4; l++) tmem_ld8(taddr + l * BN + c0, a[l]);
@@ -372,20 +390,42 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
           ok = wait_all(d_empty, seq ^ 1);  // the last tile's entries have been summed
           if (!ok) break;
           if (te == 0) tmax[(seq + 1) & 1] = 0;
-          for (int c0 = 8 * part; c0 < g.wq; c0 += 32) {
-            uint32_t a[dg::ORDERS][8];
+          // usual case: hi 2^(36 - sh) + (lo >> sh) by multiply-adds, and the constants taken off once
+          const bool usual = sh >= 5 && sh <= 36;
+          const uint32_t up = usual ? 1u << (36 - sh) : 0u;
+          const uint64_t off = usual ? dg::HI * up + (dg::LO >> sh) : 0;
+          auto group = [&](const uint32_t (&a)[dg::ORDERS][4], int c0) {
+            float far = usual ? 0.0f : dg::FAR;
+            uint64_t d[4];
 #pragma unroll
-            for (int l = 0; l < dg::ORDERS; l++) tmem_ld8(taddr + l * BN + c0, a[l]);
-            tmem_wait();
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
+            for (int c = 0; c < 4; c++) {
               float f[dg::ORDERS];
 #pragma unroll
               for (int l = 0; l < dg::ORDERS; l++) f[l] = __uint_as_float(a[l][c]);
-              int64_t hi, lo;
-              dg::combine(f, hi, lo);
-              drow[c0 + c] = (sh <= 36 ? hi << (36 - sh) : hi >> (sh - 36)) + (lo >> sh);
+              uint64_t hi, lo;
+              dg::combine_small(f, hi, lo, far);
+              d[c] = hi * up + (lo >> sh) - off;
             }
+            if (__any_sync(0xffffffffu, far >= dg::FAR)) {
+#pragma unroll
+              for (int c = 0; c < 4; c++) {
+                float f[dg::ORDERS];
+#pragma unroll
+                for (int l = 0; l < dg::ORDERS; l++) f[l] = __uint_as_float(a[l][c]);
+                int64_t hi, lo;
+                dg::combine(f, hi, lo);
+                d[c] = (uint64_t)((sh <= 36 ? hi << (36 - sh) : hi >> (sh - 36)) + (lo >> sh));
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) drow[c0 + c] = (int64_t)d[c];
+          };
+          for (int c0 = 4 * part; c0 < g.wq; c0 += EPI_WARPS) {
+            uint32_t a[dg::ORDERS][4];
+#pragma unroll
+            for (int l = 0; l < dg::ORDERS; l++) tmem_ld4(taddr + l * BN + c0, a[l]);
+            tmem_wait();
+            group(a, c0);
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
@@ -395,27 +435,38 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
           }
           ok = wait_all(d_full, seq);
           if (!ok) break;
-          const double scale = pow2_scale(ex + ew - 77 + sh);
-          for (int kb = k0 + te; kb < k1; kb += 2 * EPI) {
-            int4 ent[2];
-            ent[0] = __ldg(g.tent + kb);
-            ent[1] = kb + EPI < k1 ? __ldg(g.tent + kb + EPI) : make_int4(0, 0, 0, 0);
+          const int e = ex + ew - 77 + sh;
+          // integers below 2^60: where 2^e of them stays normal the exponent is added, else multiplied in
+          const bool plain = e > -1020 && e < 960;
+          auto total = [&](const int4 &ent) {
+            const int most = __reduce_max_sync(0xffffffffu, ent.x >> 16);  // lists run by falling count
+            const uint32_t w3[3] = {(uint32_t)ent.y, (uint32_t)ent.z, (uint32_t)ent.w};
+            // entries are sign << 15 | place in D; those past the count are ZERO_SLOT.  -x is (x ^ -1) + 1
+            int64_t sum = __popc(w3[0] & 0x80008000u) + __popc(w3[1] & 0x80008000u) + __popc(w3[2] & 0x80008000u);
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-              const int n = ent[u].x >> 16;
-              if (n == 0) continue;
-              const uint32_t w3[3] = {(uint32_t)ent[u].y, (uint32_t)ent[u].z, (uint32_t)ent[u].w};
-              int64_t sum = 0;
+            for (int i = 0; i < 6; i++)
+              if (i < most) {
+                const uint32_t w = w3[i >> 1];
+                const int64_t x = sd[(i & 1) ? (w >> 16) & 0x7fffu : w & 0x7fffu];
+                const int s = (i & 1) ? (int)w >> 31 : (int)(w << 16) >> 31;
+                sum += x ^ (int64_t)s;
+              }
+            return sum;
+          };
+          auto add = [&](int target, int64_t sum) {
+            if (target < 65536 || sum == 0) return;  // no entry here, or nothing to add
+            const double d = (double)sum;
+            atomicAdd(srow + (int64_t)(target & 0xffff) * g.es,
+                      plain ? __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d)) : d * pow2_scale(e));
+          };
+          int64_t sums[NPRE];
 #pragma unroll
-              for (int i = 0; i < 6; i++)
-                if (i < n) {
-                  // phase << 13 | beta string << 6 | pair
-                  const uint32_t en = (w3[i >> 1] >> (16 * (i & 1))) & 0xffffu;
-                  const int64_t x = sd[((en >> 6) & 127u) * LDS_D + (en & 63u)];
-                  sum += (en & 8192u) ? -x : x;
-                }
-              atomicAdd(srow + (ent[u].x & 0xffff), (double)sum * scale);
-            }
+          for (int u = 0; u < NPRE; u++) sums[u] = total(pre[u]);
+#pragma unroll
+          for (int u = 0; u < NPRE; u++) add(pre[u].x, sums[u]);
+          for (int kb = k0 + NPRE * EPI; kb < k1; kb += EPI) {  // the same rounds for every lane
+            const int4 ent = kb + te < k1 ? __ldg(g.tent + kb + te) : NO_ENTRY;
+            add(ent.x, total(ent));
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(d_empty));
@@ -446,7 +497,7 @@ struct SsArgs {
   const int32_t *kt_off, *kt_list;
   const uint32_t *xhi, *dhi;
   double *S;
-  int64_t lds;
+  int64_t es, vs;
   int *gate;
 };
 
@@ -626,7 +677,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int c = 0; c < 16; c++) {
           const int64_t ia = (int64_t)nt * BN + 16 * part + c;
           if (ia < g.na) {
-            double *y = g.S + v * g.lds + ia * g.nb + ib;
+            double *y = g.S + v * g.vs + (ia * g.nb + ib) * g.es;
             *y += digits::to_double(sh[c], (int64_t)sl[c], e);
           }
         }
@@ -821,8 +872,7 @@ static pq_status s64_side(pq_ci_handle *h, Sigma64 &S, int sp, bool with_digits)
   return PQ_OK;
 }
 
-// Scatter lists per (pass, tile of 128 beta strings): targets in ascending order, each with its contributions (six to
-// an entry): the singles of the tile's strings by pair, and their occupied orbitals onto themselves.
+// Scatter lists per (pass, tile of 128 beta strings): targets, each with its contributions (six to an entry): the singles of the tile's strings by pair, and their occupied orbitals onto themselves.
 static pq_status s64_lists(pq_ci_handle *h, Sigma64 &S) {
   using namespace s64;
   const SpinTablesDev &t = h->tab[0][1];
@@ -839,8 +889,8 @@ static pq_status s64_lists(pq_ci_handle *h, Sigma64 &S) {
   for (int64_t b = 0; b < t.n_str; b++) {
     auto put = [&](int64_t target, int pair, int neg) {
       const int p = pair / S.wq, q = pair - p * S.wq;
-      items[(size_t)p * tiles + b / BM].push_back((uint32_t)target << 16 | (uint32_t)neg << 13 | (uint32_t)(b % BM) << 6 |
-                                                  (uint32_t)q);
+      items[(size_t)p * tiles + b / BM].push_back((uint32_t)target << 16 | (uint32_t)neg << 15 |
+                                                  (uint32_t)((b % BM) * LDS_D + q));
     };
     for (int64_t s = off[b]; s < off[b + 1]; s++) put(J[s], info[s] >> 1, info[s] & 1);
     for (uint64_t m = str[b]; m; m &= m - 1) {
@@ -855,12 +905,14 @@ static pq_status s64_lists(pq_ci_handle *h, Sigma64 &S) {
     std::sort(v.begin(), v.end());
     for (size_t u = 0; u < v.size();) {
       const uint32_t target = v[u] >> 16;
-      uint32_t c[6] = {0, 0, 0, 0, 0, 0};
+      uint32_t c[6] = {ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT};
       int n = 0;
       while (u < v.size() && v[u] >> 16 == target && n < 6) c[n++] = v[u++] & 0xffffu;
       ent.push_back(make_int4((int)(target | (uint32_t)n << 16), (int)(c[0] | c[1] << 16), (int)(c[2] | c[3] << 16),
                               (int)(c[4] | c[5] << 16)));
     }
+    // by falling count, so that a warp's entries take the same steps
+    std::stable_sort(ent.begin() + toff[i], ent.end(), [](const int4 &x, const int4 &y) { return (x.x >> 16) > (y.x >> 16); });
     if (ent.size() > (size_t)INT32_MAX / 2) {
       set_error("FP64 full-CI sigma: scatter lists too large");
       return PQ_ERR_ARG;
@@ -919,8 +971,10 @@ static pq_status s64_prepare(pq_ci_handle *h) {
   return PQ_OK;
 }
 
-// S[:, 0:nv] = H C[:, 0:nv] for nv <= 4 columns of device memory; C and S must not overlap
-pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds) {
+// S = (H - shift) C for nv <= 4 vectors of device memory, vector v of determinant I at C[I es + v vs] and
+// S[I ses + v svs]; C and S must not overlap, and are either columns (es = 1) or interleaved (es = nv, vs = 1)
+pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
+                     int64_t svs) {
   using namespace s64;
   PQ_TRY(s64_prepare(h));
   Sigma64 &z = *h->s64;
@@ -930,11 +984,11 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, doub
   int *gate = z.aux.as<int>();
   uint32_t *xhi = z.aux.as<uint32_t>() + 4, *hi = z.hi.as<uint32_t>();
   PQ_CUDA_TRY(cudaMemsetAsync(z.aux.ptr, 0, 64, st));
-  x64_absmax_kernel<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 152 * 4), nv), 256, 0, st>>>(C, ldc, n, xhi);
+  x64_absmax_kernel<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 152 * 4), nv), 256, 0, st>>>(C, es, vs, n, xhi);
   // beta's exponent word is alpha's when they share the matrix (same entries)
-  x64_digits_kernel<<<dim3((unsigned)na, nv), 256, 0, st>>>(C, ldc, na, nb, nbp, nv, xhi, hi, h->tab[0][0].e_same64.as<double>(),
-                                                          h->tab[0][1].e_same64.as<double>(), z.xd.as<unsigned short>(), S,
-                                                          lds, gate);
+  x64_digits_kernel<<<dim3((unsigned)na, nv), 256, 0, st>>>(C, es, vs, na, nb, nbp, nv, xhi, hi, h->tab[0][0].e_same64.as<double>(),
+                                                          h->tab[0][1].e_same64.as<double>(), shift,
+                                                          z.xd.as<unsigned short>(), S, ses, svs, gate);
   PQ_CUDA_TRY(cudaGetLastError());
   const Sigma64::Side &A = z.side[0], &B = z.side[1];
   const DevBuf &db = z.shared ? A.d : B.d;
@@ -944,7 +998,7 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, doub
   g.n_tiles = (int)((na + BN - 1) / BN);
   g.tiles = (int64_t)nv * g.m_tiles * g.n_tiles;
   g.xhi = xhi;
-  g.S = S, g.lds = lds, g.gate = gate;
+  g.S = S, g.es = ses, g.vs = svs, g.gate = gate;
   const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, z.sms);
   CUtensorMap ma, mb;
   const int64_t xrows = (int64_t)dg::N * nv * na;
@@ -979,11 +1033,14 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, doub
   x.toff = z.toff.as<int32_t>();
   x.tent = z.tent.as<int4>();
   x.xhi = xhi, x.whi = hi + 2;
-  x.S = S, x.lds = lds, x.gate = gate;
+  x.S = S, x.es = ses, x.vs = svs, x.gate = gate;
   ab64_kernel<<<(unsigned)std::min<int64_t>(x.items, z.sms), AB_THREADS, AB_SMEM, st>>>(ma, mb, x);
   PQ_CUDA_TRY(cudaGetLastError());
-  for (int v = 0; v < nv; v++) PQ_TRY(ci_sigma_gated(h, C + (size_t)v * ldc, S + (size_t)v * lds, gate));
-  return PQ_OK;
+  if (es == 1 && ses == 1) {
+    for (int v = 0; v < nv; v++) PQ_TRY(ci_sigma_gated(h, C + v * vs, S + v * svs, 1, shift, gate));
+    return PQ_OK;
+  }
+  return ci_sigma_gated(h, C, S, nv, shift, gate);
 }
 
 }  // namespace pq

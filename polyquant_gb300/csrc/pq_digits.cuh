@@ -125,5 +125,29 @@ __device__ __forceinline__ void combine(const float (&a)[ORDERS], int64_t &hi, i
   lo = (digits::mad_wide(v[4], 512, v[5]) << 18) + digits::mad_wide(v[6], 512, v[7]);
 }
 
+// The same for sums below 2^22 by multiply-adds alone: conversions run at an eighth and integer logic and adds at half
+// of their rate.  1.5 2^23 + a_l has a_l in its low bits, so hi and lo come with the constants HI and LO added.  `far`
+// collects squares: from 2^44 on some sum may have been too large.
+constexpr uint32_t MAGIC = 0x4b400000u;  // bits of 1.5 2^23
+constexpr uint64_t HI = (uint64_t)MAGIC * 513u, LO = (uint64_t)MAGIC * 513u * ((1u << 18) + 1u);
+constexpr float FAR = 17592186044416.0f;  // 2^44
+__device__ __forceinline__ void combine_small(const float (&a)[ORDERS], uint64_t &hi, uint64_t &lo, float &far) {
+  uint32_t v[ORDERS];
+#pragma unroll
+  for (int l = 0; l < ORDERS; l++) {
+    v[l] = __float_as_uint(a[l] + 12582912.0f);
+    far = fmaf(a[l], a[l], far);
+  }
+  auto wide = [](uint32_t x, uint32_t m, uint64_t y) {
+    uint64_t d;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(x), "r"(m), "l"(y));
+    return d;
+  };
+  const int top = (int)(v[0] * 512u + v[1] - MAGIC * 513u);
+  hi = (uint64_t)digits::mad_wide(top, 1 << 18, (int64_t)wide(v[2], 512u, v[3]));
+  const uint64_t x = wide(v[4], 512u, v[5]), y = wide((uint32_t)x, 1u << 18, wide(v[6], 512u, v[7]));
+  lo = y + ((uint64_t)((uint32_t)(x >> 32) << 18) << 32);
+}
+
 }  // namespace digits9
 }  // namespace pq

@@ -178,12 +178,14 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int pre
 // ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
 pq_status ci_sigma_rows_build(pq_ci_handle *h);
 pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
-// ci_sigma64.cu: S = H C for at most 4 columns of device memory that do not overlap (FP64, column-major)
+// ci_sigma64.cu: S = (H - shift) C for at most 4 vectors of device memory that do not overlap (FP64, strides over
+// determinants and vectors)
 bool sigma64_applicable(const pq_ci_handle *h);
-pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds);
+pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
+                     int64_t svs);
 size_t sigma64_bytes(const pq_ci_handle *h);
-// ci_sigma.cu: the element-by-element kernel on one column, if *gate is not zero when it runs
-pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, const int *gate);
+// ci_sigma.cu: the element-by-element kernel on interleaved vectors (nvp = 1: a column), if *gate is not zero when it runs
+pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate);
 // FP64 sigma of a block of at most 4 columns in device memory, by the tensor cores where they apply (*done tells; the
 // explicit matrix, overlapping buffers and full device memory leave the block to the interleaved kernels)
 pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool *done);

@@ -110,3 +110,26 @@ def test_overlapping_buffers(monkeypatch):
                                  _lib.PQ_FP64)
     torch.cuda.synchronize()
     assert st == _lib.PQ_OK and torch.equal(X.t(), want)
+
+
+def test_interleaved_vectors_and_shift(monkeypatch):
+    """The native-layout entry point: widths 1, 2, 4 with a diagonal shift; three interleaved vectors stay refused."""
+    from polyquant_gb300 import _lib
+
+    p = synthetic_fci(10, 5, 5, seed=95)
+    g, r = _pair(monkeypatch, p)
+    L = _lib.load()
+    for k in (1, 2, 3, 4):
+        X = torch.randn(g.N_dets, k, device="cuda", dtype=torch.float64)
+        out = []
+        for h in (g, r):
+            Y = torch.empty_like(X)
+            st = L.pq_ci_sigma_interleaved(h._h, ctypes.c_void_p(X.data_ptr()), ctypes.c_void_p(Y.data_ptr()), k, _lib.PQ_FP64,
+                                           ctypes.c_double(-3.25))
+            torch.cuda.synchronize()
+            assert st == (_lib.PQ_ERR_ARG if k == 3 else _lib.PQ_OK)
+            out.append(Y)
+        if k != 3:
+            assert ((out[0] - out[1]).abs().amax(0) <= TOL * out[1].abs().amax(0)).all()
+            want = r.sigma(X) + 3.25 * X
+            assert ((out[0] - want).abs().amax(0) <= TOL * want.abs().amax(0)).all()
