@@ -215,7 +215,7 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
     if (precision == PQ_FP64 && h->fp64_tc && !h->use_explicit) {
       bool done = false;
       if (on_device) {
-        PQ_TRY(ci_sigma64_block(h, C + (size_t)v0 * ldc, ldc, nv, S + (size_t)v0 * lds, lds, &done));
+        PQ_TRY(ci_sigma64_block(h, C + (size_t)v0 * ldc, ldc, nv, S + (size_t)v0 * lds, lds, false, 0.0, &done));
       } else {
         // page-locked host columns pass through device columns, copied by the conversion kernels
         const size_t n = (size_t)h->n_dets, block = sizeof(double) * nv * (n + 1);
@@ -223,7 +223,7 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
         PQ_TRY(h->y_il.ensure(block));
         double *x = h->x_il.as<double>(), *y = h->y_il.as<double>();
         for (int v = 0; v < nv; v++) PQ_TRY(ci_to_il(h, C, ldc, v0 + v, 1, 1, PQ_FP64, x + v * n));
-        PQ_TRY(ci_sigma64_block(h, x, n, nv, y, n, &done));
+        PQ_TRY(ci_sigma64_block(h, x, n, nv, y, n, false, 0.0, &done));
         for (int v = 0; v < nv && done; v++) PQ_TRY(ci_from_il(h, y + v * n, v0 + v, 1, 1, PQ_FP64, S, lds));
       }
       if (done) continue;
@@ -312,15 +312,10 @@ pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32
     set_error("pq_ci_sigma_interleaved: NULL argument");
     return PQ_ERR_ARG;
   }
-  if (precision == PQ_FP64 && h->fp64_tc && (nvec == 1 || nvec == 2 || nvec == 4) && !(h->use_explicit && diag_shift == 0.0)) {
-    const double *x = (const double *)X;
-    double *y = (double *)Y;
-    const int64_t len = h->n_dets * nvec;
-    if (x + len <= y || y + len <= x) {
-      const pq_status s = ci_sigma64(h, x, nvec, 1, nvec, diag_shift, y, nvec, 1);
-      if (s != PQ_ERR_OOM) return s;
-      clear_error();
-    }
+  if (precision == PQ_FP64 && (nvec == 1 || nvec == 2 || nvec == 4 || (nvec == 3 && h->n_species == 2))) {
+    bool done = false;
+    PQ_TRY(ci_sigma64_block(h, (const double *)X, 0, nvec, (double *)Y, 0, true, diag_shift, &done));
+    if (done) return PQ_OK;
   }
   if (h->n_species == 1 && nvec == 3 && !(precision == PQ_FP64 && h->use_explicit && diag_shift == 0.0)) {
     set_error("unsupported interleave width %d / precision %d (widths 1, 2, 4)", nvec, precision);
@@ -335,7 +330,8 @@ pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes) {
     return PQ_ERR_ARG;
   }
   *bytes = (int64_t)(h->x_il.bytes + h->y_il.bytes + h->x_t.bytes + h->z_t.bytes + h->tc_btab.bytes + h->tc_aux.bytes +
-                     h->tc_toff.bytes + h->tc_tinfo.bytes + h->host_c.bytes + h->host_s.bytes + ci_sigma32_ss_bytes(h) + sigma64_bytes(h));
+                     h->tc_toff.bytes + h->tc_tinfo.bytes + h->host_c.bytes + h->host_s.bytes + ci_sigma32_ss_bytes(h) + sigma64_bytes(h) +
+                     two64_bytes(h));
   return PQ_OK;
 }
 

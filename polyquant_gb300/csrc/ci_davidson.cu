@@ -703,7 +703,7 @@ pq_status sigma_request_single(pq_ci_handle *h, const SigmaRequest &r) {
     const int c = std::min(4, r.cnt - v0), nvp = il_width(h, c, r.precision);
     if (r.precision == PQ_FP64) {
       bool done = false;
-      PQ_TRY(ci_sigma64_block(h, r.src + (size_t)v0 * n, n, c, r.dst + (size_t)v0 * n, n, &done));
+      PQ_TRY(ci_sigma64_block(h, r.src + (size_t)v0 * n, n, c, r.dst + (size_t)v0 * n, n, false, 0.0, &done));
       if (done) continue;
     }
     const size_t esz = r.precision == PQ_FP64 ? sizeof(double) : sizeof(float);

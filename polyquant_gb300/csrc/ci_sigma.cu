@@ -357,26 +357,38 @@ static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift,
   return use_tab ? launch_sigma<T, NV, false, true, 0>(a, na, smem, st) : launch_sigma<T, NV, false, false, 0>(a, na, smem, st);
 }
 
-pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate) {
+// the element-by-element kernel on interleaved vectors (nvp = 1: a column), if *gate is not zero when it runs
+static pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate) {
+  if (h->n_species == 2) return ci_two_gated(h, C, S, nvp, shift, gate);
   if (nvp == 1) return sigma_dispatch<double, 1>(h, C, S, shift, gate);
   if (nvp == 2) return sigma_dispatch<double, 2>(h, C, S, shift, gate);
   if (nvp == 3) return sigma_dispatch<double, 3>(h, C, S, shift, gate);
   return sigma_dispatch<double, 4>(h, C, S, shift, gate);
 }
 
-pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool *done) {
+pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool interleaved,
+                           double shift, bool *done) {
   *done = false;
-  if (!h->fp64_tc || h->use_explicit) return PQ_OK;
-  const double *c1 = C + (size_t)(nv - 1) * ldc + h->n_dets, *s1 = S + (size_t)(nv - 1) * lds + h->n_dets;
+  if (!h->fp64_tc || (h->use_explicit && shift == 0.0)) return PQ_OK;
+  const int64_t n = h->n_dets;
+  const double *c1 = C + (interleaved ? n * nv : (nv - 1) * ldc + n), *s1 = S + (interleaved ? n * nv : (nv - 1) * lds + n);
   if (C < s1 && S < c1) return PQ_OK;
-  const pq_status s = ci_sigma64(h, C, 1, ldc, nv, 0.0, S, 1, lds);
+  int *gate = nullptr;
+  const auto run = h->n_species == 2 ? ci_two64 : ci_sigma64;
+  const pq_status s = interleaved ? run(h, C, nv, 1, nv, shift, S, nv, 1, &gate) : run(h, C, 1, ldc, nv, shift, S, 1, lds, &gate);
   if (s == PQ_ERR_OOM) {
     cudaGetLastError();
     clear_error();
     return PQ_OK;
   }
-  *done = s == PQ_OK;
-  return s;
+  PQ_TRY(s);
+  if (interleaved) {
+    PQ_TRY(ci_sigma_gated(h, C, S, nv, shift, gate));
+  } else {
+    for (int v = 0; v < nv; v++) PQ_TRY(ci_sigma_gated(h, C + v * ldc, S + v * lds, 1, shift, gate));
+  }
+  *done = true;
+  return PQ_OK;
 }
 
 pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvp, int precision, double shift,

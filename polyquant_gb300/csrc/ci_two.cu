@@ -17,12 +17,14 @@
 //   det(ea, eb, pa, pb) = ebase[ie] + prowoff[L][pa] + pb  (pb < prowlen[L][pa]).
 // This reproduces the reference's sequential numbering of the nested loops.
 //
-// Kernel: one CTA per species-0 pair, threads over the determinants of its
-// block; each thread gathers H_IJ C_J over every connection class of the
+// Small full products in FP64 run as pair matrices on the tensor cores (ci_two64.cu).
+//
+// Kernel: a thread per determinant over the flat list; each thread gathers H_IJ C_J over every connection class of the
 // reference's singleshot builder (singles of each of the four spin lists with
 // their same-species and cross-species Coulomb terms, same-spin doubles,
 // alpha-beta doubles within a species, single x single cross doubles).
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "pq_bits.cuh"
@@ -215,7 +217,9 @@ __device__ __forceinline__ void two_conn_visit(const Args2<T> &p, const int (&t)
 // which the CTA's first determinant lies (a few steps forward through the sorted block bases).
 // WIDE: strings of more than 64 orbitals (two words); one-word spaces keep the hi words at compile-time zero.
 template <typename T, int NV, bool FULL, bool WIDE>
-__global__ void __launch_bounds__(128) sigma_two_species_kernel(Args2<T> p, int64_t n_dets, const int32_t *ie_first) {
+__global__ void __launch_bounds__(128) sigma_two_species_kernel(Args2<T> p, int64_t n_dets, const int32_t *ie_first,
+                                                                const int *gate) {
+  if (gate && *gate == 0) return;  // only behind the tensor-core path, for what that refused
   const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (I >= n_dets) return;
   int t[4];
@@ -525,6 +529,7 @@ pq_status ci_build2(pq_ci_handle *h) {
     for (int64_t ie = 0; full && ie < ne; ie++) full = h->elev[ie] >= 0 && h->psize[h->elev[ie]] == n1;
     h->full2 = full && nd == ne * n1;
   }
+  h->fp64_tc = two64_applicable(h) && getenv("PQ_SIGMA64_GATHER") == nullptr;
   PQ_TRY(upload(h->d_rowoff, rowoff32, st));
   PQ_TRY(upload(h->d_rowlen, h->rowlen, st));
   PQ_TRY(upload(h->d_e_a, h->e_a, st));
@@ -549,7 +554,7 @@ pq_status ci_build2(pq_ci_handle *h) {
 }
 
 template <typename T, int NV>
-static pq_status launch2(pq_ci_handle *h, const void *X, void *Y, double shift) {
+static pq_status launch2(pq_ci_handle *h, const void *X, void *Y, double shift, const int *gate = nullptr) {
   Args2<T> a = make_args<T>(h);
   a.shift = shift;
   a.X = (const T *)X;
@@ -557,13 +562,20 @@ static pq_status launch2(pq_ci_handle *h, const void *X, void *Y, double shift) 
   const unsigned grid = (unsigned)((h->n_dets + 127) / 128);
   // wide strings take the searched addressing, which holds for full products too
   if (h->wide)
-    sigma_two_species_kernel<T, NV, false, true><<<grid, 128, 0, h->stream>>>(a, h->n_dets, h->d_ie_first.as<int32_t>());
+    sigma_two_species_kernel<T, NV, false, true><<<grid, 128, 0, h->stream>>>(a, h->n_dets, h->d_ie_first.as<int32_t>(), gate);
   else if (h->full2)
-    sigma_two_species_kernel<T, NV, true, false><<<grid, 128, 0, h->stream>>>(a, h->n_dets, nullptr);
+    sigma_two_species_kernel<T, NV, true, false><<<grid, 128, 0, h->stream>>>(a, h->n_dets, nullptr, gate);
   else
-    sigma_two_species_kernel<T, NV, false, false><<<grid, 128, 0, h->stream>>>(a, h->n_dets, h->d_ie_first.as<int32_t>());
+    sigma_two_species_kernel<T, NV, false, false><<<grid, 128, 0, h->stream>>>(a, h->n_dets, h->d_ie_first.as<int32_t>(), gate);
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
+}
+
+pq_status ci_two_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate) {
+  if (nvp == 1) return launch2<double, 1>(h, C, S, shift, gate);
+  if (nvp == 2) return launch2<double, 2>(h, C, S, shift, gate);
+  if (nvp == 3) return launch2<double, 3>(h, C, S, shift, gate);
+  return launch2<double, 4>(h, C, S, shift, gate);
 }
 
 pq_status ci_sigma2_il(pq_ci_handle *h, const void *X, void *Y, int nvp, int precision, double shift) {

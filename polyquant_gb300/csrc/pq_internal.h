@@ -81,6 +81,8 @@ struct SigmaRows;  // ci_sigma_rows.cu
 void rows_delete(SigmaRows *r);
 struct Sigma64;  // ci_sigma64.cu
 void sigma64_delete(Sigma64 *s);
+struct Two64;  // ci_two64.cu
+void two64_delete(Two64 *t);
 struct PairLists;  // ci_props.cu
 void pairs_delete(PairLists *p);
 
@@ -129,8 +131,10 @@ struct pq_ci_handle {
   std::unique_ptr<pq::SameSpinGemm, void (*)(pq::SameSpinGemm *)> ss{nullptr, pq::ss_delete};
   // FP64 sigma with a warp per determinant (ci_sigma_rows.cu); empty where ci_sigma.cu's kernel runs
   std::unique_ptr<pq::SigmaRows, void (*)(pq::SigmaRows *)> rows{nullptr, pq::rows_delete};
-  // FP64 full-CI sigma on the tensor cores (ci_sigma64.cu), its tables made by the first such call
+  // FP64 sigma on the tensor cores (full CI of one species: ci_sigma64.cu, small two-species products: ci_two64.cu),
+  // its tables made by the first such call
   bool fp64_tc = false;
+  std::unique_ptr<pq::Two64, void (*)(pq::Two64 *)> two64{nullptr, pq::two64_delete};
   std::unique_ptr<pq::Sigma64, void (*)(pq::Sigma64 *)> s64{nullptr, pq::sigma64_delete};
   // singles by orbital pair, made by the first property call of a one-species handle (ci_props.cu)
   std::unique_ptr<pq::PairLists, void (*)(pq::PairLists *)> pairs{nullptr, pq::pairs_delete};
@@ -178,17 +182,24 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int pre
 // ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
 pq_status ci_sigma_rows_build(pq_ci_handle *h);
 pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
-// ci_sigma64.cu: S = (H - shift) C for at most 4 vectors of device memory that do not overlap (FP64, strides over
-// determinants and vectors)
+// ci_sigma64.cu, ci_two64.cu: S = (H - shift) C for at most 4 vectors of device memory that do not overlap (FP64,
+// strides over determinants and vectors).  A raised *gate afterwards means that nothing of it counts.
 bool sigma64_applicable(const pq_ci_handle *h);
+bool two64_applicable(const pq_ci_handle *h);
 pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
-                     int64_t svs);
+                     int64_t svs, int **gate);
+pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
+                   int64_t svs, int **gate);
 size_t sigma64_bytes(const pq_ci_handle *h);
-// ci_sigma.cu: the element-by-element kernel on interleaved vectors (nvp = 1: a column), if *gate is not zero when it runs
-pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate);
-// FP64 sigma of a block of at most 4 columns in device memory, by the tensor cores where they apply (*done tells; the
-// explicit matrix, overlapping buffers and full device memory leave the block to the interleaved kernels)
-pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool *done);
+size_t two64_bytes(const pq_ci_handle *h);
+// the element kernels of ci_two.cu on interleaved vectors (nvp = 1: a column), if *gate is not zero when they run
+pq_status ci_two_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate);
+// ci_sigma.cu: (H - shift) C of a block of at most 4 vectors in device memory, columns (interleaved = false, leading
+// dimensions ldc, lds) or interleaved, by the tensor cores where they apply, with the element kernels behind them for
+// what they refuse on the device.  *done tells; the explicit matrix, overlapping buffers and a full device leave the
+// block to the caller's other kernels.
+pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool interleaved,
+                           double shift, bool *done);
 // ci_explicit.cu: sigma with the explicit matrix (FP64, interleaved vectors)
 pq_status ci_ham_spmv(pq_ci_handle *h, const void *X, void *Y, int nvp);
 // exact FP64 columns H[:, dets[c]] into column-major W (one species)
