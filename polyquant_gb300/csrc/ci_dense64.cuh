@@ -56,7 +56,8 @@ struct SsArgs {
   int ksplit;                 // parts of the K list, each with its own copy of sigma, `part` values apart
   int64_t part;
   int64_t a_plane, b_plane;   // rows of one digit of either operand
-  const int32_t *kt_off, *kt_list;
+  const int32_t *kt_off, *kt_list;  // NULL: every tile has all the chunks
+  int chunks;
   const uint32_t *xhi, *dhi;
   double *S;
   int64_t es, vs;
@@ -112,18 +113,19 @@ __global__ void __launch_bounds__(THREADS, 1)
   // K list positions of a tile
   auto range_of = [&](int v, int mt, int nt, int &k0, int &k1) {
     const int rt = ALPHA ? nt : mt;
-    k0 = __ldg(g.kt_off + rt), k1 = __ldg(g.kt_off + rt + 1);
+    k0 = g.kt_list ? __ldg(g.kt_off + rt) : 0, k1 = g.kt_list ? __ldg(g.kt_off + rt + 1) : g.chunks;
     if (g.ksplit > 1) {
       const int n = k1 - k0;
       k1 = k0 + (int)((int64_t)n * (v + 1) / g.ksplit);
       k0 += (int)((int64_t)n * v / g.ksplit);
     }
   };
+  auto chunk_of = [&](int j) { return g.kt_list ? __ldg(g.kt_list + j) : j; };
   // end of the window that starts at list position j
   auto window_end = [&](int j, int k1) {
-    const int w = __ldg(g.kt_list + j) / g.win;
+    const int w = chunk_of(j) / g.win;
     int e = j + 1;
-    while (e < k1 && __ldg(g.kt_list + e) / g.win == w) e++;
+    while (e < k1 && chunk_of(e) / g.win == w) e++;
     return e;
   };
 
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((gs / SS_STAGES) & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
           if (!ok) break;
           const uint32_t a = smem_u32(smem + slot * SS_STAGE), b = a + dg::N * SS_A, bar = smem_u32(full + slot);
-          const int k = g.kt_list[j] * 32;
+          const int k = chunk_of(j) * 32;
           mbar_expect_tx(bar, SS_STAGE);
           for (int d = 0; d < dg::N; d++) {
             if (ALPHA) {

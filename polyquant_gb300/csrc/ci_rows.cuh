@@ -12,15 +12,17 @@ namespace pq {
 // Grouped tables of one spin list and the Coulomb sums of its strings.
 struct SigmaRows {
   struct Side {
-    DevBuf s1;    // int2 {partner (row offset for alpha, string for beta), info}, grouped by level change
-    DevBuf s1_F;  // same-spin part of the element
-    DevBuf s2, s2_D;
-    DevBuf cum;   // per string 8 x int32: ends of the 3 groups of singles and the 5 groups of doubles
-    DevBuf lvl;
-    DevBuf coul;  // [string][pair]: sum over the string's orbitals k of (pair of the other spin | kk); empty when large
+    int2 *s1 = nullptr;      // {partner (row offset for alpha, string for beta), info}, grouped by level change
+    double *s1_F = nullptr;  // same-spin part of the element
+    int32_t *s2 = nullptr;
+    double *s2_D = nullptr;
+    int32_t *cum = nullptr;  // per string 8: ends of the 3 groups of singles and the 5 groups of doubles
+    int32_t *lvl = nullptr;
+    double *coul = nullptr;  // [string][pair]: sum over the string's orbitals k of (pair of the other spin | kk); NULL when large
   };
   Side side[2];
-  DevBuf row;  // alpha string of every determinant
+  int32_t *row = nullptr;    // alpha string of every determinant
+  DevBuf mem;                // all of the above
   int lim = 0;
 };
 

@@ -14,11 +14,11 @@
 // over those planes for either spin.  ab64_kernel forms, per alpha string Ia and tile of 128 beta strings Jb,
 //   D[Jb][Q] = sum_{(Ja, P): e_P Ja = +-Ia} +-(P|Q) C(Ja, Jb)       K = singles and occupied orbitals of Ia
 // with both operands fetched by TMA row gathers (rows of C's planes by Ja, signed rows of the integral digits by P),
-// and adds the entries of D into sigma(Ia, Ib) along the lists of e_Q.  The gathered rows run along Jb and Q, so both
+// and adds the entries of D into sigma(Ia, Ib) along the lists of e_Q; a CTA owns the rows it adds to and their order.  The gathered rows run along Jb and Q, so both
 // operands are M- and N-major and nothing is converted or transposed on the way.
 //
 // Errors.  A sum of digits leaves out less than 2^-64 of K max|C| max|W|.  D goes through shared memory as 64-bit
-// integers with one exponent per tile, 56 bits below the tile's largest entry, and sums of its entries are exact.  An
+// integers with one exponent per tile, 55 bits below the tile's largest entry, and sums of its entries are exact.  An
 // element-by-element FP64 sum rounds each of its terms at 2^-53 of the partial sum, which holds the diagonal (-147
 // C_I at 14 orbitals).
 // Against a 64-bit evaluation of the second-quantised form the 2-norm error is 7e-16 at 13 and 14 orbitals, where the
@@ -27,9 +27,9 @@
 // Non-finite input (or integrals), and a bounded wait that runs out, raise a device flag; the element-by-element
 // kernel is launched behind with that flag as its condition and then computes the whole result, as before.
 //
-// Measured against the element-by-element kernel: four roots of FCI(14o, 7a7b) 50.1 / 345.6 ms (opposite spin 29, same
-// spin 2 x 10, digits 0.3), one root of FCI(13o, 6a5b) 1.86 / 17.0 ms, four roots of FCI(12o, 6a6b) 3.7 / 18.2,
-// FCI(11o, 5a5b) 0.95 / 2.33, FCI(10o, 5a5b) 0.21 / 0.61 ms.  Bound: the epilogue of the opposite-spin kernel, in clocks
+// Measured against the element-by-element kernel: four roots of FCI(14o, 7a7b) 51.1 / 345.6 ms (opposite spin 30, same
+// spin 2 x 10, digits 0.3), one root of FCI(13o, 6a5b) 1.93 / 17.0 ms, four roots of FCI(12o, 6a6b) 2.7 / 18.2,
+// FCI(11o, 5a5b) 0.68 / 2.33, FCI(10o, 5a5b) 0.20 / 0.61 ms.  Bound: the epilogue of the opposite-spin kernel, in clocks
 // per tile and pass of FCI(14o): MMAs 5.6 k, which overlap the sums of the entries (4.0 k), then the drain (4.6 k: the
 // integer arithmetic of eight orders), which cannot overlap MMAs because eight orders fill TMEM; the drain likewise in
 // ss64_kernel.  With one gather warp a tile took 17 k (75 clocks a row gather), with three 11 k.
@@ -47,25 +47,22 @@ namespace pq {
 
 struct Sigma64 {
   struct Side {
-    DevBuf d;                 // digits of the dense same-spin H: [digit][I][np]
-    int64_t n = 0, np = 0;    // strings, row length
-    DevBuf kt_off, kt_list;   // K chunks of 32 with an entry, per row tile (64 rows alpha, 128 rows beta)
-    int win = 2;              // chunks of a window that holds at most 80 entries of a row
+    unsigned short *d = nullptr;       // digits of the dense same-spin H: [digit][I][np]
+    int64_t n = 0, np = 0;             // strings, row length
+    int32_t *kt_off = nullptr, *kt_list = nullptr;  // K chunks of 32 with an entry, per row tile (64 rows alpha, 128 beta)
+    int win = 2;                       // chunks of a window that holds at most 80 entries of a row
   };
   Side side[2];
-  bool shared = false;        // beta uses alpha's matrix
-  DevBuf w;                   // digits of (P|Q): [digit][2 P + sign; a zero row last][pass x 64]
-  DevBuf klist;               // per alpha string kp x {row of C, row of w}
+  unsigned short *w = nullptr;         // digits of (P|Q): [digit][2 P + sign; a zero row last][pass x 64]
+  int2 *klist = nullptr;               // per alpha string kp x {row of C, row of w}
   int kp = 0, npass = 1, wq = 0;
-  DevBuf toff, tent;          // scatter lists per (pass, beta tile)
-  DevBuf hi;                  // high words of max|.|: same-spin H alpha, beta, integrals
-  DevBuf xd, aux;             // digits of C; gate and high word of max|C| per root
+  int32_t *toff = nullptr;             // scatter lists per (pass, beta tile)
+  int4 *tent = nullptr;
+  uint32_t *hi = nullptr;              // high words of max|.|: same-spin H alpha, beta, integrals
+  int *aux = nullptr;                  // gate; high words of max|C| per root from word 4 on
+  DevBuf mem, lists, xd;               // matrices and words; the chunk and scatter lists; digits of C
   int sms = 0;
-  size_t bytes() const {
-    size_t b = w.bytes + klist.bytes + toff.bytes + tent.bytes + hi.bytes + xd.bytes + aux.bytes;
-    for (const Side &s : side) b += s.d.bytes + s.kt_off.bytes + s.kt_list.bytes;
-    return b;
-  }
+  size_t bytes() const { return mem.bytes + lists.bytes + xd.bytes; }
 };
 void sigma64_delete(Sigma64 *s) { delete s; }
 
@@ -128,7 +125,7 @@ static_assert(AB_SMEM <= 232448, "shared memory per CTA");
 
 struct AbArgs {
   int64_t na, nb, items;
-  int nv, vsplit;            // vsplit: an item is one root of (alpha string, pass), else all of them
+  int nv, vsplit;            // vsplit: an item is one root of an alpha string, else all of them
   int npass, wq, kp, wrows;  // wrows: rows of one digit of w
   int m_tiles;
   const int2 *klist;
@@ -151,7 +148,7 @@ constexpr int NPRE = 3;  // list entries per epilogue thread loaded ahead of a t
 // Roles: warp 0 and the last two gather (their lanes share the row gathers of a stage; one warp
 // issues a gather in about 75 clocks), warp 1 lane 0 issues MMAs, warps 2 .. 17 drain
 // and scatter.  Per tile the epilogue finds the largest |D| from the four leading orders, so that the tile's entries
-// become 57-bit integers; stages them; releases the accumulators; and sums the entries of each target.  Every wait is
+// become 56-bit integers; stages them; releases the accumulators; and sums the entries of each target.  Every wait is
 // an mbarrier wait with a budget; one that runs out raises the gate and the CTA winds down.
 __global__ void __launch_bounds__(AB_THREADS, 1)
     ab64_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, AbArgs g) {
@@ -201,16 +198,19 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     *g.gate = ERR_WAIT;
     *abort_flag = 1;
   };
-  // item -> alpha string, pass, roots v0 .. v1 - 1
+  // (item, pass) -> alpha string, pass, roots v0 .. v1 - 1; a CTA runs the passes of an item one after the other, so
+  // that it alone adds to those rows of sigma, in a fixed order
   auto item_of = [&](int64_t it, int64_t &ia, int &p, int &v0, int &v1) {
+    p = (int)(it % g.npass);
+    it = blockIdx.x + (it / g.npass) * gridDim.x;
     v0 = 0, v1 = g.nv;
     if (g.vsplit) {
       v0 = (int)(it % g.nv), v1 = v0 + 1;
       it /= g.nv;
     }
-    ia = it / g.npass;
-    p = (int)(it - ia * g.npass);
+    ia = it;
   };
+  const int64_t mine = (int64_t)blockIdx.x < g.items ? ((g.items - 1 - blockIdx.x) / gridDim.x + 1) * g.npass : 0;
 
   if (warp == 0 || warp >= 2 + EPI_WARPS) {
     // ---- gather warps
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     int2 *kl = kl_all + pw * KMAX;  // this warp's copy of the item's K list
     int gs = 0, nit = 0;
     bool ok = true;
-    for (int64_t it = blockIdx.x; it < g.items && ok; it += gridDim.x, nit++) {
+    for (int64_t it = 0; it < mine && ok; it++, nit++) {
       int64_t ia;
       int p, v0, v1;
       item_of(it, ia, p, v0, v1);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     if (lane == 0) {
       int gs = 0, nit = 0, seq = 0;
       bool ok = true;
-      for (int64_t it = blockIdx.x; it < g.items && ok; it += gridDim.x, nit++) {
+      for (int64_t it = 0; it < mine && ok; it++, nit++) {
         int64_t ia;
         int p, v0, v1;
         item_of(it, ia, p, v0, v1);
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     int seq = 0;
     bool ok = true;
     const int ew = plane_exp(g.whi);
-    for (int64_t it = blockIdx.x; it < g.items && ok; it += gridDim.x) {
+    for (int64_t it = 0; it < mine && ok; it++) {
       int64_t ia;
       int p, v0, v1;
       item_of(it, ia, p, v0, v1);
@@ -349,9 +349,9 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
           }
           ok = wait_all(max_full, seq);
           if (!ok) break;
-          // |T| < (m (1 + 2^-20) + 2^17) 2^36 with the orders behind; the entries of T >> sh are below 2^56
+          // |T| < (m (1 + 2^-20) + 2^17) 2^36 with the orders behind; the entries of T >> sh are below 2^55
           const float mx = __uint_as_float(*(volatile uint32_t *)(tmax + (seq & 1))) * 1.00001f + 131072.0f;
-          const int sh = max(0, (int)(__float_as_uint(mx) >> 23) - 126 + 36 - 56);
+          const int sh = max(0, (int)(__float_as_uint(mx) >> 23) - 126 + 36 - 55);
           ok = wait_all(d_empty, seq ^ 1);  // the last tile's entries have been summed
           if (!ok) break;
           if (te == 0) tmax[(seq + 1) & 1] = 0;
@@ -401,10 +401,12 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
           ok = wait_all(d_full, seq);
           if (!ok) break;
           const int e = ex + ew - 77 + sh;
-          // integers below 2^60: where 2^e of them stays normal the exponent is added, else multiplied in
+          // integers below 2^63: where 2^e of them stays normal the exponent is added, else multiplied in
           const bool plain = e > -1020 && e < 960;
+          // the sum of an entry; a target with more than six contributions has its entries in neighbouring lanes, and
+          // the first one, at place 0 of the chain, gets their total
           auto total = [&](const int4 &ent) {
-            const int most = __reduce_max_sync(0xffffffffu, ent.x >> 16);  // lists run by falling count
+            const int most = __reduce_max_sync(0xffffffffu, (ent.x >> 16) & 7);  // lists run by falling count
             const uint32_t w3[3] = {(uint32_t)ent.y, (uint32_t)ent.z, (uint32_t)ent.w};
             // entries are sign << 15 | place in D; those past the count are ZERO_SLOT.  -x is (x ^ -1) + 1
             int64_t sum = __popc(w3[0] & 0x80008000u) + __popc(w3[1] & 0x80008000u) + __popc(w3[2] & 0x80008000u);
@@ -416,22 +418,33 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
                 const int s = (i & 1) ? (int)w >> 31 : (int)(w << 16) >> 31;
                 sum += x ^ (int64_t)s;
               }
-            return sum;
+            const int place = ent.x >> 19, longest = __reduce_max_sync(0xffffffffu, place);
+            int64_t all = sum;
+            for (int k = 1; k <= longest; k++) {
+              const int64_t x = __shfl_down_sync(0xffffffffu, sum, k);
+              const int q = __shfl_down_sync(0xffffffffu, place, k);
+              if (place == 0 && lane + k < 32 && q == k) all += x;
+            }
+            return all;
           };
-          auto add = [&](int target, int64_t sum) {
-            if (target < 65536 || sum == 0) return;  // no entry here, or nothing to add
+          auto value = [&](int64_t sum) {
             const double d = (double)sum;
-            atomicAdd(srow + (int64_t)(target & 0xffff) * g.es,
-                      plain ? __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d)) : d * pow2_scale(e));
+            return sum == 0 ? 0.0 : plain ? __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d)) : d * pow2_scale(e);
           };
-          int64_t sums[NPRE];
+          auto head = [](const int4 &ent) { return (ent.x >> 16) != 0 && (ent.x >> 19) == 0; };
+          // a target is one lane's in this tile, and tiles follow one another, so sigma is read and written plainly
+          double y[NPRE];
 #pragma unroll
-          for (int u = 0; u < NPRE; u++) sums[u] = total(pre[u]);
+          for (int u = 0; u < NPRE; u++) y[u] = head(pre[u]) ? srow[(int64_t)(pre[u].x & 0xffff) * g.es] : 0.0;
 #pragma unroll
-          for (int u = 0; u < NPRE; u++) add(pre[u].x, sums[u]);
+          for (int u = 0; u < NPRE; u++) {
+            const double x = value(total(pre[u]));
+            if (head(pre[u])) srow[(int64_t)(pre[u].x & 0xffff) * g.es] = y[u] + x;
+          }
           for (int kb = k0 + NPRE * EPI; kb < k1; kb += EPI) {  // the same rounds for every lane
             const int4 ent = kb + te < k1 ? __ldg(g.tent + kb + te) : NO_ENTRY;
-            add(ent.x, total(ent));
+            const double x = value(total(ent));
+            if (head(ent)) srow[(int64_t)(ent.x & 0xffff) * g.es] += x;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(d_empty));
@@ -535,72 +548,19 @@ bool sigma64_applicable(const pq_ci_handle *h) {
 
 size_t sigma64_bytes(const pq_ci_handle *h) { return h->s64 ? h->s64->bytes() : 0; }
 
-// Dense same-spin H of one spin list in the role of alpha (64-row tiles) or beta (128-row tiles).  digits = false only
-// makes the chunk lists (the matrix is the other side's).
-static pq_status s64_side(pq_ci_handle *h, Sigma64 &S, int sp, bool with_digits) {
+// Scatter lists per (pass, tile of 128 beta strings): targets, each with its contributions: the singles of the tile's
+// strings by pair, and their occupied orbitals onto themselves.  An entry is {target | count << 16 | place << 19, six
+// contributions}; a target takes as many neighbouring entries as it needs (at most 128 contributions of other
+// strings, one pair each, and its own occupied orbitals: 25 entries, and 2^7.2 terms below 2^55).
+static pq_status s64_lists(const pq_ci_handle *h, const Sigma64 &S, const std::vector<int64_t> &off,
+                           const std::vector<int32_t> &J, const std::vector<int32_t> &info, std::vector<int32_t> &toff,
+                           std::vector<int4> &ent) {
   using namespace s64;
-  const SpinTablesDev &t = h->tab[0][sp];
-  Sigma64::Side &d = S.side[sp];
-  cudaStream_t st = h->stream;
-  d.n = t.n_str;
-  d.np = up64(t.n_str, 64);
-  const int chunks = (int)((d.n + 31) / 32), tile_rows = sp == 0 ? BN : BM;
-  const int64_t rt = (d.n + tile_rows - 1) / tile_rows;
-  if (with_digits) {
-    const size_t bytes = 2 * (size_t)dg::N * d.n * d.np;
-    PQ_TRY(d.d.alloc(bytes));
-    PQ_CUDA_TRY(cudaMemsetAsync(d.d.ptr, 0, bytes, st));
-  }
-  DevBuf flags, wmax;
-  PQ_TRY(flags.alloc((size_t)rt * chunks));
-  PQ_TRY(wmax.alloc(4 * sizeof(int)));
-  PQ_CUDA_TRY(cudaMemsetAsync(flags.ptr, 0, (size_t)rt * chunks, st));
-  PQ_CUDA_TRY(cudaMemsetAsync(wmax.ptr, 0, 4 * sizeof(int), st));
-  uint32_t *hi = S.hi.as<uint32_t>() + sp;
-  const unsigned g1 = (unsigned)std::min<int64_t>((t.n1 + 255) / 256, 1216), g2 = (unsigned)std::min<int64_t>((t.n2 + 255) / 256, 1216);
-  if (t.n1) absmax_kernel<<<g1, 256, 0, st>>>(t.s1_F64.as<double>(), t.n1, hi);
-  if (t.n2) absmax_kernel<<<g2, 256, 0, st>>>(t.s2_D64.as<double>(), t.n2, hi);
-  dense_kernel<<<(unsigned)d.n, 128, chunks * sizeof(int), st>>>(
-      t.s1_off.as<int64_t>(), t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(),
-      t.s2_J.as<int32_t>(), t.s2_D64.as<double>(), d.n, d.np, hi, chunks, tile_rows,
-      with_digits ? d.d.as<unsigned short>() : nullptr, flags.as<uint8_t>(), wmax.as<int>());
-  PQ_CUDA_TRY(cudaGetLastError());
-  std::vector<uint8_t> f((size_t)rt * chunks);
-  int wm[4];
-  PQ_CUDA_TRY(cudaMemcpyAsync(f.data(), flags.ptr, f.size(), cudaMemcpyDeviceToHost, st));
-  PQ_CUDA_TRY(cudaMemcpyAsync(wm, wmax.ptr, sizeof(wm), cudaMemcpyDeviceToHost, st));
-  PQ_CUDA_TRY(cudaStreamSynchronize(st));
-  d.win = 2;
-  for (int l = 1; l < 4; l++)
-    if (wm[l] <= KMAX) d.win = 2 << l;
-  std::vector<int32_t> off(rt + 1, 0), list;
-  for (int64_t r = 0; r < rt; r++) {
-    for (int c = 0; c < chunks; c++)
-      if (f[(size_t)r * chunks + c]) list.push_back(c);
-    off[r + 1] = (int32_t)list.size();
-  }
-  if (list.empty()) list.push_back(0);
-  PQ_TRY(upload(d.kt_off, off, st));
-  PQ_TRY(upload(d.kt_list, list, st));
-  PQ_CUDA_TRY(cudaStreamSynchronize(st));
-  return PQ_OK;
-}
-
-// Scatter lists per (pass, tile of 128 beta strings): targets, each with its contributions (six to an entry): the singles of the tile's strings by pair, and their occupied orbitals onto themselves.
-static pq_status s64_lists(pq_ci_handle *h, Sigma64 &S) {
-  using namespace s64;
-  const SpinTablesDev &t = h->tab[0][1];
-  cudaStream_t st = h->stream;
-  std::vector<int64_t> off(t.n_str + 1);
-  std::vector<int32_t> J(t.n1 + 1), info(t.n1 + 1);
-  PQ_CUDA_TRY(cudaMemcpyAsync(off.data(), t.s1_off.ptr, off.size() * 8, cudaMemcpyDeviceToHost, st));
-  PQ_CUDA_TRY(cudaMemcpyAsync(J.data(), t.s1_J.ptr, t.n1 * 4, cudaMemcpyDeviceToHost, st));
-  PQ_CUDA_TRY(cudaMemcpyAsync(info.data(), t.s1_info.ptr, t.n1 * 4, cudaMemcpyDeviceToHost, st));
-  PQ_CUDA_TRY(cudaStreamSynchronize(st));
-  const int tiles = (int)((t.n_str + BM - 1) / BM);
-  std::vector<std::vector<uint32_t>> items((size_t)S.npass * tiles);  // target << 16 | contribution
   const std::vector<uint64_t> &str = h->str[0][1];
-  for (int64_t b = 0; b < t.n_str; b++) {
+  const int64_t n = (int64_t)str.size();
+  const int tiles = (int)((n + BM - 1) / BM);
+  std::vector<std::vector<uint32_t>> items((size_t)S.npass * tiles);  // target << 16 | contribution
+  for (int64_t b = 0; b < n; b++) {
     auto put = [&](int64_t target, int pair, int neg) {
       const int p = pair / S.wq, q = pair - p * S.wq;
       items[(size_t)p * tiles + b / BM].push_back((uint32_t)target << 16 | (uint32_t)neg << 15 |
@@ -612,31 +572,38 @@ static pq_status s64_lists(pq_ci_handle *h, Sigma64 &S) {
       put(b, k * (k + 3) / 2, 0);
     }
   }
-  std::vector<int32_t> toff(items.size() + 1, 0);
-  std::vector<int4> ent;
+  toff.assign(items.size() + 1, 0);
+  ent.clear();
   for (size_t i = 0; i < items.size(); i++) {
     std::vector<uint32_t> &v = items[i];
     std::sort(v.begin(), v.end());
+    std::vector<std::pair<size_t, size_t>> runs;  // ranges of one target
     for (size_t u = 0; u < v.size();) {
-      const uint32_t target = v[u] >> 16;
-      uint32_t c[6] = {ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT};
-      int n = 0;
-      while (u < v.size() && v[u] >> 16 == target && n < 6) c[n++] = v[u++] & 0xffffu;
-      ent.push_back(make_int4((int)(target | (uint32_t)n << 16), (int)(c[0] | c[1] << 16), (int)(c[2] | c[3] << 16),
-                              (int)(c[4] | c[5] << 16)));
+      size_t w = u;
+      while (w < v.size() && v[w] >> 16 == v[u] >> 16) w++;
+      runs.emplace_back(u, w);
+      u = w;
     }
     // by falling count, so that a warp's entries take the same steps
-    std::stable_sort(ent.begin() + toff[i], ent.end(), [](const int4 &x, const int4 &y) { return (x.x >> 16) > (y.x >> 16); });
+    std::stable_sort(runs.begin(), runs.end(), [](const auto &x, const auto &y) { return x.second - x.first > y.second - y.first; });
+    for (const auto &r : runs) {
+      const size_t need = (r.second - r.first + 5) / 6;
+      // the entries of a target stay within one group of 32
+      while ((ent.size() - toff[i]) % 32 + need > 32) ent.push_back(make_int4(0, ZERO2, ZERO2, ZERO2));
+      for (size_t u = r.first, place = 0; u < r.second; place++) {
+        uint32_t c[6] = {ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT, ZERO_SLOT};
+        uint32_t k = 0;
+        for (; u < r.second && k < 6; u++) c[k++] = v[u] & 0xffffu;
+        ent.push_back(make_int4((int)(v[r.first] >> 16 | k << 16 | (uint32_t)place << 19), (int)(c[0] | c[1] << 16),
+                                (int)(c[2] | c[3] << 16), (int)(c[4] | c[5] << 16)));
+      }
+    }
     if (ent.size() > (size_t)INT32_MAX / 2) {
       set_error("FP64 full-CI sigma: scatter lists too large");
       return PQ_ERR_ARG;
     }
     toff[i + 1] = (int32_t)ent.size();
   }
-  if (ent.empty()) ent.push_back(make_int4(0, 0, 0, 0));
-  PQ_TRY(upload(S.toff, toff, st));
-  PQ_TRY(upload(S.tent, ent, st));
-  PQ_CUDA_TRY(cudaStreamSynchronize(st));
   return PQ_OK;
 }
 
@@ -650,37 +617,118 @@ static pq_status s64_prepare(pq_ci_handle *h) {
   }
   cudaStream_t st = h->stream;
   const pq_ci_desc &d = h->desc;
-  const SpinTablesDev &a = h->tab[0][0];
+  const SpinTablesDev &a = h->tab[0][0], &bt = h->tab[0][1];
   const int npair = h->npair[0];
-  PQ_TRY(S->hi.alloc(16));
-  PQ_CUDA_TRY(cudaMemsetAsync(S->hi.ptr, 0, 16, st));
   // identical spin lists with identical integrals share the matrix
-  S->shared = !h->selected && h->n_blocks[0] == 1 && d.n_alpha[0] == d.n_beta[0] && d.ex_level[0][0] == d.ex_level[0][1];
-  PQ_TRY(s64_side(h, *S, 0, true));
-  PQ_TRY(s64_side(h, *S, 1, !S->shared));
+  const bool shared = !h->selected && h->n_blocks[0] == 1 && d.n_alpha[0] == d.n_beta[0] && d.ex_level[0][0] == d.ex_level[0][1];
   S->npass = (npair + BN - 1) / BN;
   S->wq = (npair + S->npass - 1) / S->npass;
-  const int ncol = S->npass * BN;
-  uint32_t *whi = S->hi.as<uint32_t>() + 2;
-  absmax_kernel<<<32, 256, 0, st>>>(h->d_eab64.as<double>(), (int64_t)npair * npair, whi);
-  PQ_TRY(S->w.alloc(2 * (size_t)dg::N * (2 * npair + 1) * ncol));
-  w_kernel<<<(unsigned)(((int64_t)(2 * npair + 1) * ncol + 255) / 256), 256, 0, st>>>(h->d_eab64.as<double>(), npair, S->wq,
-                                                                                    ncol, whi, S->w.as<unsigned short>());
-  S->kp = (int)up64(a.max1 + d.n_alpha[0], 16);
-  if (S->kp == 0) S->kp = 16;
-  PQ_TRY(S->klist.alloc(sizeof(int2) * (size_t)a.n_str * S->kp));
+  const int ncol = S->npass * BN, wrows = 2 * npair + 1;
+  S->kp = std::max<int>(16, (int)up64(a.max1 + d.n_alpha[0], 16));
+  int chunks[2], tile_rows[2] = {BN, BM};
+  int64_t rt[2];
+  for (int sp = 0; sp < 2; sp++) {
+    Sigma64::Side &z = S->side[sp];
+    z.n = h->tab[0][sp].n_str;
+    z.np = up64(z.n, 64);
+    chunks[sp] = (int)((z.n + 31) / 32);
+    rt[sp] = (z.n + tile_rows[sp] - 1) / tile_rows[sp];
+  }
+  uint8_t *flags = nullptr;  // both sides' flags, then 2 x 4 window maxima
+  const size_t nflags = (size_t)(rt[0] * chunks[0] + rt[1] * chunks[1] + 15) / 16 * 16;
+  size_t zeroed = 0;
+  auto lay = [&](DevLayout &l) {
+    l.take(S->hi, 4);
+    l.take(S->aux, 16);
+    l.take(flags, nflags + 8 * sizeof(int));
+    for (int sp = 0; sp < (shared ? 1 : 2); sp++) l.take(S->side[sp].d, (size_t)dg::N * S->side[sp].n * S->side[sp].np);
+    zeroed = l.used;
+    l.take(S->w, (size_t)dg::N * wrows * ncol);
+    l.take(S->klist, (size_t)a.n_str * S->kp);
+  };
+  DevLayout l;
+  lay(l);
+  PQ_TRY(S->mem.alloc(l.used));
+  l = DevLayout{static_cast<char *>(S->mem.ptr), 0};
+  lay(l);
+  PQ_CUDA_TRY(cudaMemsetAsync(S->mem.ptr, 0, zeroed, st));
+  int *wmax = reinterpret_cast<int *>(flags + nflags);
+  for (int sp = 0; sp < 2; sp++) {
+    const SpinTablesDev &t = h->tab[0][sp];
+    const Sigma64::Side &z = S->side[sp];
+    uint32_t *hi = S->hi + sp;
+    const unsigned g1 = (unsigned)std::min<int64_t>((t.n1 + 255) / 256, 1216), g2 = (unsigned)std::min<int64_t>((t.n2 + 255) / 256, 1216);
+    if (t.n1) absmax_kernel<<<g1, 256, 0, st>>>(t.s1_F64.as<double>(), t.n1, hi);
+    if (t.n2) absmax_kernel<<<g2, 256, 0, st>>>(t.s2_D64.as<double>(), t.n2, hi);
+    dense_kernel<<<(unsigned)z.n, 128, chunks[sp] * sizeof(int), st>>>(
+        t.s1_off.as<int64_t>(), t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(),
+        t.s2_J.as<int32_t>(), t.s2_D64.as<double>(), z.n, z.np, hi, chunks[sp], tile_rows[sp], z.d,
+        flags + (sp ? rt[0] * chunks[0] : 0), wmax + 4 * sp);
+    PQ_CUDA_TRY(cudaGetLastError());
+  }
+  absmax_kernel<<<32, 256, 0, st>>>(h->d_eab64.as<double>(), (int64_t)npair * npair, S->hi + 2);
+  w_kernel<<<(unsigned)(((int64_t)wrows * ncol + 255) / 256), 256, 0, st>>>(h->d_eab64.as<double>(), npair, S->wq, ncol, S->hi + 2, S->w);
   klist_kernel<<<(unsigned)((a.n_str + 127) / 128), 128, 0, st>>>(a.s1_off.as<int64_t>(), a.s1_J.as<int32_t>(),
                                                                 a.s1_info.as<int32_t>(), a.str.as<uint64_t>(), a.n_str, S->kp,
-                                                                npair, S->klist.as<int2>());
+                                                                npair, S->klist);
   PQ_CUDA_TRY(cudaGetLastError());
-  PQ_TRY(s64_lists(h, *S));
-  PQ_TRY(S->aux.alloc(64));
+  std::vector<uint8_t> f(nflags + 8 * sizeof(int));
+  std::vector<int64_t> off(bt.n_str + 1);
+  std::vector<int32_t> J(bt.n1 + 1), info(bt.n1 + 1);
+  PQ_CUDA_TRY(cudaMemcpyAsync(off.data(), bt.s1_off.ptr, off.size() * 8, cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaMemcpyAsync(J.data(), bt.s1_J.ptr, bt.n1 * 4, cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaMemcpyAsync(info.data(), bt.s1_info.ptr, bt.n1 * 4, cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaMemcpyAsync(f.data(), flags, f.size(), cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  // the lists, one upload: scatter entries, then the offsets and chunk lists
+  std::vector<int32_t> toff, kto[2], ktl[2];
+  std::vector<int4> ent;
+  PQ_TRY(s64_lists(h, *S, off, J, info, toff, ent));
+  const uint8_t *fl = f.data();
+  for (int sp = 0; sp < 2; sp++) {
+    int wm[4];
+    memcpy(wm, f.data() + nflags + 4 * sp * sizeof(int), sizeof(wm));
+    for (int k = 1; k < 4; k++)
+      if (wm[k] <= KMAX) S->side[sp].win = 2 << k;
+    kto[sp].assign(rt[sp] + 1, 0);
+    for (int64_t r = 0; r < rt[sp]; r++) {
+      for (int c = 0; c < chunks[sp]; c++)
+        if (fl[r * chunks[sp] + c]) ktl[sp].push_back(c);
+      kto[sp][r + 1] = (int32_t)ktl[sp].size();
+    }
+    fl += rt[sp] * chunks[sp];
+  }
+  auto lay2 = [&](DevLayout &m) {
+    m.take(S->tent, ent.size() + 1);
+    m.take(S->toff, toff.size());
+    for (int sp = 0; sp < 2; sp++) {
+      m.take(S->side[sp].kt_off, kto[sp].size());
+      m.take(S->side[sp].kt_list, ktl[sp].size() + 1);
+    }
+  };
+  DevLayout m;
+  lay2(m);
+  PQ_TRY(S->lists.alloc(m.used));
+  std::vector<char> host(m.used);
+  m = DevLayout{host.data(), 0};
+  lay2(m);
+  memcpy(S->tent, ent.data(), ent.size() * sizeof(int4));
+  memcpy(S->toff, toff.data(), toff.size() * 4);
+  for (int sp = 0; sp < 2; sp++) {
+    memcpy(S->side[sp].kt_off, kto[sp].data(), kto[sp].size() * 4);
+    memcpy(S->side[sp].kt_list, ktl[sp].data(), ktl[sp].size() * 4);
+  }
+  m = DevLayout{static_cast<char *>(S->lists.ptr), 0};
+  lay2(m);
+  PQ_CUDA_TRY(cudaMemcpyAsync(S->lists.ptr, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+  if (shared) S->side[1].d = S->side[0].d;
   int dev = 0;
   PQ_CUDA_TRY(cudaGetDevice(&dev));
   PQ_CUDA_TRY(cudaDeviceGetAttribute(&S->sms, cudaDevAttrMultiProcessorCount, dev));
   PQ_CUDA_TRY(cudaFuncSetAttribute(ab64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AB_SMEM));
   PQ_CUDA_TRY(cudaFuncSetAttribute(ss64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM));
   PQ_CUDA_TRY(cudaFuncSetAttribute(ss64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));  // the host copy of the lists ends here
   h->s64 = std::move(S);
   return PQ_OK;
 }
@@ -695,17 +743,15 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
   cudaStream_t st = h->stream;
   const int64_t na = h->tab[0][0].n_str, nb = h->tab[0][1].n_str, n = h->n_dets, nbp = up64(nb, 64);
   PQ_TRY(z.xd.ensure(2 * (size_t)dg::N * nv * na * nbp));
-  int *gate = z.aux.as<int>();
-  uint32_t *xhi = z.aux.as<uint32_t>() + 4, *hi = z.hi.as<uint32_t>();
-  PQ_CUDA_TRY(cudaMemsetAsync(z.aux.ptr, 0, 64, st));
+  int *gate = z.aux;
+  uint32_t *xhi = reinterpret_cast<uint32_t *>(z.aux) + 4, *hi = z.hi;
+  PQ_CUDA_TRY(cudaMemsetAsync(z.aux, 0, 64, st));
   x64_absmax_kernel<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 152 * 4), nv), 256, 0, st>>>(C, es, vs, n, xhi);
-  // beta's exponent word is alpha's when they share the matrix (same entries)
   x64_digits_kernel<<<dim3((unsigned)na, nv), 256, 0, st>>>(C, es, vs, na, nb, nbp, nv, xhi, hi, h->tab[0][0].e_same64.as<double>(),
                                                           h->tab[0][1].e_same64.as<double>(), shift,
                                                           z.xd.as<unsigned short>(), S, ses, svs, gate);
   PQ_CUDA_TRY(cudaGetLastError());
   const Sigma64::Side &A = z.side[0], &B = z.side[1];
-  const DevBuf &db = z.shared ? A.d : B.d;
   SsArgs g{};
   g.na = na, g.nb = nb, g.nv = nv;
   g.m_tiles = (int)((nb + BM - 1) / BM);
@@ -718,35 +764,35 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
   const int64_t xrows = (int64_t)dg::N * nv * na;
   // alpha: strips of 64 beta strings of 32 rows Ja; rows of Ha
   PQ_TRY(s64_map(&ma, z.xd.ptr, xrows, nb, nbp, 64, 32));
-  PQ_TRY(s64_map(&mb, A.d.ptr, dg::N * A.n, A.n, A.np, 32, BN));
+  PQ_TRY(s64_map(&mb, A.d, dg::N * A.n, A.n, A.np, 32, BN));
   g.ksplit = 1;
   g.win = A.win;
   g.a_plane = (int64_t)nv * na, g.b_plane = A.n;
-  g.kt_off = A.kt_off.as<int32_t>(), g.kt_list = A.kt_list.as<int32_t>();
+  g.kt_off = A.kt_off, g.kt_list = A.kt_list;
   g.dhi = hi;
   ss64_kernel<true><<<grid, THREADS, SS_SMEM, st>>>(ma, mb, g);
   // beta: rows of Hb; rows (v, Ia) of C
-  PQ_TRY(s64_map(&ma, db.ptr, dg::N * B.n, B.n, B.np, 32, BM));
+  PQ_TRY(s64_map(&ma, B.d, dg::N * B.n, B.n, B.np, 32, BM));
   PQ_TRY(s64_map(&mb, z.xd.ptr, xrows, nb, nbp, 32, BN));
   g.win = B.win;
   g.a_plane = B.n, g.b_plane = (int64_t)nv * na;
-  g.kt_off = B.kt_off.as<int32_t>(), g.kt_list = B.kt_list.as<int32_t>();
-  g.dhi = z.shared ? hi : hi + 1;
+  g.kt_off = B.kt_off, g.kt_list = B.kt_list;
+  g.dhi = hi + 1;
   ss64_kernel<false><<<grid, THREADS, SS_SMEM, st>>>(ma, mb, g);
   PQ_CUDA_TRY(cudaGetLastError());
   AbArgs x{};
   const int ncol = z.npass * BN, wrows = 2 * h->npair[0] + 1;
   PQ_TRY(s64_map(&ma, z.xd.ptr, xrows, nb, nbp, 64, 1));
-  PQ_TRY(s64_map(&mb, z.w.ptr, (int64_t)dg::N * wrows, ncol, ncol, 64, 1));
+  PQ_TRY(s64_map(&mb, z.w, (int64_t)dg::N * wrows, ncol, ncol, 64, 1));
   x.na = na, x.nb = nb, x.nv = nv;
   x.npass = z.npass, x.wq = z.wq, x.kp = z.kp, x.wrows = wrows;
   x.m_tiles = g.m_tiles;
   // few items: one per root, so that the last round of CTAs is short
-  x.vsplit = na * z.npass < 8 * z.sms;
-  x.items = na * z.npass * (x.vsplit ? nv : 1);
-  x.klist = z.klist.as<int2>();
-  x.toff = z.toff.as<int32_t>();
-  x.tent = z.tent.as<int4>();
+  x.vsplit = na < 8 * z.sms;
+  x.items = na * (x.vsplit ? nv : 1);
+  x.klist = z.klist;
+  x.toff = z.toff;
+  x.tent = z.tent;
   x.xhi = xhi, x.whi = hi + 2;
   x.S = S, x.es = ses, x.vs = svs, x.gate = gate;
   ab64_kernel<<<(unsigned)std::min<int64_t>(x.items, z.sms), AB_THREADS, AB_SMEM, st>>>(ma, mb, x);

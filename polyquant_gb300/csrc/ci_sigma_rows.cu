@@ -231,35 +231,46 @@ pq_status rows_make(pq_ci_handle *h, std::unique_ptr<SigmaRows, void (*)(SigmaRo
     return PQ_ERR_OOM;
   }
   r->lim = std::min(h->desc.ex_level[0][2], h->desc.max_collective);
+  auto lay = [&](DevLayout &l) {
+    for (int sp = 0; sp < 2; sp++) {
+      const SpinTablesDev &t = h->tab[0][sp];
+      SigmaRows::Side &s = r->side[sp];
+      const size_t coul = (size_t)npair * t.n_str;
+      l.take(s.lvl, t.n_str);
+      l.take(s.cum, 8 * t.n_str);
+      l.take(s.s1, t.n1 + 1);
+      l.take(s.s1_F, t.n1 + 1);
+      l.take(s.s2, t.n2 + 1);
+      l.take(s.s2_D, t.n2 + 1);
+      if (sizeof(double) * coul <= ROWS_COUL_MAX) l.take(s.coul, coul);
+    }
+    l.take(r->row, h->n_dets);
+  };
+  DevLayout l;
+  lay(l);
+  PQ_TRY(r->mem.alloc(l.used));
+  l = DevLayout{static_cast<char *>(r->mem.ptr), 0};
+  lay(l);
   for (int sp = 0; sp < 2; sp++) {
     const SpinTablesDev &t = h->tab[0][sp];
     SigmaRows::Side &s = r->side[sp];
-    PQ_TRY(upload(s.lvl, h->lvl[0][sp], st));
-    PQ_TRY(s.s1.alloc(sizeof(int2) * (t.n1 + 1)));
-    PQ_TRY(s.s1_F.alloc(sizeof(double) * (t.n1 + 1)));
-    PQ_TRY(s.s2.alloc(sizeof(int32_t) * (t.n2 + 1)));
-    PQ_TRY(s.s2_D.alloc(sizeof(double) * (t.n2 + 1)));
-    PQ_TRY(s.cum.alloc(sizeof(int32_t) * 8 * t.n_str));
+    PQ_CUDA_TRY(cudaMemcpyAsync(s.lvl, h->lvl[0][sp].data(), sizeof(int32_t) * t.n_str, cudaMemcpyHostToDevice, st));
     group_kernel<<<(unsigned)((t.n_str + 3) / 4), 128, 0, st>>>(
-        t.n_str, s.lvl.as<int32_t>(), sp == 0 ? h->d_rowoff.as<int64_t>() : nullptr, t.s1_off.as<int64_t>(),
-        t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(),
-        t.s2_J.as<int32_t>(), t.s2_D64.as<double>(), s.s1.as<int2>(), s.s1_F.as<double>(), s.s2.as<int32_t>(),
-        s.s2_D.as<double>(), s.cum.as<int32_t>());
+        t.n_str, s.lvl, sp == 0 ? h->d_rowoff.as<int64_t>() : nullptr, t.s1_off.as<int64_t>(), t.s1_J.as<int32_t>(),
+        t.s1_info.as<int32_t>(), t.s1_F64.as<double>(), t.s2_off.as<int64_t>(), t.s2_J.as<int32_t>(), t.s2_D64.as<double>(),
+        s.s1, s.s1_F, s.s2, s.s2_D, s.cum);
     PQ_CUDA_TRY(cudaGetLastError());
+    if (!s.coul) continue;
     const int64_t total = (int64_t)npair * t.n_str;
-    if (sizeof(double) * (size_t)total > ROWS_COUL_MAX) continue;
-    PQ_TRY(s.coul.alloc(sizeof(double) * (size_t)total));
     coulomb_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 152 * 16), 256, 0, st>>>(
         h->d_eab64.as<double>(), npair, sp == 0 ? 1 : npair, sp == 0 ? npair : 1, t.str.as<uint64_t>(),
-        t.str_hi.as<uint64_t>(), t.n_str, s.coul.as<double>());
+        t.str_hi.as<uint64_t>(), t.n_str, s.coul);
     PQ_CUDA_TRY(cudaGetLastError());
   }
   const int64_t na = h->tab[0][0].n_str;
-  PQ_TRY(r->row.alloc(sizeof(int32_t) * h->n_dets));
   row_kernel<<<(unsigned)std::min<int64_t>(na, 152 * 16), 128, 0, st>>>(h->d_rowoff.as<int64_t>(),
-                                                                       h->d_rowlen.as<int32_t>(), na, r->row.as<int32_t>());
+                                                                       h->d_rowlen.as<int32_t>(), na, r->row);
   PQ_CUDA_TRY(cudaGetLastError());
-  PQ_CUDA_TRY(cudaStreamSynchronize(st));
   out = std::move(r);
   return PQ_OK;
 }
@@ -272,12 +283,11 @@ rows::Args rows_args(const pq_ci_handle *h, const SigmaRows &r) {
     const SpinTablesDev &t = h->tab[0][sp];
     const SigmaRows::Side &s = r.side[sp];
     // strings of one spin stand beside singles of the other: eab is [pair_alpha][pair_beta]
-    *out[sp] = {t.s1_off.as<int64_t>(), t.s2_off.as<int64_t>(), s.s1.as<int2>(),     s.s1_F.as<double>(),
-                s.s2.as<int32_t>(),     s.s2_D.as<double>(),    s.cum.as<int4>(),    s.lvl.as<int32_t>(),
-                s.coul.as<double>(),    t.str.as<uint64_t>(),   t.str_hi.as<uint64_t>(),
-                sp == 0 ? 1 : p.npair,  sp == 0 ? p.npair : 1};
+    *out[sp] = {t.s1_off.as<int64_t>(), t.s2_off.as<int64_t>(), s.s1, s.s1_F, s.s2, s.s2_D,
+                reinterpret_cast<const int4 *>(s.cum), s.lvl, s.coul, t.str.as<uint64_t>(), t.str_hi.as<uint64_t>(),
+                sp == 0 ? 1 : p.npair, sp == 0 ? p.npair : 1};
   }
-  p.row = r.row.as<int32_t>();
+  p.row = r.row;
   p.rowoff = h->d_rowoff.as<int64_t>();
   p.eab = h->d_eab64.as<double>();
   p.diag = h->d_diag.as<double>();

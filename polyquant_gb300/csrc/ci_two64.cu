@@ -31,19 +31,17 @@ namespace pq {
 
 struct Two64 {
   struct Pair {
-    int x = 0, y = 1;          // lists (species-0 alpha, beta, species-1 alpha, beta)
-    int64_t M = 0, np = 0;     // rows, row length
-    DevBuf d, kt_off, kt_list, xd, part;
+    int x = 0, y = 1;                // lists (species-0 alpha, beta, species-1 alpha, beta)
+    int64_t M = 0, np = 0;           // rows, row length
+    unsigned short *d = nullptr;     // digits of H_xy
     int win = 2;
   };
-  std::vector<std::unique_ptr<Pair>> pairs;
-  DevBuf hi, aux;              // high word of max|H_xy| per pair; gate and high words of max|C|
+  std::vector<Pair> pairs;
+  uint32_t *hi = nullptr;            // high word of max|H_xy| per pair
+  int *aux = nullptr;                // gate; high words of max|C| from word 4 on
+  DevBuf mem, work;                  // the matrices and these words; digits and copies of a call
   int sms = 0;
-  size_t bytes() const {
-    size_t b = hi.bytes + aux.bytes;
-    for (const auto &p : pairs) b += p->d.bytes + p->kt_off.bytes + p->kt_list.bytes + p->xd.bytes + p->part.bytes;
-    return b;
-  }
+  size_t bytes() const { return mem.bytes + work.bytes; }
 };
 void two64_delete(Two64 *t) { delete t; }
 
@@ -63,12 +61,11 @@ struct Shape {
   int64_t st[4];  // determinant index step of each list
 };
 
-// Row m' = (x', y') of a pair matrix without its diagonal.  FILL = false: largest magnitude.  FILL: digits, flags of
-// the (128-row, chunk) blocks with an entry, largest number of entries in windows of 2, 4, 8, 16 chunks.
+// Row m' = (x', y') of a pair matrix without its diagonal.  FILL = false: largest magnitude.  FILL: digits, and the
+// largest number of entries in windows of 2, 4, 8, 16 chunks.
 template <bool FILL>
 __global__ void __launch_bounds__(256) pair_kernel(List x, List y, int ny, bool own_x, bool own_y, const double *W, int ldw,
-                                                   int64_t M, int64_t np, int chunks, uint32_t *hi, unsigned short *d,
-                                                   uint8_t *flags, int *wmax) {
+                                                   int64_t M, int64_t np, int chunks, uint32_t *hi, unsigned short *d, int *wmax) {
   extern __shared__ int cnt[];
   const int64_t row = blockIdx.x;
   const int xs = (int)(row / ny), ys = (int)(row - (int64_t)xs * ny);
@@ -85,7 +82,6 @@ __global__ void __launch_bounds__(256) pair_kernel(List x, List y, int ny, bool 
       return;
     }
     atomicAdd(cnt + m / 32, 1);
-    flags[(row / BM) * chunks + m / 32] = 1;
     if (e == digits::BAD) return;
     unsigned short h[dg::N];
     dg::to_half(digits::fixed_point<dg::BITS>(v, e), h);
@@ -265,62 +261,49 @@ static pq_status two64_prepare(pq_ci_handle *h) {
   }
   cudaStream_t st = h->stream;
   const Shape sh = shape_of(h);
-  PQ_TRY(T->hi.alloc(32));
-  PQ_CUDA_TRY(cudaMemsetAsync(T->hi.ptr, 0, 32, st));
-  PQ_TRY(T->aux.alloc(64));
-  bool owned[4] = {false, false, false, false};
   for (int x = 0; x < 4; x++)
-    for (int y = x + 1; y < 4; y++) {
-      if (sh.n[x] < 2 || sh.n[y] < 2) continue;
-      std::unique_ptr<Two64::Pair> p(new (std::nothrow) Two64::Pair());
-      if (!p) {
-        set_error("host allocation failed");
-        return PQ_ERR_OOM;
+    for (int y = x + 1; y < 4; y++)
+      if (sh.n[x] > 1 && sh.n[y] > 1) {
+        Two64::Pair p;
+        p.x = x, p.y = y;
+        p.M = (int64_t)sh.n[x] * sh.n[y];
+        p.np = up64(p.M, 64);
+        T->pairs.push_back(p);
       }
-      p->x = x, p->y = y;
-      p->M = (int64_t)sh.n[x] * sh.n[y];
-      p->np = up64(p->M, 64);
-      const bool ox = !owned[x], oy = !owned[y];
-      owned[x] = owned[y] = true;
-      const bool same = (x >> 1) == (y >> 1);
-      const double *W = same ? h->d_eabs64[x >> 1].as<double>() : h->d_epc64[x & 1][y & 1].as<double>();
-      const int ldw = h->npair[y >> 1], chunks = (int)((p->M + 31) / 32);
-      const int64_t rt = (p->M + BM - 1) / BM;
-      uint32_t *hi = T->hi.as<uint32_t>() + T->pairs.size();
-      const size_t bytes = 2 * (size_t)dg::N * p->M * p->np;
-      PQ_TRY(p->d.alloc(bytes));
-      PQ_CUDA_TRY(cudaMemsetAsync(p->d.ptr, 0, bytes, st));
-      DevBuf flags, wmax;
-      PQ_TRY(flags.alloc((size_t)rt * chunks));
-      PQ_TRY(wmax.alloc(4 * sizeof(int)));
-      PQ_CUDA_TRY(cudaMemsetAsync(flags.ptr, 0, (size_t)rt * chunks, st));
-      PQ_CUDA_TRY(cudaMemsetAsync(wmax.ptr, 0, 4 * sizeof(int), st));
-      const List lx = list_of(h, x), ly = list_of(h, y);
-      pair_kernel<false><<<(unsigned)p->M, 256, 0, st>>>(lx, ly, sh.n[y], ox, oy, W, ldw, p->M, p->np, chunks, hi, nullptr,
-                                                       nullptr, nullptr);
-      pair_kernel<true><<<(unsigned)p->M, 256, chunks * sizeof(int), st>>>(lx, ly, sh.n[y], ox, oy, W, ldw, p->M, p->np, chunks,
-                                                                          hi, p->d.as<unsigned short>(), flags.as<uint8_t>(),
-                                                                          wmax.as<int>());
-      PQ_CUDA_TRY(cudaGetLastError());
-      std::vector<uint8_t> f((size_t)rt * chunks);
-      int wm[4];
-      PQ_CUDA_TRY(cudaMemcpyAsync(f.data(), flags.ptr, f.size(), cudaMemcpyDeviceToHost, st));
-      PQ_CUDA_TRY(cudaMemcpyAsync(wm, wmax.ptr, sizeof(wm), cudaMemcpyDeviceToHost, st));
-      PQ_CUDA_TRY(cudaStreamSynchronize(st));
-      for (int l = 1; l < 4; l++)
-        if (wm[l] <= KMAX) p->win = 2 << l;
-      std::vector<int32_t> off(rt + 1, 0), list;
-      for (int64_t r = 0; r < rt; r++) {
-        for (int c = 0; c < chunks; c++)
-          if (f[(size_t)r * chunks + c]) list.push_back(c);
-        off[r + 1] = (int32_t)list.size();
-      }
-      if (list.empty()) list.push_back(0);
-      PQ_TRY(upload(p->kt_off, off, st));
-      PQ_TRY(upload(p->kt_list, list, st));
-      PQ_CUDA_TRY(cudaStreamSynchronize(st));
-      T->pairs.push_back(std::move(p));
-    }
+  const int npairs = (int)T->pairs.size();
+  int *wmax = nullptr;
+  auto lay = [&](DevLayout &l) {
+    l.take(T->hi, 8);
+    l.take(T->aux, 16);
+    l.take(wmax, 4 * npairs);
+    for (Two64::Pair &p : T->pairs) l.take(p.d, (size_t)dg::N * p.M * p.np);
+  };
+  DevLayout l;
+  lay(l);
+  PQ_TRY(T->mem.alloc(l.used));
+  l = DevLayout{static_cast<char *>(T->mem.ptr), 0};
+  lay(l);
+  PQ_CUDA_TRY(cudaMemsetAsync(T->mem.ptr, 0, l.used, st));
+  bool owned[4] = {false, false, false, false};
+  for (int i = 0; i < npairs; i++) {
+    const Two64::Pair &p = T->pairs[i];
+    const int x = p.x, y = p.y, ldw = h->npair[y >> 1], chunks = (int)((p.M + 31) / 32);
+    const bool ox = !owned[x], oy = !owned[y];  // a list's own moves belong to one pair
+    owned[x] = owned[y] = true;
+    const double *W = (x >> 1) == (y >> 1) ? h->d_eabs64[x >> 1].as<double>() : h->d_epc64[x & 1][y & 1].as<double>();
+    const List lx = list_of(h, x), ly = list_of(h, y);
+    pair_kernel<false><<<(unsigned)p.M, 256, 0, st>>>(lx, ly, sh.n[y], ox, oy, W, ldw, p.M, p.np, chunks, T->hi + i, nullptr,
+                                                    nullptr);
+    pair_kernel<true><<<(unsigned)p.M, 256, chunks * sizeof(int), st>>>(lx, ly, sh.n[y], ox, oy, W, ldw, p.M, p.np, chunks,
+                                                                       T->hi + i, p.d, wmax + 4 * i);
+    PQ_CUDA_TRY(cudaGetLastError());
+  }
+  std::vector<int> wm(4 * npairs);
+  PQ_CUDA_TRY(cudaMemcpyAsync(wm.data(), wmax, wm.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+  PQ_CUDA_TRY(cudaStreamSynchronize(st));
+  for (int i = 0; i < npairs; i++)
+    for (int k = 1; k < 4; k++)
+      if (wm[4 * i + k] <= KMAX) T->pairs[i].win = 2 << k;
   int dev = 0;
   PQ_CUDA_TRY(cudaGetDevice(&dev));
   PQ_CUDA_TRY(cudaDeviceGetAttribute(&T->sms, cudaDevAttrMultiProcessorCount, dev));
@@ -338,34 +321,44 @@ pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int
   cudaStream_t st = h->stream;
   const Shape sh = shape_of(h);
   const int64_t n = h->n_dets;
-  int *gate = T.aux.as<int>();
-  uint32_t *xhi = T.aux.as<uint32_t>() + 4, *hi = T.hi.as<uint32_t>();
+  int *gate = T.aux;
+  uint32_t *xhi = reinterpret_cast<uint32_t *>(T.aux) + 4, *hi = T.hi;
   const int npairs = (int)T.pairs.size();
   Parts q{};
   q.npairs = npairs;
-  // buffers first: a full device leaves the call to the other kernel before anything is written
+  unsigned short *xd[6];
+  double *part[6];
+  auto lay = [&](DevLayout &l) {
+    for (int i = 0; i < npairs; i++) {
+      l.take(xd[i], (size_t)dg::N * nv * q.R[i] * T.pairs[i].np);
+      l.take(part[i], (size_t)q.ksplit[i] * q.part[i]);
+    }
+  };
   for (int i = 0; i < npairs; i++) {
-    Two64::Pair &p = *T.pairs[i];
+    const Two64::Pair &p = T.pairs[i];
     const int64_t R = n / p.M, N = nv * R;
     const int64_t tiles = ((p.M + BM - 1) / BM) * ((N + BN - 1) / BN), chunks = (p.M + 31) / 32;
     // parts of the K range, of at least eight chunks, while the tiles leave SMs idle
-    const int ks = (int)std::max<int64_t>(1, std::min<int64_t>({T.sms / tiles, chunks / 8, 8}));
-    q.x[i] = p.x, q.y[i] = p.y, q.M[i] = p.M, q.R[i] = R, q.ksplit[i] = ks, q.part[i] = N * p.M;
-    PQ_TRY(p.xd.ensure(2 * (size_t)dg::N * N * p.np));
-    PQ_TRY(p.part.ensure(sizeof(double) * (size_t)ks * N * p.M));
-    q.p[i] = p.part.as<double>();
+    q.ksplit[i] = (int)std::max<int64_t>(1, std::min<int64_t>({T.sms / tiles, chunks / 8, 8}));
+    q.x[i] = p.x, q.y[i] = p.y, q.M[i] = p.M, q.R[i] = R, q.part[i] = N * p.M;
   }
-  PQ_CUDA_TRY(cudaMemsetAsync(T.aux.ptr, 0, 64, st));
+  DevLayout l;
+  lay(l);
+  PQ_TRY(T.work.ensure(l.used));  // a full device leaves the call to the other kernel before anything is written
+  l = DevLayout{static_cast<char *>(T.work.ptr), 0};
+  lay(l);
+  for (int i = 0; i < npairs; i++) q.p[i] = part[i];
+  PQ_CUDA_TRY(cudaMemsetAsync(T.aux, 0, 64, st));
   absmax_vectors_kernel<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 152 * 4), nv), 256, 0, st>>>(C, es, vs, n, xhi);
   for (int i = 0; i < npairs; i++) {
-    Two64::Pair &p = *T.pairs[i];
+    const Two64::Pair &p = T.pairs[i];
     const int64_t R = q.R[i], N = nv * R;
     pair_digits_kernel<<<(unsigned)N, 256, 0, st>>>(C, es, vs, sh, p.x, p.y, p.M, p.np, R, nv, xhi, hi, npairs,
-                                                  p.xd.as<unsigned short>(), gate);
+                                                  xd[i], gate);
     PQ_CUDA_TRY(cudaGetLastError());
     CUtensorMap ma, mb;
-    PQ_TRY(s64_map(&ma, p.d.ptr, dg::N * p.M, p.M, p.np, 32, BM));
-    PQ_TRY(s64_map(&mb, p.xd.ptr, dg::N * N, p.M, p.np, 32, BN));
+    PQ_TRY(s64_map(&ma, p.d, dg::N * p.M, p.M, p.np, 32, BM));
+    PQ_TRY(s64_map(&mb, xd[i], dg::N * N, p.M, p.np, 32, BN));
     SsArgs g{};
     g.na = N, g.nb = p.M, g.nv = 1;
     g.m_tiles = (int)((p.M + BM - 1) / BM);
@@ -376,9 +369,9 @@ pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int
     g.per = R;
     g.part = q.part[i];
     g.a_plane = p.M, g.b_plane = N;
-    g.kt_off = p.kt_off.as<int32_t>(), g.kt_list = p.kt_list.as<int32_t>();
+    g.chunks = (int)((p.M + 31) / 32);
     g.xhi = xhi, g.dhi = hi + i;
-    g.S = p.part.as<double>();
+    g.S = part[i];
     g.gate = gate;
     ss64_kernel<false><<<(unsigned)std::min<int64_t>(g.tiles, T.sms), THREADS, SS_SMEM, st>>>(ma, mb, g);
     PQ_CUDA_TRY(cudaGetLastError());

@@ -60,6 +60,18 @@ template <typename T> pq_status upload(DevBuf &b, const std::vector<T> &v, cudaS
   return PQ_OK;
 }
 
+// Arrays laid out one behind the other in one allocation (a cudaMalloc each costs more than the tables of a small
+// problem): run once from a null base for the size, then from the buffer.
+struct DevLayout {
+  char *base = nullptr;
+  size_t used = 0;
+  template <typename T> void take(T *&p, size_t n) {
+    used = (used + 255) / 256 * 256;
+    p = reinterpret_cast<T *>(base + used);
+    used += n * sizeof(T);
+  }
+};
+
 // Excitation tables of one spin list of one species (CSR over strings).
 // Single entries: J (string index), info = (pair << 1) | (phase < 0), and the
 // same-spin part of the element F = h_hp + sum_{k in occ(I)} ((hp|kk) - (hk|kp)).
