@@ -5,7 +5,11 @@
 // pair in half 2), T = C^T S C, written packed (i >= j).  Each slice costs two
 // GEMMs, both in the "A (M x K, K-major) times B (N x K, K-major)^T" form:
 //   GEMM 1:  U^T[m][nu] = sum_mu Ct[m][mu] S[nu][mu]    (A = C^T shared, B = S per slice)
-//   GEMM 2:  T[m][n]   = sum_nu U^T[m][nu] Ct[n][nu]    (A = U^T per slice, B = C^T shared)
+//   GEMM 2:  T[m][n]   = sum_nu U^T[m][nu] Ct[n][nu]    (A = U^T of all slices, B = C^T shared)
+// GEMM 1 leaves U^T with rows (m, slice).  A tile of GEMM 2 then holds 128 slices of one m, or a few m: it loads and
+// multiplies only the columns n <= m, half of the work, and its 32 lanes hold 32 slices, so that a pair (m, n) is
+// written along the slices, as half 2 reads it and as the result wants it, and no transpose is left (256 AOs, BF16x3:
+// two transposes of 13 + 8.7 GB and the FP64 expansion, 35.8 ms in all; now 25.0).
 // Operands are split into a high and a low part (x = x_hi + x_lo) in BF16 or
 // TF32 and each product is formed as hi*hi + hi*lo + lo*hi with FP32
 // accumulation in tensor memory (three MMAs per K step).  BF16 and TF32 keep
@@ -15,7 +19,7 @@
 // tiles, warp-specialised: one thread issues TMA tile loads (128-byte
 // swizzle, a ring of two stages of K = 128 bytes of each of A_hi, A_lo, B_hi,
 // B_lo), one thread issues the tcgen05.mma instructions into one of two TMEM
-// accumulators (128 lanes x 256 FP32 columns each), and four warps drain the
+// accumulators (128 lanes x 256 FP32 columns each; as many columns as the tile has), and four warps drain the
 // other accumulator with tcgen05.ld for the epilogue (BF16/TF32 split of the
 // result for the next GEMM, or the packed lower triangle).  Every mbarrier
 // wait is bounded; a wait that runs out records an error code and the kernel
@@ -43,6 +47,7 @@ constexpr int ROW_BYTES = 128;   // K extent of one stage, in bytes (one swizzle
 constexpr int STAGES = 2;
 constexpr int A_TILE = BM * ROW_BYTES;  // 16 KB
 constexpr int B_TILE = BN * ROW_BYTES;  // 32 KB
+constexpr int B_BOX = 64;               // B rows per load: a tile loads the boxes that it has columns for
 constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;
 constexpr int EPI_WARPS = 4;
 constexpr int EPI_LD = 33;                                  // per-warp 32 x 32 staging, odd stride
@@ -56,15 +61,15 @@ enum { EPI_SPLIT = 0, EPI_PACK = 1 };
 enum { ERR_TIMEOUT_FULL = 1, ERR_TIMEOUT_MMA = 2, ERR_TIMEOUT_ACC = 3 };
 
 struct GemmArgs {
-  int M, N, K;                 // logical sizes
+  int M, N, K;                 // logical sizes (EPI_PACK: M = n_mo * nbp rows)
   int m_tiles;                 // ceil(M / BM)
-  int nbatch;                  // batch entries (tiles = nbatch * m_tiles)
-  int a_batched, b_batched;    // operand varies with the batch index
-  int a_rows, b_rows;          // rows per batch in the operand tensors
+  int nbatch;                  // EPI_SPLIT: slices, one B operand of b_rows rows each (tiles = nbatch * m_tiles)
+  int b_rows;
+  int nb, nbp;                 // slices of this batch, and up to a multiple of 32
   int ld_out;                  // EPI_SPLIT: row length of the split output
-  void *out_hi, *out_lo;       // EPI_SPLIT outputs [b][M][ld_out]
-  float *out_pack;             // EPI_PACK output [b][M(M+1)/2]
-  int64_t pack_stride;         // elements per batch of out_pack
+  void *out_hi, *out_lo;       // EPI_SPLIT outputs, rows (m, slice)
+  void *out_pack;              // EPI_PACK output [pair (m, n)][ld_pack], slice b of this batch in column b
+  int64_t ld_pack;
   long long wait_cycles;       // budget of the pipeline waits (the wind-down waits keep WAIT_CYCLES)
   int *err;
 };
@@ -98,6 +103,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
   return true;
 }
 
+// EPI_PACK: rows (m, slice), so a tile holds few m; only columns n <= m are kept, and the tile takes a whole number of
+// B boxes up to the last of them
+// (the widest tiles come first, so that the last ones even the SMs out)
+template <int EPI> __device__ __forceinline__ void tile_at(const GemmArgs &g, int t, int &b, int &mt) {
+  b = EPI == EPI_SPLIT ? t / g.m_tiles : 0;
+  mt = EPI == EPI_SPLIT ? t - b * g.m_tiles : g.m_tiles - 1 - t;
+}
+template <int EPI> __device__ __forceinline__ int tile_cols(const GemmArgs &g, int64_t row0) {
+  if (EPI == EPI_SPLIT) return g.N;
+  const int64_t last = row0 + BM < g.M ? row0 + BM : g.M;
+  const int n = (int)((last - 1) / g.nbp) + 1;
+  return n < g.N ? n : g.N;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -116,9 +135,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   return d;
 }
 
-// instruction descriptor: D = F32, A/B format (1 = BF16 for kind::f16, 2 = TF32), K-major A and B
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t ab_format) {
-  return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// instruction descriptor: D = F32, A/B format (1 = BF16 for kind::f16, 2 = TF32), K-major A and B, n columns
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t ab_format, int n) {
+  return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
 template <bool TF32>
@@ -171,7 +190,7 @@ __device__ __forceinline__ float tf32_round(float x) {
 // wait is bounded; a wait that runs out sets the error word and an abort flag
 // that every role polls, the producer then waits (bounded) for its own loads
 // in flight, the MMA thread for its own MMAs, and the CTA frees TMEM.
-template <bool TF32, int EPI>
+template <bool TF32, int EPI, typename TO>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
                    const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo, GemmArgs g) {
@@ -219,9 +238,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     // ---- producer
     int gs = 0;
     for (int t = blockIdx.x; t < n_tiles && !*abort_flag; t += gridDim.x) {
-      const int b = t / g.m_tiles, mt = t - b * g.m_tiles;
-      const int ya = (g.a_batched ? b * g.a_rows : 0) + mt * BM;
-      const int yb = g.b_batched ? b * g.b_rows : 0;
+      int b, mt;
+      tile_at<EPI>(g, t, b, mt);
+      const int ya = mt * BM, yb = b * g.b_rows;
+      const int boxes = (tile_cols<EPI>(g, ya) + B_BOX - 1) / B_BOX;
       for (int s = 0; s < nst; s++, gs++) {
         const int slot = gs % STAGES;
         const uint32_t ph = (uint32_t)((gs / STAGES) & 1);
@@ -233,12 +253,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         if (*abort_flag) break;
         unsigned char *st = smem + slot * STAGE_BYTES;
         const uint32_t bar = smem_u32(full + slot);
-        mbar_expect_tx(bar, STAGE_BYTES);
+        mbar_expect_tx(bar, 2 * A_TILE + 2 * boxes * B_BOX * ROW_BYTES);
         const int x = s * BK;
         tma_load_2d(smem_u32(st), &tmA_hi, x, ya, bar);
         tma_load_2d(smem_u32(st + A_TILE), &tmA_lo, x, ya, bar);
-        tma_load_2d(smem_u32(st + 2 * A_TILE), &tmB_hi, x, yb, bar);
-        tma_load_2d(smem_u32(st + 2 * A_TILE + B_TILE), &tmB_lo, x, yb, bar);
+        for (int i = 0; i < boxes; i++) {
+          tma_load_2d(smem_u32(st + 2 * A_TILE + i * B_BOX * ROW_BYTES), &tmB_hi, x, yb + i * B_BOX, bar);
+          tma_load_2d(smem_u32(st + 2 * A_TILE + B_TILE + i * B_BOX * ROW_BYTES), &tmB_lo, x, yb + i * B_BOX, bar);
+        }
       }
     }
     // the loads of the last stages must have landed before the CTA exits
@@ -246,7 +268,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       mbar_wait(smem_u32(full + (j % STAGES)), (uint32_t)((j / STAGES) & 1));
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
-    const uint32_t idesc = instr_desc(TF32 ? 2u : 1u);
     int gs = 0, i = 0;
     for (int t = blockIdx.x; t < n_tiles && !*abort_flag; t += gridDim.x, i++) {
       const int a = i & 1;
@@ -258,6 +279,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + (uint32_t)(a * BN);
+      int b, mt;
+      tile_at<EPI>(g, t, b, mt);
+      const uint32_t idesc = instr_desc(TF32 ? 2u : 1u, (tile_cols<EPI>(g, (int64_t)mt * BM) + 15) / 16 * 16);
       bool ok = true;
       for (int s = 0; s < nst; s++, gs++) {
         const int slot = gs % STAGES;
@@ -303,16 +327,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int b = t / g.m_tiles, mt = t - b * g.m_tiles;
+      int b, mt;
+      tile_at<EPI>(g, t, b, mt);
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN);
       const int row0 = mt * BM + q * 32;
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      const int cols = tile_cols<EPI>(g, (int64_t)mt * BM);
+      // EPI_PACK: 32 rows of one m, lanes are slices
+      const int pm = EPI == EPI_PACK ? row0 / g.nbp : 0, pb = EPI == EPI_PACK ? row0 - pm * g.nbp + lane : 0;
+      for (int c0 = 0; c0 < cols; c0 += 32) {
         float v[32];
         tmem_ld32(taddr + c0, v);  // v[j] = D[row0 + lane][c0 + j]
-#pragma unroll
-        for (int j = 0; j < 32; j++) stg[lane * EPI_LD + j] = v[j];
-        __syncwarp();
         if constexpr (EPI == EPI_SPLIT) {
+#pragma unroll
+          for (int j = 0; j < 32; j++) stg[lane * EPI_LD + j] = v[j];
+          __syncwarp();
           // four lanes per row, eight consecutive columns per lane: 16-byte stores
           // (rows of ld_out = a multiple of 8 elements, so n0 keeps them aligned)
           const int cq = (lane & 3) * 8, n0 = c0 + cq;
@@ -323,7 +351,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             float x[8];
 #pragma unroll
             for (int k = 0; k < 8; k++) x[k] = stg[rr * EPI_LD + cq + k];
-            const int64_t o = ((int64_t)b * g.M + m) * g.ld_out + n0;
+            const int64_t o = ((int64_t)m * g.nbp + b) * g.ld_out + n0;
             if constexpr (TF32) {
               float h[8], l[8];
 #pragma unroll
@@ -359,16 +387,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
               }
             }
           }
-        } else {
-          const int n = c0 + lane;
-          for (int rr = 0; rr < 32; rr++) {
-            const int m = row0 + rr;
-            if (m >= g.M) break;
-            if (n <= m && n < g.N)
-              g.out_pack[(int64_t)b * g.pack_stride + (int64_t)m * (m + 1) / 2 + n] = stg[rr * EPI_LD + lane];
-          }
+          __syncwarp();
+        } else if (row0 < g.M && pb < g.nb) {
+          TO *o = static_cast<TO *>(g.out_pack) + ((int64_t)pm * (pm + 1) / 2 + c0) * g.ld_pack + pb;
+#pragma unroll
+          for (int j = 0; j < 32; j++)
+            if (c0 + j <= pm) o[(int64_t)j * g.ld_pack] = (TO)v[j];
         }
-        __syncwarp();
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -475,43 +500,28 @@ __global__ void __launch_bounds__(256) split_slices_kernel(const double *src64, 
   }
 }
 
-// full column-major pair matrix from the 8-fold packed vector: one block per
+// full symmetric pair matrix (rows of ld) from the 8-fold packed vector, rounded to FP32 as every slice is before it is
+// split: one block per
 // 32x32 tile of the lower triangle (row tile >= column tile), read along
 // packed rows, written to both triangles through a shared-memory transpose
-__global__ void __launch_bounds__(256) expand_packed8_kernel(const double *packed, int64_t np, double *full) {
-  __shared__ double tile[32][33];
+__global__ void __launch_bounds__(256) expand_packed8_kernel(const double *packed, int64_t np, int64_t ld, float *full) {
+  __shared__ float tile[32][33];
   const int64_t tr = blockIdx.y, tcol = blockIdx.x;
   if (tcol > tr) return;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int y = ty; y < 32; y += 8) {
     const int64_t r = tr * 32 + y, c = tcol * 32 + tx;
-    double x = 0.0;
+    float x = 0.0f;
     if (r < np && c <= r) {
-      x = packed[r * (r + 1) / 2 + c];
-      full[r * np + c] = x;  // element (c, r): column r, contiguous in c
+      x = (float)packed[r * (r + 1) / 2 + c];
+      full[r * ld + c] = x;  // element (c, r): column r, contiguous in c
     }
     tile[y][tx] = x;
   }
   __syncthreads();
   for (int y = ty; y < 32; y += 8) {
     const int64_t c = tcol * 32 + y, r = tr * 32 + tx;
-    if (r < np && c < r) full[c * np + r] = tile[tx][y];  // element (r, c): column c, contiguous in r
-  }
-}
-
-// out[c*rows + r] = in[r*cols + c] (FP32 tiles), optionally widened to FP64
-template <typename TO>
-__global__ void transpose32_kernel(const float *in, int64_t rows, int64_t cols, TO *out) {
-  __shared__ float tile[32][33];
-  int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    int64_t r = r0 + y, c = c0 + threadIdx.x;
-    if (r < rows && c < cols) tile[y][threadIdx.x] = in[r * cols + c];
-  }
-  __syncthreads();
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    int64_t c = c0 + y, r = r0 + threadIdx.x;
-    if (r < rows && c < cols) out[c * rows + r] = (TO)tile[threadIdx.x][y];
+    if (r < np && c < r) full[c * ld + r] = tile[tx][y];  // element (r, c): column c, contiguous in r
   }
 }
 
@@ -563,26 +573,24 @@ struct Operand {
   int64_t ld;    // row length in elements
 };
 
-template <bool TF32, int EPI>
-static pq_status run_gemm(const Operand &A, const Operand &B, bool a_batched, bool b_batched, int M, int N, int K,
-                          int nbatch, const tc::GemmArgs &gin, cudaStream_t st) {
+// EPI_SPLIT: U^T of nbatch slices (A = C^T, B = the slices); EPI_PACK: M = n_mo * nbp rows of U^T times C
+template <bool TF32, int EPI, typename TO>
+static pq_status run_gemm(const Operand &A, const Operand &B, int M, int N, int K, int nbatch, const tc::GemmArgs &gin,
+                          cudaStream_t st) {
   CUtensorMap ma_hi, ma_lo, mb_hi, mb_lo;
   PQ_TRY(make_map(&ma_hi, A.hi, TF32, A.rows, K, A.ld, tc::BM));
   PQ_TRY(make_map(&ma_lo, A.lo, TF32, A.rows, K, A.ld, tc::BM));
-  PQ_TRY(make_map(&mb_hi, B.hi, TF32, B.rows, K, B.ld, tc::BN));
-  PQ_TRY(make_map(&mb_lo, B.lo, TF32, B.rows, K, B.ld, tc::BN));
+  PQ_TRY(make_map(&mb_hi, B.hi, TF32, B.rows, K, B.ld, tc::B_BOX));
+  PQ_TRY(make_map(&mb_lo, B.lo, TF32, B.rows, K, B.ld, tc::B_BOX));
   tc::GemmArgs g = gin;
   g.M = M;
   g.N = N;
   g.K = K;
   g.m_tiles = (M + tc::BM - 1) / tc::BM;
-  g.a_batched = a_batched;
-  g.b_batched = b_batched;
-  g.a_rows = M;
   g.b_rows = N;
   g.nbatch = nbatch;
   g.wait_cycles = g_gemm_wait_cycles;
-  auto kern = tc::tc_gemm_kernel<TF32, EPI>;
+  auto kern = tc::tc_gemm_kernel<TF32, EPI, TO>;
   PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES));
   int dev = 0, sms = 0;
   PQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -598,10 +606,10 @@ static pq_status run_gemm(const Operand &A, const Operand &B, bool a_batched, bo
 // transforms allocate nothing; calls on one device are serialised by the mutex (they share the buffers, and
 // each call synchronises its stream before it returns).  pq_ao2mo_release_workspace frees them.
 struct Ao2moWorkspace {
-  DevBuf full, cth, ctl, sh, sl, uh, ul, H1, H1t, Erow, err;
+  DevBuf full, cth, ctl, sh, sl, uh, ul, H1, err;
   Ao2moF64 f64;
   void release() {
-    for (DevBuf *b : {&full, &cth, &ctl, &sh, &sl, &uh, &ul, &H1, &H1t, &Erow, &err}) b->release();
+    for (DevBuf *b : {&full, &cth, &ctl, &sh, &sl, &uh, &ul, &H1, &err}) b->release();
     f64.release();
   }
 };
@@ -650,18 +658,21 @@ static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, cons
   std::lock_guard<std::mutex> lock(g_ws_mu);
   Ao2moWorkspace &w = g_ws[dev];
   DevBuf &full = w.full, &cth = w.cth, &ctl = w.ctl, &sh = w.sh, &sl = w.sl, &uh = w.uh, &ul = w.ul, &H1 = w.H1,
-         &H1t = w.H1t, &err = w.err;
+         &err = w.err;
   const double *pairs = eri_ao;
+  const float *pairs32 = nullptr;
+  const int64_t ld1 = (npa + 31) / 32 * 32;  // AO pairs in a row of the FP32 pair matrices
   if (layout == PQ_AO_PACKED8) {
-    PQ_TRY(full.ensure(sizeof(double) * npa * npa));
+    PQ_TRY(full.ensure(sizeof(float) * npa * ld1));
     const unsigned nt = (unsigned)((npa + 31) / 32);
     if (nt > 65535) {
       set_error("ao2mo: too many pairs for the expansion grid");
       return PQ_ERR_ARG;
     }
-    tc::expand_packed8_kernel<<<dim3(nt, nt), 256, 0, st>>>(eri_ao, npa, full.as<double>());
+    tc::expand_packed8_kernel<<<dim3(nt, nt), 256, 0, st>>>(eri_ao, npa, ld1, full.as<float>());
     PQ_CUDA_TRY(cudaGetLastError());
-    pairs = full.as<double>();
+    pairs = nullptr;
+    pairs32 = full.as<float>();
   }
   PQ_TRY(err.ensure(sizeof(int)));
   PQ_CUDA_TRY(cudaMemsetAsync(err.ptr, 0, sizeof(int), st));
@@ -672,70 +683,46 @@ static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, cons
                                                                                ctl.as<E>());
   PQ_CUDA_TRY(cudaGetLastError());
   // slices per batch: S (n x ld) and U^T (nm x ld) in hi/lo
-  const int64_t bt = std::max<int64_t>(1, std::min<int64_t>(std::max(npa, npm), 4096));
+  // (BF16x3, 200 AOs to 160 MOs: 12.1 ms with 4096 slices in a batch, 10.6 with 1216, 10.5 with 608, 11.8 with 304;
+  // 128 AOs: 1.81 / 1.84 / 2.10 / 2.72)
+  const int64_t bt = std::min<int64_t>(npa, 1216), btp = (bt + 31) / 32 * 32;
   PQ_TRY(sh.ensure(sizeof(E) * bt * n * ld));
   PQ_TRY(sl.ensure(sizeof(E) * bt * n * ld));
-  PQ_TRY(uh.ensure(sizeof(E) * bt * nm * ld));
-  PQ_TRY(ul.ensure(sizeof(E) * bt * nm * ld));
-  PQ_TRY(H1.ensure(sizeof(float) * npa * npm));
+  PQ_TRY(uh.ensure(sizeof(E) * btp * nm * ld));
+  PQ_TRY(ul.ensure(sizeof(E) * btp * nm * ld));
+  PQ_TRY(H1.ensure(sizeof(float) * npm * ld1));
   tc::GemmArgs g{};
   g.err = err.as<int>();
   Operand ct{cth.ptr, ctl.ptr, nm, ld};
-  auto half = [&](const double *src64, const float *src32, int64_t ld_src, int64_t nslices, float *out) -> pq_status {
+  auto half = [&](auto *out, const double *src64, const float *src32, int64_t ld_src, int64_t nslices,
+                  int64_t ld_out) -> pq_status {
+    using TO = std::remove_pointer_t<decltype(out)>;
     for (int64_t b0 = 0; b0 < nslices; b0 += bt) {
       const int nb = (int)std::min(bt, nslices - b0);
       const unsigned ntile = (unsigned)((n + 31) / 32);
       tc::split_slices_kernel<TF32><<<dim3((unsigned)nb, ntile * ntile), 256, 0, st>>>(src64, src32, ld_src, (int)n, ld,
                                                                                       b0, sh.as<E>(), sl.as<E>());
       PQ_CUDA_TRY(cudaGetLastError());
-      // GEMM 1: U^T[b] (nm x n) = Ct (nm x n) . S[b]^T, K = n
+      tc::GemmArgs gb = g;
+      gb.nb = nb;
+      gb.nbp = (nb + 31) / 32 * 32;
+      // GEMM 1: U^T[b] (nm x n) = Ct (nm x n) . S[b]^T, K = n, row (m, b)
       Operand S{sh.ptr, sl.ptr, (int64_t)nb * n, ld};
-      tc::GemmArgs g1 = g;
-      g1.out_hi = uh.ptr;
-      g1.out_lo = ul.ptr;
-      g1.ld_out = ld;
-      PQ_TRY((run_gemm<TF32, tc::EPI_SPLIT>(ct, S, false, true, (int)nm, (int)n, (int)n, nb, g1, st)));
-      // GEMM 2: T[b] (nm x nm) = U^T[b] . Ct^T, K = n; packed lower triangle
-      Operand U{uh.ptr, ul.ptr, (int64_t)nb * nm, ld};
-      tc::GemmArgs g2 = g;
-      g2.out_pack = out + b0 * npm;
-      g2.pack_stride = npm;
-      PQ_TRY((run_gemm<TF32, tc::EPI_PACK>(U, ct, true, false, (int)nm, (int)nm, (int)n, nb, g2, st)));
+      gb.out_hi = uh.ptr;
+      gb.out_lo = ul.ptr;
+      gb.ld_out = ld;
+      PQ_TRY((run_gemm<TF32, tc::EPI_SPLIT, float>(ct, S, (int)nm, (int)n, (int)n, nb, gb, st)));
+      // GEMM 2: T (rows (m, b) x nm) = U^T . Ct^T, K = n; the pairs n <= m
+      Operand U{uh.ptr, ul.ptr, nm * gb.nbp, ld};
+      gb.out_pack = out + b0;
+      gb.ld_pack = ld_out;
+      PQ_TRY((run_gemm<TF32, tc::EPI_PACK, TO>(U, ct, (int)nm * gb.nbp, (int)nm, (int)n, 1, gb, st)));
     }
     return PQ_OK;
   };
-  // half 1 over AO ket pairs: H1[ket][ij]
-  PQ_TRY(half(pairs, nullptr, npa, npa, H1.as<float>()));
-  // H1t[ij][ket], in the expanded pair matrix's memory when there is one (it is not read again):
-  // each reuse saves an allocation and a synchronising free inside the call
-  float *h1t = nullptr;
-  if (layout == PQ_AO_PACKED8 && full.bytes >= sizeof(float) * npa * npm) {
-    h1t = full.as<float>();
-  } else {
-    PQ_TRY(H1t.ensure(sizeof(float) * npa * npm));
-    h1t = H1t.as<float>();
-  }
-  {
-    dim3 grid((unsigned)((npm + 31) / 32), (unsigned)((npa + 31) / 32));
-    if (grid.y > 65535) {
-      set_error("ao2mo: too many pairs for the transpose grid");
-      return PQ_ERR_ARG;
-    }
-    tc::transpose32_kernel<float><<<grid, dim3(32, 8), 0, st>>>(H1.as<float>(), npa, npm, h1t);
-    PQ_CUDA_TRY(cudaGetLastError());
-  }
-  // half 2 over MO bra pairs: Erow[ij][kl], in H1's memory when it fits (npm <= npa); slices read from rows of H1t
-  float *erow = H1.as<float>();
-  if (npm > npa) {
-    PQ_TRY(w.Erow.ensure(sizeof(float) * npm * npm));
-    erow = w.Erow.as<float>();
-  }
-  PQ_TRY(half(nullptr, h1t, npa, npm, erow));
-  {
-    dim3 grid((unsigned)((npm + 31) / 32), (unsigned)((npm + 31) / 32));
-    tc::transpose32_kernel<double><<<grid, dim3(32, 8), 0, st>>>(erow, npm, npm, eri_mo);
-    PQ_CUDA_TRY(cudaGetLastError());
-  }
+  // half 1 over AO ket pairs: H1[ij][ket]; half 2 over its rows, MO bra pairs: eri_mo[kl][ij]
+  PQ_TRY(half(H1.as<float>(), pairs, pairs32, pairs32 ? ld1 : npa, npa, ld1));
+  PQ_TRY(half(eri_mo, nullptr, H1.as<float>(), ld1, npm, npm));
   int herr = 0;
   PQ_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   PQ_CUDA_TRY(cudaStreamSynchronize(st));
