@@ -9,7 +9,8 @@
 // GEMM 1 leaves U^T with rows (m, slice).  A tile of GEMM 2 then holds 128 slices of one m, or a few m: it loads and
 // multiplies only the columns n <= m, half of the work, and its 32 lanes hold 32 slices, so that a pair (m, n) is
 // written along the slices, as half 2 reads it and as the result wants it, and no transpose is left (256 AOs, BF16x3:
-// two transposes of 13 + 8.7 GB and the FP64 expansion, 35.8 ms in all; now 25.0).
+// two transposes of 13 + 8.7 GB and the FP64 expansion, 35.8 ms in all; without them 24.7).  In BF16 GEMM 1 reads the
+// slices from their pair rows (slice_gemm_kernel); in TF32 they are split in memory first.
 // Operands are split into a high and a low part (x = x_hi + x_lo) in BF16 or
 // TF32 and each product is formed as hi*hi + hi*lo + lo*hi with FP32
 // accumulation in tensor memory (three MMAs per K step).  BF16 and TF32 keep
@@ -67,7 +68,7 @@ struct GemmArgs {
   int b_rows;
   int nb, nbp;                 // slices of this batch, and up to a multiple of 32
   int ld_out;                  // EPI_SPLIT: row length of the split output
-  void *out_hi, *out_lo;       // EPI_SPLIT outputs, rows (m, slice)
+  float *out_hi, *out_lo;      // EPI_SPLIT outputs (TF32), rows (m, slice)
   void *out_pack;              // EPI_PACK output [pair (m, n)][ld_pack], slice b of this batch in column b
   int64_t ld_pack;
   long long wait_cycles;       // budget of the pipeline waits (the wind-down waits keep WAIT_CYCLES)
@@ -194,6 +195,7 @@ template <bool TF32, int EPI, typename TO>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
                    const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo, GemmArgs g) {
+  static_assert(TF32 || EPI == EPI_PACK, "BF16 slices go through slice_gemm_kernel");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // 1024-byte alignment of the shared-window address (128-byte swizzle atoms)
   unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -352,39 +354,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
             for (int k = 0; k < 8; k++) x[k] = stg[rr * EPI_LD + cq + k];
             const int64_t o = ((int64_t)m * g.nbp + b) * g.ld_out + n0;
-            if constexpr (TF32) {
-              float h[8], l[8];
+            float h[8], l[8];
 #pragma unroll
-              for (int k = 0; k < 8; k++) {
-                h[k] = tf32_round(x[k]);
-                l[k] = tf32_round(x[k] - h[k]);
-              }
-              float *oh = static_cast<float *>(g.out_hi) + o, *ol = static_cast<float *>(g.out_lo) + o;
-              if (n0 + 8 <= g.N) {
-                reinterpret_cast<float4 *>(oh)[0] = make_float4(h[0], h[1], h[2], h[3]);
-                reinterpret_cast<float4 *>(oh)[1] = make_float4(h[4], h[5], h[6], h[7]);
-                reinterpret_cast<float4 *>(ol)[0] = make_float4(l[0], l[1], l[2], l[3]);
-                reinterpret_cast<float4 *>(ol)[1] = make_float4(l[4], l[5], l[6], l[7]);
-              } else {
-                for (int k = 0; k < g.N - n0; k++) oh[k] = h[k], ol[k] = l[k];
-              }
+            for (int k = 0; k < 8; k++) {
+              h[k] = tf32_round(x[k]);
+              l[k] = tf32_round(x[k] - h[k]);
+            }
+            float *oh = g.out_hi + o, *ol = g.out_lo + o;
+            if (n0 + 8 <= g.N) {
+              reinterpret_cast<float4 *>(oh)[0] = make_float4(h[0], h[1], h[2], h[3]);
+              reinterpret_cast<float4 *>(oh)[1] = make_float4(h[4], h[5], h[6], h[7]);
+              reinterpret_cast<float4 *>(ol)[0] = make_float4(l[0], l[1], l[2], l[3]);
+              reinterpret_cast<float4 *>(ol)[1] = make_float4(l[4], l[5], l[6], l[7]);
             } else {
-              __nv_bfloat162 h2[4], l2[4];
-#pragma unroll
-              for (int k = 0; k < 4; k++) {
-                h2[k] = __floats2bfloat162_rn(x[2 * k], x[2 * k + 1]);
-                l2[k] = __floats2bfloat162_rn(x[2 * k] - __low2float(h2[k]), x[2 * k + 1] - __high2float(h2[k]));
-              }
-              __nv_bfloat16 *oh = static_cast<__nv_bfloat16 *>(g.out_hi) + o;
-              __nv_bfloat16 *ol = static_cast<__nv_bfloat16 *>(g.out_lo) + o;
-              if (n0 + 8 <= g.N) {
-                *reinterpret_cast<uint4 *>(oh) = *reinterpret_cast<const uint4 *>(h2);
-                *reinterpret_cast<uint4 *>(ol) = *reinterpret_cast<const uint4 *>(l2);
-              } else {
-                const __nv_bfloat16 *hs = reinterpret_cast<const __nv_bfloat16 *>(h2);
-                const __nv_bfloat16 *ls = reinterpret_cast<const __nv_bfloat16 *>(l2);
-                for (int k = 0; k < g.N - n0; k++) oh[k] = hs[k], ol[k] = ls[k];
-              }
+              for (int k = 0; k < g.N - n0; k++) oh[k] = h[k], ol[k] = l[k];
             }
           }
           __syncwarp();
@@ -438,30 +421,19 @@ __global__ void split_ct_kernel(const double *C, int64_t ldc, int n_ao, int n_mo
   Split<TF32>::run(x, hi[i], lo[i]);
 }
 
-__device__ __forceinline__ int64_t tri64(int64_t i, int64_t j) { return i > j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
-
-// slice b of a pair-matrix source, split: S[b][nu][mu] = src(tri(mu,nu), b0 + b)
+// slice b of a pair-matrix source, split (TF32): S[b][nu][mu] = src(tri(mu,nu), b0 + b)
 // src64: column-major (ld x ncols) FP64 pair matrix (element (r, c) at r + c*ld)
 // src32: row-major FP32 pair rows (element (r, c) at c*ld + r), i.e. row c holds the slice
-// Split two consecutive row elements (a at o, b at o + 1; o even, so the pair
-// is 4-byte (BF16) or 8-byte (TF32) aligned) into hi/lo with one vector store
+// Two consecutive row elements (a at o, b at o + 1; o even, so the pair is 8-byte aligned) go with one vector store
 // each when both are wanted.
-template <bool TF32>
-__device__ __forceinline__ void split_store2(typename Split<TF32>::T *H, typename Split<TF32>::T *L, int64_t o, float a,
-                                             float b, bool va, bool vb) {
+__device__ __forceinline__ void split_store2(float *H, float *L, int64_t o, float a, float b, bool va, bool vb) {
   if (va && vb) {
-    if constexpr (TF32) {
-      const float ha = tf32_round(a), hb = tf32_round(b);
-      *reinterpret_cast<float2 *>(H + o) = make_float2(ha, hb);
-      *reinterpret_cast<float2 *>(L + o) = make_float2(tf32_round(a - ha), tf32_round(b - hb));
-    } else {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-      *reinterpret_cast<__nv_bfloat162 *>(H + o) = h;
-      *reinterpret_cast<__nv_bfloat162 *>(L + o) = __floats2bfloat162_rn(a - __low2float(h), b - __high2float(h));
-    }
+    const float ha = tf32_round(a), hb = tf32_round(b);
+    *reinterpret_cast<float2 *>(H + o) = make_float2(ha, hb);
+    *reinterpret_cast<float2 *>(L + o) = make_float2(tf32_round(a - ha), tf32_round(b - hb));
   } else {
-    if (va) Split<TF32>::run(a, H[o], L[o]);
-    if (vb) Split<TF32>::run(b, H[o + 1], L[o + 1]);
+    if (va) Split<true>::run(a, H[o], L[o]);
+    if (vb) Split<true>::run(b, H[o + 1], L[o + 1]);
   }
 }
 
@@ -470,16 +442,14 @@ __device__ __forceinline__ void split_store2(typename Split<TF32>::T *H, typenam
 // upper one through a shared-memory transpose, so loads and stores are
 // coalesced and every slice spreads over many SMs.  Each thread handles two
 // consecutive columns (16 column pairs x 16 rows per pass).
-template <bool TF32>
 __global__ void __launch_bounds__(256) split_slices_kernel(const double *src64, const float *src32, int64_t ld, int n,
-                                                           int ld_row, int64_t b0, typename Split<TF32>::T *hi,
-                                                           typename Split<TF32>::T *lo) {
+                                                           int ld_row, int64_t b0, float *hi, float *lo) {
   __shared__ float tile[32][33];
   const int nt = (n + 31) / 32;
   const int tv = blockIdx.y / nt, tm = blockIdx.y - tv * nt;
   if (tm > tv) return;
   const int64_t b = blockIdx.x, c = b0 + b;
-  typename Split<TF32>::T *H = hi + b * (int64_t)n * ld_row, *L = lo + b * (int64_t)n * ld_row;
+  float *H = hi + b * (int64_t)n * ld_row, *L = lo + b * (int64_t)n * ld_row;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   for (int y = ty; y < 32; y += 16) {
     const int nu = tv * 32 + y, mu = tm * 32 + 2 * tx;
@@ -488,7 +458,7 @@ __global__ void __launch_bounds__(256) split_slices_kernel(const double *src64, 
     const int64_t pr = (int64_t)nu * (nu + 1) / 2 + mu;
     if (va) xa = src64 ? (float)src64[pr + c * ld] : src32[c * ld + pr];
     if (vb) xb = src64 ? (float)src64[pr + 1 + c * ld] : src32[c * ld + pr + 1];
-    split_store2<TF32>(H, L, (int64_t)nu * ld_row + mu, xa, xb, va, vb);
+    split_store2(H, L, (int64_t)nu * ld_row + mu, xa, xb, va, vb);
     tile[y][2 * tx] = xa;
     tile[y][2 * tx + 1] = xb;
   }
@@ -496,7 +466,7 @@ __global__ void __launch_bounds__(256) split_slices_kernel(const double *src64, 
   for (int y = ty; y < 32; y += 16) {
     const int row = tm * 32 + y, nu = tv * 32 + 2 * tx;
     const bool va = nu < n && row < nu, vb = nu + 1 < n && row < nu + 1;
-    split_store2<TF32>(H, L, (int64_t)row * ld_row + nu, tile[2 * tx][y], tile[2 * tx + 1][y], va, vb);
+    split_store2(H, L, (int64_t)row * ld_row + nu, tile[2 * tx][y], tile[2 * tx + 1][y], va, vb);
   }
 }
 
@@ -524,6 +494,296 @@ __global__ void __launch_bounds__(256) expand_packed8_kernel(const double *packe
     if (r < np && c < r) full[c * ld + r] = tile[tx][y];  // element (r, c): column c, contiguous in r
   }
 }
+
+// ---------------------------------------------------------------------------
+// GEMM 1 for BF16 straight from the pair rows: the slices S are not written anywhere.  A CTA keeps its 128 rows of C^T
+// (hi and lo, all of K: 128 KB) and takes one slice after another.  16 producer warps read the packed symmetric slice
+// (FP32 rows, or a caller's FP64 pair matrix), 16 rows nu each, 32 columns mu a stage: below the diagonal along mu,
+// above it along nu, a stage ahead of the one being written; they split the values and write both parts as K-major
+// rows of 64 bytes (64-byte swizzle).  Values, split, K order and the three products of a step are those of
+// tc_gemm_kernel, so are the results.  Four warps turn an accumulator into the split U^T, 32 columns at a time through
+// swizzled staging that TMA stores (rows (m, slice)), while the MMAs of the next slice fill the other accumulator.
+// The pair of CTAs that shares a slice reads it through L2, where one of them prefetches it (one slice ahead): 45 GB of
+// 128-byte requests over both halves at 256 AOs are what bounds it (5.4 of 10 ms go with the loads, 1.7 with the split
+// and its stores, 0.5 with the TMA stores).  256 AOs: 24.7 ms with the slices split in memory, 20.2 so, 18.6 with the
+// prefetch (19.3 with the values two stages ahead); 200 AOs to 160 MOs 10.6 -> 6.6, 128 AOs 1.84 -> 1.29, 24 AOs
+// 0.14 -> 0.12.  In TF32 C^T takes twice the room and does not stay in shared memory: it keeps the other way.
+namespace slices {
+constexpr int KC = 32;                        // K of a stage
+constexpr int PROD_WARPS = 16, EPI0 = PROD_WARPS, MMA_WARP = EPI0 + EPI_WARPS;
+constexpr int THREADS = 32 * (MMA_WARP + 1);
+constexpr int A_BYTES = 2 * (BN / 64) * A_TILE;  // [hi, lo][block of 64 k][128 rows]
+constexpr int B_HALF = BN * KC * 2;              // 16 KB: hi or lo of a stage
+constexpr int NSTAGE = 2;
+constexpr int STG = 32 * KC * 2;                 // 2 KB: 32 rows x 32 columns of one part
+constexpr int SMEM = A_BYTES + NSTAGE * 2 * B_HALF + EPI_WARPS * 2 * 2 * STG + 1024 + 256;
+static_assert(SMEM <= 227 * 1024, "shared memory");
+
+struct Args {
+  int n, nm, m_tiles, nslices;  // slices of this launch
+  int64_t ld;                   // source row length
+  const void *src;              // first slice
+  long long wait_cycles;
+  int *err;
+};
+
+__device__ __forceinline__ uint64_t desc_k64(uint32_t addr) {  // rows of 64 bytes, 64-byte swizzle, 8 rows 512 B
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)4 << 61;
+}
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(src), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+__device__ __forceinline__ void split2(float a, float b, uint32_t &h, uint32_t &l) {
+  const __nv_bfloat162 hh = __floats2bfloat162_rn(a, b);
+  const __nv_bfloat162 ll = __floats2bfloat162_rn(a - __low2float(hh), b - __high2float(hh));
+  h = *reinterpret_cast<const uint32_t *>(&hh);
+  l = *reinterpret_cast<const uint32_t *>(&ll);
+}
+
+// 16 rows nu0 .. of the slice and 32 columns mu0 ..; over: the whole block is above the diagonal.
+// Below or on it lane = mu and v[r] = S[nu0 + r][mu]; above it lane = (half of mu, row) and v[k] = S[nu][mu of the half + k]
+template <typename TS>
+__device__ __forceinline__ void load16(const TS *s, int n, int nu0, int mu0, bool over, int lane, float (&v)[16]) {
+  if (over) {
+    const int nu = nu0 + (lane & 15), m0 = mu0 + (lane & 16);
+    int o = m0 * (m0 + 1) / 2 + nu;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      v[k] = m0 + k < n ? (float)s[o] : 0.0f;  // nu < m0
+      o += m0 + k + 1;
+    }
+  } else {
+    const int mu = mu0 + lane;
+    const int up = mu * (mu + 1) / 2;
+    int row = nu0 * (nu0 + 1) / 2;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      const int nu = nu0 + r;
+      v[r] = nu < n && mu < n ? (float)s[mu <= nu ? row + mu : up + nu] : 0.0f;
+      row += nu + 1;
+    }
+  }
+}
+__device__ __forceinline__ void store16(unsigned char *hi, int nu0, bool over, int lane, const float (&v)[16]) {
+  unsigned char *lo = hi + B_HALF;
+  if (over) {
+    const int r = nu0 + (lane & 15), c = (lane & 16) >> 3;  // 16-byte chunks c, c + 1 of the row
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      uint4 h, l;
+      split2(v[8 * q], v[8 * q + 1], h.x, l.x);
+      split2(v[8 * q + 2], v[8 * q + 3], h.y, l.y);
+      split2(v[8 * q + 4], v[8 * q + 5], h.z, l.z);
+      split2(v[8 * q + 6], v[8 * q + 7], h.w, l.w);
+      const int o = r * 64 + (((c + q) ^ ((r >> 1) & 3)) << 4);
+      *reinterpret_cast<uint4 *>(hi + o) = h;
+      *reinterpret_cast<uint4 *>(lo + o) = l;
+    }
+  } else {
+    // lanes exchange in pairs: the even one packs (mu, mu + 1) of row 2 k, the odd one (mu - 1, mu) of row 2 k + 1
+    const int odd = lane & 1, c = lane >> 3, w = (lane >> 1) & 3;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const float mine = odd ? v[2 * k + 1] : v[2 * k];
+      const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * k] : v[2 * k + 1], 1);
+      uint32_t h, l;
+      split2(odd ? got : mine, odd ? mine : got, h, l);
+      const int r = nu0 + 2 * k + odd;
+      const int o = r * 64 + ((c ^ ((r >> 1) & 3)) << 4) + w * 4;
+      *reinterpret_cast<uint32_t *>(hi + o) = h;
+      *reinterpret_cast<uint32_t *>(lo + o) = l;
+    }
+  }
+}
+
+template <typename TS>
+__global__ void __launch_bounds__(THREADS, 1)
+    slice_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
+                      const __grid_constant__ CUtensorMap tmU_hi, const __grid_constant__ CUtensorMap tmU_lo, Args g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  unsigned char *smB = smem + A_BYTES, *smE = smB + NSTAGE * 2 * B_HALF;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smE + EPI_WARPS * 2 * 2 * STG);
+  uint64_t *afull = bars, *full = bars + 1, *empty = full + NSTAGE, *accf = empty + NSTAGE, *acce = accf + 2,
+           *drain = acce + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nst = (g.n + KC - 1) / KC, cols = (g.n + 15) / 16 * 16;
+  const int mt = blockIdx.x % g.m_tiles, first = blockIdx.x / g.m_tiles, step = gridDim.x / g.m_tiles;
+
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(afull), 1);
+    for (int i = 0; i < NSTAGE; i++) {
+      mbar_init(smem_u32(full + i), PROD_WARPS);
+      mbar_init(smem_u32(empty + i), 1);
+    }
+    for (int a = 0; a < 2; a++) {
+      mbar_init(smem_u32(accf + a), 1);
+      mbar_init(smem_u32(acce + a), EPI_WARPS);
+    }
+    mbar_init(smem_u32(drain), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(2 * BN)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp < PROD_WARPS) {
+    // ---- producers: 16 rows each, one stage of values ahead
+    const int nu0 = warp * 16;
+    const bool mine = nu0 < g.n;
+    const TS *src = static_cast<const TS *>(g.src);
+    float v0[16], v1[16];
+    int lb = first, ls = 0;  // the next values to load
+    auto load = [&](float (&v)[16]) {
+      if (lb < g.nslices) {
+        if (mine) load16(src + lb * g.ld, g.n, nu0, ls * KC, nu0 + 16 <= ls * KC, lane, v);
+        if (++ls == nst) ls = 0, lb += step;
+      }
+    };
+    load(v0);
+    // FP32 rows start at multiples of 128 bytes; a bulk prefetch takes multiples of 16
+    const uint32_t pf = sizeof(TS) == 4 && threadIdx.x == 0 && mt == 0 ? (uint32_t)(g.n * (g.n + 1) / 2 * 4) & ~15u : 0u;
+    int b = first, s = 0, it = 0;
+    while (b < g.nslices) {
+      // the slice after this one into L2, once for the tiles that share it
+      if (pf && s == 0 && b + step < g.nslices)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + (b + step) * g.ld), "r"(pf) : "memory");
+      load(v1);
+      const int slot = it % NSTAGE;
+      const bool ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((it / NSTAGE) & 1) ^ 1u, g.wait_cycles);
+      if (!ok || *abort_flag) {
+        if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_MMA);
+        *abort_flag = 1;
+        break;
+      }
+      if (mine) store16(smB + slot * 2 * B_HALF, nu0, nu0 + 16 <= s * KC, lane, v0);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(full + slot));
+#pragma unroll
+      for (int k = 0; k < 16; k++) v0[k] = v1[k];
+      if (++s == nst) s = 0, b += step;
+      it++;
+    }
+  } else if (warp == MMA_WARP) {
+    if (lane == 0) {
+      mbar_expect_tx(smem_u32(afull), (uint32_t)(2 * ((g.n + 63) / 64) * A_TILE));
+      for (int k = 0; k * 64 < g.n; k++) {
+        tma_load_2d(smem_u32(smem + k * A_TILE), &tmA_hi, k * 64, mt * BM, smem_u32(afull));
+        tma_load_2d(smem_u32(smem + A_BYTES / 2 + k * A_TILE), &tmA_lo, k * 64, mt * BM, smem_u32(afull));
+      }
+      if (!mbar_wait(smem_u32(afull), 0, g.wait_cycles)) {
+        atomicCAS(g.err, 0, ERR_TIMEOUT_FULL);
+        *abort_flag = 1;
+      }
+      const uint32_t idesc = instr_desc(1u, cols);
+      int it = 0, i = 0;
+      for (int b = first; b < g.nslices && !*abort_flag; b += step, i++) {
+        const int a = i & 1;
+        if (!mbar_wait(smem_u32(acce + a), (uint32_t)((i >> 1) & 1) ^ 1u, g.wait_cycles)) {
+          atomicCAS(g.err, 0, ERR_TIMEOUT_ACC);
+          *abort_flag = 1;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d = tmem + (uint32_t)(a * BN);
+        bool ok = true;
+        for (int s = 0; s < nst; s++, it++) {
+          const int slot = it % NSTAGE;
+          if (!mbar_wait(smem_u32(full + slot), (uint32_t)((it / NSTAGE) & 1), g.wait_cycles)) {
+            atomicCAS(g.err, 0, ERR_TIMEOUT_FULL);
+            *abort_flag = 1;
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a_hi = smem_u32(smem + (s >> 1) * A_TILE) + (s & 1) * 64, a_lo = a_hi + A_BYTES / 2;
+          const uint32_t b_hi = smem_u32(smB + slot * 2 * B_HALF), b_lo = b_hi + B_HALF;
+#pragma unroll
+          for (int kk = 0; kk < KC / 16; kk++) {
+            const uint32_t o = kk * 32;
+            mma<false>(d, smem_desc(a_hi + o), desc_k64(b_hi + o), idesc, s > 0 || kk > 0);
+            mma<false>(d, smem_desc(a_hi + o), desc_k64(b_lo + o), idesc, 1u);
+            mma<false>(d, smem_desc(a_lo + o), desc_k64(b_hi + o), idesc, 1u);
+          }
+          mma_commit(smem_u32(empty + slot));
+        }
+        if (!ok) break;
+        mma_commit(smem_u32(accf + a));
+      }
+      // no load or MMA of this CTA is in flight when it leaves
+      mma_commit(smem_u32(drain));
+      mbar_wait(smem_u32(drain), 0);
+      mbar_wait(smem_u32(afull), 0);
+    }
+  } else {
+    // ---- epilogue
+    const int q = warp & 3;
+    unsigned char *stg = smE + (warp - EPI0) * 2 * 2 * STG;
+    const int m0 = mt * BM + q * 32;
+    int i = 0, buf = 0;
+    for (int b = first; b < g.nslices; b += step, i++) {
+      const int a = i & 1;
+      const bool ok = mbar_wait(smem_u32(accf + a), (uint32_t)((i >> 1) & 1), g.wait_cycles);
+      if (!ok || *abort_flag) {
+        if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_ACC);
+        *abort_flag = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (m0 < g.nm) {
+        for (int c0 = 0; c0 < g.n; c0 += KC, buf ^= 1) {
+          float x[32];
+          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + c0), x);
+          unsigned char *hi = stg + buf * 2 * STG, *lo = hi + STG;
+          // the stores that last read this buffer are through with it
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            uint4 h, l;
+            split2(x[8 * c], x[8 * c + 1], h.x, l.x);
+            split2(x[8 * c + 2], x[8 * c + 3], h.y, l.y);
+            split2(x[8 * c + 4], x[8 * c + 5], h.z, l.z);
+            split2(x[8 * c + 6], x[8 * c + 7], h.w, l.w);
+            const int o = lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4);
+            *reinterpret_cast<uint4 *>(hi + o) = h;
+            *reinterpret_cast<uint4 *>(lo + o) = l;
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmU_hi, smem_u32(hi), c0, b, m0);
+            tma_store_3d(&tmU_lo, smem_u32(lo), c0, b, m0);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(acce + a));
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == MMA_WARP)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+}
+}  // namespace slices
 
 }  // namespace tc
 
@@ -598,6 +858,38 @@ static pq_status run_gemm(const Operand &A, const Operand &B, int M, int N, int 
   const int64_t tiles = (int64_t)nbatch * g.m_tiles;
   const int grid = (int)std::min<int64_t>(tiles, sms);  // persistent: one CTA per SM
   kern<<<grid, tc::GEMM_THREADS, tc::SMEM_BYTES, st>>>(ma_hi, ma_lo, mb_hi, mb_lo, g);
+  PQ_CUDA_TRY(cudaGetLastError());
+  return PQ_OK;
+}
+
+// GEMM 1 of nb slices (BF16) from their pair rows src (FP32 or FP64, ld apart)
+template <typename TS>
+static pq_status run_slices(const Operand &ct, void *uh, void *ul, const TS *src, int64_t ld_src, int n, int nm, int nb,
+                            int nbp, int64_t ld, int *err, cudaStream_t st) {
+  auto fn = encode_fn();
+  CUtensorMap ma[2], mu[2];
+  PQ_TRY(make_map(&ma[0], ct.hi, false, ct.rows, n, ct.ld, tc::BM));
+  PQ_TRY(make_map(&ma[1], ct.lo, false, ct.rows, n, ct.ld, tc::BM));
+  for (int k = 0; k < 2; k++) {
+    cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)nb, (cuuint64_t)nm};
+    cuuint64_t strides[2] = {(cuuint64_t)(2 * ld), (cuuint64_t)(2 * ld * nbp)};
+    cuuint32_t box[3] = {(cuuint32_t)tc::slices::KC, 1, 32}, es[3] = {1, 1, 1};
+    CUresult r = fn(&mu[k], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, k ? ul : uh, dims, strides, box, es,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+      set_error("cuTensorMapEncodeTiled failed (%d): U^T of %d x %d, %d slices", (int)r, nm, n, nb);
+      return PQ_ERR_CUDA;
+    }
+  }
+  tc::slices::Args g{n, nm, (nm + tc::BM - 1) / tc::BM, nb, ld_src, src, g_gemm_wait_cycles, err};
+  auto kern = tc::slices::slice_gemm_kernel<TS>;
+  PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::slices::SMEM));
+  int dev = 0, sms = 0;
+  PQ_CUDA_TRY(cudaGetDevice(&dev));
+  PQ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int groups = std::min(nb, std::max(1, sms / g.m_tiles));
+  kern<<<groups * g.m_tiles, tc::slices::THREADS, tc::slices::SMEM, st>>>(ma[0], ma[1], mu[0], mu[1], g);
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
 }
@@ -686,8 +978,10 @@ static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, cons
   // (BF16x3, 200 AOs to 160 MOs: 12.1 ms with 4096 slices in a batch, 10.6 with 1216, 10.5 with 608, 11.8 with 304;
   // 128 AOs: 1.81 / 1.84 / 2.10 / 2.72)
   const int64_t bt = std::min<int64_t>(npa, 1216), btp = (bt + 31) / 32 * 32;
-  PQ_TRY(sh.ensure(sizeof(E) * bt * n * ld));
-  PQ_TRY(sl.ensure(sizeof(E) * bt * n * ld));
+  if (TF32) {
+    PQ_TRY(sh.ensure(sizeof(E) * bt * n * ld));
+    PQ_TRY(sl.ensure(sizeof(E) * bt * n * ld));
+  }
   PQ_TRY(uh.ensure(sizeof(E) * btp * nm * ld));
   PQ_TRY(ul.ensure(sizeof(E) * btp * nm * ld));
   PQ_TRY(H1.ensure(sizeof(float) * npm * ld1));
@@ -699,19 +993,29 @@ static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, cons
     using TO = std::remove_pointer_t<decltype(out)>;
     for (int64_t b0 = 0; b0 < nslices; b0 += bt) {
       const int nb = (int)std::min(bt, nslices - b0);
-      const unsigned ntile = (unsigned)((n + 31) / 32);
-      tc::split_slices_kernel<TF32><<<dim3((unsigned)nb, ntile * ntile), 256, 0, st>>>(src64, src32, ld_src, (int)n, ld,
-                                                                                      b0, sh.as<E>(), sl.as<E>());
-      PQ_CUDA_TRY(cudaGetLastError());
       tc::GemmArgs gb = g;
       gb.nb = nb;
       gb.nbp = (nb + 31) / 32 * 32;
       // GEMM 1: U^T[b] (nm x n) = Ct (nm x n) . S[b]^T, K = n, row (m, b)
-      Operand S{sh.ptr, sl.ptr, (int64_t)nb * n, ld};
-      gb.out_hi = uh.ptr;
-      gb.out_lo = ul.ptr;
-      gb.ld_out = ld;
-      PQ_TRY((run_gemm<TF32, tc::EPI_SPLIT, float>(ct, S, (int)nm, (int)n, (int)n, nb, gb, st)));
+      if constexpr (!TF32) {
+        if (src64) {
+          PQ_TRY(run_slices(ct, uh.ptr, ul.ptr, src64 + b0 * ld_src, ld_src, (int)n, (int)nm, nb, gb.nbp, ld,
+                            err.as<int>(), st));
+        } else {
+          PQ_TRY(run_slices(ct, uh.ptr, ul.ptr, src32 + b0 * ld_src, ld_src, (int)n, (int)nm, nb, gb.nbp, ld,
+                            err.as<int>(), st));
+        }
+      } else {
+        const unsigned ntile = (unsigned)((n + 31) / 32);
+        tc::split_slices_kernel<<<dim3((unsigned)nb, ntile * ntile), 256, 0, st>>>(
+            src64, src32, ld_src, (int)n, ld, b0, sh.as<float>(), sl.as<float>());
+        PQ_CUDA_TRY(cudaGetLastError());
+        Operand S{sh.ptr, sl.ptr, (int64_t)nb * n, ld};
+        gb.out_hi = uh.as<float>();
+        gb.out_lo = ul.as<float>();
+        gb.ld_out = ld;
+        PQ_TRY((run_gemm<TF32, tc::EPI_SPLIT, float>(ct, S, (int)nm, (int)n, (int)n, nb, gb, st)));
+      }
       // GEMM 2: T (rows (m, b) x nm) = U^T . Ct^T, K = n; the pairs n <= m
       Operand U{uh.ptr, ul.ptr, nm * gb.nbp, ld};
       gb.out_pack = out + b0;
