@@ -499,15 +499,16 @@ __global__ void __launch_bounds__(256) expand_packed8_kernel(const double *packe
 // GEMM 1 for BF16 straight from the pair rows: the slices S are not written anywhere.  A CTA keeps its 128 rows of C^T
 // (hi and lo, all of K: 128 KB) and takes one slice after another.  16 producer warps read the packed symmetric slice
 // (FP32 rows, or a caller's FP64 pair matrix), 16 rows nu each, 32 columns mu a stage: below the diagonal along mu,
-// above it along nu, a stage ahead of the one being written; they split the values and write both parts as K-major
+// above it along nu, two stages ahead; they split the values and write both parts as K-major
 // rows of 64 bytes (64-byte swizzle).  Values, split, K order and the three products of a step are those of
 // tc_gemm_kernel, so are the results.  Four warps turn an accumulator into the split U^T, 32 columns at a time through
 // swizzled staging that TMA stores (rows (m, slice)), while the MMAs of the next slice fill the other accumulator.
 // The pair of CTAs that shares a slice reads it through L2, where one of them prefetches it (one slice ahead): 45 GB of
-// 128-byte requests over both halves at 256 AOs are what bounds it (5.4 of 10 ms go with the loads, 1.7 with the split
-// and its stores, 0.5 with the TMA stores).  256 AOs: 24.7 ms with the slices split in memory, 20.2 so, 18.6 with the
-// prefetch (19.3 with the values two stages ahead); 200 AOs to 160 MOs 10.6 -> 6.6, 128 AOs 1.84 -> 1.29, 24 AOs
-// 0.14 -> 0.12.  In TF32 C^T takes twice the room and does not stay in shared memory: it keeps the other way.
+// requests of 128 unaligned bytes over both halves at 256 AOs are what bounds it (without the loads 5.4 ms less, without
+// the split and its stores 1.7, without the TMA stores 0.5).  256 AOs: 24.7 ms with the slices split in memory, 20.2 so,
+// 18.6 with the prefetch, 17.7 with two stages of values in flight and batches of 2432 slices; 200 AOs to 160 MOs
+// 10.6 -> 6.3, 128 AOs 1.84 -> 1.2, 24 AOs 0.14 -> 0.13.  In TF32 C^T takes twice the room and does not stay in shared
+// memory: it keeps the other way.
 namespace slices {
 constexpr int KC = 32;                        // K of a stage
 constexpr int PROD_WARPS = 16, EPI0 = PROD_WARPS, MMA_WARP = EPI0 + EPI_WARPS;
@@ -641,7 +642,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp < PROD_WARPS) {
-    // ---- producers: 16 rows each, one stage of values ahead
+    // ---- producers: 16 rows each, two stages of values in registers
     const int nu0 = warp * 16;
     const bool mine = nu0 < g.n;
     const TS *src = static_cast<const TS *>(g.src);
@@ -653,30 +654,33 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (++ls == nst) ls = 0, lb += step;
       }
     };
-    load(v0);
     // FP32 rows start at multiples of 128 bytes; a bulk prefetch takes multiples of 16
     const uint32_t pf = sizeof(TS) == 4 && threadIdx.x == 0 && mt == 0 ? (uint32_t)(g.n * (g.n + 1) / 2 * 4) & ~15u : 0u;
     int b = first, s = 0, it = 0;
-    while (b < g.nslices) {
+    // write a stage from v, then fill v for the stage after the next: no register is waited for before it is used
+    auto stage = [&](float (&v)[16]) {
       // the slice after this one into L2, once for the tiles that share it
       if (pf && s == 0 && b + step < g.nslices)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + (b + step) * g.ld), "r"(pf) : "memory");
-      load(v1);
       const int slot = it % NSTAGE;
       const bool ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((it / NSTAGE) & 1) ^ 1u, g.wait_cycles);
       if (!ok || *abort_flag) {
         if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_MMA);
         *abort_flag = 1;
-        break;
+        return false;
       }
-      if (mine) store16(smB + slot * 2 * B_HALF, nu0, nu0 + 16 <= s * KC, lane, v0);
+      if (mine) store16(smB + slot * 2 * B_HALF, nu0, nu0 + 16 <= s * KC, lane, v);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(full + slot));
-#pragma unroll
-      for (int k = 0; k < 16; k++) v0[k] = v1[k];
+      load(v);
       if (++s == nst) s = 0, b += step;
       it++;
+      return true;
+    };
+    load(v0);
+    load(v1);
+    while (b < g.nslices && stage(v0) && b < g.nslices && stage(v1)) {
     }
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
@@ -975,9 +979,9 @@ static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, cons
                                                                                ctl.as<E>());
   PQ_CUDA_TRY(cudaGetLastError());
   // slices per batch: S (n x ld) and U^T (nm x ld) in hi/lo
-  // (BF16x3, 200 AOs to 160 MOs: 12.1 ms with 4096 slices in a batch, 10.6 with 1216, 10.5 with 608, 11.8 with 304;
-  // 128 AOs: 1.81 / 1.84 / 2.10 / 2.72)
-  const int64_t bt = std::min<int64_t>(npa, 1216), btp = (bt + 31) / 32 * 32;
+  // (BF16x3, 256 AOs: 19.9 ms with 608 slices in a batch, 18.6 with 1216, 17.9 with 2432, 18.1 with 4864; 128 AOs:
+  // 1.48 / 1.26 / 1.18 / 1.11; TF32x3, 200 AOs: 14.1 with 1216, 14.5 with 4096)
+  const int64_t bt = std::min<int64_t>(npa, 2432), btp = (bt + 31) / 32 * 32;
   if (TF32) {
     PQ_TRY(sh.ensure(sizeof(E) * bt * n * ld));
     PQ_TRY(sl.ensure(sizeof(E) * bt * n * ld));
