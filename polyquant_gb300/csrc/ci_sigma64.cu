@@ -37,6 +37,7 @@
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <numeric>
 #include <utility>
 #include <vector>
 
@@ -574,13 +575,20 @@ static pq_status s64_lists(const pq_ci_handle *h, const Sigma64 &S, const std::v
   }
   toff.assign(items.size() + 1, 0);
   ent.clear();
+  std::vector<uint32_t> v;
+  std::vector<int32_t> at(n + 1);
+  std::vector<std::pair<size_t, size_t>> runs;
   for (size_t i = 0; i < items.size(); i++) {
-    std::vector<uint32_t> &v = items[i];
-    std::sort(v.begin(), v.end());
-    std::vector<std::pair<size_t, size_t>> runs;  // ranges of one target
+    // in order of target and contribution: counted by target, then sorted within each one's few
+    std::fill(at.begin(), at.end(), 0);
+    for (uint32_t x : items[i]) at[(x >> 16) + 1]++;
+    std::partial_sum(at.begin(), at.end(), at.begin());
+    v.resize(items[i].size());
+    for (uint32_t x : items[i]) v[at[x >> 16]++] = x;
+    runs.clear();  // ranges of one target
     for (size_t u = 0; u < v.size();) {
-      size_t w = u;
-      while (w < v.size() && v[w] >> 16 == v[u] >> 16) w++;
+      const size_t w = at[v[u] >> 16];
+      std::sort(v.begin() + u, v.begin() + w);
       runs.emplace_back(u, w);
       u = w;
     }

@@ -224,7 +224,7 @@ static Shape shape_of(const pq_ci_handle *h) {
 // a connection half a clock of an SM's FP64 pipe, and a pair some 25 us of launches and of a chip that is not full.
 // us a sigma of three roots, this path / the element kernel: 864 determinants of 258 connections in three pairs
 // 100 / 110, 4 000 of 740 146 / 301, 18 000 of 2 020 170 / 787; four lists, 82 944 of 721 (3.5 rows a connection)
-// 301 / 463; 36 504 of 863 (8.1 rows a connection) 357 / 351.
+// 301 / 463, but 640 / 415 with the matrices that its first call makes; 36 504 of 863 (8.1 rows a connection) 357 / 351.
 bool two64_applicable(const pq_ci_handle *h) {
   if (h->n_species != 2 || !h->full2 || h->wide || h->n_dets > (16 << 20)) return false;
   double rows = 0.0, conn = 0.0;
@@ -246,7 +246,7 @@ bool two64_applicable(const pq_ci_handle *h) {
   }
   if (npairs == 0) return false;
   if (getenv("PQ_TWO64_ALWAYS")) return true;  // tests of small spaces, read when a handle is created
-  return rows <= 4.0 * conn && (double)h->n_dets * conn >= 6e5 * npairs;
+  return rows <= 2.5 * conn && (double)h->n_dets * conn >= 6e5 * npairs;
 }
 
 size_t two64_bytes(const pq_ci_handle *h) { return h->two64 ? h->two64->bytes() : 0; }
