@@ -17,7 +17,7 @@
 //               pairs, K = 64 singles; hi*hi + hi*lo + lo*hi in FP16 with FP32
 //               accumulation; two accumulators so the epilogue overlaps);
 //   warps 1-4   converters: thread (c, kq) owns beta string c of a 32-string tile
-//               (operand rows 4c .. 4c + 3) and alpha singles 16 kq .. 16 kq + 15;
+//               (an operand row for each root) and alpha singles 16 kq .. 16 kq + 15;
 //               it copies the 16-byte vectors X[Ja][Jb][0..3] of its singles into a
 //               shared stage with asynchronous copies, one tile ahead, then scales
 //               them, splits them into FP16 hi/lo and writes its part of the K-major
@@ -229,6 +229,11 @@ __device__ __forceinline__ void store_quarter(unsigned char *th, unsigned char *
   }
 }
 
+// operand row of beta string c and root v of a tile: eight strings, root by root.  The lanes of a converter warp (32
+// strings of one root) then write rows of all eight swizzle phases, and those of a staging warp (eight strings, four
+// roots) all 32 banks.
+__device__ __forceinline__ int op_row(int c, int v) { return (c & ~7) * NV + 8 * v + (c & 7); }
+
 // power of two 2^e with x * 2^e in [2^14, 2^15) (1 for x == 0)
 __device__ __forceinline__ float fp16_scale(float x) {
   if (!(x > 0.0f) || !isfinite(x)) return 1.0f;
@@ -347,7 +352,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
     __syncwarp();
   } else if (warp < EPI0) {
     // ---- converters.  A: thread (c = lane, kq = warp - CONV0) owns beta string c of the tile (its four
-    // operand rows 4c .. 4c + 3) and alpha singles 16 kq .. 16 kq + 15: it copies the 16-byte vectors
+    // operand rows op_row(c, v)) and alpha singles 16 kq .. 16 kq + 15: it copies the 16-byte vectors
     // X[Ja(k)][Jb][0..3] of its singles into the raw stage, one tile ahead, and converts only what it copied
     // (no cross-thread wait).  B: thread r = 32 kq + c owns the off-diagonal beta pair q = r.
     const int kq = warp - CONV0, c = lane;
@@ -447,7 +452,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
             x[3][j] = v4.w * sx;
           }
 #pragma unroll
-          for (int v = 0; v < NV; v++) store_quarter(a_hi + s * OP_TILE, a_lo + s * OP_TILE, 4 * c + v, kq, x[v]);
+          for (int v = 0; v < NV; v++) store_quarter(a_hi + s * OP_TILE, a_lo + s * OP_TILE, op_row(c, v), kq, x[v]);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -471,7 +476,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
     bool dead = false;
     // the two inverse scales are powers of two inside the FP32 range, and so is their product
     const float unscale = (1.0f / g.sw) * (1.0f / fp16_scale(*g.xmax));
-    const int jl = 8 * q4 + (lane >> 2), vv = lane & 3;  // a staging lane's accumulator row (beta string, root)
+    const int jl = 8 * q4 + (lane & 7), vv = lane >> 3;  // a staging lane's accumulator row (beta string, root)
     for (int64_t ia = blockIdx.x; ia < g.na; ia += gridDim.x) {
       float *yrow = g.Y + ia * row_len;
       for (int t = 0; t < mt; t++, seq++) {
