@@ -23,9 +23,9 @@
 //               them, splits them into FP16 hi/lo and writes its part of the K-major
 //               128-byte-swizzled operand tile (two stages); they also build B per
 //               alpha string from the cross-spin integrals (one buffer);
-//   warps 5-8   epilogue: tcgen05.ld of the accumulator into a shared staging copy
+//   warps 5-12  epilogue: tcgen05.ld of the accumulator into a shared staging copy
 //               of the whole tile ([Jb][q][v]), which frees the accumulator at once;
-//   warps 5-11  then each thread takes targets from the tile's precomputed scatter
+//   warps 5-15  then each thread takes targets from the tile's precomputed scatter
 //               list (the distinct Ib reached from the tile's 32 beta strings, each
 //               with its (Jb, q, phase) contributions: 2.1 per target at 16
 //               orbitals), sums them and adds the sum into sigma(Ia, Ib) with one
@@ -65,10 +65,11 @@ constexpr int OP_TILE = BM * BK * 2;          // 16 KB: one FP16 operand tile (A
 constexpr int RAW_TILE = BK * BM * 4;         // 32 KB: the gathered FP32 rows of one tile
 constexpr int STG_BYTES = TJB * BN * NV * 4;  // 64 KB: the whole accumulator tile, [Jb][q][v]
 constexpr int KQ = BK / 4;                    // alpha singles per converter thread (16)
-constexpr int NPRE = 6;                       // scatter-list entries per processing thread loaded ahead of a tile
-constexpr int NTHREADS = 384;                    // 12 warps
-constexpr int CONV0 = 1, EPI0 = 5, PROC0 = 9;    // first converter / epilogue (staging) / list-only warp
-constexpr int NPROC = (NTHREADS / 32 - EPI0) * 32;  // threads that process the scatter lists (224)
+constexpr int NPRE = 4;                       // scatter-list entries per processing thread loaded ahead of a tile
+constexpr int NTHREADS = 512;                    // 16 warps
+constexpr int STAGERS = 8;                       // staging warps: two for each TMEM lane quadrant
+constexpr int CONV0 = 1, EPI0 = 5, PROC0 = EPI0 + STAGERS;  // first converter / epilogue (staging) / list-only warp
+constexpr int NPROC = (NTHREADS / 32 - EPI0) * 32;  // threads that process the scatter lists (352)
 constexpr long long WAIT_CYCLES = 4000000000LL;  // ~2 s at 2 GHz
 // shared memory: A hi/lo x ASTAGES, B hi/lo (one buffer), raw rows x 2, accumulator staging, per-warp alpha
 // partner lists, barriers
@@ -271,12 +272,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
     }
     for (int s = 0; s < 2; s++) {
       mbar_init(smem_u32(acc_full + s), 1);
-      mbar_init(smem_u32(acc_empty + s), 4);
+      mbar_init(smem_u32(acc_empty + s), STAGERS);
     }
     mbar_init(smem_u32(b_full), 4);
     mbar_init(smem_u32(b_empty), 1);
     mbar_init(smem_u32(drain), 1);
-    mbar_init(smem_u32(stg_full), 4);
+    mbar_init(smem_u32(stg_full), STAGERS);
     mbar_init(smem_u32(stg_empty), NPROC / 32);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -470,7 +471,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
     // add each sum into sigma(Ia, target) with one vector reduction.  Staging full / empty are mbarriers
     // with bounded waits.
     const bool stager = warp < PROC0;
-    const int q4 = warp & 3;                 // TMEM lane quadrant of a staging warp
+    const int q4 = warp & 3, half = (warp - EPI0) >> 2;  // TMEM lane quadrant and columns of a staging warp
     const int te = threadIdx.x - 32 * EPI0;  // 0 .. NPROC - 1
     int seq = 0;
     bool dead = false;
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
           const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(a * BN);
           float *srow = stg + (int64_t)jl * BN * NV + vv;
 #pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 32) {
+          for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
             float d[32];
             tmem_ld32(taddr + c0, d);
 #pragma unroll
