@@ -31,6 +31,13 @@
 //               orbitals), sums them and adds the sum into sigma(Ia, Ib) with one
 //               vector reduction (red.global.add.v4.f32).  Staging full / empty are
 //               mbarriers, so every wait in the kernel is bounded.
+// What bounds it: shared memory and the reductions.  A tile of 14 orbitals takes 4.0 k cycles, of which the epilogue's
+// staging 1.1 k and its lists 2.2 k in turn; the MMAs take 0.8 k, the converters have a third of the time to spare.
+// Four roots of 16 orbitals, the whole sigma: 188.7 ms with 12 warps and operand rows 4 c + v (16-way bank conflicts of
+// the converters' stores), 179.7 without the conflicts, 169.7 with 16 warps, 160.4 with two staging warps a quadrant
+// (20 warps 160.1).  Two staging areas, so that the next tile is staged while the lists run, with the gathered rows in
+// registers instead of a shared stage, do not help: 176.0 with four warps staging and seven on the lists, 177.7 with
+// the staging warps taking a share of the lists; the two then compete for the same shared-memory cycles.
 // A CTA is the only writer of its sigma rows, so the reductions never contend
 // between CTAs.  On this GPU a shared-memory float atomic adds fewer values
 // per clock than a global vector reduction, which carries all four roots.
@@ -465,7 +472,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ab_tc_kernel(Args g) {
       __syncwarp();
     }
   } else {
-    // ---- epilogue.  Per tile: warps EPI0 .. EPI0 + 3 copy the accumulator into the staging area ([Jb][q][v],
+    // ---- epilogue.  Per tile: warps EPI0 .. PROC0 - 1 copy the accumulator into the staging area ([Jb][q][v],
     // the column swizzled by the row) and release the accumulator; then they and the list-only warps
     // PROC0 .. take targets of the tile's scatter list, sum their contributions from the staging area and
     // add each sum into sigma(Ia, target) with one vector reduction.  Staging full / empty are mbarriers
