@@ -7,7 +7,7 @@ spin, 165,636,900 determinants, 4 roots, seeded synthetic integrals
 than L2, so no flush is needed between steps.
 
 Printed JSON line (rank 0):
-  value    : sigma dets/s = n_dets * roots / t_sigma, FP64 kernel, inputs resident in HBM
+  value    : sigma dets/s = n_dets * roots / t_sigma, FP64, inputs resident in HBM
   e2e      : the same metric through pq_ci_sigma_host with pinned host buffers (H2D + sigma + D2H)
   mixed    : the FP32 sigma (the bulk sigma of the mixed-precision Davidson), with its own roofline
   roofline : compulsory bytes B = n_dets*roots*(8+8) + n_dets*8 per FP64 sigma over the kernel time,
@@ -424,9 +424,12 @@ def fp64_dgemm_tflops(n=8192, reps=5):
     return 2.0 * n ** 3 / best / 1e12
 
 
-# DRAM traffic of one FP64 sigma launch (4 roots) per determinant, from an ncu capture of FCI(14o, 7a7b):
-# 117.73e9 B read + 0.39e9 B written over 11,778,624 determinants.
-FP64_SIGMA_DRAM_BYTES_PER_DET = (117.73e9 + 0.39e9) / 11_778_624
+# DRAM traffic of one FP64 sigma (4 roots, six kernels) per determinant, from an ncu capture of FCI(14o, 7a7b):
+# 31.92e9 B read + 2.60e9 B written over 11,778,624 determinants.
+FP64_SIGMA_DRAM_BYTES_PER_DET = (31.92e9 + 2.60e9) / 11_778_624
+# kernels of one interleaved FP64 sigma: maximum, digits, the same-spin product of either spin, the opposite-spin
+# kernel, and the element kernel behind the flag
+FP64_SIGMA_LAUNCHES = 6
 
 
 def bench_batch(n_problems=256, seed=0, roots=2, nsub=4, max_subspace=0, tol=1e-5):
@@ -674,18 +677,19 @@ def main():
                                                "allows; per-kernel ncu figures in profiles/"}},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                              "frac": achieved / hbm, "traffic": FP64_SIGMA_DRAM_BYTES_PER_DET * n,
-                             "traffic_note": "ncu dram__bytes_read+write of one FP64 sigma launch on FCI(14o, 7a7b) "
-                                             "(118.1 GB for 11,778,624 determinants x 4 roots), scaled by the "
+                             "traffic_note": "ncu dram__bytes_read+write of one FP64 sigma on FCI(14o, 7a7b) "
+                                             "(34.5 GB for 11,778,624 determinants x 4 roots), scaled by the "
                                              "determinant count; a lower bound (connections per determinant grow "
                                              "from 3381 to 5793)",
                              "peak_source": peak_kind, "algorithmic_bytes_per_launch": bytes_alg,
                              "fp64": {"fma_per_launch": fmas, "achieved_tflops": 2 * fmas / (ms64 * 1e-3) / 1e12,
                                       "dgemm_tflops_measured": dgemm,
                                       "frac_of_dgemm": (2 * fmas / (ms64 * 1e-3) / 1e12 / dgemm) if dgemm else None,
-                                      "fp64_pipe_active_ncu": 0.93,
-                                      "note": "the FP64 sigma is bound by the FP64 pipe, not HBM: every FMA is a "
-                                              "matrix element applied; DGEMM measured live as the FP64 rate"}},
-                "gpu_launches": args.steps,
+                                      "tensor_pipe_active_ncu": 0.38,
+                                      "note": "FMAs of the sparse sigma over its time; the products run as exact "
+                                              "FP16 digit products on the tensor cores, which the drain of their "
+                                              "accumulators bounds, not HBM; DGEMM measured live as the FP64 rate"}},
+                "gpu_launches": FP64_SIGMA_LAUNCHES * args.steps,
                 "clocks": clk.summary(),
                 "ao2mo": ao,
                 "psh_like": psh,

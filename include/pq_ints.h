@@ -42,9 +42,9 @@ pq_status pq_ao2mo(const double *eri_ao, int32_t layout, int64_t n_ao_a, int64_t
                    int64_t ldc_a, int64_t n_mo_a, const double *C_b, int64_t ldc_b, int64_t n_mo_b, int32_t mode,
                    double *eri_mo, void *stream);
 
-/* The transforms keep their work buffers (split-precision modes about 2.5 x
- * the FP64 pair matrix, e.g. 20 GB at n_ao = n_mo = 256; FP64 mode up to 256
- * functions one FP64 pair matrix and about 1.5 GB) on the device between
+/* The transforms keep their work buffers (split-precision modes about the size
+ * of the FP64 pair matrix, e.g. 9 to 11 GB at n_ao = n_mo = 256; FP64 mode up
+ * to 256 functions one FP64 pair matrix and about 1.5 GB) on the device between
  * calls, so repeated transforms allocate nothing; calls on one device share
  * them and run one at a time.  This frees them for the current device (no
  * reference counterpart: the reference's transform holds its buffers only
