@@ -90,6 +90,27 @@ template <> __device__ __forceinline__ const ProbT<double> &pt<double>(const Pro
 
 __device__ __forceinline__ int pairdiag(int k) { return k * (k + 3) / 2; }  // idx2(k, k)
 
+// Lanes of a group for rows of L values.  Above 32 values: the width that pads a row least with at most JMAX values a
+// lane, the widest of equals.  Rows of 72 values (36 positron determinants, two roots) take two groups of 16 and pad to
+// 80, where one of 32 padded to 96 and the FP64 pipe ran the padding; rows of 36 four groups of 8.  Sixteen uneven
+// problems, one / two roots: FP64 8.87 / 12.64 ms with one group of 32, 7.69 / 12.00 so; FP32 2.93 / 4.73 and 2.57 / 4.44.
+// Up to 32 values one group takes the row: four groups of 8 for rows of 24 gain an eighth in FP64, but the compiler
+// contracts the positron terms of three values a lane into other roundings, which FP32 results show, and work units of
+// four rows without them cost FP32 a tenth.
+__host__ __device__ inline int group_lanes(int L) {
+  if (L <= 32) {
+    int G = 1;
+    while (G < L) G <<= 1;
+    return G;
+  }
+  int best = 32, pad = (L + 31) / 32 * 32;
+  for (int G = 16; G >= 1; G >>= 1) {
+    const int p = (L + G - 1) / G * G;
+    if (p <= JMAX * G && p < pad) best = G, pad = p;
+  }
+  return best;
+}
+
 // One work unit: rows (ia, b0 .. b0+nrows-1) of one problem, one warp.
 // Lanes form R = 32 / G groups of G lanes; a group owns one row and lane gl of
 // the group owns the row's columns gl + j * G (j < J, < L).  Matrix elements
@@ -110,7 +131,7 @@ __device__ void do_rows(const Prob &p, const Call &cl, const Unit &U, T *stg, in
   const uint64_t amask = p.astr[ia];
   const T cf = (T)p.cf;
   const int rowa = ia * nb;
-  T *srow = stg + g * G;  // staging of one row (L <= G when R > 1)
+  T *srow = stg + g * G * J;  // staging of one row
   for (int r0 = 0; r0 < U.nrows; r0 += R) {
     const bool rok = r0 + g < U.nrows;
     const int ib = rok ? U.b0 + r0 + g : 0;
@@ -487,7 +508,7 @@ __device__ __forceinline__ void do_unit(const Prob &p, const Call &cl, const Uni
       do_rows_lane<T, 16>(p, cl, U, stg, lane);
     return;
   }
-  const int G = L >= 32 ? 32 : (L <= 1 ? 1 : 1 << (32 - __clz(L - 1)));
+  const int G = group_lanes(L);
   switch ((L + G - 1) / G) {
     case 1: do_rows<T, 1>(p, cl, U, stg, lane, G); break;
     case 2: do_rows<T, 2>(p, cl, U, stg, lane, G); break;
@@ -885,7 +906,7 @@ pq_status make_plan(pq_ci_batch *B, const std::vector<int> &members, int warps, 
   for (int pi : members) {
     const Prob &pr = B->prob[pi];
     const int L = pr.P * B->wmax;
-    const int G = L >= 32 ? 32 : (L <= 1 ? 1 : 1 << (32 - __builtin_clz((unsigned)(L - 1))));
+    const int G = group_lanes(L);
     const int nrows = (lane_rows(B, pi) ? 32 : 32 / G) * rows_mult;
     const double rc = row_cost(B->h[pi], pr, B->wmax);
     for (int ia = 0; ia < pr.na; ia++)
