@@ -20,7 +20,7 @@ def _pairs(B, C):
 
 @pytest.mark.parametrize("mode", ["bf16x3", "tf32x3"])
 @pytest.mark.parametrize("n,m", [(1, 1), (2, 2), (7, 5), (8, 8), (31, 16), (33, 31), (33, 32), (64, 63), (65, 65), (97, 3),
-                                (129, 128), (129, 40)])
+                                (129, 128), (129, 40), (150, 141)])
 def test_sizes_and_layouts(mode, n, m):
     from polyquant_gb300._lib import PQ_AO_PAIRS, PQ_XFORM_BF16X3, PQ_XFORM_TF32X3
     from polyquant_gb300.integral import ao2mo
