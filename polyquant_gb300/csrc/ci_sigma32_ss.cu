@@ -582,9 +582,9 @@ static pq_status ss_prepare(pq_ci_handle *h) {
     return PQ_ERR_OOM;
   }
   h->ss.reset(g);
-  const pq_ci_desc &d = h->desc;
-  // identical spin lists with identical integrals: the beta doubles are the alpha ones
-  g->shared_beta = h->n_blocks[0] == 1 && d.n_alpha[0] == d.n_beta[0] && d.ex_level[0][0] == d.ex_level[0][1];
+  // identical spin lists with identical integrals: the beta doubles are the alpha ones (the lists themselves are
+  // compared, since a caller may have chosen them)
+  g->shared_beta = h->n_blocks[0] == 1 && h->str[0][0] == h->str[0][1];
   pq_status s = ss_build_side(h, 0, g->side[0]);
   if (s == PQ_OK && !g->shared_beta) s = ss_build_side(h, 1, g->side[1]);
   if (s == PQ_OK) s = g->aux.alloc(16);
