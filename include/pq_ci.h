@@ -161,6 +161,19 @@ pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32
  * same-spin GEMM buffers of the FP32 full-CI sigma).  Meant for tests. */
 pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes);
 
+/* Diagnostics of the FP64 sigma, no reference counterpart, meant for tests.
+ * pq_debug_sigma_path: which kernels the handle's last FP64 sigma was given to
+ * and, for PQ_PATH_TENSOR, the word that the element kernel behind it looked
+ * at: 0 = the digit products' result stands, 1 = a non-finite value, 2 = a
+ * bounded wait ran out (the element kernel has then computed the result).
+ * Blocking.
+ * pq_debug_set_sigma_wait_budget: budgets, in SM clock cycles, of the pipeline
+ * waits of the same-spin (and pair matrix) kernel and of the opposite-spin
+ * kernel (<= 0: the default of about 2 s). */
+enum { PQ_PATH_NONE = 0, PQ_PATH_ELEMENT = 1, PQ_PATH_ROWS = 2, PQ_PATH_TENSOR = 3, PQ_PATH_MATRIX = 4 };
+pq_status pq_debug_sigma_path(pq_ci_handle *h, int32_t *path, int32_t *gate);
+pq_status pq_debug_set_sigma_wait_budget(long long same_spin, long long opposite_spin);
+
 /* Block Davidson on the GPU (replaces Spectra::DavidsonSymEigsSolver with the
  * reference's parameters: initial = num_subspace_vec, max = max(2*initial,
  * 10*num_states), epci.cpp:589-590). */

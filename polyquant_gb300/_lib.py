@@ -13,6 +13,7 @@ LIB_PATH = os.path.join(_PKG, "lib", "libpq_gb300.so")
 
 PQ_OK, PQ_ERR_ARG, PQ_ERR_CUDA, PQ_ERR_OOM, PQ_NOT_CONVERGED, PQ_TIMEOUT, PQ_ERR_STATE = range(7)
 PQ_FP64, PQ_FP32 = 0, 1
+PQ_PATH_NONE, PQ_PATH_ELEMENT, PQ_PATH_ROWS, PQ_PATH_TENSOR, PQ_PATH_MATRIX = range(5)
 PQ_AO_PACKED8, PQ_AO_PAIRS = 0, 1
 PQ_XFORM_FP64, PQ_XFORM_BF16X3, PQ_XFORM_TF32X3 = 0, 1, 2
 
@@ -23,7 +24,7 @@ EXPORTS = [
     "pq_ci_davidson", "pq_ci_ham_build", "pq_ci_ham_release", "pq_ci_ham_csr", "pq_ci_s2", "pq_ci_rdm1",
     "pq_ci_batch_create", "pq_ci_batch_destroy", "pq_ci_batch_num_dets", "pq_ci_batch_sigma",
     "pq_ci_batch_tuning", "pq_ci_batch_davidson", "pq_ao2mo", "pq_mo1", "pq_debug_set_wait_budget",
-    "pq_ao2mo_release_workspace",
+    "pq_ao2mo_release_workspace", "pq_debug_sigma_path", "pq_debug_set_sigma_wait_budget",
 ]
 
 
@@ -112,6 +113,10 @@ def load(path: str = LIB_PATH):
     L.pq_ci_elements.argtypes = [P, I64, P, P, P]
     L.pq_debug_scratch_bytes.restype = I32
     L.pq_debug_scratch_bytes.argtypes = [P, ctypes.POINTER(I64)]
+    L.pq_debug_sigma_path.restype = I32
+    L.pq_debug_sigma_path.argtypes = [P, ctypes.POINTER(I32), ctypes.POINTER(I32)]
+    L.pq_debug_set_sigma_wait_budget.restype = I32
+    L.pq_debug_set_sigma_wait_budget.argtypes = [ctypes.c_longlong, ctypes.c_longlong]
     L.pq_ci_sigma_interleaved.restype = I32
     L.pq_ci_sigma_interleaved.argtypes = [P, P, P, I32, I32, D]
     L.pq_ci_davidson.restype = I32

@@ -324,6 +324,22 @@ pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32
   return ci_sigma_il(h, X, Y, nvec, precision, diag_shift);
 }
 
+pq_status pq_debug_sigma_path(pq_ci_handle *h, int32_t *path, int32_t *gate) {
+  clear_error();
+  if (!h || !path || !gate) {
+    set_error("pq_debug_sigma_path: NULL argument");
+    return PQ_ERR_ARG;
+  }
+  *path = h->last_path;
+  *gate = 0;
+  if (h->last_path != PQ_PATH_TENSOR) return PQ_OK;
+  int g = 0;
+  PQ_CUDA_TRY(cudaMemcpyAsync(&g, h->last_gate, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  *gate = g;
+  return PQ_OK;
+}
+
 pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes) {
   if (!h || !bytes) {
     set_error("pq_debug_scratch_bytes: NULL argument");

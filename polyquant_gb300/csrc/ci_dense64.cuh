@@ -61,6 +61,7 @@ struct SsArgs {
   const uint32_t *xhi, *dhi;
   double *S;
   int64_t es, vs;
+  long long wait;             // budget of the pipeline waits (the wind-down waits keep WAIT_CYCLES)
   int *gate;
 };
 
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         range_of(v, mt, nt, k0, k1);
         for (int j = k0; j < k1; j++, gs++) {
           const int slot = gs % SS_STAGES;
-          ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((gs / SS_STAGES) & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
+          ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((gs / SS_STAGES) & 1) ^ 1u, g.wait) && !*abort_flag;
           if (!ok) break;
           const uint32_t a = smem_u32(smem + slot * SS_STAGE), b = a + dg::N * SS_A, bar = smem_u32(full + slot);
           const int k = chunk_of(j) * 32;
@@ -174,12 +175,12 @@ __global__ void __launch_bounds__(THREADS, 1)
         range_of(v, mt, nt, k0, k1);
         for (int j = k0; j < k1 && ok; seq++) {
           const int e = window_end(j, k1);
-          ok = mbar_wait(smem_u32(acce), (uint32_t)(seq & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
+          ok = mbar_wait(smem_u32(acce), (uint32_t)(seq & 1) ^ 1u, g.wait) && !*abort_flag;
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           for (int j0 = j; j < e; j++, gs++) {
             const int slot = gs % SS_STAGES;
-            ok = mbar_wait(smem_u32(full + slot), (uint32_t)((gs / SS_STAGES) & 1), WAIT_CYCLES);
+            ok = mbar_wait(smem_u32(full + slot), (uint32_t)((gs / SS_STAGES) & 1), g.wait);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_u32(smem + slot * SS_STAGE), b = a + dg::N * SS_A;
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int c = 0; c < 16; c++) sh[c] = 0, sl[c] = 0;
       for (int j = k0; j < k1; seq++) {
         j = window_end(j, k1);
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(accf), (uint32_t)(seq & 1), WAIT_CYCLES) && !*abort_flag);
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(accf), (uint32_t)(seq & 1), g.wait) && !*abort_flag);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll

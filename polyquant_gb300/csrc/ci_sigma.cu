@@ -382,6 +382,7 @@ pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv
     return PQ_OK;
   }
   PQ_TRY(s);
+  h->last_path = PQ_PATH_TENSOR, h->last_gate = gate;
   if (interleaved) {
     PQ_TRY(ci_sigma_gated(h, C, S, nv, shift, gate));
   } else {
@@ -393,7 +394,11 @@ pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv
 
 pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvp, int precision, double shift,
                       bool allow_scratch) {
-  if (h->use_explicit && precision == PQ_FP64 && shift == 0.0) return ci_ham_spmv(h, X, Y, nvp);
+  if (h->use_explicit && precision == PQ_FP64 && shift == 0.0) {
+    h->last_path = PQ_PATH_MATRIX;
+    return ci_ham_spmv(h, X, Y, nvp);
+  }
+  if (precision == PQ_FP64) h->last_path = h->rows ? PQ_PATH_ROWS : PQ_PATH_ELEMENT;
   if (h->n_species == 2) return ci_sigma2_il(h, X, Y, nvp, precision, shift);
   if (precision == PQ_FP32 && allow_scratch && h->fp32_v2) return ci_sigma32_v2(h, X, Y, nvp, shift);
   if (precision == PQ_FP64) {

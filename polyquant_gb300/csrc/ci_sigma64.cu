@@ -46,6 +46,9 @@
 
 namespace pq {
 
+static long long g_sigma_wait[2] = {tcx::WAIT_CYCLES, tcx::WAIT_CYCLES};
+long long sigma_wait_cycles(int kernel) { return g_sigma_wait[kernel]; }
+
 struct Sigma64 {
   struct Side {
     unsigned short *d = nullptr;       // digits of the dense same-spin H: [digit][I][np]
@@ -135,6 +138,7 @@ struct AbArgs {
   const uint32_t *xhi, *whi;
   double *S;
   int64_t es, vs;            // strides of sigma over determinants and roots
+  long long wait;            // budget of the pipeline waits (the wind-down waits keep WAIT_CYCLES)
   int *gate;
 };
 
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
       __syncwarp();
       for (int k = lane; k < g.kp; k += 32) kl[k] = __ldg(g.klist + ia * g.kp + k);
       __syncwarp();
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(b_empty), (uint32_t)(nit & 1) ^ 1u, WAIT_CYCLES)) && !*abort_flag;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(b_empty), (uint32_t)(nit & 1) ^ 1u, g.wait)) && !*abort_flag;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       if (pw == 0 && lane == 0) mbar_expect_tx(smem_u32(b_full), dg::N * g.kp * 128);
@@ -241,7 +245,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
         for (int t = 0; t < g.m_tiles && ok; t++)
           for (int s = 0; s < steps; s++, gs++) {
             const int slot = gs % A_STAGES;
-            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(a_empty + slot), (uint32_t)((gs / A_STAGES) & 1) ^ 1u, WAIT_CYCLES) &&
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(a_empty + slot), (uint32_t)((gs / A_STAGES) & 1) ^ 1u, g.wait) &&
                                              !*abort_flag);
             if (!ok) break;
             if (pw == 0 && lane == 0) mbar_expect_tx(smem_u32(a_full + slot), A_STAGE);
@@ -274,14 +278,14 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
         int64_t ia;
         int p, v0, v1;
         item_of(it, ia, p, v0, v1);
-        ok = mbar_wait(smem_u32(b_full), (uint32_t)(nit & 1), WAIT_CYCLES) && !*abort_flag;
+        ok = mbar_wait(smem_u32(b_full), (uint32_t)(nit & 1), g.wait) && !*abort_flag;
         for (int u = 0; u < (v1 - v0) * g.m_tiles && ok; u++, seq++) {
-          ok = mbar_wait(smem_u32(acc_empty), (uint32_t)(seq & 1) ^ 1u, WAIT_CYCLES) && !*abort_flag;
+          ok = mbar_wait(smem_u32(acc_empty), (uint32_t)(seq & 1) ^ 1u, g.wait) && !*abort_flag;
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           for (int s = 0; s < steps; s++, gs++) {
             const int slot = gs % A_STAGES;
-            ok = mbar_wait(smem_u32(a_full + slot), (uint32_t)((gs / A_STAGES) & 1), WAIT_CYCLES);
+            ok = mbar_wait(smem_u32(a_full + slot), (uint32_t)((gs / A_STAGES) & 1), g.wait);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_u32(sa + slot * A_STAGE), b = smem_u32(sb) + s * 2048;
@@ -306,7 +310,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16);
     int64_t *drow = sd + (int64_t)(q4 * 32 + lane) * LDS_D;
     auto wait_all = [&](uint64_t *bar, int phase) {
-      return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), (uint32_t)(phase & 1), WAIT_CYCLES) && !*abort_flag);
+      return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), (uint32_t)(phase & 1), g.wait) && !*abort_flag);
     };
     int seq = 0;
     bool ok = true;
@@ -767,6 +771,7 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
   g.tiles = (int64_t)nv * g.m_tiles * g.n_tiles;
   g.xhi = xhi;
   g.S = S, g.es = ses, g.vs = svs, g.gate = gate;
+  g.wait = sigma_wait_cycles(0);
   const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, z.sms);
   CUtensorMap ma, mb;
   const int64_t xrows = (int64_t)dg::N * nv * na;
@@ -803,6 +808,7 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
   x.tent = z.tent;
   x.xhi = xhi, x.whi = hi + 2;
   x.S = S, x.es = ses, x.vs = svs, x.gate = gate;
+  x.wait = sigma_wait_cycles(1);
   ab64_kernel<<<(unsigned)std::min<int64_t>(x.items, z.sms), AB_THREADS, AB_SMEM, st>>>(ma, mb, x);
   PQ_CUDA_TRY(cudaGetLastError());
   *gate_out = gate;
@@ -810,3 +816,9 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
 }
 
 }  // namespace pq
+
+extern "C" pq_status pq_debug_set_sigma_wait_budget(long long same_spin, long long opposite_spin) {
+  pq::g_sigma_wait[0] = same_spin > 0 ? same_spin : pq::tcx::WAIT_CYCLES;
+  pq::g_sigma_wait[1] = opposite_spin > 0 ? opposite_spin : pq::tcx::WAIT_CYCLES;
+  return PQ_OK;
+}

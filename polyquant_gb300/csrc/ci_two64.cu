@@ -372,6 +372,7 @@ pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int
     g.chunks = (int)((p.M + 31) / 32);
     g.xhi = xhi, g.dhi = hi + i;
     g.S = part[i];
+    g.wait = sigma_wait_cycles(0);
     g.gate = gate;
     ss64_kernel<false><<<(unsigned)std::min<int64_t>(g.tiles, T.sms), THREADS, SS_SMEM, st>>>(ma, mb, g);
     PQ_CUDA_TRY(cudaGetLastError());

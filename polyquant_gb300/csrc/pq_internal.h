@@ -148,6 +148,9 @@ struct pq_ci_handle {
   bool fp64_tc = false;
   std::unique_ptr<pq::Two64, void (*)(pq::Two64 *)> two64{nullptr, pq::two64_delete};
   std::unique_ptr<pq::Sigma64, void (*)(pq::Sigma64 *)> s64{nullptr, pq::sigma64_delete};
+  // what computed the last FP64 sigma (PQ_PATH_*) and, for the tensor cores, its gate word: pq_debug_sigma_path
+  int last_path = PQ_PATH_NONE;
+  const int *last_gate = nullptr;
   // singles by orbital pair, made by the first property call of a one-species handle (ci_props.cu)
   std::unique_ptr<pq::PairLists, void (*)(pq::PairLists *)> pairs{nullptr, pq::pairs_delete};
   // two species: addressing of the product space (see ci_two.cu)
@@ -202,6 +205,8 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
                      int64_t svs, int **gate);
 pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
                    int64_t svs, int **gate);
+// budget of the waits of the same-spin products, pair matrices included (0), and of the opposite-spin kernel (1)
+long long sigma_wait_cycles(int kernel);
 size_t sigma64_bytes(const pq_ci_handle *h);
 size_t two64_bytes(const pq_ci_handle *h);
 // the element kernels of ci_two.cu on interleaved vectors (nvp = 1: a column), if *gate is not zero when they run
