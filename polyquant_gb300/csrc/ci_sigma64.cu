@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + AB_BARS);
   uint32_t *tmax = tmem_slot + 1;  // [2]
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 3);
-  if (*g.gate) return;
+  if (gate_raised(g.gate)) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
