@@ -169,15 +169,16 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + AB_BARS);
   uint32_t *tmax = tmem_slot + 1;  // [2]
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 3);
+  volatile int *issued = abort_flag + 1;  // at the end: stages and items that each gather warp has issued
   if (gate_raised(g.gate)) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < A_STAGES; i++) {
-      mbar_init(smem_u32(a_full + i), 1);
+      mbar_init(smem_u32(a_full + i), GATHER_WARPS);
       mbar_init(smem_u32(a_empty + i), 1);
     }
-    mbar_init(smem_u32(b_full), 1);
+    mbar_init(smem_u32(b_full), GATHER_WARPS);
     mbar_init(smem_u32(b_empty), 1);
     mbar_init(smem_u32(acc_full), 1);
     mbar_init(smem_u32(acc_empty), EPI_WARPS);
@@ -223,7 +224,9 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
     int2 *kl = kl_all + pw * KMAX;  // this warp's copy of the item's K list
     int gs = 0, nit = 0;
     bool ok = true;
-    for (int64_t it = 0; it < mine && ok; it++, nit++) {
+    // each warp announces the bytes of its own gathers: four rows of 128 bytes each
+    auto share = [&](int gathers) { return (uint32_t)((gathers - pw + GATHER_WARPS - 1) / GATHER_WARPS * 512); };
+    for (int64_t it = 0; it < mine && ok; it++) {
       int64_t ia;
       int p, v0, v1;
       item_of(it, ia, p, v0, v1);
@@ -233,7 +236,8 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(b_empty), (uint32_t)(nit & 1) ^ 1u, g.wait)) && !*abort_flag;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      if (pw == 0 && lane == 0) mbar_expect_tx(smem_u32(b_full), dg::N * g.kp * 128);
+      if (lane == 0) mbar_expect_tx(smem_u32(b_full), share(dg::N * (g.kp / 4)));
+      nit++;
       __syncwarp();
       for (int i = GATHER_WARPS * lane + pw; i < dg::N * (g.kp / 4); i += 32 * GATHER_WARPS) {
         const int d = i / (g.kp / 4), k = 4 * (i - d * (g.kp / 4));
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
             ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(a_empty + slot), (uint32_t)((gs / A_STAGES) & 1) ^ 1u, g.wait) &&
                                              !*abort_flag);
             if (!ok) break;
-            if (pw == 0 && lane == 0) mbar_expect_tx(smem_u32(a_full + slot), A_STAGE);
+            if (lane == 0) mbar_expect_tx(smem_u32(a_full + slot), share(dg::N * 8));
             __syncwarp();
             // 56 gathers: digit, half of the 128 strings, group of four K values
             for (int i = GATHER_WARPS * lane + pw; i < dg::N * 8; i += 32 * GATHER_WARPS) {
@@ -260,14 +264,23 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
             }
           }
     }
-    if (!ok) {
-      if (lane == 0) fail();
+    // The gathers in flight land before the CTA exits.  A warp that gave up first arrives, without bytes, for the
+    // stages and the item that others had gone on to (at most the ring ahead of it), so that their phases complete;
+    // the abort flag is up by then, and what is made of such a stage is not used.
+    if (lane == 0) {
+      if (!ok) fail();
+      issued[2 * pw] = gs, issued[2 * pw + 1] = nit;
     }
-    // the gathers in flight land before the CTA exits
-    if (pw == 0 && lane == 0) {
-      for (int j = gs > A_STAGES ? gs - A_STAGES : 0; j < gs; j++)
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * GATHER_WARPS) : "memory");
+    if (lane == 0) {
+      int gmax = 0, nmax = 0;
+      for (int w = 0; w < GATHER_WARPS; w++) gmax = max(gmax, issued[2 * w]), nmax = max(nmax, issued[2 * w + 1]);
+      for (int j = gs; j < gmax; j++) mbar_arrive(smem_u32(a_full + j % A_STAGES));
+      for (int j = nit; j < nmax; j++) mbar_arrive(smem_u32(b_full));
+      for (int j = gmax > A_STAGES ? gmax - A_STAGES : 0; j < gmax; j++)
         mbar_wait(smem_u32(a_full + (j % A_STAGES)), (uint32_t)((j / A_STAGES) & 1), WAIT_CYCLES);
-      if (nit > 0) mbar_wait(smem_u32(b_full), (uint32_t)((nit - 1) & 1), WAIT_CYCLES);
+      if (nmax > 0) mbar_wait(smem_u32(b_full), (uint32_t)((nmax - 1) & 1), WAIT_CYCLES);
     }
     __syncwarp();
   } else if (warp == 1) {

@@ -49,3 +49,10 @@ def test_pair_matrices(monkeypatch):
 
 def test_same_spin_products(monkeypatch):
     _expire(monkeypatch, synthetic_fci(12, 6, 6, seed=2), [(b, 0) for b in (1, 300, 1000, 3000, 10000, 30000)])
+
+
+@pytest.mark.parametrize("n,a,b", [(12, 6, 6), (12, 6, 3), (13, 8, 2), (17, 2, 4)])
+def test_opposite_spin_kernel(monkeypatch, n, a, b):
+    """Its three gather warps give up at different stages: the gathers that some have issued and others have not are
+    waited for before the CTA leaves."""
+    _expire(monkeypatch, synthetic_fci(n, a, b, seed=3), [(0, w) for w in (1, 100, 300, 700, 1000, 2000, 3000, 10000, 30000)])
