@@ -151,14 +151,23 @@ pq_status pq_ci_elements(pq_ci_handle *h, int64_t n, const int64_t *I, const int
 
 /* Native-layout sigma on DEVICE buffers interleaved by determinant:
  * X[det * nvec + v].  T = double (precision PQ_FP64) or float (PQ_FP32).
- * diag_shift is subtracted from H_II (sigma = (H - shift*1) X). */
+ * diag_shift is subtracted from H_II (sigma = (H - shift*1) X).
+ * FP64 calls that take the tensor cores (full CI of one species, small
+ * two-species products) allocate and synchronise when the handle first makes
+ * its tables and when more vectors than before need larger work memory: for
+ * FCI(16o) about 12 GB.  While the stream is captured into a CUDA graph a call
+ * allocates nothing: before the tables are there it records the element
+ * kernel, and memory that a graph addresses is kept until the handle is
+ * destroyed.  The same holds for pq_ci_sigma, whose first calls also allocate
+ * its work vectors (pq_ci_sigma_noalloc allocates nothing at any time). */
 pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32_t nvec, int32_t precision,
                                   double diag_shift);
 
 /* Diagnostic, no reference counterpart: device bytes the handle holds as
  * grow-on-demand work memory (the interleaved vectors of pq_ci_sigma, the
  * host-sigma staging copies, the transposed copies, tensor-core tables and
- * same-spin GEMM buffers of the FP32 full-CI sigma).  Meant for tests. */
+ * same-spin GEMM buffers of the FP32 full-CI sigma, the tables, digits and
+ * copies of the FP64 tensor-core sigma).  Meant for tests. */
 pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes);
 
 /* Diagnostics of the FP64 sigma, no reference counterpart, meant for tests.

@@ -209,6 +209,7 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
     return PQ_ERR_ARG;
   }
   size_t esz = precision == PQ_FP64 ? sizeof(double) : sizeof(float);
+  ci_capturing(h);
   for (int v0 = 0; v0 < nvec; v0 += 4) {
     int nv = nvec - v0 < 4 ? nvec - v0 : 4;
     int nvp = il_width(h, nv, precision);
@@ -219,8 +220,8 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
       } else {
         // page-locked host columns pass through device columns, copied by the conversion kernels
         const size_t n = (size_t)h->n_dets, block = sizeof(double) * nv * (n + 1);
-        PQ_TRY(h->x_il.ensure(block));
-        PQ_TRY(h->y_il.ensure(block));
+        PQ_TRY(ci_grow(h, h->x_il, block));
+        PQ_TRY(ci_grow(h, h->y_il, block));
         double *x = h->x_il.as<double>(), *y = h->y_il.as<double>();
         for (int v = 0; v < nv; v++) PQ_TRY(ci_to_il(h, C, ldc, v0 + v, 1, 1, PQ_FP64, x + v * n));
         PQ_TRY(ci_sigma64_block(h, x, n, nv, y, n, false, 0.0, &done));
@@ -237,8 +238,8 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
       }
     }
     size_t bytes = esz * (size_t)nvp * (size_t)(h->n_dets + 1);
-    PQ_TRY(h->x_il.ensure(bytes));
-    PQ_TRY(h->y_il.ensure(bytes));
+    PQ_TRY(ci_grow(h, h->x_il, bytes));
+    PQ_TRY(ci_grow(h, h->y_il, bytes));
     PQ_TRY(ci_to_il(h, C, ldc, v0, nv, nvp, precision, h->x_il.ptr));
     PQ_TRY(ci_sigma_il(h, h->x_il.ptr, h->y_il.ptr, nvp, precision, 0.0));
     PQ_TRY(ci_from_il(h, h->y_il.ptr, v0, nv, nvp, precision, S, lds));
@@ -348,6 +349,7 @@ pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes) {
   *bytes = (int64_t)(h->x_il.bytes + h->y_il.bytes + h->x_t.bytes + h->z_t.bytes + h->tc_btab.bytes + h->tc_aux.bytes +
                      h->tc_toff.bytes + h->tc_tinfo.bytes + h->host_c.bytes + h->host_s.bytes + ci_sigma32_ss_bytes(h) + sigma64_bytes(h) +
                      two64_bytes(h));
+  for (const auto &b : h->retired) *bytes += (int64_t)b->bytes;
   return PQ_OK;
 }
 

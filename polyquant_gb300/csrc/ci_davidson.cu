@@ -707,8 +707,8 @@ pq_status sigma_request_single(pq_ci_handle *h, const SigmaRequest &r) {
       if (done) continue;
     }
     const size_t esz = r.precision == PQ_FP64 ? sizeof(double) : sizeof(float);
-    PQ_TRY(h->x_il.ensure(esz * nvp * (size_t)(n + 1)));
-    PQ_TRY(h->y_il.ensure(esz * nvp * (size_t)(n + 1)));
+    PQ_TRY(ci_grow(h, h->x_il, esz * nvp * (size_t)(n + 1)));
+    PQ_TRY(ci_grow(h, h->y_il, esz * nvp * (size_t)(n + 1)));
     PQ_TRY(ci_to_il(h, r.src, n, v0, c, nvp, r.precision, h->x_il.ptr));
     PQ_TRY(ci_sigma_il(h, h->x_il.ptr, h->y_il.ptr, nvp, r.precision, r.precision == PQ_FP64 ? 0.0 : r.shift));
     if (r.precision == PQ_FP64) {

@@ -366,6 +366,26 @@ static pq_status ci_sigma_gated(pq_ci_handle *h, const double *C, double *S, int
   return sigma_dispatch<double, 4>(h, C, S, shift, gate);
 }
 
+bool ci_capturing(pq_ci_handle *h) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &s) != cudaSuccess) {  // the default stream beside another stream's capture
+    cudaGetLastError();
+    return false;
+  }
+  if (s == cudaStreamCaptureStatusNone) return false;
+  h->captured = true;
+  return true;
+}
+
+pq_status ci_grow(pq_ci_handle *h, DevBuf &b, size_t n) {
+  if (n <= b.bytes) return PQ_OK;
+  if (b.ptr && h->captured) {
+    h->retired.emplace_back(new DevBuf());
+    h->retired.back()->swap(b);
+  }
+  return b.alloc(n);
+}
+
 pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool interleaved,
                            double shift, bool *done) {
   *done = false;
@@ -374,8 +394,10 @@ pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv
   const double *c1 = C + (interleaved ? n * nv : (nv - 1) * ldc + n), *s1 = S + (interleaved ? n * nv : (nv - 1) * lds + n);
   if (C < s1 && S < c1) return PQ_OK;
   int *gate = nullptr;
+  const bool fixed = ci_capturing(h);
   const auto run = h->n_species == 2 ? ci_two64 : ci_sigma64;
-  const pq_status s = interleaved ? run(h, C, nv, 1, nv, shift, S, nv, 1, &gate) : run(h, C, 1, ldc, nv, shift, S, 1, lds, &gate);
+  const pq_status s = interleaved ? run(h, C, nv, 1, nv, shift, S, nv, 1, fixed, &gate)
+                                  : run(h, C, 1, ldc, nv, shift, S, 1, lds, fixed, &gate);
   if (s == PQ_ERR_OOM) {
     cudaGetLastError();
     clear_error();

@@ -761,13 +761,16 @@ static pq_status s64_prepare(pq_ci_handle *h) {
 // S = (H - shift) C for nv <= 4 vectors of device memory, vector v of determinant I at C[I es + v vs] and
 // S[I ses + v svs]; C and S must not overlap, and are either columns (es = 1) or interleaved (es = nv, vs = 1)
 pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
-                     int64_t svs, int **gate_out) {
+                     int64_t svs, bool fixed, int **gate_out) {
   using namespace s64;
+  if (fixed && !h->s64) return PQ_ERR_OOM;
   PQ_TRY(s64_prepare(h));
   Sigma64 &z = *h->s64;
   cudaStream_t st = h->stream;
   const int64_t na = h->tab[0][0].n_str, nb = h->tab[0][1].n_str, n = h->n_dets, nbp = up64(nb, 64);
-  PQ_TRY(z.xd.ensure(2 * (size_t)dg::N * nv * na * nbp));
+  const size_t xbytes = 2 * (size_t)dg::N * nv * na * nbp;
+  if (fixed && z.xd.bytes < xbytes) return PQ_ERR_OOM;
+  PQ_TRY(ci_grow(h, z.xd, xbytes));
   int *gate = z.aux;
   uint32_t *xhi = reinterpret_cast<uint32_t *>(z.aux) + 4, *hi = z.hi;
   PQ_CUDA_TRY(cudaMemsetAsync(z.aux, 0, 64, st));

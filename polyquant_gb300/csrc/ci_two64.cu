@@ -314,8 +314,9 @@ static pq_status two64_prepare(pq_ci_handle *h) {
 
 // as ci_sigma64
 pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
-                   int64_t svs, int **gate_out) {
+                   int64_t svs, bool fixed, int **gate_out) {
   using namespace two64;
+  if (fixed && !h->two64) return PQ_ERR_OOM;
   PQ_TRY(two64_prepare(h));
   Two64 &T = *h->two64;
   cudaStream_t st = h->stream;
@@ -344,7 +345,8 @@ pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int
   }
   DevLayout l;
   lay(l);
-  PQ_TRY(T.work.ensure(l.used));  // a full device leaves the call to the other kernel before anything is written
+  if (fixed && T.work.bytes < l.used) return PQ_ERR_OOM;
+  PQ_TRY(ci_grow(h, T.work, l.used));  // a full device leaves the call to the other kernel before anything is written
   l = DevLayout{static_cast<char *>(T.work.ptr), 0};
   lay(l);
   for (int i = 0; i < npairs; i++) q.p[i] = part[i];

@@ -6,6 +6,7 @@
 #include <chrono>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "pq_ci.h"
@@ -49,6 +50,10 @@ struct DevBuf {
   // grow-only allocation used for scratch; contents are not preserved
   pq_status ensure(size_t n) { return n <= bytes ? PQ_OK : alloc(n); }
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
+  void swap(DevBuf &o) {
+    std::swap(ptr, o.ptr);
+    std::swap(bytes, o.bytes);
+  }
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
@@ -153,6 +158,10 @@ struct pq_ci_handle {
   const int *last_gate = nullptr;
   // singles by orbital pair, made by the first property call of a one-species handle (ci_props.cu)
   std::unique_ptr<pq::PairLists, void (*)(pq::PairLists *)> pairs{nullptr, pq::pairs_delete};
+  // a sigma of this handle was recorded into a CUDA graph, which holds the addresses that it used: work memory that
+  // grows later leaves them in `retired` until the handle goes
+  bool captured = false;
+  std::vector<std::unique_ptr<pq::DevBuf>> retired;
   // two species: addressing of the product space (see ci_two.cu)
   std::vector<int32_t> e_a, e_b;        // species-0 (alpha, beta) string pair of each kept pair ie
   std::vector<int64_t> ebase;           // first determinant of pair ie's species-1 block
@@ -194,17 +203,23 @@ pq_status ci_ham_rows2(pq_ci_handle *h, double thr, int32_t *cnt, const int64_t 
 // allow_scratch = false keeps sigma on kernels that need no work memory beyond X and Y
 pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int precision, double shift,
                       bool allow_scratch = true);
+// whether the handle's stream is being captured into a graph (then nothing may be allocated or waited for); remembered
+// in h->captured
+bool ci_capturing(pq_ci_handle *h);
+// grow-only work memory of a sigma; contents are not preserved
+pq_status ci_grow(pq_ci_handle *h, DevBuf &b, size_t n);
 // ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
 pq_status ci_sigma_rows_build(pq_ci_handle *h);
 pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
 // ci_sigma64.cu, ci_two64.cu: S = (H - shift) C for at most 4 vectors of device memory that do not overlap (FP64,
-// strides over determinants and vectors).  A raised *gate afterwards means that nothing of it counts.
+// strides over determinants and vectors).  A raised *gate afterwards means that nothing of it counts.  fixed: with the
+// tables and work memory of earlier calls or not at all (PQ_ERR_OOM).
 bool sigma64_applicable(const pq_ci_handle *h);
 bool two64_applicable(const pq_ci_handle *h);
 pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
-                     int64_t svs, int **gate);
+                     int64_t svs, bool fixed, int **gate);
 pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
-                   int64_t svs, int **gate);
+                   int64_t svs, bool fixed, int **gate);
 // budget of the waits of the same-spin products, pair matrices included (0), and of the opposite-spin kernel (1)
 long long sigma_wait_cycles(int kernel);
 size_t sigma64_bytes(const pq_ci_handle *h);
@@ -213,8 +228,8 @@ size_t two64_bytes(const pq_ci_handle *h);
 pq_status ci_two_gated(pq_ci_handle *h, const double *C, double *S, int nvp, double shift, const int *gate);
 // ci_sigma.cu: (H - shift) C of a block of at most 4 vectors in device memory, columns (interleaved = false, leading
 // dimensions ldc, lds) or interleaved, by the tensor cores where they apply, with the element kernels behind them for
-// what they refuse on the device.  *done tells; the explicit matrix, overlapping buffers and a full device leave the
-// block to the caller's other kernels.
+// what they refuse on the device.  *done tells; the explicit matrix, overlapping buffers, a full device, and a capture
+// before tables and work memory are there leave the block to the caller's other kernels.
 pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv, double *S, int64_t lds, bool interleaved,
                            double shift, bool *done);
 // ci_explicit.cu: sigma with the explicit matrix (FP64, interleaved vectors)
