@@ -12,7 +12,7 @@
 // rows of one species come from the grouped tables of ci_rows.cuh: a warp per
 // determinant, kept entries packed with a ballot, so the writes are coalesced
 // and no partner outside the list is looked up.  CISD of 5a5b in 24 orbitals
-// (11.2 M elements): the whole build and one product take 372 us, against
+// (11.2 M elements): the whole build and one product take 364 us, against
 // 13 380 us with a thread per determinant and host offsets.  sigma with the
 // explicit matrix is a warp-per-row gather over the interleaved vectors.
 // pq_ci_ham_csr exports the reference's layout (upper triangle with the
@@ -64,34 +64,40 @@ __device__ __forceinline__ int ham_part(int64_t I, double thr, int t0, int t1, M
   return c;
 }
 
-// Warp per determinant: counts the row's kept elements, or writes them at row_ptr in list order.  Determinants with
-// more than HEAVY connections are shared by the CTA's warps: each takes a slice of every list, and when writing
+// Warp per determinant: counts the row's kept elements, or writes them at row_ptr in list order.  Determinants that
+// outweigh their neighbours (shared_row) are shared by the CTA's warps: each takes a slice of every list, and when writing
 // counts the slices first to know where its own begin.
 template <bool FILL>
 __global__ void __launch_bounds__(32 * rows::WARPS) ham_rows_kernel(rows::Args p, double thr, int32_t *cnt,
                                                                     const int64_t *row_ptr, int32_t *col, double *val) {
   constexpr int W = rows::WARPS, LISTS = 7;
-  __shared__ int slice[LISTS * W + 1];
+  __shared__ int slice[LISTS * W + 1], len[W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t I0 = (int64_t)blockIdx.x * W, I = I0 + warp;
   bool heavy = false;
-  if (I < p.n) {
-    const rows::Det d = rows::load_det(p, I);
-    heavy = d.total > rows::HEAVY;
-    if (!heavy) {
-      const int64_t w = FILL ? row_ptr[I] : 0;
-      const double h = p.diag[I];
-      const bool keep = keep_elem(I, I, h, thr);
-      if (FILL && keep && lane == 0) col[w] = (int32_t)I, val[w] = h;
-      int c = keep;
-      rows::for_lists(p, d, [&](int n, auto &&make) { c += ham_part<FILL>(I, thr, 0, n, make, w + c, col, val); });
-      if (!FILL && lane == 0) cnt[I] = c;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {  // light rows, then the heavy ones that are not shared
+    if (pass ? heavy && !rows::shared_row(len, warp) : I < p.n) {
+      const rows::Det d = rows::load_det(p, I);
+      heavy = d.total > rows::HEAVY;
+      if (pass == 0 && lane == 0) len[warp] = d.total;
+      if (!heavy || pass) {
+        const int64_t w = FILL ? row_ptr[I] : 0;
+        const double h = p.diag[I];
+        const bool keep = keep_elem(I, I, h, thr);
+        if (FILL && keep && lane == 0) col[w] = (int32_t)I, val[w] = h;
+        int c = keep;
+        rows::for_lists(p, d, [&](int n, auto &&make) { c += ham_part<FILL>(I, thr, 0, n, make, w + c, col, val); });
+        if (!FILL && lane == 0) cnt[I] = c;
+      }
+    } else if (pass == 0 && lane == 0) {
+      len[warp] = 0;
     }
+    if (pass == 0 && !__syncthreads_or(heavy)) return;
   }
-  if (!__syncthreads_or(heavy)) return;
-  for (int k = 0; k < W && I0 + k < p.n; k++) {
+  for (int k = 0; k < W; k++) {
+    if (!rows::shared_row(len, k)) continue;  // the same for every thread
     const rows::Det d = rows::load_det(p, I0 + k);
-    if (d.total <= rows::HEAVY) continue;  // the same for every thread
     const double h = p.diag[d.I];
     const bool keep = keep_elem(d.I, d.I, h, thr);
     // this warp's slice of a list of n: whole groups of 32 entries
@@ -219,12 +225,13 @@ __device__ __forceinline__ void spmv_part(const int64_t k0, const int64_t e, con
 }
 
 // Y[I][v] = sum_k val[k] X[col[k]][v], interleaved vectors (NV per determinant): warp per row, and the CTA's warps
-// together on rows of more than HEAVY entries
+// together on rows that outweigh their neighbours (shared_row)
 template <int NV>
 __global__ void __launch_bounds__(32 * rows::WARPS) ham_spmv_kernel(const int64_t *row_ptr, const int32_t *col,
                                                                     const double *val, int64_t n, const double *X,
                                                                     double *Y) {
   __shared__ double part[rows::WARPS][NV];
+  __shared__ int len[rows::WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t I0 = (int64_t)blockIdx.x * rows::WARPS, I = I0 + warp;
   double acc[NV];
@@ -234,23 +241,29 @@ __global__ void __launch_bounds__(32 * rows::WARPS) ham_spmv_kernel(const int64_
       for (int o = 16; o; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
   };
   bool heavy = false;
-  if (I < n) {
-    const int64_t k0 = row_ptr[I], e = row_ptr[I + 1];
-    heavy = e - k0 > rows::HEAVY;
-    if (!heavy) {
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {  // light rows, then the heavy ones that are not shared
+    if (pass ? heavy && !rows::shared_row(len, warp) : I < n) {
+      const int64_t k0 = row_ptr[I], e = row_ptr[I + 1];
+      heavy = e - k0 > rows::HEAVY;
+      if (pass == 0 && lane == 0) len[warp] = (int)(e - k0);  // at most n entries
+      if (!heavy || pass) {
 #pragma unroll
-      for (int v = 0; v < NV; v++) acc[v] = 0.0;
-      spmv_part<NV>(k0, e, col, val, X, lane, 32, acc);
-      sum();
-      if (lane == 0)
+        for (int v = 0; v < NV; v++) acc[v] = 0.0;
+        spmv_part<NV>(k0, e, col, val, X, lane, 32, acc);
+        sum();
+        if (lane == 0)
 #pragma unroll
-        for (int v = 0; v < NV; v++) Y[I * NV + v] = acc[v];
+          for (int v = 0; v < NV; v++) Y[I * NV + v] = acc[v];
+      }
+    } else if (pass == 0 && lane == 0) {
+      len[warp] = 0;
     }
+    if (pass == 0 && !__syncthreads_or(heavy)) return;
   }
-  if (!__syncthreads_or(heavy)) return;
-  for (int r = 0; r < rows::WARPS && I0 + r < n; r++) {
+  for (int r = 0; r < rows::WARPS; r++) {
+    if (!rows::shared_row(len, r)) continue;  // the same for every thread
     const int64_t k0 = row_ptr[I0 + r], e = row_ptr[I0 + r + 1];
-    if (e - k0 <= rows::HEAVY) continue;  // the same for every thread
 #pragma unroll
     for (int v = 0; v < NV; v++) acc[v] = 0.0;
     spmv_part<NV>(k0, e, col, val, X, threadIdx.x, blockDim.x, acc);

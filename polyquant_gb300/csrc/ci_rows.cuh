@@ -54,7 +54,20 @@ struct Args {
 };
 
 constexpr int WARPS = 8;     // determinants per CTA
-constexpr int HEAVY = 1536;  // connections above which the CTA's warps share a determinant
+constexpr int HEAVY = 1536;  // connections above which the CTA's warps may share a determinant
+
+// Whether the CTA's warps share row k, the same for every thread; len: the CTA's row lengths, 0 past the last row.  A
+// heavy row of more than twice the mean would keep its warp long after the others have left; rows alike are one warp's
+// each, since a list split over 256 lanes leaves more of them idle and each row costs a block-wide sum.  Shared
+// whenever heavy, truncated spaces of long rows took up to 3.5 times as long (12o 6a6b, level 10 of 12, four roots 49.8
+// ms against 14.3; products with the explicit matrix of 30o 2a2b 7.3 against 5.3), CISD of 5a5b in 24 orbitals 146 us
+// against 125, and 201 with three times the mean.
+__device__ __forceinline__ bool shared_row(const int *len, int k) {
+  int64_t sum = 0;
+#pragma unroll
+  for (int w = 0; w < WARPS; w++) sum += len[w];
+  return len[k] > HEAVY && (int64_t)len[k] * WARPS > 2 * sum;
+}
 
 template <int NV> __device__ __forceinline__ void load_x(const double *X, int64_t j, double (&x)[NV]) {
   const double *p = X + j * NV;

@@ -10,8 +10,8 @@
 // goes with the Fermi beta string alone), so its CTAs ran one live thread
 // through some 10^3 connections, and a small full space has fewer
 // determinants than the chip has warps.  Here the 32 lanes of a warp share one
-// determinant's connections, and determinants with more than HEAVY
-// connections (the Fermi determinant of a truncated space has all of them) are
+// determinant's connections, and a determinant with far more of them than its
+// neighbours (the Fermi determinant of a truncated space has all of them) is
 // shared by the 8 warps of the CTA.
 //
 // A truncated space keeps the pairs with level(alpha) + level(beta) <= limit.
@@ -24,8 +24,8 @@
 // Coulomb sums of the singles come from tables [string][pair].
 //
 // Bound: FP64 pipe and L2 gathers.  CISD of 5a5b in 24 orbitals (12 636
-// determinants, 11.2 M elements), three roots: 144 us a sigma against 3914 us
-// with the thread-per-determinant kernel, 0.47 TFLOP/s; full CI of water in 7
+// determinants, 11.2 M elements), three roots: 125 us a sigma against 3914 us
+// with the thread-per-determinant kernel, 0.54 TFLOP/s; full CI of water in 7
 // orbitals (441 determinants), one root: 18 against 41 us.
 #include <algorithm>
 
@@ -110,26 +110,33 @@ template <int NV> __device__ __forceinline__ int root_of_lane(int lane) {  // -1
 
 template <int NV> __global__ void __launch_bounds__(32 * WARPS, 3) sigma_rows_kernel(Args p) {
   __shared__ double part[WARPS][4];
+  __shared__ int len[WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t I0 = (int64_t)blockIdx.x * WARPS, I = I0 + warp;
   bool heavy = false;
-  if (I < p.n) {
-    const Det d = load_det(p, I);
-    heavy = d.total > HEAVY;
-    if (!heavy) {
-      double acc[NV];
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {  // light rows, then the heavy ones that are not shared
+    if (pass ? heavy && !shared_row(len, warp) : I < p.n) {
+      const Det d = load_det(p, I);
+      heavy = d.total > HEAVY;
+      if (pass == 0 && lane == 0) len[warp] = d.total;
+      if (!heavy || pass) {
+        double acc[NV];
 #pragma unroll
-      for (int v = 0; v < NV; v++) acc[v] = 0.0;
-      accumulate<NV>(p, d, lane, 32, acc);
-      warp_sum<NV>(acc, lane);
-      const int v = root_of_lane<NV>(lane);
-      if (v >= 0) p.Y[I * NV + v] = acc[0];
+        for (int v = 0; v < NV; v++) acc[v] = 0.0;
+        accumulate<NV>(p, d, lane, 32, acc);
+        warp_sum<NV>(acc, lane);
+        const int v = root_of_lane<NV>(lane);
+        if (v >= 0) p.Y[I * NV + v] = acc[0];
+      }
+    } else if (pass == 0 && lane == 0) {
+      len[warp] = 0;
     }
+    if (pass == 0 && !__syncthreads_or(heavy)) return;
   }
-  if (!__syncthreads_or(heavy)) return;
-  for (int k = 0; k < WARPS && I0 + k < p.n; k++) {
+  for (int k = 0; k < WARPS; k++) {
+    if (!shared_row(len, k)) continue;  // the same for every thread
     const Det d = load_det(p, I0 + k);
-    if (d.total <= HEAVY) continue;  // the same for every thread
     double acc[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) acc[v] = 0.0;
