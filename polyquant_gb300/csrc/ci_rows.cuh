@@ -24,6 +24,7 @@ struct SigmaRows {
   int32_t *row = nullptr;    // alpha string of every determinant
   DevBuf mem;                // all of the above
   int lim = 0;
+  int min_width = 1;         // sigma of fewer vectors is the other kernel's
 };
 
 namespace rows {

@@ -313,6 +313,19 @@ static pq_status launch_sigma(const SigmaArgs<T> &a, int64_t na, size_t smem, cu
   return PQ_OK;
 }
 
+// shared memory of the element kernel: the alpha string's Coulomb rows, and its table of coefficients
+static size_t element_base(const pq_ci_handle *h, size_t esz) {
+  return esz * ((size_t)h->npair[0] + (size_t)h->tab[0][0].max1 * h->n_orb[0]);
+}
+static size_t element_tab(const pq_ci_handle *h, size_t esz) { return esz * (size_t)h->tab[0][0].max1 * h->npair[0]; }
+// packed-register alpha-beta path when the beta singles fit the encoding: registers, 0 without
+static int element_pack(const pq_ci_handle *h, size_t esz) {
+  if (element_base(h, esz) + element_tab(h, esz) > 100 * 1024 || h->tab[0][1].n_str >= (1 << 22) || h->npair[0] > 511) return 0;
+  const int max1b = h->tab[0][1].max1;
+  return max1b <= 32 ? 32 : (max1b <= 64 ? 64 : 0);
+}
+int ci_sigma_pack(const pq_ci_handle *h) { return element_pack(h, sizeof(double)); }
+
 template <typename T, int NV>
 static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift, const int *gate = nullptr) {
   SigmaArgs<T> a{};
@@ -326,13 +339,13 @@ static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift,
   a.n_orb = h->n_orb[0];
   a.npair = h->npair[0];
   a.max1a = h->tab[0][0].max1;
-  int64_t nb = h->tab[0][1].n_str, na = h->tab[0][0].n_str;
+  const int64_t nb = h->tab[0][1].n_str, na = h->tab[0][0].n_str;
   a.nblk_b = (nb + SIGMA_THREADS - 1) / SIGMA_THREADS;
   a.X = X;
   a.Y = Y;
   a.gate = gate;
-  size_t base = sizeof(T) * ((size_t)a.npair + (size_t)a.max1a * a.n_orb);
-  size_t tab = sizeof(T) * (size_t)a.max1a * a.npair;
+  size_t base = element_base(h, sizeof(T));
+  const size_t tab = element_tab(h, sizeof(T));
   const bool use_tab = base + tab <= 100 * 1024;
   // large orbital spaces: the Coulomb rows of the alpha singles stay in global memory (L2)
   a.jrow_global = base > 160 * 1024;
@@ -343,10 +356,7 @@ static pq_status sigma_dispatch(pq_ci_handle *h, const T *X, T *Y, double shift,
     return PQ_ERR_ARG;
   }
   cudaStream_t st = h->stream;
-  // packed-register alpha-beta path when the beta singles fit the encoding
-  const int max1b = h->tab[0][1].max1;
-  const bool pack_ok = use_tab && nb < (1 << 22) && a.npair <= 511;
-  const int pk = !pack_ok ? 0 : (max1b <= 32 ? 32 : (max1b <= 64 ? 64 : 0));
+  const int pk = element_pack(h, sizeof(T));
   if (h->full) {
     if (pk == 32) return launch_sigma<T, NV, true, true, 32>(a, na, smem, st);
     if (pk == 64) return launch_sigma<T, NV, true, true, 64>(a, na, smem, st);
@@ -420,11 +430,11 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvp, int prec
     h->last_path = PQ_PATH_MATRIX;
     return ci_ham_spmv(h, X, Y, nvp);
   }
-  if (precision == PQ_FP64) h->last_path = h->rows ? PQ_PATH_ROWS : PQ_PATH_ELEMENT;
+  if (precision == PQ_FP64) h->last_path = ci_rows_apply(h, nvp) ? PQ_PATH_ROWS : PQ_PATH_ELEMENT;
   if (h->n_species == 2) return ci_sigma2_il(h, X, Y, nvp, precision, shift);
   if (precision == PQ_FP32 && allow_scratch && h->fp32_v2) return ci_sigma32_v2(h, X, Y, nvp, shift);
   if (precision == PQ_FP64) {
-    if (h->rows) return ci_sigma_rows(h, X, Y, nvp, shift);
+    if (ci_rows_apply(h, nvp)) return ci_sigma_rows(h, X, Y, nvp, shift);
     if (nvp == 1) return sigma_dispatch<double, 1>(h, (const double *)X, (double *)Y, shift);
     if (nvp == 2) return sigma_dispatch<double, 2>(h, (const double *)X, (double *)Y, shift);
     if (nvp == 3) return sigma_dispatch<double, 3>(h, (const double *)X, (double *)Y, shift);

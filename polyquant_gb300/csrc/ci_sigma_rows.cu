@@ -220,12 +220,24 @@ __global__ void __launch_bounds__(128) row_kernel(const int64_t *rowoff, const i
 
 }  // namespace rows
 
-// Rule.  Truncated spaces always take this kernel (32-bit determinant indices).  Full spaces take it up to
-// ROWS_FULL_MAX determinants, where the other kernel has too few threads to hide the latency of its serial walk;
-// beyond, that one's staged coefficients and coalesced alpha rows win.  us a sigma (whole call, four roots), this
-// kernel / the other: 441 determinants 22 / 78, 4 900 55 / 126, 15 876 159 / 170, 63 504 657 / 619, 213 444
-// 2955 / 2328.
+// Rules (32-bit determinant indices throughout).  Full spaces take this kernel up to ROWS_FULL_MAX determinants, where
+// the other kernel has too few threads to hide the latency of its serial walk; beyond, that one's staged coefficients
+// and coalesced alpha rows win.  us a sigma (whole call, four roots), this kernel / the other: 441 determinants
+// 22 / 78, 4 900 55 / 126, 15 876 159 / 170, 63 504 657 / 619, 213 444 2955 / 2328.
+// Truncated spaces take it unless they are large and nearly full, so that the other kernel's CTAs of 256 beta strings
+// have few idle threads (`busy`, the share of threads with a determinant), and its packed registers hold the beta
+// singles.  With one to four roots, us, this kernel / the other:
+//   at most 32 singles  11o 5a5b, level 6 of 10 (busy 0.73): 827 / 688 ... 2224 / 1966; level 5 (0.49) 472 / 471 ...
+//                       1265 / 1387; 12o 4a4b, level 7 (0.95) 1300 / 1144 ... 3448 / 2745, level 5 (0.53) 623 / 685 ...
+//                       1661 / 1789; 10o 5a5b, level 7 (0.97, 62 628 determinants) 256 / 225 ... 667 / 634; 10o 4a4b,
+//                       level 7 (0.82, 43 875) 178 / 188 ... 478 / 537: the other kernel from PACK32_MIN on
+//   at most 64 singles  one root only: 14o 7a7b, level 8 of 14 (0.83) 113 / 98 ms, four roots 267 / 303 ms; 13o 5a5b,
+//                       level 8 (0.82) 13.4 / 12.7, four 31.7 / 39.0; 14o 5a5b, level 7 (0.79) 29.5 / 28.3; 12o 6a6b,
+//                       level 6 (0.59) 3.34 / 4.04, level 8 (0.88, 834 957) 5.80 / 5.82; 13o 4a4b, level 7 (0.90,
+//                       495 349) 3.36 / 3.56: the other kernel from PACK64_MIN on
 constexpr int64_t ROWS_FULL_MAX = 1 << 15;
+constexpr int64_t PACK32_MIN = 50000, PACK64_MIN = 800000;
+constexpr double PACK32_BUSY = 0.7, PACK64_BUSY = 0.75;
 constexpr size_t ROWS_COUL_MAX = (size_t)1 << 30;  // larger Coulomb tables are summed in the kernel instead
 
 pq_status rows_make(pq_ci_handle *h, std::unique_ptr<SigmaRows, void (*)(SigmaRows *)> &out) {
@@ -282,6 +294,8 @@ pq_status rows_make(pq_ci_handle *h, std::unique_ptr<SigmaRows, void (*)(SigmaRo
   return PQ_OK;
 }
 
+bool ci_rows_apply(const pq_ci_handle *h, int nvp) { return h->rows && nvp >= h->rows->min_width; }
+
 rows::Args rows_args(const pq_ci_handle *h, const SigmaRows &r) {
   rows::Args p{};
   rows::Side *out[2] = {&p.a, &p.b};
@@ -306,7 +320,14 @@ rows::Args rows_args(const pq_ci_handle *h, const SigmaRows &r) {
 pq_status ci_sigma_rows_build(pq_ci_handle *h) {
   if (h->n_species != 1 || h->n_dets <= 0 || h->n_dets > 0x7fffffffLL) return PQ_OK;
   if (h->full && h->n_dets > ROWS_FULL_MAX) return PQ_OK;
-  return rows_make(h, h->rows);
+  int64_t threads = 0;
+  for (int32_t len : h->rowlen) threads += (len + 255) / 256 * 256;
+  const double busy = (double)h->n_dets / (double)threads;
+  const int pack = h->full ? 0 : ci_sigma_pack(h);
+  if (pack == 32 && h->n_dets >= PACK32_MIN && busy > PACK32_BUSY) return PQ_OK;
+  PQ_TRY(rows_make(h, h->rows));
+  h->rows->min_width = pack == 64 && h->n_dets >= PACK64_MIN && busy > PACK64_BUSY ? 2 : 1;
+  return PQ_OK;
 }
 
 pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift) {

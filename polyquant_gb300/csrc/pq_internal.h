@@ -210,6 +210,9 @@ bool ci_capturing(pq_ci_handle *h);
 pq_status ci_grow(pq_ci_handle *h, DevBuf &b, size_t n);
 // ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
 pq_status ci_sigma_rows_build(pq_ci_handle *h);
+bool ci_rows_apply(const pq_ci_handle *h, int nvp);
+// ci_sigma.cu: beta singles that the FP64 element kernel packs into registers (32 or 64; 0: none)
+int ci_sigma_pack(const pq_ci_handle *h);
 pq_status ci_sigma_rows(pq_ci_handle *h, const void *X, void *Y, int nvp, double shift);
 // ci_sigma64.cu, ci_two64.cu: S = (H - shift) C for at most 4 vectors of device memory that do not overlap (FP64,
 // strides over determinants and vectors).  A raised *gate afterwards means that nothing of it counts.  fixed: with the
