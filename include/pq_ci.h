@@ -79,6 +79,8 @@ typedef struct pq_ci_handle pq_ci_handle;
 
 /* Build strings, excitation tables, determinant addressing and the diagonal
  * on the device (replaces setup_determinants + precompute_diagonal).
+ * The grouped tables of the FP64 row kernel (truncated and small full spaces)
+ * are left out where they do not fit; sigma then takes the element kernel.
  * stream: a cudaStream_t, or NULL for the default stream. */
 pq_status pq_ci_create(const pq_ci_desc *desc, void *stream, pq_ci_handle **out);
 /* Selected-string space (an extension with no reference counterpart: heat-bath
@@ -169,6 +171,12 @@ pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32
  * same-spin GEMM buffers of the FP32 full-CI sigma, the tables, digits and
  * copies of the FP64 tensor-core sigma).  Meant for tests. */
 pq_status pq_debug_scratch_bytes(const pq_ci_handle *h, int64_t *bytes);
+
+/* Diagnostic, no reference counterpart, meant for tests of a full device:
+ * device allocations beyond `room` bytes on top of what the library holds now
+ * fail as cudaMalloc does on a full device (negative: no such limit); *held
+ * (may be NULL) is what it holds, over all handles. */
+pq_status pq_debug_set_alloc_room(long long room, int64_t *held);
 
 /* Diagnostics of the FP64 sigma, no reference counterpart, meant for tests.
  * pq_debug_sigma_path: which kernels the handle's last FP64 sigma was given to

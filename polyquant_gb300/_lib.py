@@ -25,6 +25,7 @@ EXPORTS = [
     "pq_ci_batch_create", "pq_ci_batch_destroy", "pq_ci_batch_num_dets", "pq_ci_batch_sigma",
     "pq_ci_batch_tuning", "pq_ci_batch_davidson", "pq_ao2mo", "pq_mo1", "pq_debug_set_wait_budget",
     "pq_ao2mo_release_workspace", "pq_debug_sigma_path", "pq_debug_set_sigma_wait_budget",
+    "pq_debug_set_alloc_room",
 ]
 
 
@@ -113,6 +114,8 @@ def load(path: str = LIB_PATH):
     L.pq_ci_elements.argtypes = [P, I64, P, P, P]
     L.pq_debug_scratch_bytes.restype = I32
     L.pq_debug_scratch_bytes.argtypes = [P, ctypes.POINTER(I64)]
+    L.pq_debug_set_alloc_room.restype = I32
+    L.pq_debug_set_alloc_room.argtypes = [ctypes.c_longlong, ctypes.POINTER(I64)]
     L.pq_debug_sigma_path.restype = I32
     L.pq_debug_sigma_path.argtypes = [P, ctypes.POINTER(I32), ctypes.POINTER(I32)]
     L.pq_debug_set_sigma_wait_budget.restype = I32

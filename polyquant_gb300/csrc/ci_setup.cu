@@ -10,6 +10,7 @@
 //   elements     src/ci/detset/slater_condon_singleparticle.cpp:4-175
 //   diagonal     src/ci/detset/slater_condon.cpp:102-153
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -22,16 +23,29 @@
 
 namespace pq {
 
+// bytes in all device buffers, and the most there may be (negative: no limit; pq_debug_set_alloc_room)
+static std::atomic<long long> g_held{0}, g_limit{-1};
+
+void DevBuf::release() {
+  if (ptr) cudaFree(ptr);
+  g_held -= (long long)bytes;
+  ptr = nullptr;
+  bytes = 0;
+}
+
 pq_status DevBuf::alloc(size_t n) {
   release();
   if (n == 0) n = 16;
-  cudaError_t e = cudaMalloc(&ptr, n);
+  const long long limit = g_limit;
+  cudaError_t e = limit >= 0 && g_held + (long long)n > limit ? cudaErrorMemoryAllocation : cudaMalloc(&ptr, n);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // not left behind for the check after a launch
     ptr = nullptr;
     set_error("cudaMalloc(%zu) failed: %s", n, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? PQ_ERR_OOM : PQ_ERR_CUDA;
   }
   bytes = n;
+  g_held += (long long)n;
   return PQ_OK;
 }
 
@@ -466,3 +480,9 @@ pq_status ci_build(pq_ci_handle *h) {
 }
 
 }  // namespace pq
+
+extern "C" pq_status pq_debug_set_alloc_room(long long room, int64_t *held) {
+  if (held) *held = pq::g_held;
+  pq::g_limit = room < 0 ? -1 : pq::g_held + room;
+  return PQ_OK;
+}

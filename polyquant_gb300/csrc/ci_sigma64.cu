@@ -553,7 +553,7 @@ __global__ void klist_kernel(const int64_t *o1, const int32_t *J1, const int32_t
 // alpha string within one exact sum of 80, 16-bit beta strings in the scatter lists, dense same-spin matrices of at
 // most 4 GiB of digits that are at least 2.5 % filled (a digit product of a zero costs 1/60 of an FP64 FMA).
 bool sigma64_applicable(const pq_ci_handle *h) {
-  if (h->n_species != 1 || !h->full || h->wide || h->rows) return false;
+  if (h->n_species != 1 || !h->full || h->wide || h->n_dets <= ROWS_FULL_MAX) return false;
   const SpinTablesDev &a = h->tab[0][0], &b = h->tab[0][1];
   if (a.max1 + h->desc.n_alpha[0] > s64::KMAX || b.n_str >= 65536) return false;
   for (int sp = 0; sp < 2; sp++) {

@@ -235,7 +235,6 @@ __global__ void __launch_bounds__(128) row_kernel(const int64_t *rowoff, const i
 //                       level 8 (0.82) 13.4 / 12.7, four 31.7 / 39.0; 14o 5a5b, level 7 (0.79) 29.5 / 28.3; 12o 6a6b,
 //                       level 6 (0.59) 3.34 / 4.04, level 8 (0.88, 834 957) 5.80 / 5.82; 13o 4a4b, level 7 (0.90,
 //                       495 349) 3.36 / 3.56: the other kernel from PACK64_MIN on
-constexpr int64_t ROWS_FULL_MAX = 1 << 15;
 constexpr int64_t PACK32_MIN = 50000, PACK64_MIN = 800000;
 constexpr double PACK32_BUSY = 0.7, PACK64_BUSY = 0.75;
 constexpr size_t ROWS_COUL_MAX = (size_t)1 << 30;  // larger Coulomb tables are summed in the kernel instead
@@ -325,7 +324,12 @@ pq_status ci_sigma_rows_build(pq_ci_handle *h) {
   const double busy = (double)h->n_dets / (double)threads;
   const int pack = h->full ? 0 : ci_sigma_pack(h);
   if (pack == 32 && h->n_dets >= PACK32_MIN && busy > PACK32_BUSY) return PQ_OK;
-  PQ_TRY(rows_make(h, h->rows));
+  const pq_status s = rows_make(h, h->rows);
+  if (s == PQ_ERR_OOM) {
+    clear_error();
+    return PQ_OK;
+  }
+  PQ_TRY(s);
   h->rows->min_width = pack == 64 && h->n_dets >= PACK64_MIN && busy > PACK64_BUSY ? 2 : 1;
   return PQ_OK;
 }

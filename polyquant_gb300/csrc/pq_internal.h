@@ -41,11 +41,7 @@ struct DevBuf {
   void *ptr = nullptr;
   size_t bytes = 0;
   ~DevBuf() { release(); }
-  void release() {
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-  }
+  void release();
   pq_status alloc(size_t n);
   // grow-only allocation used for scratch; contents are not preserved
   pq_status ensure(size_t n) { return n <= bytes ? PQ_OK : alloc(n); }
@@ -208,7 +204,9 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int pre
 bool ci_capturing(pq_ci_handle *h);
 // grow-only work memory of a sigma; contents are not preserved
 pq_status ci_grow(pq_ci_handle *h, DevBuf &b, size_t n);
-// ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle), FP64 sigma on them
+// ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle, unless the device is too
+// full for them: the element kernel needs none), FP64 sigma on them
+constexpr int64_t ROWS_FULL_MAX = 1 << 15;  // full spaces of more determinants leave them out
 pq_status ci_sigma_rows_build(pq_ci_handle *h);
 bool ci_rows_apply(const pq_ci_handle *h, int nvp);
 // ci_sigma.cu: beta singles that the FP64 element kernel packs into registers (32 or 64; 0: none)

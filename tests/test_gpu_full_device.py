@@ -1,0 +1,60 @@
+"""A device that is too full for tables which only make a call faster (allocations beyond a limit fail as on a full
+device, pq_debug_set_alloc_room): the call is answered without them."""
+import ctypes
+
+import pytest
+
+from cases import synthetic_ep, synthetic_fci
+from test_gpu_sigma_path import _make, path
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+class Room:
+    """`with Room(bytes)`: the library may allocate that much more."""
+
+    def __init__(self, room):
+        self.room = room
+
+    def __enter__(self):
+        set_room(self.room)
+
+    def __exit__(self, *a):
+        set_room(-1)
+
+
+def set_room(room):
+    from polyquant_gb300 import _lib
+
+    held = ctypes.c_int64()
+    assert _lib.load().pq_debug_set_alloc_room(ctypes.c_longlong(room), ctypes.byref(held)) == _lib.PQ_OK
+    return held.value
+
+
+def _x(g, k):
+    return torch.randn(k, g.N_dets, device="cuda", dtype=torch.float64).t()
+
+
+def test_row_tables_do_not_fit():
+    from polyquant_gb300 import _lib
+
+    p = synthetic_fci(16, 4, 4, seed=2, ex=[2, 2, 2])
+    before = set_room(-1)
+    g = _make(p)
+    size = set_room(-1) - before
+    X = _x(g, 3)
+    want = g.sigma(X)
+    assert path(g)[0] == _lib.PQ_PATH_ROWS
+    with Room(size - 1):
+        r = _make(p)
+    S = r.sigma(X)
+    assert path(r)[0] == _lib.PQ_PATH_ELEMENT
+    assert (S - want).abs().max().item() <= TOL * want.abs().max().item()
+    nnz = r.create_ham()
+    assert nnz == g.create_ham()
+    with pytest.raises(_lib.PQError) as e, Room(0):
+        _make(p)
+    assert e.value.status == _lib.PQ_ERR_OOM
