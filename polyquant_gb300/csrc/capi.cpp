@@ -40,6 +40,12 @@ const char *pq_last_error(void) { return g_err; }
 const char *pq_version(void) { return "polyquant-gb300 0.1 (sm_103a)"; }
 
 pq_status pq_ci_create(const pq_ci_desc *desc, void *stream, pq_ci_handle **out) {
+  return ci_create(desc, stream, false, out);
+}
+
+}  // extern "C"
+
+pq_status pq::ci_create(const pq_ci_desc *desc, void *stream, bool batched, pq_ci_handle **out) {
   clear_error();
   if (!desc || !out) {
     set_error("pq_ci_create: NULL argument");
@@ -54,6 +60,7 @@ pq_status pq_ci_create(const pq_ci_desc *desc, void *stream, pq_ci_handle **out)
   }
   h->desc = *desc;
   h->stream = (cudaStream_t)stream;
+  h->batched = batched;
   pq_status s = ci_build(h);
   if (s != PQ_OK) {
     delete h;
@@ -62,6 +69,8 @@ pq_status pq_ci_create(const pq_ci_desc *desc, void *stream, pq_ci_handle **out)
   *out = h;
   return PQ_OK;
 }
+
+extern "C" {
 
 pq_status pq_ci_create_selected(const pq_ci_desc *desc, const uint64_t *const *strings, const int64_t *n_strings,
                                 void *stream, pq_ci_handle **out) {

@@ -1087,7 +1087,7 @@ pq_status pq_ci_batch_create(const pq_ci_desc *descs, int32_t n, void *stream, p
   B->prob.resize(n);
   for (int i = 0; i < n; i++) {
     pq_ci_handle *h = nullptr;
-    pq_status s = pq_ci_create(&descs[i], B->stream, &h);
+    pq_status s = ci_create(&descs[i], B->stream, true, &h);
     if (s != PQ_OK) return s;
     B->h.push_back(h);
     s = make_prob(h, *B->tabs[i], B->prob[i], B->stream);

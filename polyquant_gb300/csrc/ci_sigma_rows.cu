@@ -317,7 +317,7 @@ rows::Args rows_args(const pq_ci_handle *h, const SigmaRows &r) {
 }
 
 pq_status ci_sigma_rows_build(pq_ci_handle *h) {
-  if (h->n_species != 1 || h->n_dets <= 0 || h->n_dets > 0x7fffffffLL) return PQ_OK;
+  if (h->batched || h->n_species != 1 || h->n_dets <= 0 || h->n_dets > 0x7fffffffLL) return PQ_OK;
   if (h->full && h->n_dets > ROWS_FULL_MAX) return PQ_OK;
   int64_t threads = 0;
   for (int32_t len : h->rowlen) threads += (len + 255) / 256 * 256;

@@ -109,6 +109,7 @@ struct pq_ci_handle {
   int npair[2] = {0, 0};
   int n_words = 1;     // words per string in the reference layout, (max n_orb >> 6) + 1
   bool wide = false;   // some species has more than 64 orbitals: strings keep a second word
+  bool batched = false;   // member of a batch, whose sigma runs in ci_batch.cu
   bool selected = false;  // strings given by the caller (pq_ci_create_selected): full product, no levels
   int n_blocks[2] = {1, 1};  // spin blocks of integrals per species
   // host strings (occupation masks, reference order) and their levels
@@ -180,6 +181,8 @@ struct pq_ci_handle {
 };
 
 namespace pq {
+// capi.cpp: pq_ci_create; batched: without the tables that only a handle's own sigma reads
+pq_status ci_create(const pq_ci_desc *desc, void *stream, bool batched, pq_ci_handle **out);
 // ci_setup.cu
 pq_status ci_build(pq_ci_handle *h);
 pq_status make_strings(int n_orb, int n_e, int ex_max, std::vector<uint64_t> &out, std::vector<int32_t> &lvl,

@@ -58,3 +58,19 @@ def test_row_tables_do_not_fit():
     with pytest.raises(_lib.PQError) as e, Room(0):
         _make(p)
     assert e.value.status == _lib.PQ_ERR_OOM
+
+
+def test_batch_members_hold_no_row_tables():
+    """Their sigma is the batched kernel's: a batch of one holds less than a handle, which has the row tables."""
+    from polyquant_gb300.batch import CIBatch
+
+    p = synthetic_fci(9, 4, 4, seed=3)
+    start = set_room(-1)
+    g = _make(p)
+    handle = set_room(-1) - start
+    b = CIBatch([dict(n_orb=p.n_orb, n_alpha=p.n_alpha, n_beta=p.n_beta, h1=p.h1, eri=p.eri, excitation_level=p.ex_level,
+                      restricted=p.restricted, charge=p.charge)])
+    batch = set_room(-1) - start - handle
+    assert batch < handle, (batch, handle)
+    b.close()
+    g.close()
