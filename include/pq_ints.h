@@ -48,7 +48,8 @@ pq_status pq_ao2mo(const double *eri_ao, int32_t layout, int64_t n_ao_a, int64_t
  * calls, so repeated transforms allocate nothing; calls on one device share
  * them and run one at a time.  This frees them for the current device (no
  * reference counterpart: the reference's transform holds its buffers only
- * during the call). */
+ * during the call).  An allocation of this library that does not fit frees
+ * them too; allocations of other libraries cannot. */
 pq_status pq_ao2mo_release_workspace(void);
 
 /* MO one-body integrals h_MO = C^T F C for an n_ao x n_ao operator F

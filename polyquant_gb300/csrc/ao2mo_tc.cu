@@ -908,9 +908,34 @@ struct Ao2moWorkspace {
     for (DevBuf *b : {&full, &cth, &ctl, &sh, &sl, &uh, &ul, &H1, &err}) b->release();
     f64.release();
   }
+  size_t bytes() const {
+    size_t n = f64.bytes();
+    for (const DevBuf *b : {&full, &cth, &ctl, &sh, &sl, &uh, &ul, &H1, &err}) n += b->bytes;
+    return n;
+  }
 };
 static std::mutex g_ws_mu;
 static Ao2moWorkspace g_ws[64];
+static thread_local bool t_transform = false;  // this thread is inside a transform and holds the lock
+struct WorkspaceLock {
+  std::lock_guard<std::mutex> lock{g_ws_mu};
+  cudaStream_t st;
+  explicit WorkspaceLock(cudaStream_t s) : st(s) { t_transform = true; }
+  ~WorkspaceLock() {
+    cudaStreamSynchronize(st);  // also after an error, with kernels under way: the next call may be on another stream
+    t_transform = false;
+  }
+};
+
+// For an allocation that did not fit: frees this device's buffers between transforms; whether there were any.
+bool ao2mo_give_back() {
+  if (t_transform) return false;
+  std::unique_lock<std::mutex> lock(g_ws_mu, std::try_to_lock);
+  int dev = 0;
+  if (!lock || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || g_ws[dev].bytes() == 0) return false;
+  g_ws[dev].release();
+  return true;
+}
 
 long long ao2mo_wait_cycles() { return g_gemm_wait_cycles; }
 
@@ -924,7 +949,7 @@ pq_status ao2mo_f64_shared(const double *eri_ao, int layout, int64_t n_ao_a, int
     set_error("pq_ao2mo: device ordinal %d out of range", dev);
     return PQ_ERR_STATE;
   }
-  std::lock_guard<std::mutex> lock(g_ws_mu);
+  WorkspaceLock lock(st);
   auto run = [&] {
     return ao2mo_f64(g_ws[dev].f64, eri_ao, layout, n_ao_a, n_ao_b, Ca, lda, nmo_a, Cb, ldb, nmo_b, eri_mo, st);
   };
@@ -951,7 +976,7 @@ static pq_status ao2mo_tc_impl(const double *eri_ao, int layout, int64_t n, cons
     set_error("pq_ao2mo: device ordinal %d out of range", dev);
     return PQ_ERR_STATE;
   }
-  std::lock_guard<std::mutex> lock(g_ws_mu);
+  WorkspaceLock lock(st);
   Ao2moWorkspace &w = g_ws[dev];
   DevBuf &full = w.full, &cth = w.cth, &ctl = w.ctl, &sh = w.sh, &sl = w.sl, &uh = w.uh, &ul = w.ul, &H1 = w.H1,
          &err = w.err;

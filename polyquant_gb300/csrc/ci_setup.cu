@@ -25,6 +25,7 @@ namespace pq {
 
 // bytes in all device buffers, and the most there may be (negative: no limit; pq_debug_set_alloc_room)
 static std::atomic<long long> g_held{0}, g_limit{-1};
+bool ao2mo_give_back();  // ao2mo_tc.cu
 
 void DevBuf::release() {
   if (ptr) cudaFree(ptr);
@@ -36,8 +37,12 @@ void DevBuf::release() {
 pq_status DevBuf::alloc(size_t n) {
   release();
   if (n == 0) n = 16;
-  const long long limit = g_limit;
-  cudaError_t e = limit >= 0 && g_held + (long long)n > limit ? cudaErrorMemoryAllocation : cudaMalloc(&ptr, n);
+  auto get = [&] {
+    const long long limit = g_limit;
+    return limit >= 0 && g_held + (long long)n > limit ? cudaErrorMemoryAllocation : cudaMalloc(&ptr, n);
+  };
+  cudaError_t e = get();
+  if (e == cudaErrorMemoryAllocation && ao2mo_give_back()) e = get();  // kept between transforms only to save time
   if (e != cudaSuccess) {
     cudaGetLastError();  // not left behind for the check after a launch
     ptr = nullptr;

@@ -270,6 +270,11 @@ struct Ao2moF64 {
   void release() {
     for (DevBuf *b : {&ct, &s, &u, &e, &h1, &err}) b->release();
   }
+  size_t bytes() const {
+    size_t n = 0;
+    for (const DevBuf *b : {&ct, &s, &u, &e, &h1, &err}) n += b->bytes;
+    return n;
+  }
 };
 pq_status ao2mo_f64(Ao2moF64 &w, const double *eri_ao, int layout, int64_t n_ao_a, int64_t n_ao_b, const double *Ca,
                     int64_t lda, int64_t nmo_a, const double *Cb, int64_t ldb, int64_t nmo_b, double *eri_mo,

@@ -74,3 +74,33 @@ def test_batch_members_hold_no_row_tables():
     assert batch < handle, (batch, handle)
     b.close()
     g.close()
+
+
+def test_transform_buffers_are_given_back():
+    """What the transforms keep between calls goes when another allocation of the library does not fit."""
+    from polyquant_gb300 import _lib
+    from polyquant_gb300.integral import ao2mo
+
+    n = 60
+    npair = n * (n + 1) // 2
+    P = torch.randn(npair * (npair + 1) // 2, device="cuda", dtype=torch.float64)
+    C = torch.randn(n, n, device="cuda", dtype=torch.float64)
+    assert _lib.load().pq_ao2mo_release_workspace() == _lib.PQ_OK
+    before = set_room(-1)
+    out = ao2mo(P, C, layout=_lib.PQ_AO_PACKED8, mode=_lib.PQ_XFORM_FP64)
+    kept = set_room(-1) - before
+    assert kept > 8 * npair * npair
+    with Room(0):
+        g = _make(synthetic_fci(10, 5, 5, seed=4))
+    assert g.N_dets == 63504
+    assert set_room(-1) - before < kept
+    again = ao2mo(P, C, layout=_lib.PQ_AO_PACKED8, mode=_lib.PQ_XFORM_FP64)
+    assert torch.equal(out, again)
+    # a transform that does not fit beside its own buffers of an earlier call frees them and fails only then
+    with Room(0), pytest.raises(_lib.PQError) as e:
+        m = 90
+        q = m * (m + 1) // 2
+        ao2mo(torch.randn(q * (q + 1) // 2, device="cuda", dtype=torch.float64),
+              torch.randn(m, m, device="cuda", dtype=torch.float64), layout=_lib.PQ_AO_PACKED8, mode=_lib.PQ_XFORM_FP64)
+    assert e.value.status == _lib.PQ_ERR_OOM
+    assert torch.equal(out, ao2mo(P, C, layout=_lib.PQ_AO_PACKED8, mode=_lib.PQ_XFORM_FP64))
