@@ -219,7 +219,7 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
   }
   size_t esz = precision == PQ_FP64 ? sizeof(double) : sizeof(float);
   ci_capturing(h);
-  for (int v0 = 0; v0 < nvec; v0 += 4) {
+  auto block = [&](int v0) -> pq_status {
     int nv = nvec - v0 < 4 ? nvec - v0 : 4;
     int nvp = il_width(h, nv, precision);
     if (precision == PQ_FP64 && h->fp64_tc && !h->use_explicit) {
@@ -228,22 +228,21 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
         PQ_TRY(ci_sigma64_block(h, C + (size_t)v0 * ldc, ldc, nv, S + (size_t)v0 * lds, lds, false, 0.0, &done));
       } else {
         // page-locked host columns pass through device columns, copied by the conversion kernels
-        const size_t n = (size_t)h->n_dets, block = sizeof(double) * nv * (n + 1);
-        PQ_TRY(ci_grow(h, h->x_il, block));
-        PQ_TRY(ci_grow(h, h->y_il, block));
+        const size_t n = (size_t)h->n_dets, cols = sizeof(double) * nv * (n + 1);
+        PQ_TRY(ci_grow(h, h->x_il, cols));
+        PQ_TRY(ci_grow(h, h->y_il, cols));
         double *x = h->x_il.as<double>(), *y = h->y_il.as<double>();
         for (int v = 0; v < nv; v++) PQ_TRY(ci_to_il(h, C, ldc, v0 + v, 1, 1, PQ_FP64, x + v * n));
         PQ_TRY(ci_sigma64_block(h, x, n, nv, y, n, false, 0.0, &done));
         for (int v = 0; v < nv && done; v++) PQ_TRY(ci_from_il(h, y + v * n, v0 + v, 1, 1, PQ_FP64, S, lds));
       }
-      if (done) continue;
+      if (done) return PQ_OK;
     }
     if (on_device && nvp == 1 && precision == PQ_FP64) {
       const double *c = C + (size_t)v0 * ldc;
       double *s = S + (size_t)v0 * lds;
       if (s + h->n_dets <= c || c + h->n_dets <= s) {  // sigma over its own input needs the copies below
-        PQ_TRY(ci_sigma_il(h, c, s, 1, precision, 0.0));
-        continue;
+        return ci_sigma_il(h, c, s, 1, precision, 0.0);
       }
     }
     size_t bytes = esz * (size_t)nvp * (size_t)(h->n_dets + 1);
@@ -251,8 +250,9 @@ static pq_status sigma_device(pq_ci_handle *h, const double *C, int64_t ldc, int
     PQ_TRY(ci_grow(h, h->y_il, bytes));
     PQ_TRY(ci_to_il(h, C, ldc, v0, nv, nvp, precision, h->x_il.ptr));
     PQ_TRY(ci_sigma_il(h, h->x_il.ptr, h->y_il.ptr, nvp, precision, 0.0));
-    PQ_TRY(ci_from_il(h, h->y_il.ptr, v0, nv, nvp, precision, S, lds));
-  }
+    return ci_from_il(h, h->y_il.ptr, v0, nv, nvp, precision, S, lds);
+  };
+  for (int v0 = 0; v0 < nvec; v0 += 4) PQ_TRY(with_room(h, [&] { return block(v0); }));
   return PQ_OK;
 }
 
@@ -293,8 +293,8 @@ pq_status pq_ci_sigma_host(pq_ci_handle *h, const double *C, int64_t ldc, int32_
   // pageable buffers: device copies of C and sigma stay with the handle (grow-only), so repeated calls
   // allocate nothing; with ldc == n (and lds == n) each block moves in one copy
   const size_t bytes = sizeof(double) * (size_t)n * nvec + 16;
-  PQ_TRY(h->host_c.ensure(bytes));
-  PQ_TRY(h->host_s.ensure(bytes));
+  PQ_TRY(with_room(h, [&] { return h->host_c.ensure(bytes); }));
+  PQ_TRY(with_room(h, [&] { return h->host_s.ensure(bytes); }));
   double *dc = h->host_c.as<double>(), *ds = h->host_s.as<double>();
   if (ldc == n) {
     PQ_CUDA_TRY(cudaMemcpyAsync(dc, C, sizeof(double) * (size_t)n * nvec, cudaMemcpyHostToDevice, h->stream));
@@ -331,7 +331,7 @@ pq_status pq_ci_sigma_interleaved(pq_ci_handle *h, const void *X, void *Y, int32
     set_error("unsupported interleave width %d / precision %d (widths 1, 2, 4)", nvec, precision);
     return PQ_ERR_ARG;
   }
-  return ci_sigma_il(h, X, Y, nvec, precision, diag_shift);
+  return with_room(h, [&] { return ci_sigma_il(h, X, Y, nvec, precision, diag_shift); });
 }
 
 pq_status pq_debug_sigma_path(pq_ci_handle *h, int32_t *path, int32_t *gate) {

@@ -722,14 +722,14 @@ pq_status sigma_request_single(pq_ci_handle *h, const SigmaRequest &r) {
   return PQ_OK;
 }
 
-pq_status ci_davidson(pq_ci_handle *h, const pq_davidson_params *p, double *energies, double *vecs,
-                      pq_davidson_report *rep_out) {
+static pq_status davidson_run(pq_ci_handle *h, const pq_davidson_params *p, double *energies, double *vecs,
+                              pq_davidson_report *rep_out) {
   DavidsonRun D;
   PQ_TRY(D.init(h, *p));
   while (!D.done) {
     if (D.pending) {
       const auto t0 = std::chrono::steady_clock::now();
-      PQ_TRY(sigma_request_single(h, D.req));
+      PQ_TRY(with_room(h, [&] { return sigma_request_single(h, D.req); }));
       PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
       D.rep.sigma_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     }
@@ -740,6 +740,11 @@ pq_status ci_davidson(pq_ci_handle *h, const pq_davidson_params *p, double *ener
   if (D.result != PQ_OK)
     set_error("davidson: not converged after %d iterations (max residual %.3e)", D.iter_max, D.rep.max_residual);
   return D.result;
+}
+
+pq_status ci_davidson(pq_ci_handle *h, const pq_davidson_params *p, double *energies, double *vecs,
+                      pq_davidson_report *rep_out) {
+  return with_room(h, [&] { return davidson_run(h, p, energies, vecs, rep_out); });
 }
 
 }  // namespace pq

@@ -532,7 +532,7 @@ pq_status pq_ci_s2(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, 
   const int ns = h->n_species;
   DevBuf own;
   if (ns == 1)
-    PQ_TRY(pair_lists(h));
+    PQ_TRY(with_room(h, [&] { return pair_lists(h); }));
   else
     PQ_TRY(own.alloc(sizeof(double) * S2_MAXV));
   double *out = ns == 1 ? h->pairs->out.as<double>() : own.as<double>();
@@ -563,7 +563,7 @@ pq_status pq_ci_rdm1(pq_ci_handle *h, const double *C, int32_t species, int32_t 
   }
   const int n = h->n_orb[species];
   if (h->n_species == 1) {
-    PQ_TRY(pair_lists(h));
+    PQ_TRY(with_room(h, [&] { return pair_lists(h); }));
     PQ_TRY(rdm_one(h, C, spin));
     std::vector<double> d(h->npair[0]);
     PQ_CUDA_TRY(cudaMemcpyAsync(d.data(), h->pairs->out.ptr, sizeof(double) * d.size(), cudaMemcpyDeviceToHost, h->stream));

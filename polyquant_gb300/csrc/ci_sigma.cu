@@ -387,6 +387,21 @@ bool ci_capturing(pq_ci_handle *h) {
   return true;
 }
 
+bool ci_drop_tables(pq_ci_handle *h) {
+  const bool made = h->s64 || h->two64 || h->pairs;
+  if (h->captured || !(made || h->rows)) return false;
+  cudaStreamSynchronize(h->stream);
+  if (h->last_path == PQ_PATH_TENSOR) h->last_path = PQ_PATH_NONE;
+  if (made) {
+    h->s64.reset();
+    h->two64.reset();
+    h->pairs.reset();
+  } else {
+    h->rows.reset();
+  }
+  return true;
+}
+
 pq_status ci_grow(pq_ci_handle *h, DevBuf &b, size_t n) {
   if (n <= b.bytes) return PQ_OK;
   if (b.ptr && h->captured) {

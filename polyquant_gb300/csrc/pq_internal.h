@@ -205,6 +205,18 @@ pq_status ci_sigma_il(pq_ci_handle *h, const void *X, void *Y, int nvec, int pre
 // whether the handle's stream is being captured into a graph (then nothing may be allocated or waited for); remembered
 // in h->captured
 bool ci_capturing(pq_ci_handle *h);
+// Frees tables of the handle that only make calls faster: first those of the tensor-core sigma and the properties, which
+// are made again when they fit, then those of the row kernel.  False: nothing left, or a graph may hold their addresses.
+bool ci_drop_tables(pq_ci_handle *h);
+// f(), again after each step of ci_drop_tables while it runs out of device memory
+template <typename F> pq_status with_room(pq_ci_handle *h, F &&f) {
+  pq_status s = f();
+  while (s == PQ_ERR_OOM && ci_drop_tables(h)) {
+    clear_error();
+    s = f();
+  }
+  return s;
+}
 // grow-only work memory of a sigma; contents are not preserved
 pq_status ci_grow(pq_ci_handle *h, DevBuf &b, size_t n);
 // ci_sigma_rows.cu: grouped tables of truncated and small full spaces (built with the handle, unless the device is too

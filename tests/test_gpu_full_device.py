@@ -104,3 +104,78 @@ def test_transform_buffers_are_given_back():
               torch.randn(m, m, device="cuda", dtype=torch.float64), layout=_lib.PQ_AO_PACKED8, mode=_lib.PQ_XFORM_FP64)
     assert e.value.status == _lib.PQ_ERR_OOM
     assert torch.equal(out, ao2mo(P, C, layout=_lib.PQ_AO_PACKED8, mode=_lib.PQ_XFORM_FP64))
+
+
+def _need(make, run):
+    """Device bytes that run(handle) takes from the library on a fresh handle, to within 2 %."""
+    from polyquant_gb300 import _lib
+
+    _lib.load().pq_ao2mo_release_workspace()  # else the first failure would free it
+    lo, hi = 0, 1 << 20
+    while True:
+        g = make()
+        try:
+            with Room(hi):
+                run(g)
+            break
+        except Exception:
+            lo, hi = hi, 2 * hi
+    while hi - lo > hi // 50:
+        mid = (lo + hi) // 2
+        g = make()
+        try:
+            with Room(mid):
+                run(g)
+            hi = mid
+        except Exception:
+            lo = mid
+    return hi
+
+
+@pytest.mark.parametrize("what", ["fp32", "davidson", "ham"])
+@pytest.mark.parametrize("p", [lambda: synthetic_fci(11, 5, 5, seed=5), lambda: synthetic_ep(33, 1, 1, 9, 1, 0, seed=6)],
+                         ids=["full", "two species"])
+def test_tables_of_the_tensor_cores_make_room(monkeypatch, p, what):
+    """A call that fits a handle without them fits one that has used them."""
+    from polyquant_gb300 import _lib
+
+    monkeypatch.setenv("PQ_TWO64_ALWAYS", "1")
+    p = p()
+    if what == "ham" and p.n_orb[0] == 11:
+        p = synthetic_fci(10, 5, 4, seed=5)
+    runs = {"fp32": lambda g: g.sigma(torch.ones(g.N_dets, 4, device="cuda", dtype=torch.float64), precision=_lib.PQ_FP32),
+            "davidson": lambda g: g.davidson(num_states=1, num_subspace_vec=3, convergence_E=1e-6)[0],
+            "ham": lambda g: g.create_ham()}
+    run = runs[what]
+    monkeypatch.setenv("PQ_SIGMA64_GATHER", "1")
+    room = _need(lambda: _make(p), run)
+    monkeypatch.delenv("PQ_SIGMA64_GATHER")
+    g = _make(p)
+    X = _x(g, 4)
+    before = set_room(-1)
+    S = g.sigma(X)
+    tables = set_room(-1) - before
+    assert path(g)[0] == _lib.PQ_PATH_TENSOR
+    with Room(max(0, room - tables // 2)):
+        out = run(g)
+    if what == "davidson":
+        assert abs(out - run(g)).max() < 1e-6
+    g.release_ham()
+    assert (g.sigma(X) - S).abs().max().item() <= TOL * S.abs().max().item()
+    g.close()
+
+
+def test_row_tables_make_room():
+    """Likewise the row kernel's, when a solve does not fit beside them."""
+    p = synthetic_fci(16, 4, 4, seed=7, ex=[2, 2, 2])
+    g = _make(p)
+
+    def run(h):
+        return h.davidson(num_states=1, num_subspace_vec=3, convergence_E=1e-8)[0]
+
+    e = run(g)
+    room = _need(lambda: _make(p), run)  # with them
+    with Room(room * 4 // 5):
+        low = run(g)
+    assert abs(low - e).max() < 1e-8
+    g.close()
