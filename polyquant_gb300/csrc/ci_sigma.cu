@@ -421,8 +421,9 @@ pq_status ci_sigma64_block(pq_ci_handle *h, const double *C, int64_t ldc, int nv
   int *gate = nullptr;
   const bool fixed = ci_capturing(h);
   const auto run = h->n_species == 2 ? ci_two64 : ci_sigma64;
-  const pq_status s = interleaved ? run(h, C, nv, 1, nv, shift, S, nv, 1, fixed, &gate)
-                                  : run(h, C, 1, ldc, nv, shift, S, 1, lds, fixed, &gate);
+  const pq_status s = host_guard([&] {
+    return interleaved ? run(h, C, nv, 1, nv, shift, S, nv, 1, fixed, &gate) : run(h, C, 1, ldc, nv, shift, S, 1, lds, fixed, &gate);
+  });
   if (s == PQ_ERR_OOM) {
     cudaGetLastError();
     clear_error();

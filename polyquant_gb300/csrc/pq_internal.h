@@ -5,6 +5,7 @@
 
 #include <chrono>
 #include <memory>
+#include <new>
 #include <string>
 #include <utility>
 #include <vector>
@@ -208,12 +209,21 @@ bool ci_capturing(pq_ci_handle *h);
 // Frees tables of the handle that only make calls faster: first those of the tensor-core sigma and the properties, which
 // are made again when they fit, then those of the row kernel.  False: nothing left, or a graph may hold their addresses.
 bool ci_drop_tables(pq_ci_handle *h);
-// f(), again after each step of ci_drop_tables while it runs out of device memory
+// f(), with a failed host allocation as PQ_ERR_OOM: no exception leaves a C entry
+template <typename F> pq_status host_guard(F &&f) {
+  try {
+    return f();
+  } catch (const std::bad_alloc &) {
+    set_error("host allocation failed");
+    return PQ_ERR_OOM;
+  }
+}
+// f(), again after each step of ci_drop_tables while it runs out of memory
 template <typename F> pq_status with_room(pq_ci_handle *h, F &&f) {
-  pq_status s = f();
+  pq_status s = host_guard(f);
   while (s == PQ_ERR_OOM && ci_drop_tables(h)) {
     clear_error();
-    s = f();
+    s = host_guard(f);
   }
   return s;
 }
