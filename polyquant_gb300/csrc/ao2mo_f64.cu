@@ -392,21 +392,9 @@ __global__ void __launch_bounds__(512) slice_digits_kernel(const double *src, in
 
 }  // namespace f64
 
-static PFN_cuTensorMapEncodeTiled_v12000 f64_encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      return (PFN_cuTensorMapEncodeTiled_v12000)p;
-    return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
-  }();
-  return fn;
-}
-
 // digit rows: boxes of 64 FP16 (two digits of a chunk) x box_rows, 128-byte swizzle, zeros past the last row
 static pq_status f64_map(CUtensorMap *m, const void *base, int64_t rows, int64_t row_len, int box_rows) {
-  auto fn = f64_encode_fn();
+  auto fn = tcx::encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return PQ_ERR_CUDA;

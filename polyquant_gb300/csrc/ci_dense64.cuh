@@ -287,22 +287,10 @@ static __global__ void __launch_bounds__(256) absmax_kernel(const double *x, int
 
 }  // namespace s64
 
-inline PFN_cuTensorMapEncodeTiled_v12000 s64_encode_fn() {
-  inline PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      return (PFN_cuTensorMapEncodeTiled_v12000)p;
-    return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
-  }();
-  return fn;
-}
-
 // FP16 matrix of `rows` rows of `cols` values, ld values apart; reads outside give zeros
 inline pq_status s64_map(CUtensorMap *m, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_cols,
                          int box_rows) {
-  auto fn = s64_encode_fn();
+  auto fn = tcx::encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return PQ_ERR_CUDA;
