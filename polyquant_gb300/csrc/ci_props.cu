@@ -39,48 +39,124 @@ constexpr int S2_MAXV = 8;
 // between i and j, at the string with the larger index, in its order: {I << 1 | phase, J << 1 | (I holds i)}; for
 // i = j the strings that hold i, {I << 1, I << 1}.
 struct PairLists {
-  DevBuf off[2], ent[2];     // int64 [npair + 1], uint2
-  std::vector<int64_t> hoff[2];
-  DevBuf out;                // sums of a call
+  struct Side {
+    int64_t *off = nullptr;  // [npair + 1]
+    uint2 *ent = nullptr;
+    int64_t n_ent = 0;       // half of the singles, and every string's occupied orbitals
+  };
+  Side side[2];
+  double *out = nullptr;     // sums of a call
+  DevBuf mem;                // all of the above
 };
 void pairs_delete(PairLists *p) { delete p; }
 
-// warp per pair: counts (ent == NULL) or writes its list
-__global__ void __launch_bounds__(128) pair_lists_kernel(int npair, int64_t n_str, const uint64_t *str,
-                                                         const uint64_t *str_hi, const int64_t *s1_off,
-                                                         const int32_t *s1_J, const int32_t *s1_info, int64_t *cnt,
-                                                         const int64_t *off, uint2 *ent) {
-  const int lane = threadIdx.x & 31, q = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (q >= npair) return;
-  int i = 0;
+// The lists are made in three launches for both spins, without a word from the device: a chunk of strings is counted
+// by pair, the counts are summed over the chunks and then over the pairs, and each chunk's warp writes its strings'
+// entries one string after the other, 32 lanes over its singles (which belong to different pairs).  The first property
+// call of a handle then takes little longer than one that made no lists; with a warp per pair searching every string's
+// singles, counts read back and five allocations, first calls of <S^2> took up to 1.5 ms more (14o 7a1b, 48 048
+// determinants: 503 us without lists, 1974 so, 246 now; 9o 4a4b 143 / 205 / 114; CISD of 5a5b in 100 orbitals
+// 175 / 89 / 10 ms).
+struct PairBuild {
+  const uint64_t *str[2], *str_hi[2];
+  const int64_t *o1[2];
+  const int32_t *J[2], *info[2];
+  int64_t n[2];
+  int chunks[2], per[2];  // chunks of `per` strings
+  uint32_t *cnt[2];       // [chunk][pair]: entries, then those of the same pair in earlier chunks
+  int64_t *off[2];
+  uint2 *ent[2];
+  int npair;
+};
+constexpr int PAIR_CHUNKS = 304;
+
+__device__ __forceinline__ int pair_row(int q) {  // i of q = i (i + 1) / 2 + j, j <= i
+  int i = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
+  while (i * (i + 1) / 2 > q) i--;
   while ((i + 1) * (i + 2) / 2 <= q) i++;
-  const int j = q - i * (i + 1) / 2;
-  int64_t w = ent ? off[q] : 0;
-  for (int64_t I0 = 0; I0 < n_str; I0 += 32) {
-    const int64_t I = I0 + lane;
-    bool there = false;
-    uint2 e = make_uint2(0u, 0u);
-    if (I < n_str) {
-      const uint64_t m = str[I], mh = hiword(str_hi, I);
-      const bool hi = occupied(m, mh, i);
-      if (i == j) {
-        there = hi;
-        e = make_uint2((uint32_t)I << 1, (uint32_t)I << 1);
-      } else if (hi != occupied(m, mh, j)) {
-        for (int64_t s = s1_off[I]; s < s1_off[I + 1]; s++)
-          if (s1_info[s] >> 1 == q) {
-            const int J = s1_J[s];
-            there = J < I;
-            e = make_uint2((uint32_t)I << 1 | (uint32_t)(s1_info[s] & 1), (uint32_t)J << 1 | (uint32_t)hi);
-            break;  // a string moves between i and j in one direction only
-          }
+  return i;
+}
+
+// f(pair, string, partner, phase bit) for the entries of string I, lanes over its singles and its orbitals
+template <typename F> __device__ __forceinline__ void pair_entries(const PairBuild &b, int sp, int64_t I, int lane, F &&f) {
+  for (int64_t e = b.o1[sp][I] + lane; e < b.o1[sp][I + 1]; e += 32) {
+    const int J = b.J[sp][e], info = b.info[sp][e];
+    if (J < I) f(info >> 1, (uint32_t)J, (uint32_t)(info & 1));
+  }
+  const uint64_t m = b.str[sp][I], mh = hiword(b.str_hi[sp], I);
+  for (int k = lane; k < 128; k += 32)
+    if (occupied(m, mh, k)) f(k * (k + 3) / 2, (uint32_t)I, 0u);
+}
+
+__global__ void __launch_bounds__(128) pair_count_kernel(PairBuild b) {
+  extern __shared__ uint32_t hist[];
+  const int sp = blockIdx.y, c = blockIdx.x, lane = threadIdx.x & 31;
+  if (c >= b.chunks[sp]) return;
+  for (int q = threadIdx.x; q < b.npair; q += blockDim.x) hist[q] = 0;
+  __syncthreads();
+  const int64_t end = min(b.n[sp], (int64_t)(c + 1) * b.per[sp]);
+  for (int64_t I = (int64_t)c * b.per[sp] + (threadIdx.x >> 5); I < end; I += blockDim.x >> 5)
+    pair_entries(b, sp, I, lane, [&](int q, uint32_t, uint32_t) { atomicAdd(hist + q, 1u); });
+  __syncthreads();
+  for (int q = threadIdx.x; q < b.npair; q += blockDim.x) b.cnt[sp][(int64_t)c * b.npair + q] = hist[q];
+}
+
+// block per spin: counts to places
+__global__ void __launch_bounds__(1024) pair_scan_kernel(PairBuild b) {
+  __shared__ int64_t part[33];
+  const int sp = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t base = 0;
+  for (int q0 = 0; q0 < b.npair; q0 += blockDim.x) {
+    const int q = q0 + threadIdx.x;
+    int64_t total = 0;
+    if (q < b.npair) {
+      uint32_t *p = b.cnt[sp] + q;
+      constexpr int U = 8;
+      for (int c0 = 0; c0 < b.chunks[sp]; c0 += U) {
+        uint32_t x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) x[u] = c0 + u < b.chunks[sp] ? p[(int64_t)(c0 + u) * b.npair] : 0u;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (c0 + u < b.chunks[sp]) p[(int64_t)(c0 + u) * b.npair] = (uint32_t)total;
+          total += x[u];
+        }
       }
     }
-    const unsigned b = __ballot_sync(0xffffffffu, there);
-    if (ent && there) ent[w + __popc(b & ((1u << lane) - 1u))] = e;
-    w += __popc(b);
+    int64_t inc = total;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    __syncthreads();  // the last round's sums have been read
+    if (lane == 31) part[warp + 1] = inc;
+    if (threadIdx.x == 0) part[0] = 0;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 1; w <= 32; w++) part[w] += part[w - 1];
+    __syncthreads();
+    if (q < b.npair) b.off[sp][q] = base + part[warp] + inc - total;
+    base += part[32];
   }
-  if (!ent && lane == 0) cnt[q] = w;
+  if (threadIdx.x == 0) b.off[sp][b.npair] = base;
+}
+
+// warp per chunk
+__global__ void __launch_bounds__(32) pair_fill_kernel(PairBuild b) {
+  extern __shared__ uint32_t next[];
+  const int sp = blockIdx.y, c = blockIdx.x, lane = threadIdx.x;
+  if (c >= b.chunks[sp]) return;
+  for (int q = lane; q < b.npair; q += 32) next[q] = b.cnt[sp][(int64_t)c * b.npair + q];
+  __syncwarp();
+  const int64_t end = min(b.n[sp], (int64_t)(c + 1) * b.per[sp]);
+  for (int64_t I = (int64_t)c * b.per[sp]; I < end; I++) {
+    const uint64_t m = b.str[sp][I], mh = hiword(b.str_hi[sp], I);
+    pair_entries(b, sp, I, lane, [&](int q, uint32_t J, uint32_t neg) {
+      const uint32_t holds = J != (uint32_t)I && occupied(m, mh, pair_row(q));
+      b.ent[sp][b.off[sp][q] + next[q]++] = make_uint2((uint32_t)I << 1 | neg, J << 1 | holds);
+    });
+    __syncwarp();
+  }
 }
 
 __device__ __forceinline__ double xflip(double v, uint32_t neg) {
@@ -279,30 +355,39 @@ static pq_status pair_lists(pq_ci_handle *h) {
     set_error("host allocation failed");
     return PQ_ERR_OOM;
   }
-  const int npair = h->npair[0];
-  cudaStream_t st = h->stream;
-  PQ_TRY(p->out.alloc(sizeof(double) * std::max(npair, S2_MAXV)));
-  DevBuf cnt;
-  PQ_TRY(cnt.alloc(sizeof(int64_t) * npair));
-  const unsigned grid = (unsigned)((npair + 3) / 4);
+  PairBuild b{};
+  b.npair = h->npair[0];
+  const int ne[2] = {h->desc.n_alpha[0], h->desc.n_beta[0]};
+  int most = 0;
   for (int sp = 0; sp < 2; sp++) {
     const SpinTablesDev &t = h->tab[0][sp];
-    auto run = [&](int64_t *c, const int64_t *o, uint2 *e) -> pq_status {
-      pair_lists_kernel<<<grid, 128, 0, st>>>(npair, t.n_str, t.str.as<uint64_t>(), t.str_hi.as<uint64_t>(),
-                                             t.s1_off.as<int64_t>(), t.s1_J.as<int32_t>(), t.s1_info.as<int32_t>(), c, o, e);
-      PQ_CUDA_TRY(cudaGetLastError());
-      return PQ_OK;
-    };
-    PQ_TRY(run(cnt.as<int64_t>(), nullptr, nullptr));
-    std::vector<int64_t> &o = p->hoff[sp];
-    o.assign(npair + 1, 0);
-    PQ_CUDA_TRY(cudaMemcpyAsync(o.data() + 1, cnt.ptr, sizeof(int64_t) * npair, cudaMemcpyDeviceToHost, st));
-    PQ_CUDA_TRY(cudaStreamSynchronize(st));
-    for (int q = 0; q < npair; q++) o[q + 1] += o[q];
-    PQ_TRY(upload(p->off[sp], o, st));
-    PQ_TRY(p->ent[sp].alloc(sizeof(uint2) * (size_t)(o[npair] + 1)));
-    PQ_TRY(run(nullptr, p->off[sp].as<int64_t>(), p->ent[sp].as<uint2>()));
+    b.str[sp] = t.str.as<uint64_t>(), b.str_hi[sp] = t.str_hi.as<uint64_t>();
+    b.o1[sp] = t.s1_off.as<int64_t>(), b.J[sp] = t.s1_J.as<int32_t>(), b.info[sp] = t.s1_info.as<int32_t>();
+    b.n[sp] = t.n_str;
+    b.per[sp] = (int)std::max<int64_t>(8, (t.n_str + PAIR_CHUNKS - 1) / PAIR_CHUNKS);
+    b.chunks[sp] = (int)((t.n_str + b.per[sp] - 1) / b.per[sp]);
+    most = std::max(most, b.chunks[sp]);
+    p->side[sp].n_ent = t.n1 / 2 + t.n_str * ne[sp];
   }
+  auto lay = [&](DevLayout &l) {
+    l.take(p->out, std::max(b.npair, S2_MAXV));
+    for (int sp = 0; sp < 2; sp++) {
+      l.take(p->side[sp].off, b.npair + 1);
+      l.take(p->side[sp].ent, p->side[sp].n_ent + 1);
+      l.take(b.cnt[sp], (size_t)b.chunks[sp] * b.npair);
+    }
+  };
+  DevLayout l;
+  lay(l);
+  PQ_TRY(p->mem.alloc(l.used));
+  l = DevLayout{static_cast<char *>(p->mem.ptr), 0};
+  lay(l);
+  for (int sp = 0; sp < 2; sp++) b.off[sp] = p->side[sp].off, b.ent[sp] = p->side[sp].ent;
+  const size_t smem = sizeof(uint32_t) * b.npair;  // at most 33 KB
+  pair_count_kernel<<<dim3(most, 2), 128, smem, h->stream>>>(b);
+  pair_scan_kernel<<<2, 1024, 0, h->stream>>>(b);
+  pair_fill_kernel<<<dim3(most, 2), 32, smem, h->stream>>>(b);
+  PQ_CUDA_TRY(cudaGetLastError());
   h->pairs = std::move(p);
   return PQ_OK;
 }
@@ -313,16 +398,16 @@ static pq_status s2_one(pq_ci_handle *h, const double *C, int64_t ldc, int nvec)
   const SpinTablesDev &A = h->tab[0][0], &B = h->tab[0][1];
   const int npair = h->npair[0], na = h->desc.n_alpha[0], nb = h->desc.n_beta[0];
   cudaStream_t st = h->stream;
-  double *out = p.out.as<double>();
+  double *out = p.out;
   const double sz = 0.5 * (na - nb);
   PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * S2_MAXV, st));
   s2_diag_kernel<<<(unsigned)A.n_str, PROP_THREADS, 0, st>>>(
       A.str.as<uint64_t>(), A.str_hi.as<uint64_t>(), B.str.as<uint64_t>(), B.str_hi.as<uint64_t>(),
       h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), sz * sz + 0.5 * (na + nb), C, ldc, nvec, out);
-  const int64_t n_ent = p.hoff[0][npair];
+  const int64_t n_ent = p.side[0].n_ent;
   if (n_ent > 0)
     s2_flip_kernel<<<(unsigned)((n_ent + 8 * FLIP_PER - 1) / (8 * FLIP_PER)), 256, 0, st>>>(
-        p.off[0].as<int64_t>(), p.ent[0].as<uint2>(), p.off[1].as<int64_t>(), p.ent[1].as<uint2>(), npair, n_ent,
+        p.side[0].off, p.side[0].ent, p.side[1].off, p.side[1].ent, npair, n_ent,
         h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), C, ldc, nvec, out);
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
@@ -333,13 +418,13 @@ static pq_status rdm_one(pq_ci_handle *h, const double *C, int spin) {
   const PairLists &p = *h->pairs;
   const int npair = h->npair[0];
   cudaStream_t st = h->stream;
-  double *out = p.out.as<double>();
+  double *out = p.out;
   const int64_t *ro = h->d_rowoff.as<int64_t>();
   const int32_t *rl = h->d_rowlen.as<int32_t>();
   PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * npair, st));
-  const int64_t *off = p.off[spin].as<int64_t>();
-  const uint2 *ent = p.ent[spin].as<uint2>();
-  const int64_t n_ent = p.hoff[spin][npair], na = h->tab[0][0].n_str;
+  const int64_t *off = p.side[spin].off;
+  const uint2 *ent = p.side[spin].ent;
+  const int64_t n_ent = p.side[spin].n_ent, na = h->tab[0][0].n_str;
   if (n_ent == 0) return PQ_OK;
   if (spin == 0) {
     const int64_t per = 8 * ROWS_PER;
@@ -535,7 +620,7 @@ pq_status pq_ci_s2(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, 
     PQ_TRY(with_room(h, [&] { return pair_lists(h); }));
   else
     PQ_TRY(own.alloc(sizeof(double) * S2_MAXV));
-  double *out = ns == 1 ? h->pairs->out.as<double>() : own.as<double>();
+  double *out = ns == 1 ? h->pairs->out : own.as<double>();
   std::vector<double> part(S2_MAXV);
   for (int sp = 0; sp < ns; sp++)
     for (int v0 = 0; v0 < nvec; v0 += S2_MAXV) {
@@ -566,7 +651,7 @@ pq_status pq_ci_rdm1(pq_ci_handle *h, const double *C, int32_t species, int32_t 
     PQ_TRY(with_room(h, [&] { return pair_lists(h); }));
     PQ_TRY(rdm_one(h, C, spin));
     std::vector<double> d(h->npair[0]);
-    PQ_CUDA_TRY(cudaMemcpyAsync(d.data(), h->pairs->out.ptr, sizeof(double) * d.size(), cudaMemcpyDeviceToHost, h->stream));
+    PQ_CUDA_TRY(cudaMemcpyAsync(d.data(), h->pairs->out, sizeof(double) * d.size(), cudaMemcpyDeviceToHost, h->stream));
     PQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
     for (int i = 0, q = 0; i < n; i++)
       for (int j = 0; j <= i; j++, q++) rdm[i + (size_t)j * n] = rdm[j + (size_t)i * n] = d[q];
