@@ -256,6 +256,25 @@ __global__ void __launch_bounds__(512) rdm_cols_kernel(const int64_t *off, const
   }
 }
 
+// Beta 1-RDM with lists of a few entries: thread per entry, over the `per` rows of blockIdx.y; one atomic each
+__global__ void __launch_bounds__(256) rdm_entries_kernel(const int64_t *off, const uint2 *ent, int npair, int64_t n_ent,
+                                                          int64_t na, int per, const int64_t *rowoff, const int32_t *rowlen,
+                                                          const double *C, double *out) {
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (e >= n_ent) return;
+  const uint2 x = __ldg(ent + e);
+  const int I = (int)(x.x >> 1), J = (int)(x.y >> 1);  // J <= I
+  const int64_t end = min(na, (int64_t)(blockIdx.y + 1) * per);
+  double acc = 0.0;
+#pragma unroll 4
+  for (int64_t a = (int64_t)blockIdx.y * per; a < end; a++)
+    if (I < __ldg(rowlen + a)) {
+      const double *row = C + __ldg(rowoff + a);
+      acc = fma(__ldg(row + I), __ldg(row + J), acc);
+    }
+  if (acc != 0.0) atomicAdd(out + pair_of(off, npair, e), xflip(acc, x.x & 1u));
+}
+
 // <S^2>, diagonal: sum of C_I^2 (s_z^2 + (n_alpha + n_beta)/2 - doubly occupied orbitals); block per alpha string
 __global__ void __launch_bounds__(PROP_THREADS) s2_diag_kernel(const uint64_t *astr, const uint64_t *astr_hi,
                                                               const uint64_t *bstr, const uint64_t *bstr_hi,
@@ -429,6 +448,20 @@ static pq_status rdm_one(pq_ci_handle *h, const double *C, int spin) {
   if (spin == 0) {
     const int64_t per = 8 * ROWS_PER;
     rdm_rows_kernel<<<(unsigned)((n_ent + per - 1) / per), 256, 0, st>>>(off, ent, npair, n_ent, ro, rl, C, out);
+    PQ_CUDA_TRY(cudaGetLastError());
+    return PQ_OK;
+  }
+  // With few entries a pair, a warp per pair idles and the blocks' sums meet in the same few atomics.  us a call, thread
+  // per determinant (before there were lists) / warp per pair / thread per entry: 30o 4a1b (1 entry a pair, 465 pairs)
+  // 556 / 1367 / 68; 40o 2a1b (1, 820 pairs) 109 / 229 / 48; 20o 3a1b (1) 84 / 109 / 47; 16o 8a2b (14) 1059 / 233 / 127;
+  // 30o 2a2b (28) 300 / 117 / 76; CISD of 40o 2a2b (38, 820 pairs) 177 / 209 / 102; but 9o 4a4b (39, 45 pairs) 98 / 50 /
+  // 59; 10o 5a5b (80) 154 / 53 / 104.
+  if (n_ent < (npair >= 256 ? 64 : 32) * (int64_t)npair) {
+    const int64_t blocks = (n_ent + 255) / 256;
+    const int64_t chunks = std::min<int64_t>((na + 7) / 8, std::max<int64_t>(1, 1216 / blocks));
+    const int per = (int)((na + chunks - 1) / chunks);
+    rdm_entries_kernel<<<dim3((unsigned)blocks, (unsigned)((na + per - 1) / per)), 256, 0, st>>>(off, ent, npair, n_ent, na,
+                                                                                               per, ro, rl, C, out);
     PQ_CUDA_TRY(cudaGetLastError());
     return PQ_OK;
   }
