@@ -551,11 +551,15 @@ __global__ void klist_kernel(const int64_t *o1, const int32_t *J1, const int32_t
 
 // One-species full CI of more than 32 768 determinants (below, ci_sigma_rows.cu), singles and occupied orbitals of an
 // alpha string within one exact sum of 80, 16-bit beta strings in the scatter lists, dense same-spin matrices of at
-// most 4 GiB of digits that are at least 2.5 % filled (a digit product of a zero costs 1/60 of an FP64 FMA).
+// most 4 GiB of digits that are at least 2.5 % filled (a digit product of a zero costs 1/60 of an FP64 FMA), and at
+// least one tile of 64 alpha strings: fewer leave most of the chip without an item and the dense product of the beta
+// side with padding.  One / four roots, us, here / element kernel: 16o 1a6b (16 alpha strings) 1736 / 657, 2376 / 1870;
+// 24o 1a4b (24) 3218 / 2329, 5070 / 5694; 12o 2a6b (66) 234 / 308, 331 / 952; 13o 2a6b (78) 370 / 660, 661 / 2110.
+// The tables of such a handle take as long as 10 to 15 of its sigmas.
 bool sigma64_applicable(const pq_ci_handle *h) {
   if (h->n_species != 1 || !h->full || h->wide || h->n_dets <= ROWS_FULL_MAX) return false;
   const SpinTablesDev &a = h->tab[0][0], &b = h->tab[0][1];
-  if (a.max1 + h->desc.n_alpha[0] > s64::KMAX || b.n_str >= 65536) return false;
+  if (a.max1 + h->desc.n_alpha[0] > s64::KMAX || a.n_str < s64::BN || b.n_str >= 65536) return false;
   for (int sp = 0; sp < 2; sp++) {
     const SpinTablesDev &t = h->tab[0][sp];
     const double n = (double)t.n_str;

@@ -92,3 +92,13 @@ def test_other_paths(monkeypatch):
     g = _make(synthetic_fci(10, 5, 5, seed=2))
     g.sigma(_x(g, 2))
     assert path(g) == (PQ_PATH_ELEMENT, 0)
+
+
+@pytest.mark.parametrize("n,a,b,tensor", [(16, 1, 5, False), (20, 1, 5, False), (12, 2, 6, True), (16, 8, 1, True)])
+def test_few_alpha_strings_stay_with_the_element_kernel(n, a, b, tensor):
+    """Fewer than a tile of 64 alpha strings leave the tensor-core kernels idle."""
+    from polyquant_gb300._lib import PQ_PATH_ELEMENT, PQ_PATH_TENSOR
+
+    g = _make(synthetic_fci(n, a, b, seed=7))
+    g.sigma(_x(g, 2))
+    assert path(g)[0] == (PQ_PATH_TENSOR if tensor else PQ_PATH_ELEMENT)
