@@ -56,7 +56,7 @@ void pairs_delete(PairLists *p) { delete p; }
 // call of a handle then takes little longer than one that made no lists; with a warp per pair searching every string's
 // singles, counts read back and five allocations, first calls of <S^2> took up to 1.5 ms more (14o 7a1b, 48 048
 // determinants: 503 us without lists, 1974 so, 246 now; 9o 4a4b 143 / 205 / 114; CISD of 5a5b in 100 orbitals
-// 175 / 89 / 10 ms).
+// 175 / 89 / 9 ms).  A warp loads 128 singles at a time (CISD of 5a1b in 64 orbitals 1348 -> 1142 us).
 struct PairBuild {
   const uint64_t *str[2], *str_hi[2];
   const int64_t *o1[2];
@@ -79,9 +79,18 @@ __device__ __forceinline__ int pair_row(int q) {  // i of q = i (i + 1) / 2 + j,
 
 // f(pair, string, partner, phase bit) for the entries of string I, lanes over its singles and its orbitals
 template <typename F> __device__ __forceinline__ void pair_entries(const PairBuild &b, int sp, int64_t I, int lane, F &&f) {
-  for (int64_t e = b.o1[sp][I] + lane; e < b.o1[sp][I + 1]; e += 32) {
-    const int J = b.J[sp][e], info = b.info[sp][e];
-    if (J < I) f(info >> 1, (uint32_t)J, (uint32_t)(info & 1));
+  constexpr int U = 4;
+  const int64_t end = b.o1[sp][I + 1];
+  for (int64_t e = b.o1[sp][I] + lane; e < end; e += 32 * U) {
+    int J[U], info[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      J[u] = e + 32 * u < end ? __ldg(b.J[sp] + e + 32 * u) : INT32_MAX;
+      info[u] = e + 32 * u < end ? __ldg(b.info[sp] + e + 32 * u) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (J[u] < I) f(info[u] >> 1, (uint32_t)J[u], (uint32_t)(info[u] & 1));
   }
   const uint64_t m = b.str[sp][I], mh = hiword(b.str_hi[sp], I);
   for (int k = lane; k < 128; k += 32)
@@ -143,17 +152,17 @@ __global__ void __launch_bounds__(1024) pair_scan_kernel(PairBuild b) {
 
 // warp per chunk
 __global__ void __launch_bounds__(32) pair_fill_kernel(PairBuild b) {
-  extern __shared__ uint32_t next[];
+  extern __shared__ int64_t next[];
   const int sp = blockIdx.y, c = blockIdx.x, lane = threadIdx.x;
   if (c >= b.chunks[sp]) return;
-  for (int q = lane; q < b.npair; q += 32) next[q] = b.cnt[sp][(int64_t)c * b.npair + q];
+  for (int q = lane; q < b.npair; q += 32) next[q] = b.off[sp][q] + b.cnt[sp][(int64_t)c * b.npair + q];
   __syncwarp();
   const int64_t end = min(b.n[sp], (int64_t)(c + 1) * b.per[sp]);
   for (int64_t I = (int64_t)c * b.per[sp]; I < end; I++) {
     const uint64_t m = b.str[sp][I], mh = hiword(b.str_hi[sp], I);
     pair_entries(b, sp, I, lane, [&](int q, uint32_t J, uint32_t neg) {
       const uint32_t holds = J != (uint32_t)I && occupied(m, mh, pair_row(q));
-      b.ent[sp][b.off[sp][q] + next[q]++] = make_uint2((uint32_t)I << 1 | neg, J << 1 | holds);
+      b.ent[sp][next[q]++] = make_uint2((uint32_t)I << 1 | neg, J << 1 | holds);
     });
     __syncwarp();
   }
@@ -180,7 +189,7 @@ __device__ __forceinline__ int pair_of(const int64_t *off, int npair, int64_t e)
   return lo;
 }
 
-// Alpha 1-RDM: sum over the list of pair q of phase * (row I . row J), warp per ROWS_PER entries
+// Alpha 1-RDM: sum over the list of pair q of phase * (row I . row J), warp per ROWS_PER entries and part of the columns
 constexpr int ROWS_PER = 8;
 __global__ void __launch_bounds__(256) rdm_rows_kernel(const int64_t *off, const uint2 *ent, int npair, int64_t n_ent,
                                                        const int64_t *rowoff, const int32_t *rowlen, const double *C,
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(256) rdm_rows_kernel(const int64_t *off, const
       const int len = min(rowlen[I], rowlen[J]);
       double part = 0.0;
 #pragma unroll 4
-      for (int b = lane; b < len; b += 32) part = fma(__ldg(ri + b), __ldg(rj + b), part);
+      for (int b = 32 * blockIdx.y + lane; b < len; b += 32 * gridDim.y) part = fma(__ldg(ri + b), __ldg(rj + b), part);
       acc += xflip(part, x.x & 1u);
     }
     acc = warp_total(acc);
@@ -314,7 +323,7 @@ __global__ void __launch_bounds__(PROP_THREADS) s2_diag_kernel(const uint64_t *a
 
 // <S^2>, spin flips: each unordered pair of determinants (A_lo, B_hi), (A_hi, B_lo) of a pair of orbitals, where lo
 // and hi are the strings that hold the lower and the higher of the two, adds -2 phase C C.  Warp per FLIP_PER alpha
-// entries, lanes over the beta list of the same pair.
+// entries and part of the beta list of the same pair, lanes over that part.
 constexpr int FLIP_PER = 4;
 __global__ void __launch_bounds__(256) s2_flip_kernel(const int64_t *aoff, const uint2 *aent, const int64_t *boff,
                                                       const uint2 *bent, int npair, int64_t n_ent,
@@ -341,7 +350,7 @@ __global__ void __launch_bounds__(256) s2_flip_kernel(const int64_t *aoff, const
     const int alo = (x.y & 1u) ? J : I, ahi = (x.y & 1u) ? I : J;
     const int64_t rlo = rowoff[alo], rhi = rowoff[ahi];
     const int llo = rowlen[alo], lhi = rowlen[ahi];
-    for (int64_t f = boff[q] + lane; f < boff[q + 1]; f += 32) {
+    for (int64_t f = boff[q] + 32 * blockIdx.y + lane; f < boff[q + 1]; f += 32 * gridDim.y) {
       const uint2 y = __ldg(bent + f);
       const int K = (int)(y.x >> 1), L = (int)(y.y >> 1);
       const int blo = (y.y & 1u) ? L : K, bhi = (y.y & 1u) ? K : L;
@@ -402,32 +411,41 @@ static pq_status pair_lists(pq_ci_handle *h) {
   l = DevLayout{static_cast<char *>(p->mem.ptr), 0};
   lay(l);
   for (int sp = 0; sp < 2; sp++) b.off[sp] = p->side[sp].off, b.ent[sp] = p->side[sp].ent;
-  const size_t smem = sizeof(uint32_t) * b.npair;  // at most 33 KB
-  pair_count_kernel<<<dim3(most, 2), 128, smem, h->stream>>>(b);
+  const size_t places = sizeof(int64_t) * b.npair;  // at most 66 KB
+  if (places > 48 * 1024)
+    PQ_CUDA_TRY(cudaFuncSetAttribute(pair_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)places));
+  pair_count_kernel<<<dim3(most, 2), 128, sizeof(uint32_t) * b.npair, h->stream>>>(b);
   pair_scan_kernel<<<2, 1024, 0, h->stream>>>(b);
-  pair_fill_kernel<<<dim3(most, 2), 32, smem, h->stream>>>(b);
+  pair_fill_kernel<<<dim3(most, 2), 32, places, h->stream>>>(b);
   PQ_CUDA_TRY(cudaGetLastError());
   h->pairs = std::move(p);
   return PQ_OK;
 }
 
-// <S^2> of nvec <= S2_MAXV states into the device sums of the lists
-static pq_status s2_one(pq_ci_handle *h, const double *C, int64_t ldc, int nvec) {
-  const PairLists &p = *h->pairs;
+// Parts of the columns (or beta entries, `most` of them for an alpha entry): as many as fill the chip twice where the
+// alpha entries alone leave it idle, of at least 64 columns.  16o 1a8b (136 alpha entries, 12 870 columns), us a call,
+// thread per determinant / undivided / so: <S^2> of four states 276 / 623 / 177, alpha 1-RDM 423 / 734 / 80;
+// 20o 1a5b (210, 15 504) 461 / 598 / 199, 628 / 866 / 91.
+static unsigned column_parts(int64_t blocks, int64_t most) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((most + 63) / 64, 304 / std::max<int64_t>(blocks, 1)));
+}
+
+// <S^2> of nvec <= S2_MAXV states into device sums; lists: NULL without particles of either spin, which cannot flip
+static pq_status s2_one(pq_ci_handle *h, const PairLists *lists, const double *C, int64_t ldc, int nvec, double *out) {
   const SpinTablesDev &A = h->tab[0][0], &B = h->tab[0][1];
   const int npair = h->npair[0], na = h->desc.n_alpha[0], nb = h->desc.n_beta[0];
   cudaStream_t st = h->stream;
-  double *out = p.out;
   const double sz = 0.5 * (na - nb);
   PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * S2_MAXV, st));
   s2_diag_kernel<<<(unsigned)A.n_str, PROP_THREADS, 0, st>>>(
       A.str.as<uint64_t>(), A.str_hi.as<uint64_t>(), B.str.as<uint64_t>(), B.str_hi.as<uint64_t>(),
       h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), sz * sz + 0.5 * (na + nb), C, ldc, nvec, out);
-  const int64_t n_ent = p.side[0].n_ent;
-  if (n_ent > 0)
-    s2_flip_kernel<<<(unsigned)((n_ent + 8 * FLIP_PER - 1) / (8 * FLIP_PER)), 256, 0, st>>>(
-        p.side[0].off, p.side[0].ent, p.side[1].off, p.side[1].ent, npair, n_ent,
-        h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), C, ldc, nvec, out);
+  if (lists) {
+    const PairLists::Side &a = lists->side[0], &b = lists->side[1];
+    const int64_t blocks = (a.n_ent + 8 * FLIP_PER - 1) / (8 * FLIP_PER);
+    s2_flip_kernel<<<dim3((unsigned)blocks, column_parts(blocks, b.n_ent / npair)), 256, 0, st>>>(
+        a.off, a.ent, b.off, b.ent, npair, a.n_ent, h->d_rowoff.as<int64_t>(), h->d_rowlen.as<int32_t>(), C, ldc, nvec, out);
+  }
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
 }
@@ -446,8 +464,9 @@ static pq_status rdm_one(pq_ci_handle *h, const double *C, int spin) {
   const int64_t n_ent = p.side[spin].n_ent, na = h->tab[0][0].n_str;
   if (n_ent == 0) return PQ_OK;
   if (spin == 0) {
-    const int64_t per = 8 * ROWS_PER;
-    rdm_rows_kernel<<<(unsigned)((n_ent + per - 1) / per), 256, 0, st>>>(off, ent, npair, n_ent, ro, rl, C, out);
+    const int64_t blocks = (n_ent + 8 * ROWS_PER - 1) / (8 * ROWS_PER);
+    const dim3 grid((unsigned)blocks, column_parts(blocks, h->tab[0][1].n_str));
+    rdm_rows_kernel<<<grid, 256, 0, st>>>(off, ent, npair, n_ent, ro, rl, C, out);
     PQ_CUDA_TRY(cudaGetLastError());
     return PQ_OK;
   }
@@ -648,18 +667,20 @@ pq_status pq_ci_s2(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, 
     return PQ_ERR_ARG;
   }
   const int ns = h->n_species;
+  const bool flips = ns == 1 && h->desc.n_alpha[0] > 0 && h->desc.n_beta[0] > 0;
   DevBuf own;
-  if (ns == 1)
+  if (flips)
     PQ_TRY(with_room(h, [&] { return pair_lists(h); }));
   else
     PQ_TRY(own.alloc(sizeof(double) * S2_MAXV));
-  double *out = ns == 1 ? h->pairs->out : own.as<double>();
+  const PairLists *lists = flips ? h->pairs.get() : nullptr;
+  double *out = flips ? lists->out : own.as<double>();
   std::vector<double> part(S2_MAXV);
   for (int sp = 0; sp < ns; sp++)
     for (int v0 = 0; v0 < nvec; v0 += S2_MAXV) {
       const int c = std::min(S2_MAXV, nvec - v0);
       if (ns == 1) {
-        PQ_TRY(s2_one(h, C + (size_t)v0 * ldc, ldc, c));
+        PQ_TRY(s2_one(h, lists, C + (size_t)v0 * ldc, ldc, c, out));
       } else {
         PQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * S2_MAXV, h->stream));
         s2_two_kernel<<<(unsigned)h->e_a.size(), PROP_THREADS, 0, h->stream>>>(make_two(h), sp, C + (size_t)v0 * ldc,
