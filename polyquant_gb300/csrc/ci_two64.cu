@@ -225,6 +225,10 @@ static Shape shape_of(const pq_ci_handle *h) {
 // us a sigma of three roots, this path / the element kernel: 864 determinants of 258 connections in three pairs
 // 100 / 110, 4 000 of 740 146 / 301, 18 000 of 2 020 170 / 787; four lists, 82 944 of 721 (3.5 rows a connection)
 // 301 / 463, but 640 / 415 with the matrices that its first call makes; 36 504 of 863 (8.1 rows a connection) 357 / 351.
+// With four lists the six products are smaller, and rows that stand for few connections weigh more; one / three roots:
+// 19 200 of 405 (2.3 rows a connection, 1.3e6 connections a pair) 208 / 154, 238 / 190; 22 400 of 559 (1.9, 2.1e6)
+// 230 / 196, 260 / 255; 22 050 of 545 (2.3, 2.0e6) 254 / 195, 281 / 246; 12 544 of 622 (1.1, 1.3e6) 206 / 212, 229 / 258;
+// 19 600 of 903 (1.1, 3.0e6) 247 / 307, 267 / 381.
 bool two64_applicable(const pq_ci_handle *h) {
   if (h->n_species != 2 || !h->full2 || h->wide || h->n_dets > (16 << 20)) return false;
   double rows = 0.0, conn = 0.0;
@@ -246,7 +250,8 @@ bool two64_applicable(const pq_ci_handle *h) {
   }
   if (npairs == 0) return false;
   if (getenv("PQ_TWO64_ALWAYS")) return true;  // tests of small spaces, read when a handle is created
-  return rows <= 2.5 * conn && (double)h->n_dets * conn >= 6e5 * npairs;
+  const double least = npairs == 6 ? std::max(6e5, 1e6 * (rows / conn) * (rows / conn)) : 6e5;
+  return rows <= 2.5 * conn && (double)h->n_dets * conn >= least * npairs;
 }
 
 size_t two64_bytes(const pq_ci_handle *h) { return h->two64 ? h->two64->bytes() : 0; }

@@ -102,3 +102,14 @@ def test_few_alpha_strings_stay_with_the_element_kernel(n, a, b, tensor):
     g = _make(synthetic_fci(n, a, b, seed=7))
     g.sigma(_x(g, 2))
     assert path(g)[0] == (PQ_PATH_TENSOR if tensor else PQ_PATH_ELEMENT)
+
+
+@pytest.mark.parametrize("args,tensor", [((6, 3, 2, 8, 1, 1), False), ((8, 1, 2, 10, 1, 1), False), ((20, 1, 1, 7, 1, 1), True),
+                                         ((11, 2, 1, 18, 1, 0), True)])
+def test_size_rule_of_two_species(args, tensor):
+    """Four lists of which few strings are connected stay with the element kernel."""
+    from polyquant_gb300._lib import PQ_PATH_ELEMENT, PQ_PATH_TENSOR
+
+    g = _make(synthetic_ep(*args, seed=9))
+    g.sigma(_x(g, 3))
+    assert path(g)[0] == (PQ_PATH_TENSOR if tensor else PQ_PATH_ELEMENT)
