@@ -112,7 +112,19 @@ pq_status pq_ci_diag(pq_ci_handle *h, double *out_device);
 /* sigma = H C for nvec vectors (operator*).  C and S are DEVICE buffers,
  * column-major n_dets x nvec with leading dimensions ldc, lds (the Eigen layout
  * the reference passes).  precision: PQ_FP64 or PQ_FP32 (FP32 tables and
- * arithmetic, inputs/outputs still FP64). */
+ * arithmetic, inputs/outputs still FP64).
+ * Accuracy of PQ_FP64.  Where the tensor cores take it (full CI of one species,
+ * small two-species products) each column of C and each matrix of H is held as
+ * 61-bit fixed-point numbers below its own largest value, so the error of every
+ * entry of a column is absolute: below 1e-15 * (largest row sum of |H|) *
+ * (largest |C| of that column), and in the 2-norm smaller than that of a sum in
+ * FP64.  Entries of C more than 2^-8 below the largest therefore enter with
+ * fewer than 53 significant bits, and ones below 2^-62 of it as zero; entries
+ * of sigma that only such values feed carry the column's error, not their own.
+ * A vector whose small part has to keep its own accuracy is passed as two
+ * columns, each with its own scale.  The other FP64 kernels (truncated and
+ * small spaces, pq_ci_sigma_noalloc, the explicit matrix) sum in FP64 and are
+ * accurate relative to each entry's own terms. */
 pq_status pq_ci_sigma(pq_ci_handle *h, const double *C, int64_t ldc, int32_t nvec, double *S, int64_t lds,
                       int32_t precision);
 /* Same with HOST buffers (blocking).  Page-locked buffers (cudaHostAlloc or

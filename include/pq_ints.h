@@ -30,7 +30,14 @@ enum {
 };
 
 enum {
-  PQ_XFORM_FP64 = 0,   /* plain FP64 quarter transforms */
+  /* FP64.  Up to 256 functions by exact digit products: each slice (the AO
+   * integrals of one ket pair, the half-transformed ones of one MO pair) is held
+   * as 62-bit fixed-point numbers below its largest value and each column of C
+   * below its own, so the error of (ij|kl) is absolute, below 1e-16 * n_ao *
+   * (largest integral of the slice) * (largest |C_i|) * (largest |C_j|) in
+   * either half, smaller than a sum's in FP64 but not relative to integrals far
+   * below their slice's largest.  Larger bases: library DGEMM. */
+  PQ_XFORM_FP64 = 0,
   PQ_XFORM_BF16X3 = 1, /* split-BF16 (hi*hi + hi*lo + lo*hi) on tcgen05, FP32 accumulate */
   PQ_XFORM_TF32X3 = 2  /* split-TF32 (hi*hi + hi*lo + lo*hi) on tcgen05, FP32 accumulate */
 };

@@ -1,5 +1,6 @@
 // FP64 numbers as eight signed base-256 digits held in FP16, so that products of FP64 matrices run on the tensor
-// cores without rounding: x = 2^(e - 6) sum_i d_i 256^-i for a common exponent e of a row with |x| < 2^e.
+// cores without rounding (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012, here
+// with digits of one common exponent): x = 2^(e - 6) sum_i d_i 256^-i for a common exponent e of a row with |x| < 2^e.
 //
 // A number becomes the integer t = round(x 2^(62 - e)), |t| <= 2^62, and its balanced bytes d_i in [-128, 127]
 // (|d_0| <= 64).  A product of two rows is sum_l 256^-l a_l with a_l = sum_{i + j = l} sum_k d_i d'_j.  For K <= 256
