@@ -103,6 +103,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
   }
   return true;
 }
+// the same for a whole warp, which goes on or gives up as one: lanes that parted here would miss each other in the
+// shuffles and TMEM loads that follow
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long budget) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, budget));
+}
+__device__ __forceinline__ bool warp_aborted(volatile int *flag) { return __any_sync(0xffffffffu, *flag != 0); }
 
 // EPI_PACK: rows (m, slice), so a tile holds few m; only columns n <= m are kept, and the tile takes a whole number of
 // B boxes up to the last of them
@@ -322,8 +328,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, i++) {
       const int a = i & 1;
       const uint32_t aph = (uint32_t)((i >> 1) & 1);
-      const bool ok = mbar_wait(smem_u32(accf + a), aph, g.wait_cycles);
-      if (!ok || *abort_flag) {
+      const bool ok = warp_wait(smem_u32(accf + a), aph, g.wait_cycles);
+      if (!ok || warp_aborted(abort_flag)) {
         if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_ACC);
         *abort_flag = 1;
         break;
@@ -663,8 +669,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (pf && s == 0 && b + step < g.nslices)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + (b + step) * g.ld), "r"(pf) : "memory");
       const int slot = it % NSTAGE;
-      const bool ok = mbar_wait(smem_u32(empty + slot), (uint32_t)((it / NSTAGE) & 1) ^ 1u, g.wait_cycles);
-      if (!ok || *abort_flag) {
+      const bool ok = warp_wait(smem_u32(empty + slot), (uint32_t)((it / NSTAGE) & 1) ^ 1u, g.wait_cycles);
+      if (!ok || warp_aborted(abort_flag)) {
         if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_MMA);
         *abort_flag = 1;
         return false;
@@ -741,8 +747,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     int i = 0, buf = 0;
     for (int b = first; b < g.nslices; b += step, i++) {
       const int a = i & 1;
-      const bool ok = mbar_wait(smem_u32(accf + a), (uint32_t)((i >> 1) & 1), g.wait_cycles);
-      if (!ok || *abort_flag) {
+      const bool ok = warp_wait(smem_u32(accf + a), (uint32_t)((i >> 1) & 1), g.wait_cycles);
+      if (!ok || warp_aborted(abort_flag)) {
         if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_ACC);
         *abort_flag = 1;
         break;
