@@ -197,8 +197,9 @@ pq_status pq_debug_set_alloc_room(long long room, int64_t *held);
  * bounded wait ran out (the element kernel has then computed the result).
  * Blocking.
  * pq_debug_set_sigma_wait_budget: budgets, in SM clock cycles, of the pipeline
- * waits of the same-spin (and pair matrix) kernel and of the opposite-spin
- * kernel (<= 0: the default of about 2 s). */
+ * waits of the same-spin (and pair matrix) kernels and of the FP64 opposite-spin
+ * kernel (<= 0: the default of about 2 s).  An FP32 sigma whose wait runs out
+ * returns PQ_TIMEOUT. */
 enum { PQ_PATH_NONE = 0, PQ_PATH_ELEMENT = 1, PQ_PATH_ROWS = 2, PQ_PATH_TENSOR = 3, PQ_PATH_MATRIX = 4 };
 pq_status pq_debug_sigma_path(pq_ci_handle *h, int32_t *path, int32_t *gate);
 pq_status pq_debug_set_sigma_wait_budget(long long same_spin, long long opposite_spin);

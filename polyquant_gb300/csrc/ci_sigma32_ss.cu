@@ -291,8 +291,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int a = i & 1;
       const uint32_t aph = (uint32_t)((i >> 1) & 1);
       i++;
-      const bool ok = mbar_wait(smem_u32(accf + a), aph, g.wait_cycles);
-      if (!ok || *abort_flag) {
+      // the warp goes on or gives up as one: tmem_ld32 needs all of its lanes
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(accf + a), aph, g.wait_cycles));
+      if (!ok || __any_sync(0xffffffffu, *abort_flag != 0)) {
         if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_ACC);
         *abort_flag = 1;
         break;
@@ -621,7 +622,7 @@ static pq_status ss_run(pq_ci_handle *h, const SameSpinGemm::Side &S, int64_t n_
   a.mode = mode;
   a.xmax = g.aux.as<unsigned>();
   a.inv_sd = S.inv_sd;
-  a.wait_cycles = WAIT_CYCLES;
+  a.wait_cycles = sigma_wait_cycles(0);
   a.err = reinterpret_cast<int *>(g.aux.as<unsigned>() + 1);
   const int64_t tiles = (int64_t)a.m_tiles * a.n_tiles;
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, h->tc_sms > 0 ? h->tc_sms : 148);

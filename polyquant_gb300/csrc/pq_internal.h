@@ -246,7 +246,8 @@ pq_status ci_sigma64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, i
                      int64_t svs, bool fixed, int **gate);
 pq_status ci_two64(pq_ci_handle *h, const double *C, int64_t es, int64_t vs, int nv, double shift, double *S, int64_t ses,
                    int64_t svs, bool fixed, int **gate);
-// budget of the waits of the same-spin products, pair matrices included (0), and of the opposite-spin kernel (1)
+// budget of the waits of the same-spin products, pair matrices and FP32 included (0), and of the FP64 opposite-spin
+// kernel (1)
 long long sigma_wait_cycles(int kernel);
 size_t sigma64_bytes(const pq_ci_handle *h);
 size_t two64_bytes(const pq_ci_handle *h);
