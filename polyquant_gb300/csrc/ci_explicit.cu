@@ -367,7 +367,11 @@ pq_status pq_ci_ham_build(pq_ci_handle *h, double screening_threshold, int32_t u
     return PQ_ERR_ARG;
   }
   h->use_explicit = false;
-  PQ_TRY(with_room(h, [&] { return ham_build(h, screening_threshold); }));
+  const pq_status s = with_room(h, [&] { return ham_build(h, screening_threshold); });
+  if (s != PQ_OK) {
+    pq_ci_ham_release(h);  // row offsets without their entries are no matrix (pq_ci_ham_csr)
+    return s;
+  }
   h->use_explicit = use_for_sigma != 0;
   if (nnz) *nnz = h->h_nnz;
   return PQ_OK;
