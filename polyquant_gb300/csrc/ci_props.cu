@@ -193,8 +193,8 @@ __device__ __forceinline__ int pair_of(const int64_t *off, int npair, int64_t e)
 constexpr int ROWS_PER = 8;
 __global__ void __launch_bounds__(256) rdm_rows_kernel(const int64_t *off, const uint2 *ent, int npair, int64_t n_ent,
                                                        const int64_t *rowoff, const int32_t *rowlen, const double *C,
-                                                       double *out) {
-  const int lane = threadIdx.x & 31;
+                                                       int width, double *out) {
+  const int lane = threadIdx.x & 31, b0 = blockIdx.y * width;
   int64_t e = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * ROWS_PER;
   const int64_t e1 = min(e + ROWS_PER, n_ent);
   if (e >= e1) return;
@@ -206,10 +206,10 @@ __global__ void __launch_bounds__(256) rdm_rows_kernel(const int64_t *off, const
       const uint2 x = __ldg(ent + e);
       const int64_t I = x.x >> 1, J = x.y >> 1;
       const double *ri = C + rowoff[I], *rj = C + rowoff[J];
-      const int len = min(rowlen[I], rowlen[J]);
+      const int len = min(min(rowlen[I], rowlen[J]), b0 + width);
       double part = 0.0;
 #pragma unroll 4
-      for (int b = 32 * blockIdx.y + lane; b < len; b += 32 * gridDim.y) part = fma(__ldg(ri + b), __ldg(rj + b), part);
+      for (int b = b0 + lane; b < len; b += 32) part = fma(__ldg(ri + b), __ldg(rj + b), part);
       acc += xflip(part, x.x & 1u);
     }
     acc = warp_total(acc);
@@ -350,7 +350,13 @@ __global__ void __launch_bounds__(256) s2_flip_kernel(const int64_t *aoff, const
     const int alo = (x.y & 1u) ? J : I, ahi = (x.y & 1u) ? I : J;
     const int64_t rlo = rowoff[alo], rhi = rowoff[ahi];
     const int llo = rowlen[alo], lhi = rowlen[ahi];
-    for (int64_t f = boff[q] + 32 * blockIdx.y + lane; f < boff[q + 1]; f += 32 * gridDim.y) {
+    int64_t f0 = boff[q], f1 = boff[q + 1];
+    if (gridDim.y > 1) {
+      const int64_t width = ((f1 - f0 + gridDim.y - 1) / gridDim.y + 31) & ~31;
+      f0 += blockIdx.y * width;
+      f1 = min(f1, f0 + width);
+    }
+    for (int64_t f = f0 + lane; f < f1; f += 32) {
       const uint2 y = __ldg(bent + f);
       const int K = (int)(y.x >> 1), L = (int)(y.y >> 1);
       const int blo = (y.y & 1u) ? L : K, bhi = (y.y & 1u) ? K : L;
@@ -423,9 +429,10 @@ static pq_status pair_lists(pq_ci_handle *h) {
 }
 
 // Parts of the columns (or beta entries, `most` of them for an alpha entry): as many as fill the chip twice where the
-// alpha entries alone leave it idle, of at least 64 columns.  16o 1a8b (136 alpha entries, 12 870 columns), us a call,
-// thread per determinant / undivided / so: <S^2> of four states 276 / 623 / 177, alpha 1-RDM 423 / 734 / 80;
-// 20o 1a5b (210, 15 504) 461 / 598 / 199, 628 / 866 / 91.
+// alpha entries alone leave it idle, of at least 64 columns each.  us a call, undivided / so: 16o 1a8b (136 alpha
+// entries, 12 870 columns) <S^2> of four states 574 / 129, alpha 1-RDM 582 / 33; 20o 1a5b (210, 15 504) 544 / 154,
+// 688 / 41; also full CI 10o 5a5b, alpha 1-RDM 41 / 28.  A part is one range: with 32 columns in turn the loops of an
+// undivided call had a stride that is not known when they are compiled, and FCI(12o) took 378 us instead of 362.
 static unsigned column_parts(int64_t blocks, int64_t most) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((most + 63) / 64, 304 / std::max<int64_t>(blocks, 1)));
 }
@@ -465,8 +472,10 @@ static pq_status rdm_one(pq_ci_handle *h, const double *C, int spin) {
   if (n_ent == 0) return PQ_OK;
   if (spin == 0) {
     const int64_t blocks = (n_ent + 8 * ROWS_PER - 1) / (8 * ROWS_PER);
-    const dim3 grid((unsigned)blocks, column_parts(blocks, h->tab[0][1].n_str));
-    rdm_rows_kernel<<<grid, 256, 0, st>>>(off, ent, npair, n_ent, ro, rl, C, out);
+    const int64_t nb = h->tab[0][1].n_str;
+    const dim3 grid((unsigned)blocks, column_parts(blocks, nb));
+    const int width = (int)((nb + grid.y - 1) / grid.y + 31) & ~31;
+    rdm_rows_kernel<<<grid, 256, 0, st>>>(off, ent, npair, n_ent, ro, rl, C, width, out);
     PQ_CUDA_TRY(cudaGetLastError());
     return PQ_OK;
   }
