@@ -34,10 +34,13 @@
 #include <vector>
 
 #include "pq_internal.h"
+#include "pq_tc.cuh"
 
 namespace pq {
 
 namespace tc {
+
+using namespace tcx;
 
 constexpr int BM = 128;          // output rows per CTA (TMEM lanes)
 constexpr int BN = 256;          // output columns per CTA (TMEM columns, UMMA N)
@@ -56,7 +59,6 @@ constexpr int EPI_BYTES = EPI_WARPS * 32 * EPI_LD * 4;      // 16.5 KB
 constexpr int NBARS = 2 * STAGES + 4 + 1;                   // full, empty, acc_full[2], acc_empty[2], drain
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers, slots*/;
 constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;           // producer warp, MMA warp, epilogue warps
-constexpr long long WAIT_CYCLES = 4000000000LL;  // ~2 s at 2 GHz
 
 enum { EPI_SPLIT = 0, EPI_PACK = 1 };
 enum { ERR_TIMEOUT_FULL = 1, ERR_TIMEOUT_MMA = 2, ERR_TIMEOUT_ACC = 3 };
@@ -75,41 +77,6 @@ struct GemmArgs {
   int *err;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait: true when the phase completed, false when the budget (SM clock cycles) ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long budget = WAIT_CYCLES) {
-  const long long t0 = clock64();
-  while (!mbar_try(bar, parity)) {
-    if (clock64() - t0 > budget) return false;
-  }
-  return true;
-}
-// the same for a whole warp, which goes on or gives up as one: lanes that parted here would miss each other in the
-// shuffles and TMEM loads that follow
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long budget) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, budget));
-}
-__device__ __forceinline__ bool warp_aborted(volatile int *flag) { return __any_sync(0xffffffffu, *flag != 0); }
-
 // EPI_PACK: rows (m, slice), so a tile holds few m; only columns n <= m are kept, and the tile takes a whole number of
 // B boxes up to the last of them
 // (the widest tiles come first, so that the last ones even the SMs out)
@@ -122,24 +89,6 @@ template <int EPI> __device__ __forceinline__ int tile_cols(const GemmArgs &g, i
   const int64_t last = row0 + BM < g.M ? row0 + BM : g.M;
   const int n = (int)((last - 1) / g.nbp) + 1;
   return n < g.N ? n : g.N;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-
-// UMMA shared-memory descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);        // start address
-  d |= (uint64_t)1 << 16;                         // leading byte offset (unused for this layout)
-  d |= (uint64_t)(1024 >> 4) << 32;               // stride byte offset: 8 rows x 128 B
-  d |= (uint64_t)1 << 46;                         // descriptor version for tcgen05
-  d |= (uint64_t)2 << 61;                         // 128-byte swizzle
-  return d;
 }
 
 // instruction descriptor: D = F32, A/B format (1 = BF16 for kind::f16, 2 = TF32), K-major A and B, n columns
@@ -160,25 +109,6 @@ __device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t a, uint64_t b, uin
         "l"(a), "l"(b), "r"(idesc), "r"(accum)
         : "memory");
   }
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
 __device__ __forceinline__ float tf32_round(float x) {
@@ -273,7 +203,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
     // the loads of the last stages must have landed before the CTA exits
     for (int j = gs > STAGES ? gs - STAGES : 0; j < gs; j++)
-      mbar_wait(smem_u32(full + (j % STAGES)), (uint32_t)((j / STAGES) & 1));
+      mbar_wait(smem_u32(full + (j % STAGES)), (uint32_t)((j / STAGES) & 1), WAIT_CYCLES);
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
     int gs = 0, i = 0;
@@ -319,7 +249,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
     // every MMA issued by this thread has completed before TMEM is freed
     mma_commit(smem_u32(drain));
-    mbar_wait(smem_u32(drain), 0);
+    mbar_wait(smem_u32(drain), 0, WAIT_CYCLES);
   } else if (warp >= 2) {
     // ---- epilogue
     const int q = warp & 3;  // TMEM lane quadrant of this warp
@@ -534,10 +464,6 @@ struct Args {
   int *err;
 };
 
-__device__ __forceinline__ uint64_t desc_k64(uint32_t addr) {  // rows of 64 bytes, 64-byte swizzle, 8 rows 512 B
-  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 |
-         (uint64_t)4 << 61;
-}
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src, int x, int y, int z) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(map)),
@@ -725,9 +651,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
           for (int kk = 0; kk < KC / 16; kk++) {
             const uint32_t o = kk * 32;
-            mma<false>(d, smem_desc(a_hi + o), desc_k64(b_hi + o), idesc, s > 0 || kk > 0);
-            mma<false>(d, smem_desc(a_hi + o), desc_k64(b_lo + o), idesc, 1u);
-            mma<false>(d, smem_desc(a_lo + o), desc_k64(b_hi + o), idesc, 1u);
+            mma<false>(d, smem_desc(a_hi + o), smem_desc_k64(b_hi + o), idesc, s > 0 || kk > 0);
+            mma<false>(d, smem_desc(a_hi + o), smem_desc_k64(b_lo + o), idesc, 1u);
+            mma<false>(d, smem_desc(a_lo + o), smem_desc_k64(b_hi + o), idesc, 1u);
           }
           mma_commit(smem_u32(empty + slot));
         }
@@ -736,8 +662,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       // no load or MMA of this CTA is in flight when it leaves
       mma_commit(smem_u32(drain));
-      mbar_wait(smem_u32(drain), 0);
-      mbar_wait(smem_u32(afull), 0);
+      mbar_wait(smem_u32(drain), 0, WAIT_CYCLES);
+      mbar_wait(smem_u32(afull), 0, WAIT_CYCLES);
     }
   } else {
     // ---- epilogue
@@ -799,24 +725,12 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 // ---------------------------------------------------------------------------
 // budget of the GEMM pipeline waits; pq_debug_set_wait_budget changes it for tests of the timeout path
-static long long g_gemm_wait_cycles = tc::WAIT_CYCLES;
-
-static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
-  return fn;
-}
+static long long g_gemm_wait_cycles = tcx::WAIT_CYCLES;
 
 // 2-D tensor map over a row-major (rows x kdim) operand, box (BK x box_rows), 128-byte swizzle
 static pq_status make_map(CUtensorMap *m, const void *base, bool tf32, int64_t rows, int64_t kdim, int64_t ld,
                           int box_rows) {
-  auto fn = encode_fn();
+  auto fn = tcx::encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return PQ_ERR_CUDA;
@@ -876,7 +790,7 @@ static pq_status run_gemm(const Operand &A, const Operand &B, int M, int N, int 
 template <typename TS>
 static pq_status run_slices(const Operand &ct, void *uh, void *ul, const TS *src, int64_t ld_src, int n, int nm, int nb,
                             int nbp, int64_t ld, int *err, cudaStream_t st) {
-  auto fn = encode_fn();
+  auto fn = tcx::encode_fn();
   CUtensorMap ma[2], mu[2];
   PQ_TRY(make_map(&ma[0], ct.hi, false, ct.rows, n, ct.ld, tc::BM));
   PQ_TRY(make_map(&ma[1], ct.lo, false, ct.rows, n, ct.ld, tc::BM));
@@ -1096,6 +1010,6 @@ extern "C" pq_status pq_ao2mo_release_workspace(void) {
 }
 
 extern "C" pq_status pq_debug_set_wait_budget(long long cycles) {
-  pq::g_gemm_wait_cycles = cycles > 0 ? cycles : pq::tc::WAIT_CYCLES;
+  pq::g_gemm_wait_cycles = cycles > 0 ? cycles : pq::tcx::WAIT_CYCLES;
   return PQ_OK;
 }

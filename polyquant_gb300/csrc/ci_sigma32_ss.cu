@@ -41,9 +41,12 @@
 #include <vector>
 
 #include "pq_internal.h"
+#include "pq_tc.cuh"
 
 namespace pq {
 namespace ssg {
+
+using namespace tcx;
 
 constexpr int BM = 128;          // output rows per tile (TMEM lanes)
 constexpr int BN = 256;          // output columns per tile (TMEM columns per accumulator)
@@ -57,7 +60,6 @@ constexpr int THREADS = 64 + 32 * EPI_WARPS;  // producer warp, MMA warp, epilog
 constexpr int NBARS = 2 * STAGES + 4 + 1;     // full, empty, acc_full[2], acc_empty[2], drain
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers, slots*/;
 constexpr int NGROUP = 8;                     // n tiles per scheduling group (L2 reuse of the A panels)
-constexpr long long WAIT_CYCLES = 4000000000LL;  // ~2 s at 2 GHz
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 
 enum { ERR_TIMEOUT_FULL = 1, ERR_TIMEOUT_MMA = 2, ERR_TIMEOUT_ACC = 3 };
@@ -77,49 +79,6 @@ struct Args {
   int *err;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait: true when the phase completed, false when the budget (SM clock cycles) ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long budget = WAIT_CYCLES) {
-  const long long t0 = clock64();
-  while (!mbar_try(bar, parity)) {
-    if (clock64() - t0 > budget) return false;
-  }
-  return true;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-// UMMA shared-memory descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 // instruction descriptor: D = F32, A = B = F16, both K-major, N = BN, M = BM
 constexpr uint32_t IDESC = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 
@@ -128,23 +87,6 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b,
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(IDESC), "r"(accum)
       : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
 // power of two 2^e with x * 2^e in [2^14, 2^15) (1 for x == 0)
@@ -230,7 +172,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     // the loads of the last stages must have landed before the CTA exits
     for (int j = gs > STAGES ? gs - STAGES : 0; j < gs; j++)
-      mbar_wait(smem_u32(full + (j % STAGES)), (uint32_t)((j / STAGES) & 1));
+      mbar_wait(smem_u32(full + (j % STAGES)), (uint32_t)((j / STAGES) & 1), WAIT_CYCLES);
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
     int gs = 0, i = 0;
@@ -278,7 +220,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     // every MMA issued by this thread has completed before TMEM is freed
     mma_commit(smem_u32(drain));
-    mbar_wait(smem_u32(drain), 0);
+    mbar_wait(smem_u32(drain), 0, WAIT_CYCLES);
   } else if (warp >= 2) {
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31
     const int q = warp & 3;
@@ -291,9 +233,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int a = i & 1;
       const uint32_t aph = (uint32_t)((i >> 1) & 1);
       i++;
-      // the warp goes on or gives up as one: tmem_ld32 needs all of its lanes
-      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(accf + a), aph, g.wait_cycles));
-      if (!ok || __any_sync(0xffffffffu, *abort_flag != 0)) {
+      const bool ok = warp_wait(smem_u32(accf + a), aph, g.wait_cycles);
+      if (!ok || warp_aborted(abort_flag)) {
         if (!ok && lane == 0) atomicCAS(g.err, 0, ERR_TIMEOUT_ACC);
         *abort_flag = 1;
         break;
@@ -446,22 +387,10 @@ struct SameSpinGemm {
 
 void ss_delete(SameSpinGemm *g) { delete g; }
 
-static PFN_cuTensorMapEncodeTiled_v12000 ss_encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
-  return fn;
-}
-
 // 2-D tensor map over a row-major FP16 (rows x kdim) operand with row pitch ld, box (BK x box_rows),
 // 128-byte swizzle; reads past kdim or rows return zeros
 static pq_status ss_map(CUtensorMap *m, const void *base, int64_t rows, int64_t kdim, int64_t ld, int box_rows) {
-  auto fn = ss_encode_fn();
+  auto fn = tcx::encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return PQ_ERR_CUDA;

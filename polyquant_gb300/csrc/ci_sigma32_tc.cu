@@ -58,9 +58,12 @@
 #include <vector>
 
 #include "pq_internal.h"
+#include "pq_tc.cuh"
 
 namespace pq {
 namespace abtc {
+
+using namespace tcx;
 
 constexpr int BM = 128;       // (Jb, v) rows per tile (TMEM lanes)
 constexpr int BN = 128;       // off-diagonal beta pairs (TMEM columns per accumulator)
@@ -77,7 +80,6 @@ constexpr int NTHREADS = 512;                    // 16 warps
 constexpr int STAGERS = 8;                       // staging warps: two for each TMEM lane quadrant
 constexpr int CONV0 = 1, EPI0 = 5, PROC0 = EPI0 + STAGERS;  // first converter / epilogue (staging) / list-only warp
 constexpr int NPROC = (NTHREADS / 32 - EPI0) * 32;  // threads that process the scatter lists (352)
-constexpr long long WAIT_CYCLES = 4000000000LL;  // ~2 s at 2 GHz
 // shared memory: A hi/lo x ASTAGES, B hi/lo (one buffer), raw rows x 2, accumulator staging, per-warp alpha
 // partner lists, barriers
 constexpr int SMEM_OPS = ASTAGES * 2 * OP_TILE + 2 * OP_TILE + 2 * RAW_TILE + STG_BYTES;
@@ -120,38 +122,6 @@ struct Args {
 #define PACC(slot, v)
 #endif
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait: true when the phase completed, false when the budget (SM clock cycles) ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long budget) {
-  const long long t0 = clock64();
-  while (!mbar_try(bar, parity)) {
-    if (clock64() - t0 > budget) return false;
-  }
-  return true;
-}
-// warp-uniform bounded wait: every lane polls; the warp agrees on success only if every lane saw the phase
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long budget) {
-  const bool ok = mbar_wait(bar, parity, budget);
-  return __all_sync(0xffffffffu, ok);
-}
-__device__ __forceinline__ bool warp_aborted(volatile int *flag) { return __any_sync(0xffffffffu, *flag != 0); }
-
 // 4-byte / 16-byte asynchronous copies global -> shared (each thread waits for its own groups)
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -162,17 +132,6 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// UMMA shared-memory descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
 // instruction descriptor: D = F32, A = B = F16 (format 0 of kind::f16), both K-major, N = BN, M = BM
 constexpr uint32_t IDESC = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 
@@ -181,23 +140,6 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b,
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(IDESC), "r"(accum)
       : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
 // K values of row r of an operand tile (scaled FP32) -> FP16 hi/lo tiles in the 128-byte-swizzled K-major
