@@ -41,12 +41,6 @@ __device__ __forceinline__ void mma_step(uint32_t tmem, A &&adesc, B &&bdesc, ui
   }
 }
 
-// A CTA's decision not to start, taken once for all its threads: a CTA of the same launch whose wait runs out raises the
-// gate, so threads that each read it could part ways before the barriers and the warp-wide TMEM allocation.
-__device__ __forceinline__ bool gate_raised(const int *gate) {
-  return __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<const volatile int *>(gate) != 0);
-}
-
 constexpr int SS_A = BM * 64, SS_B = BN * 64;                  // one digit of 32 K values: 8 KB, 4 KB
 constexpr int SS_STAGE = dg::N * (SS_A + SS_B);                // 84 KB
 constexpr int SS_STAGES = 2;
@@ -85,7 +79,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint64_t *full = bars, *empty = bars + SS_STAGES, *accf = bars + 2 * SS_STAGES, *acce = accf + 1, *drain = accf + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + SS_BARS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  if (gate_raised(g.gate)) return;
+  // A CTA decides once for all its threads whether to start: a CTA of the same launch whose wait runs out raises the gate,
+  // so threads that each read it could part ways before the barriers.  Thread 0 reads it, the barrier after the setup
+  // tells the others (one of its own before the setup cost 1 us a launch).
+  const int gate = threadIdx.x == 0 ? *reinterpret_cast<const volatile int *>(g.gate) : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < SS_STAGES; i++) {
@@ -103,7 +100,11 @@ __global__ void __launch_bounds__(THREADS, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  __syncthreads();
+  if (__syncthreads_or(gate)) {
+    if (warp == 0)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(512) : "memory");
+    return;
+  }
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   auto fail = [&] {
