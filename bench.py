@@ -11,7 +11,7 @@ Printed JSON line (rank 0):
   e2e      : the same metric through pq_ci_sigma_host with pinned host buffers (H2D + sigma + D2H)
   mixed    : the FP32 sigma (the bulk sigma of the mixed-precision Davidson), with its own roofline
   roofline : compulsory bytes B = n_dets*roots*(8+8) + n_dets*8 per FP64 sigma over the kernel time,
-             against the measured HBM copy bandwidth; `fp64` adds the FMA rate against a live DGEMM
+             against the measured HBM copy bandwidth (`bound` names what does bound the kernels); `fp64` adds the FMA rate against a live DGEMM
   time_to_1uEh : FP64 vs mixed Davidson for the lowest 4 roots (residual 1e-4), each energy's error
              against a 1e-7 FP64 solve
   psh_like : the electron-positron product space (60 x 40 orbitals, 144,000 determinants); its heat_bath
@@ -360,7 +360,7 @@ def bench_psh_like(seed=0, cpu_budget=5.0):
     b64 = n * roots * 16 + n * 8
     ach = b64 / (res["sigma_fp64_ms"] * 1e-3) / 1e9
     fmas = n * roots * (1 + conn)
-    res["roofline"] = {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
+    res["roofline"] = {"bound": "accumulator drain", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                        "traffic": None, "peak_source": src, "algorithmic_bytes_per_launch": b64,
                        "note": "FP64 sigma call (layout conversion of the column-major block included); "
                                f"{conn} off-diagonal connections per determinant",
@@ -667,7 +667,7 @@ def main():
                 "setup_seconds": setup_s,
                 "e2e": e2e,
                 "mixed": {"value": units / (ms32 * 1e-3), "unit": UNIT, "ms_per_step": ms32, "dtype": "f32",
-                          "roofline": {"bound": "hbm", "achieved": bytes32 / (ms32 * 1e-3) / 1e9, "peak": hbm,
+                          "roofline": {"bound": "tensor pipe and shared memory of the epilogue", "achieved": bytes32 / (ms32 * 1e-3) / 1e9, "peak": hbm,
                                        "unit": "GB/s", "frac": bytes32 / (ms32 * 1e-3) / 1e9 / hbm,
                                        "algorithmic_bytes_per_launch": bytes32,
                                        "fp32_fma_per_launch": fmas,
@@ -675,7 +675,7 @@ def main():
                                        "note": "the alpha-beta and same-spin doubles run on the tcgen05 tensor "
                                                "cores (FP16 hi/lo split, FP32 accumulation) where the space "
                                                "allows; per-kernel ncu figures in profiles/"}},
-                "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+                "roofline": {"bound": "accumulator drain", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                              "frac": achieved / hbm, "traffic": FP64_SIGMA_DRAM_BYTES_PER_DET * n,
                              "traffic_note": "ncu dram__bytes_read+write of one FP64 sigma on FCI(14o, 7a7b) "
                                              "(34.5 GB for 11,778,624 determinants x 4 roots), scaled by the "

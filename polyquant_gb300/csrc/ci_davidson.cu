@@ -84,7 +84,8 @@ static void jacobi_eigh(int n, std::vector<double> A, std::vector<double> &w, st
 // CI (63 504 determinants) issued 448 norms of 35 us and about 500 DGEMV and dot launches.  Here one launch does
 // what belongs together (Ritz vectors, residuals and their norms; all projections of a vector and its norm), sums
 // are finished by the last block to arrive, in block order, so results do not vary between runs, and Gram-Schmidt
-// takes its decisions on the device.  That solve takes 21.4 ms against 41.4, 9.4 of them in sigma (before: the same 9.4).
+// takes its decisions on the device.  That solve took 21.4 ms against 41.4 with the sigma of the time (9.4 ms in either);
+// with the tensor-core sigma 12 to 17 ms, by the number of iterations that the integrals need.
 constexpr int TS_THREADS = 256;
 constexpr int TS_MI = 8, TS_Q = 4;  // register tile of the products: columns of V x columns of the other block
 
